@@ -10,8 +10,11 @@
 // per expanded child and playout index, the reference's thread (tree, action, t)), so the lanes of a warp wait for
 // each other once per step, not once per game.
 //
-// Position encoding: column c of the 6x7 board owns bits 7c .. 7c+5 (bit 7c = bottom cell) and a guard bit 7c+6 that
-// stays 0, so that shifts by 1, 6, 7, 8 test the four line directions without wrapping between columns.
+// Position encoding: column c of the 6x7 board owns byte c + 1 of a 64-bit word: bits 8c + 8 .. 8c + 13 (bottom cell first) and
+// two guard bits that stay 0, so that shifts by 1, 7, 8, 9 test the four line directions without wrapping between columns;
+// byte 0 holds no cell.  Four columns are exactly the high 32-bit word: a horizontal or diagonal four ends in one of them,
+// so its test needs one funnel shift per stone and word-wide ANDs of the high word only, and the column of a stone is one
+// byte permute away.
 #pragma once
 #include <cooperative_groups.h>
 
@@ -22,38 +25,48 @@ namespace mctsnc {
 namespace c4 {
 
 constexpr int ROWS = 6, COLS = 7, A = 7;
-constexpr int LEGAL_SHIFT = 6;       // the playout loop keeps the set of open columns times 64 = byte offset of its row of move_lut
+__host__ __device__ constexpr int column_shift(int c) { return 8 * c + 8; }
+// plies of a playout between two looks at whether the game is over
 #ifndef MCTSNC_PLIES_PER_CHECK
 #define MCTSNC_PLIES_PER_CHECK 4
 #endif
-constexpr int PLIES_PER_CHECK = MCTSNC_PLIES_PER_CHECK;  // plies of a playout between two looks at whether the game is over
-constexpr unsigned long long BOTTOM_ROW = 0x0000040810204081ULL;  // bit 7c for c = 0..6
-constexpr unsigned long long TOP_ROW = BOTTOM_ROW << 5;
+#ifndef MCTSNC_STRAIGHT_PLIES
+#define MCTSNC_STRAIGHT_PLIES 4
+#endif
+constexpr int PLIES_PER_CHECK = MCTSNC_PLIES_PER_CHECK, STRAIGHT_PLIES = MCTSNC_STRAIGHT_PLIES;
+constexpr unsigned long long BOTTOM_ROW = 0x0101010101010100ULL;
 constexpr unsigned long long FULL_BOARD = BOTTOM_ROW * 0x3FULL;
-constexpr unsigned long long MOVE_LUT_NO_COLUMN = 1ULL << 63;
+constexpr unsigned BOTTOM_LO = 0x01010100u, BOTTOM_HI = 0x01010101u;   // of the columns 0..2 and 3..6
+constexpr unsigned TOP_LO = 0x20202000u, TOP_HI = 0x20202020u;
 
-// four in a row anywhere in the stone set p.  Left shifts: the low word of a 64-bit left shift is a plain 32-bit
-// shift, which the integer multiply-add pipe can execute, taking load off the logic pipe that limits this kernel.
-// Bits shifted past bit 48 meet zeros of p in the AND.
+// four in a row that end in the high word's columns (horizontal and both diagonals) of the stone set (lo, hi)
+__host__ __device__ __forceinline__ unsigned fours_across(unsigned lo, unsigned hi) {
+    const unsigned long long p = ((unsigned long long)hi << 32) | lo;   // the high word of p << k is the low word of p >> (32 - k)
+    unsigned r = hi & (unsigned)(p >> 24) & (unsigned)(p >> 16) & (unsigned)(p >> 8);
+    r |= hi & (unsigned)(p >> 23) & (unsigned)(p >> 14) & (unsigned)(p >> 5);
+    r |= hi & (unsigned)(p >> 25) & (unsigned)(p >> 18) & (unsigned)(p >> 11);
+    return r;
+}
+
+// four in a row anywhere in the stone set p
 __host__ __device__ __forceinline__ bool has_four(unsigned long long p) {
-    unsigned long long m, r;
-    m = p & (p << 7);
-    r = m & (m << 14);
-    m = p & (p << 6);
-    r |= m & (m << 12);
-    m = p & (p << 8);
-    r |= m & (m << 16);
-    m = p & (p << 1);
-    r |= m & (m << 2);
-    return r != 0;
+    unsigned long long v = p & (p >> 1);
+    v &= v >> 2;
+    return (fours_across((unsigned)p, (unsigned)(p >> 32)) | (unsigned)v | (unsigned)(v >> 32)) != 0u;
 }
 
 // set of columns that still have room, from the occupancy bitboard
 __host__ __device__ __forceinline__ unsigned legal_columns(unsigned long long all) {
     unsigned l = 0;
 #pragma unroll
-    for (int c = 0; c < COLS; c++) l |= ((all >> (7 * c + 5)) & 1ULL) ? 0u : (1u << c);
+    for (int c = 0; c < COLS; c++) l |= ((all >> (column_shift(c) + 5)) & 1ULL) ? 0u : (1u << c);
     return l;
+}
+
+// index of the n-th set bit (n = 0 is the lowest)
+__device__ __forceinline__ int nth_set(int mask, int n) {
+    for (; n > 0; n--) mask &= mask - 1;
+    return __ffs(mask) - 1;
 }
 
 // among tied maxima the reference's stride-halving reduction keeps the left operand (src/mctsnc.py:1343-1351), which
@@ -117,7 +130,7 @@ __device__ __noinline__ EmuResult playout_emulated(unsigned long long neg, unsig
     for (int j = 0; j < COLS; j++) {
         int f = 0;
         for (int h = 0; h < ROWS; h++) {
-            int bit = 7 * j + h;
+            int bit = column_shift(j) + h;
             int v = ((pos >> bit) & 1ULL) ? 1 : (((neg >> bit) & 1ULL) ? -1 : 0);
             board[(ROWS - 1 - h) * COLS + j] = (signed char)v;
             f += v != 0;
@@ -180,35 +193,55 @@ __device__ __noinline__ EmuResult playout_emulated(unsigned long long neg, unsig
 
 // everything a thread needs to start a game from one child, fetched with two 16-byte shared-memory loads
 struct __align__(16) GameSlot {
-    unsigned long long cur;  // stones of the side to move
-    unsigned long long top;  // one bit per column: its lowest empty cell (the guard bit of a full column) = all stones + BOTTOM_ROW
-    unsigned legal;          // columns with room, shifted left by LEGAL_SHIFT
-    int rng_base;            // index of the child's first stream in the block's stream array
-    int stones;              // stones on the board
-    float count;             // number of columns with room times 2^-64 (the playout loop draws uniforms scaled by 2^64)
+    unsigned long long cur;    // stones of the side to move
+    unsigned long long other;  // stones of the other side
+    float row;                 // move_row(set of columns with room)
+    float count;               // number of columns with room times 2^-64 (the playout loop draws uniforms scaled by 2^64)
+    int rng_base;              // index of the child's first stream in the block's stream array
+    int stones;                // stones on the board
 };
+
+// move_lut[(set ^ 1) * 8 + ord]: the ord-th column (ascending) of the column set `set`, as the six cells of that column in
+// the two words of a position.  The low bits of `lo`, where no cell is, hold the number of the column's byte.  The index is
+// computed in float: the playout loop keeps row = 2^23 + 8 * (set ^ 1), and row + u * count added with rounding towards zero is
+// 2^23 + the index, in the low bits of the mantissa.
+// An ordinal the set does not have (only a uniform draw of exactly 1.0f gives one: ord == number of columns) is a move to
+// MARK, a bit of byte 0, which stays in the position and tells the end of the game.  The empty set has no move at all.
+struct __align__(8) MoveEntry {
+    unsigned lo, hi;
+};
+constexpr float MOVE_LUT_BASE = 8388608.f;
+constexpr unsigned MOVE_LUT_BASE_BITS = 0x4B000000u;
+constexpr unsigned MARK = 0x10u;
+__host__ __device__ constexpr float move_row(unsigned set) { return MOVE_LUT_BASE + (float)(8u * (set ^ 1u)); }
+constexpr float NO_MOVES = MOVE_LUT_BASE + 8.f;   // move_row(0)
+
+// one level of the selected path, as far as the backup can know it while the games are still being played; the last entry of a
+// path: its children, which all get the same counts
+struct PathTerm {
+    double explore;      // sqrt(log N / n) of the child on the path, with the counts the backup will leave
+    double n, reciprocal;  // n (as the float32 the UCB divides by) and 1 / n
+    unsigned other_key;  // ordered key of the best UCB among the other children (0: there is none)
+    int other;           // that child's rank, and bit 8: on equal UCB the child on the path wins
+};
+
+constexpr int MAX_PATH = 48;
 
 struct Shared {
     GameSlot slot[A];        // children that need real playouts, in expansion order
+    int4 path_rec[MAX_PATH]; // the records of the selected path as the select read them
+    PathTerm term[MAX_PATH];
+    MoveEntry move_lut[128 * 8];
     int tally[A][2];         // per slot: games won by -1, by +1 (of the games this block played)
     int gather[A][2];        // cluster of blocks per tree: the sums over the blocks, kept by the first block
-    int path[48];
-    int path_ns[48];
-    int path_wins[48];
-    int child_action[A];     // per expanded child (expansion order): its action,
-    int child_outcome[A];    // its outcome (2 = ongoing)
+    int path[MAX_PATH];
+    int child_outcome[A];    // per expanded child (expansion order): its outcome (2 = ongoing)
     int child_slot[A];       // and its slot (-1: no playouts: terminal, or not picked in OCP)
     int child_out[A][2];     // trees_playout_outcomes_children (persists over steps)
     short ae[A + 2];         // trees_actions_expanded row (persists over steps)
-    // move_lut[set * 8 + ord]: for the ord-th column (ascending) of the column set `set`, the six cells of the column
-    // (0x3F << 7 * column) in bits 0..47 and the column's bit in bits 54..60, i.e. where it sits in the pre-shifted column
-    // set the playout loop keeps (GameSlot::legal), moved up by 48.  An ordinal the set does not have (only a uniform
-    // draw of exactly 1.0f gives one: ord == number of columns) maps to MOVE_LUT_NO_COLUMN: no cell, bit 63 set.
-    unsigned long long move_lut[128 * 8];
     int job;                 // tree of the slice being run (-1: none left)
     int n_slots;
     int next_item;           // next game to hand out in the playout phase
-    int n_exp;
     int mode;
     int first_child;
     int exp_mask;
@@ -236,9 +269,101 @@ __device__ __forceinline__ void rec_store(int4 *rec, int4 *cache, int cache_n, i
     rec[i] = v;
     if (i < cache_n) cache[i] = v;
 }
-__device__ __forceinline__ void rec_store_stats(int4 *rec, int4 *cache, int cache_n, int i, int ns, int wins) {
-    *reinterpret_cast<int2 *>(&rec[i]) = make_int2(ns, wins);
-    if (i < cache_n) *reinterpret_cast<int2 *>(&cache[i]) = make_int2(ns, wins);
+
+// w / n from the correctly rounded reciprocal of n: one Newton correction of w * (1 / n) with its exact remainder gives the
+// correctly rounded quotient (Markstein, "Computation of elementary functions on the IBM RISC System/6000", 1990), in three
+// dependent operations.  Both operands are whole numbers below 2^53 here, so nothing overflows or is lost.
+__device__ __forceinline__ double divide_by_reciprocal(double w, double n, double reciprocal) {
+    const double q = w * reciprocal;
+    return fma(fma(-q, n, w), reciprocal, q);
+}
+
+// UCB of a child (src/mctsnc.py:1337), evaluated in float64 (numba promotes int32/float32 and log(int32) to float64), fused
+// multiply-add as NVVM contracts it, rounded once to float32; `explore` is sqrt(log(N) / n), `n` is rounded to float32 first
+__device__ __forceinline__ float ucb_value(double c_ucb, double explore, double n, double reciprocal, int wins) {
+    return __double2float_rn(fma(c_ucb, explore, divide_by_reciprocal((double)wins, n, reciprocal)));
+}
+
+// What the backup of the selected path needs and what does not depend on how the games end: the visit counts it will leave
+// are known as soon as the leaf is, so every logarithm, division and square root of the UCBs can be done while the games
+// are being played.  Eight lanes per level (lane = action), four levels at a time.
+template <bool OCP>
+__device__ __forceinline__ void prepare_backup(Shared &s, const int4 *rec, const int4 *cache, int cache_n, double c_ucb, int lane,
+                                               int plen, int n_tot, int leaf_playouts) {
+    const int a = lane & 7, shift = lane & 24;
+    for (int base = 0; base < plen - 1; base += 4) {
+        const int e = base + (lane >> 3);
+        const bool level = e < plen - 1;
+        const int4 pr = s.path_rec[level ? e : 0];
+        const int n_path = s.path_rec[level ? e + 1 : 0].x + n_tot;
+        const unsigned mask = pr.w & 0x7F;
+        const bool has = level && ((mask >> a) & 1u);
+        const int rank = __popc(mask & ((1u << a) - 1u));
+        const bool on_path = rank == meta_best(pr.w);
+        int n = n_path, w = 0;
+        if (has && !on_path) {
+            const int4 cr = rec_load(rec, cache, cache_n, pr.z + rank);
+            n = cr.x;
+            w = cr.y;
+        }
+        const double explore = sqrt(log((double)(pr.x + n_tot)) / (double)n);
+        const double n_f = (double)__int2float_rn(n), reciprocal = 1.0 / n_f;
+        unsigned key = 0;
+        if (has && !on_path) key = ordered_key(n == 0 ? __int_as_float(0x7f800000) : ucb_value(c_ucb, explore, n_f, reciprocal, w));
+        unsigned best = max(key, __shfl_xor_sync(0xFFFFFFFFu, key, 1));
+        best = max(best, __shfl_xor_sync(0xFFFFFFFFu, best, 2));
+        best = max(best, __shfl_xor_sync(0xFFFFFFFFu, best, 4));
+        const unsigned tied = (__ballot_sync(0xFFFFFFFFu, key != 0u && key == best) >> shift) & 0x7Fu;
+        if (has && on_path) {
+            PathTerm t;
+            t.explore = explore;
+            t.n = n_f;
+            t.reciprocal = reciprocal;
+            t.other_key = best;
+            const int o = pick_among_tied(tied);
+            t.other = __popc(mask & ((1u << o) - 1u)) | (pick_among_tied((1u << o) | (1u << a)) == a ? 256 : 0);
+            s.term[e] = t;
+        }
+    }
+    if (leaf_playouts > 0) {
+        PathTerm t;
+        t.n = (double)leaf_playouts;   // at most 512: the same as a float32
+        t.explore = sqrt(log((double)(s.path_rec[plen - 1].x + n_tot)) / t.n);
+        t.reciprocal = 1.0 / t.n;
+        t.other_key = 0u;
+        t.other = 0;
+        if (lane == 0) s.term[plen - 1] = t;
+    }
+}
+
+// Shared-memory address of the table less the offset of the float exponent: address of entry i = base + 8 * (bits of the
+// float 2^23 + i), modulo 2^32
+__device__ __forceinline__ unsigned move_lut_base(const Shared &s) {
+    return (unsigned)__cvta_generic_to_shared(s.move_lut) - MOVE_LUT_BASE_BITS * (unsigned)sizeof(MoveEntry);
+}
+__device__ __forceinline__ MoveEntry load_move(unsigned base, unsigned float_bits) {
+    MoveEntry m;
+    asm("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(m.lo), "=r"(m.hi) : "r"(base + float_bits * (unsigned)sizeof(MoveEntry)));
+    return m;
+}
+
+// A column that has just been filled (`filled` != 0) leaves the set of columns with room: `row` drops by 8 << column, a power of
+// two whose exponent is the column's byte number in the entry's low bits (the shift's other bits fall out, but for the
+// bottom cell of column 0, which flips the sign: that is why the set's bit 0 is kept inverted).  Two predicated additions:
+// the branch the compiler makes of it cost the warp its resolving on every ply.
+__device__ __forceinline__ void close_column(unsigned filled, float &row, float &count, unsigned entry_lo) {
+    const unsigned drop = entry_lo * (1u << 23) + (0x80000000u + (129u << 23));
+    asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p add.rn.f32 %0, %0, %3;\n\t@p add.rn.f32 %1, %1, %4;\n\t}"
+        : "+f"(row), "+f"(count) : "r"(filled), "f"(__uint_as_float(drop)), "f"(-RNG_2M64));
+}
+
+// fours of the side that has just put a stone into the column of entry `entry_lo`: a new vertical four can only be in that
+// column, whose byte is tested alone (20 logic operations in all; the four directions over the whole board take 32)
+// (the permute takes the entry as it is: its other selectors name byte 0 or columns that hold no four)
+__device__ __forceinline__ unsigned fours_with(unsigned lo, unsigned hi, unsigned entry_lo) {
+    unsigned v = __byte_perm(lo, hi, entry_lo);
+    v &= v >> 1;
+    return fours_across(lo, hi) | (v & (v >> 2));
 }
 
 // `n_steps` steps of tree g by the whole block, from the state the tree has in global memory and back to it.
@@ -251,12 +376,15 @@ __device__ __forceinline__ void rec_store_stats(int4 *rec, int4 *cache, int cach
 // playout indices of every child -- it keeps the streams of exactly those in its shared memory -- and adds its tallies
 // to the first block's `gather`.  Two cluster barriers per step; all blocks run the same loop, so every block reaches
 // every barrier.
-template <bool OCP, int CL>
+//
+// STRAIGHT: how a game is played, see the playouts.
+template <bool OCP, int CL, bool STRAIGHT>
 __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulonglong2 *s_rng, int4 *cache, const int g,
                                           const int n_steps, const bool first) {
     namespace cg = cooperative_groups;
     const int cache_n = CL > 1 ? p.cache_nodes : 0;
     static_assert(CL == 1 || CL == 2 || CL == 4 || CL == 8, "cluster sizes");
+    constexpr int PLIES = STRAIGHT ? STRAIGHT_PLIES : PLIES_PER_CHECK;
     constexpr int LOG_CL = CL == 8 ? 3 : (CL == 4 ? 2 : (CL == 2 ? 1 : 0));
     const int tid = threadIdx.x;
     const int nt = blockDim.x;
@@ -272,6 +400,9 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
     TreeState *st = p.state + g;
     const bool thrifty = (p.variant == 0 || p.variant == 2);
     const bool walker = warp == 0 && rank == 0;   // the warp that selects, expands and backs up
+    // threads whose first game of a step is fixed by their number: all, but for the walker where it is not the only warp
+    const int first_free_item = rank == 0 && nt > 32 ? nt - 32 : nt;
+    const unsigned lut_base = move_lut_base(s);
 
     const int n_streams = OCP ? P : A * P;
     ulonglong2 *g_rng = p.rng_playout + (long long)g * n_streams;
@@ -323,6 +454,8 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
 
     const double c_ucb = (double)p.ucb_c;
     unsigned my_plies = 0, my_ub = 0, my_err = 0;
+    ulonglong2 pick_stream = make_ulonglong2(0ULL, 0ULL);   // OCP: the stream of the child picks (lane 0 of the walker)
+    if (OCP && walker && lane == 0) pick_stream = p.rng_expand[g];
 
     // The walker warp runs steps on its own for as long as they select a terminal node (nothing to play: the backup follows
     // at once) and meets the other threads only for a step with games, or when the steps are done (MODE_DONE).
@@ -337,39 +470,41 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
                 const unsigned c_backup = (unsigned)clock();
                 const int (*tally)[2] = CL > 1 ? s.gather : s.tally;
                 const int mode = s.mode;
-                const int n_exp = s.n_exp;
+                const int exp_mask = s.exp_mask;
                 const int sel_meta = s.sel_meta;
                 const int child_turn = -meta_turn(sel_meta);
+                const int plen = s.path_len;
+                // Lanes 0..6: the children of the expanded node (lane = action).  The other lanes: the levels of the path.
                 int neg_tot = 0, pos_tot = 0;
-                long long n_tot = P;
-                if (mode == MODE_ALL_CHILDREN) {
-                    int my_neg = 0, my_pos = 0;
-                    if (lane < n_exp) {
-                        const int o = s.child_outcome[lane];
-                        const int j = s.child_slot[lane];
-                        const bool played = !OCP || lane == s.pick;
-                        if (j >= 0) {
-                            my_neg = tally[j][0];
-                            my_pos = tally[j][1];
-                        } else if (played) {
-                            // a terminal child: its stored outcome stands for all P playouts (src/mctsnc.py:2016-2021)
-                            my_neg = o == -1 ? P : 0;
-                            my_pos = o == 1 ? P : 0;
-                        }
-                        // children start from ns = ns_wins = 0 (src/mctsnc.py:1819-1820), then _backup_1_acp_* / the
-                        // thread-0 part of _backup_ocp credit them (:2172-2177, :2104-2114)
-                        const int cns = played ? P : 0;
-                        const int cw = played ? (child_turn == 1 ? my_neg : my_pos) : 0;
-                        rec_store(rec, cache, cache_n, s.first_child + lane,
-                                  make_int4(cns, cw, -1, make_meta(0, o != 2, o, child_turn, meta_depth(sel_meta) + 1)));
-                        if (!OCP) {
-                            s.child_out[s.child_action[lane]][0] = my_neg;
-                            s.child_out[s.child_action[lane]][1] = my_pos;
-                        }
+                int n_tot = P;
+                int my_neg = 0, my_pos = 0;
+                const int k = __popc(exp_mask & ((1 << lane) - 1));
+                const bool child = mode == MODE_ALL_CHILDREN && lane < A && ((exp_mask >> lane) & 1);
+                bool played = false;
+                int outcome = 2;
+                if (child) {
+                    outcome = s.child_outcome[k];
+                    const int j = s.child_slot[k];
+                    played = !OCP || k == s.pick;
+                    if (j >= 0) {
+                        my_neg = tally[j][0];
+                        my_pos = tally[j][1];
+                    } else if (played) {
+                        // a terminal child: its stored outcome stands for all P playouts (src/mctsnc.py:2016-2021)
+                        my_neg = outcome == -1 ? P : 0;
+                        my_pos = outcome == 1 ? P : 0;
                     }
-                    neg_tot = __reduce_add_sync(0xFFFFFFFFu, my_neg);
-                    pos_tot = __reduce_add_sync(0xFFFFFFFFu, my_pos);
-                    if (!OCP) n_tot = (long long)P * n_exp;
+                    if (!OCP) {
+                        s.child_out[lane][0] = my_neg;
+                        s.child_out[lane][1] = my_pos;
+                    }
+                }
+                if (mode == MODE_ALL_CHILDREN) {
+                    // the sums of the children's games, both in one reduction (at most 7 * 512 games a side)
+                    const int both = __reduce_add_sync(0xFFFFFFFFu, my_neg | (my_pos << 16));
+                    neg_tot = both & 0xFFFF;
+                    pos_tot = both >> 16;
+                    if (!OCP) n_tot = P * __popc(exp_mask);
                 } else if (mode == MODE_TERMINAL) {
                     neg_tot = s.out_neg;
                     pos_tot = s.out_pos;
@@ -381,16 +516,47 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
                         s.child_out[0][1] = pos_tot;
                     }
                 }
-                const int plen = s.path_len;
-                for (int e = lane; e < plen; e += 32) {
-                    const int node = s.path[e];
-                    const int turn_e = (e & 1) ? -s.root_turn : s.root_turn;
-                    const int ns = s.path_ns[e] + (int)n_tot;
-                    const int wins = s.path_wins[e] + (turn_e == 1 ? neg_tot : pos_tot);
-                    if (e == plen - 1 && mode == MODE_ALL_CHILDREN) {
-                        rec_store(rec, cache, cache_n, node, make_int4(ns, wins, s.first_child, sel_meta | s.exp_mask));
-                    } else {
-                        rec_store_stats(rec, cache, cache_n, node, ns, wins);
+                // The counts and wins of the path change the UCBs of its own nodes' children only, so this is where the child
+                // that the next select goes on to is decided: on every level of the path the child on the path against the
+                // best of the others, at its end the best of the new children.
+                constexpr int LEVEL_LANES = 32 - 8;
+                const int root_turn = s.root_turn;
+                for (int base = 0; base < plen; base += LEVEL_LANES) {
+                    const int e = lane < 8 ? plen - 1 : base + lane - 8;
+                    const bool level = lane >= 8 && e < plen - 1;
+                    const int turn_e = (e & 1) ? -root_turn : root_turn;
+                    int wins_n = turn_e == 1 ? pos_tot : neg_tot;   // of the child on the path: the other side's
+                    if (level) wins_n += s.path_rec[e + 1].y;
+                    else wins_n = turn_e == 1 ? my_pos : my_neg;
+                    const PathTerm t = s.term[min(e, plen - 1)];
+                    const bool evaluate = level || (child && played);
+                    unsigned key = evaluate ? ordered_key(ucb_value(c_ucb, t.explore, t.n, t.reciprocal, wins_n)) : 0u;
+                    if (child && !played) key = ordered_key(__int_as_float(0x7f800000));
+                    int leaf_best = 0;
+                    if (base == 0 && mode == MODE_ALL_CHILDREN) {
+                        const unsigned leaf_key = lane < 8 ? key : 0u;
+                        const unsigned best = __reduce_max_sync(0xFFFFFFFFu, leaf_key);
+                        const int a = pick_among_tied(__ballot_sync(0xFFFFFFFFu, leaf_key != 0u && leaf_key == best));
+                        leaf_best = __popc(exp_mask & ((1 << a) - 1));
+                        // children start from ns = ns_wins = 0 (src/mctsnc.py:1819-1820), then _backup_1_acp_* / the
+                        // thread-0 part of _backup_ocp credit them (:2172-2177, :2104-2114)
+                        if (child)
+                            rec_store(rec, cache, cache_n, s.first_child + k,
+                                      make_int4(played ? P : 0, played ? wins_n : 0, -1,
+                                                make_meta(0, outcome != 2, outcome, child_turn, meta_depth(sel_meta) + 1)));
+                    }
+                    if (level || (lane == 7 && base == 0)) {   // lane 7: the end of the path
+                        int4 r = s.path_rec[e];
+                        r.x += n_tot;
+                        r.y += turn_e == 1 ? neg_tot : pos_tot;
+                        if (level) {
+                            if (key < t.other_key || (key == t.other_key && !(t.other & 256)))
+                                r.w = (r.w & ~META_BEST_MASK) | ((t.other & 7) << META_BEST_SHIFT);
+                        } else if (mode == MODE_ALL_CHILDREN) {
+                            r.z = s.first_child;
+                            r.w |= exp_mask | (leaf_best << META_BEST_SHIFT);
+                        }
+                        rec_store(rec, cache, cache_n, s.path[e], r);
                     }
                 }
                 __syncwarp();
@@ -408,55 +574,24 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
                 if (CL > 1 && lane > 0 && lane < CL) cg::this_cluster().map_shared_rank(&s, lane)->mode = MODE_DONE;
                 break;
             }
+            // =========================================================== select
+            // A node names the child that the arg-max over its children's UCBs picks (the backup of every path keeps that up to
+            // date), so the walk is one dependent load per level.
             const unsigned c_step = (unsigned)clock();   // 32-bit cycle counts: differences are right modulo 2^32
             int node = 0;
             int4 r = rec_load(rec, cache, cache_n, 0);
             int depth = 0;
             if (lane == 0) {
                 s.path[0] = 0;
-                s.path_ns[0] = r.x;
-                s.path_wins[0] = r.y;
+                s.path_rec[0] = r;
             }
-            // log(N) of the node being left is needed by every child's UCB; each lane computes the logarithm of ITS child's
-            // count while it evaluates the child's UCB (two independent float64 chains), so the winner's value is ready
-            // for the next level instead of starting that level with a ~100-operation dependent chain
-            double log_parent = (r.w & 0x7F) != 0 ? log((double)r.x) : 0.0;
-            while ((r.w & 0x7F) != 0 && depth < 46) {
-                const unsigned mask = r.w & 0x7F;
-                int child = -1;
-                int4 cr = make_int4(0, 0, -1, 0);
-                unsigned key = 0;
-                double log_child = 0.0;
-                if (lane < A && ((mask >> lane) & 1u)) {
-                    child = r.z + __popc(mask & ((1u << lane) - 1u));
-                    cr = rec_load(rec, cache, cache_n, child);
-                    float v;
-                    if (cr.x == 0) {
-                        v = __int_as_float(0x7f800000);
-                    } else {
-                        // src/mctsnc.py:1337 -- evaluated in float64 (numba promotes int32/float32 and log(int32) to
-                        // float64), fused multiply-add as NVVM contracts it, rounded once to float32
-                        const double q = (double)cr.y / (double)__int2float_rn(cr.x);
-                        const double e = sqrt(log_parent / (double)cr.x);
-                        v = __double2float_rn(fma(c_ucb, e, q));
-                        log_child = log((double)cr.x);
-                    }
-                    key = ordered_key(v);
-                }
-                const unsigned best = __reduce_max_sync(0xFFFFFFFFu, key);
-                const unsigned tied = __ballot_sync(0xFFFFFFFFu, key == best && child >= 0) & 0x7Fu;
-                const int w = pick_among_tied(tied);
-                node = __shfl_sync(0xFFFFFFFFu, child, w);
-                r.x = __shfl_sync(0xFFFFFFFFu, cr.x, w);
-                r.y = __shfl_sync(0xFFFFFFFFu, cr.y, w);
-                r.z = __shfl_sync(0xFFFFFFFFu, cr.z, w);
-                r.w = __shfl_sync(0xFFFFFFFFu, cr.w, w);
-                log_parent = __shfl_sync(0xFFFFFFFFu, log_child, w);
+            while ((r.w & 0x7F) != 0 && depth < MAX_PATH - 2) {
+                node = r.z + meta_best(r.w);
+                r = rec_load(rec, cache, cache_n, node);
                 depth++;
                 if (lane == 0) {
                     s.path[depth] = node;
-                    s.path_ns[depth] = r.x;
-                    s.path_wins[depth] = r.y;
+                    s.path_rec[depth] = r;
                 }
             }
             // ------------------------------------------------------- expand (_expand_1_* and _expand_2_*)
@@ -488,9 +623,7 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
                     if (OCP) {
                         // src/mctsnc.py:1435 / :1511 -- float32 * int64 is a float64 product, truncated
                         if (lane == 0) {
-                            ulonglong2 es = p.rng_expand[g];
-                            const float u = rng_uniform_f32(es.x, es.y);
-                            p.rng_expand[g] = es;
+                            const float u = rng_uniform_f32(pick_stream.x, pick_stream.y);
                             pick = __double2int_rz((double)u * (double)n_exp);
                             if (pick >= n_exp) {  // u == 1.0f: undefined in the reference, clamped
                                 pick = n_exp - 1;
@@ -505,7 +638,7 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
                     unsigned long long cneg = bb.x, cpos = bb.y, call = all;
                     int outcome = 2;
                     if (has_child) {
-                        const unsigned long long move = (all + (1ULL << (7 * lane))) & (0x3FULL << (7 * lane));
+                        const unsigned long long move = (all + (1ULL << column_shift(lane))) & (0x3FULL << column_shift(lane));
                         if (sel_turn > 0) cpos |= move;
                         else cneg |= move;
                         call = all | move;
@@ -519,17 +652,17 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
                     n_slots = __popc(play_mask);
                     if (has_child) {
                         const int j = plays ? __popc(play_mask & ((1u << lane) - 1u)) : -1;
-                        s.child_action[k] = lane;
                         s.child_outcome[k] = outcome;
                         s.child_slot[k] = j;
                         if (plays) {
                             GameSlot gs;
+                            const unsigned open = legal_columns(call);
                             gs.cur = sel_turn > 0 ? cneg : cpos;  // the child is to be moved in by the other side
-                            gs.top = call + BOTTOM_ROW;
-                            gs.legal = legal_columns(call) << LEGAL_SHIFT;
+                            gs.other = sel_turn > 0 ? cpos : cneg;
+                            gs.row = move_row(open);
+                            gs.count = (float)__popc(open) * RNG_2M64;
                             gs.rng_base = OCP ? 0 : lane * P;
                             gs.stones = __popcll(call);
-                            gs.count = (float)__popc(gs.legal) * RNG_2M64;
                             s.slot[j] = gs;
                             s.tally[j][0] = 0;
                             s.tally[j][1] = 0;
@@ -544,11 +677,11 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
                     if (lane == 0) {
                         GameSlot gs;
                         gs.cur = sel_turn > 0 ? bb.y : bb.x;
-                        gs.top = all + BOTTOM_ROW;
-                        gs.legal = legal << LEGAL_SHIFT;
+                        gs.other = sel_turn > 0 ? bb.x : bb.y;
+                        gs.row = move_row(legal);
+                        gs.count = (float)n_legal * RNG_2M64;
                         gs.rng_base = 0;
                         gs.stones = __popcll(all);
-                        gs.count = (float)n_legal * RNG_2M64;
                         s.slot[0] = gs;
                         s.tally[0][0] = 0;
                         s.tally[0][1] = 0;
@@ -573,14 +706,13 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
                 if (mode == MODE_ALL_CHILDREN) s.size += n_exp;
                 s.ae[A + 1] = (short)(mode == MODE_ALL_CHILDREN ? n_exp : 1);
                 int m2 = mode;
-                if (OCP && mode == MODE_ALL_CHILDREN) m2 = thrifty ? pick : s.child_action[pick];
+                if (OCP && mode == MODE_ALL_CHILDREN) m2 = thrifty ? pick : nth_set(exp_mask, pick);
                 s.ae[A] = (short)m2;
                 if (!OCP && mode != MODE_ALL_CHILDREN) s.ae[0] = 0;
-                s.next_item = 0;
+                s.next_item = first_free_item;
                 s.n_slots = n_slots;
                 s.pick = pick;
                 s.mode = mode;
-                s.n_exp = n_exp;
                 s.exp_mask = exp_mask;
                 s.first_child = first_child;
                 s.selected = node;
@@ -593,7 +725,11 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
             }
             step++;
             backup_due = true;
-            if (mode == MODE_TERMINAL) continue;
+            if (mode == MODE_TERMINAL) {
+                __syncwarp();
+                prepare_backup<OCP>(s, rec, cache, cache_n, c_ucb, lane, depth + 1, P, 0);
+                continue;
+            }
             if (CL > 1) {
                 // the step's games for the other blocks of the cluster: stores into their shared memory, made visible by
                 // the barrier below
@@ -605,7 +741,7 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
                         rs->n_slots = n_slots;
                         rs->mode = mode;
                         rs->sel_meta = r.w;
-                        rs->next_item = 0;
+                        rs->next_item = nt;
                     }
                 }
             }
@@ -621,109 +757,127 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
         // item / P; it draws from the stream the reference's thread (tree, action, t) owns (src/mctsnc.py:1938, :2028;
         // OCP: cuda.grid(1), :1849), so which thread plays it does not matter.
         //
-        // The board of a game in progress is three words: the stones of the side that moves at the even plies of a
-        // block of PLIES_PER_CHECK plies (a game starts at ply 0 of a block, so that is the side to move in the game's
-        // first position), the stones of the other side, and `top`, one bit per column at its lowest empty cell (the
-        // guard bit once the column is full; top = all stones + BOTTOM_ROW).  A move in a column with room is then
-        // top & (six cells of the column), and top + move puts the marker one cell up.
+        // The first game of every thread is its own number.  The walker has the counts and logarithms of the backup to work
+        // out first and takes what games are left after that.
+        //
+        // The board of a game in progress is three pairs of words: the stones of the side that moves at the even plies of a
+        // block of PLIES plies (a game starts at ply 0 of a block, so that is the side to move in the game's first
+        // position), the stones of the other side, and `top`, one bit per column at its lowest empty cell (the guard bit
+        // once the column is full; top = all stones + bottom row).  A move in a column with room is then top & (six cells
+        // of the column), and top + move puts the marker one cell up; columns are bytes, so the two words never carry.
         {
             const int n_items = s.n_slots << log2_local;
             // the side to move in the played-out positions: the other side than at the selected node, unless the
             // selected node itself is played out
             const int first_mover = (s.mode == MODE_TREE_FULL) ? meta_turn(s.sel_meta) : -meta_turn(s.sel_meta);
-            unsigned long long side_even = 0, side_odd = 0, top = 0, s0 = 0, s1 = 0;
-            unsigned legal = 0;
-            float count = 0.f;
+            unsigned even_lo = 0, even_hi = 0, odd_lo = 0, odd_hi = 0, top_lo = 0, top_hi = 0;
+            unsigned long long s0 = 0, s1 = 0;
+            float row = 0.f, count = 0.f;
             int rng_idx = 0, stones = 0, j = 0;
-            int item = atomicAdd(&s.next_item, 1);
-            if (item < n_items) {
+            int item = tid - (nt - first_free_item);
+            if (walker) {
+                const int sel_n = s.mode == MODE_ALL_CHILDREN && !OCP ? P * __popc(s.exp_mask) : P;
+                prepare_backup<OCP>(s, rec, cache, cache_n, c_ucb, lane, s.path_len, sel_n, s.mode == MODE_ALL_CHILDREN ? P : 0);
+                if (item < 0) item = atomicAdd(&s.next_item, 1);
+            }
+            auto start_game = [&]() {
                 j = item >> log2_local;
                 const GameSlot gs = s.slot[j];
-                side_even = gs.cur;
-                side_odd = (gs.top - BOTTOM_ROW) ^ gs.cur;
-                top = gs.top;
-                legal = gs.legal;
+                even_lo = (unsigned)gs.cur;
+                even_hi = (unsigned)(gs.cur >> 32);
+                odd_lo = (unsigned)gs.other;
+                odd_hi = (unsigned)(gs.other >> 32);
+                top_lo = (even_lo | odd_lo) + BOTTOM_LO + MARK;
+                top_hi = (even_hi | odd_hi) + BOTTOM_HI;
+                row = gs.row;
                 count = gs.count;
                 stones = gs.stones;
                 rng_idx = (gs.rng_base >> LOG_CL) + (item & (P_local - 1));
                 const ulonglong2 rs = s_rng[rng_idx];
                 s0 = rs.x;
                 s1 = rs.y;
-            }
-            while (item < n_items) {
-                // A finished game is noticed only every PLIES_PER_CHECK plies: its lane sits out the plies in between.  The
-                // code that closes a game and fetches the next one (about 30 instructions) runs for the few lanes whose
-                // games have just ended while the others wait, and with a check after every ply it ran in nearly every
-                // iteration; checking after every fourth ply costs a little lane time and saved 10 % of the run time
-                // (13.8 -> 15.3 G playouts/s on the headline workload; 2: 14.9, 3: 15.3, 5: 15.4, 8: 14.1).
-                bool win = false, over = false;
-                unsigned no_column = 0;   // bit 31 set once a draw of 1.0f asked for a column the position does not have
-                static_assert(PLIES_PER_CHECK % 2 == 0, "the two sides alternate by the parity of the ply within a block");
+            };
+            // PLIES plies.  STRAIGHT: no branch; a game that is over has no move left (`row` names the empty column set) and draws
+            // on to the end of the block, which is put right when it is closed.  So the generator runs ahead of the moves,
+            // which shortens a ply from the whole chain to the part from the table to the four test.
+            unsigned fours = 0u;
+            auto play_block = [&]() {
+                fours = 0u;
+                static_assert(PLIES % 2 == 0, "the two sides alternate by the parity of the ply within a block");
 #pragma unroll
-                for (int k = 0; k < PLIES_PER_CHECK; k++) {
-                    if (over) continue;
+                for (int k = 0; k < PLIES; k++) {
+                    if (!STRAIGHT && fours != 0u) continue;
                     // ---- one ply (src/mctsnc.py:2059-2064, :2069)
-                    // float32 u * int16 count -> float32 (:2061); here (u * 2^64) * (count * 2^-64): the same product.
-                    // u == 1.0f gives ord == count, which the table answers with MOVE_LUT_NO_COLUMN: nothing is played, the flag
-                    // sticks, and the game is replayed from its start through the byte-level emulation when it is closed
+                    // float32 u * int16 count -> float32 (:2061); here (u * 2^64) * (count * 2^-64): the same product
                     const float f = rng_uniform_times_2p64(s0, s1);
-                    const int ord = __float2int_rz(__fmul_rn(f, count));
-                    const unsigned long long e = *reinterpret_cast<const unsigned long long *>(
-                        reinterpret_cast<const char *>(s.move_lut) + (legal + ord * 8));
-                    no_column |= (unsigned)(e >> 32);
-                    const unsigned long long move = top & e;
-                    top += move;
+                    const MoveEntry m = load_move(lut_base, __float_as_uint(__fadd_rz(__fmul_rn(f, count), row)));
+                    const unsigned move_lo = top_lo & m.lo, move_hi = top_hi & m.hi;
+                    top_lo += move_lo;
+                    top_hi += move_hi;
                     // the sides take turns with the plies of the unrolled block: no swap of "mine" and "theirs"
-                    unsigned long long mine;
                     if (k & 1) {
-                        side_odd |= move;
-                        mine = side_odd;
+                        odd_lo |= move_lo;
+                        odd_hi |= move_hi;
+                        fours |= fours_with(odd_lo, odd_hi, m.lo);
                     } else {
-                        side_even |= move;
-                        mine = side_even;
+                        even_lo |= move_lo;
+                        even_hi |= move_hi;
+                        fours |= fours_with(even_lo, even_hi, m.lo);
                     }
-                    win = has_four(mine);
-                    if ((move & TOP_ROW) != 0) {
-                        legal ^= (unsigned)(e >> 48);
-                        count -= RNG_2M64;
-                    }
-                    over = win || count == 0.0f;
+                    close_column((move_lo & TOP_LO) | (move_hi & TOP_HI), row, count, m.lo);
+                    if (STRAIGHT && fours != 0u) row = NO_MOVES;
                 }
-                if (over || (no_column & 0x80000000u)) {
-                    int n = __popcll(side_even | side_odd) - stones;  // plies of this game; the last one was made by the
-                    int winner = 0;                                    // first mover iff n is odd
-                    if (win) winner = (n & 1) ? first_mover : -first_mover;
-                    if (no_column & 0x80000000u) {
-                        // u == 1.0f somewhere in this game: replay it through the byte-level emulation of the reference
-                        const GameSlot gs = s.slot[j];
-                        const ulonglong2 rs = s_rng[rng_idx];
-                        const unsigned long long other = (gs.top - BOTTOM_ROW) ^ gs.cur;
-                        const EmuResult er = playout_emulated(first_mover > 0 ? other : gs.cur, first_mover > 0 ? gs.cur : other,
-                                                              first_mover, rs.x, rs.y);
-                        s0 = er.s0;
-                        s1 = er.s1;
-                        winner = er.outcome == 2 ? 0 : er.outcome;
-                        n = (int)er.plies;
-                        my_ub += er.ub;
-                        my_err |= er.err;
-                    }
-                    s_rng[rng_idx] = make_ulonglong2(s0, s1);
-                    my_plies += n;
-                    if (winner != 0) atomicAdd(&s.tally[j][winner > 0 ? 1 : 0], 1);
-                    item = atomicAdd(&s.next_item, 1);
+            };
+            auto marked = [&]() { return ((even_lo | odd_lo) & MARK) != 0u; };   // a draw of 1.0f, see MoveEntry
+            auto over = [&]() { return fours != 0u || marked() || row == NO_MOVES; };
+            auto close_game = [&]() {
+                int n = __popc(even_lo | odd_lo) + __popc(even_hi | odd_hi) - stones;  // plies of this game; the last one was made
+                int winner = 0;                                                        // by the first mover iff n is odd
+                if (fours != 0u) winner = (n & 1) ? first_mover : -first_mover;
+                if (STRAIGHT || fours == 0u)
+                    for (int k = n % PLIES; k != 0 && k < PLIES; k++) rng_back(s0, s1);
+                if (marked()) {
+                    // u == 1.0f somewhere in this game: replay it through the byte-level emulation of the reference
+                    const GameSlot gs = s.slot[j];
+                    const ulonglong2 rs = s_rng[rng_idx];
+                    const EmuResult er = playout_emulated(first_mover > 0 ? gs.other : gs.cur, first_mover > 0 ? gs.cur : gs.other,
+                                                          first_mover, rs.x, rs.y);
+                    s0 = er.s0;
+                    s1 = er.s1;
+                    winner = er.outcome == 2 ? 0 : er.outcome;
+                    n = (int)er.plies;
+                    my_ub += er.ub;
+                    my_err |= er.err;
+                }
+                s_rng[rng_idx] = make_ulonglong2(s0, s1);
+                my_plies += n;
+                if (winner != 0) atomicAdd(&s.tally[j][winner > 0 ? 1 : 0], 1);
+                item = atomicAdd(&s.next_item, 1);
+            };
+            if (STRAIGHT) {
+                // About one game per thread: a warp plays its games to the end together and closes them together.  Closed one by
+                // one, every game that ends would hold up the ones still going on in its warp by the closing (a few hundred
+                // cycles of shared-memory atomics and the generator's way back, nine times per 32 games).
+                while (__any_sync(0xFFFFFFFFu, item < n_items)) {
                     if (item < n_items) {
-                        j = item >> log2_local;
-                        const GameSlot gs = s.slot[j];
-                        side_even = gs.cur;
-                        side_odd = (gs.top - BOTTOM_ROW) ^ gs.cur;
-                        top = gs.top;
-                        legal = gs.legal;
-                        count = gs.count;
-                        stones = gs.stones;
-                        rng_idx = (gs.rng_base >> LOG_CL) + (item & (P_local - 1));
-                        const ulonglong2 rs = s_rng[rng_idx];
-                        s0 = rs.x;
-                        s1 = rs.y;
+                        start_game();
+                        do play_block();
+                        while (!over());
+                    }
+                    __syncwarp();
+                    if (item < n_items) close_game();
+                }
+            } else {
+                // Several games per thread: a lane takes its next game at once.  A finished game is noticed only every PLIES
+                // plies (its lane sits out the plies in between): the code that closes a game and starts the next one (about 40
+                // instructions) runs for the few lanes whose games have just ended while the others wait, and with a look
+                // after every ply it ran in nearly every iteration.
+                if (item < n_items) start_game();
+                while (item < n_items) {
+                    play_block();
+                    if (over()) {
+                        close_game();
+                        if (item < n_items) start_game();
                     }
                 }
             }
@@ -754,6 +908,7 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
         }
         if (my_err) atomicOr(&home->status, STATUS_INTERNAL);
     }
+    if (OCP && walker && lane == 0) p.rng_expand[g] = pick_stream;
     if (CL > 1) cg::this_cluster().sync();   // also: no block leaves while another may still write to its shared memory
     else __syncthreads();
     for (int i = tid; i < (n_streams >> LOG_CL); i += nt)
@@ -789,22 +944,25 @@ __device__ __forceinline__ long long global_timer_ns() {
 
 __device__ __forceinline__ void build_move_lut(Shared &s) {
     for (int i = threadIdx.x; i < 128 * 8; i += blockDim.x) {
-        const int set = i >> 3, ord = i & 7;
-        int col = -1, seen = 0;
-        for (int c = 0; c < COLS; c++)
-            if (set & (1 << c)) {
-                if (seen == ord) col = c;
-                seen++;
-            }
-        s.move_lut[i] = col < 0 ? MOVE_LUT_NO_COLUMN
-                                : (0x3FULL << (7 * col)) | ((unsigned long long)((1 << col) << LEGAL_SHIFT) << 48);
+        const int set = (i >> 3) ^ 1, ord = i & 7;
+        MoveEntry m;
+        m.lo = m.hi = 0u;
+        if (ord < __popc(set)) {
+            const int col = nth_set(set, ord);
+            const unsigned long long cells = 0x3FULL << column_shift(col);
+            m.lo = (unsigned)cells | (unsigned)(col + 1);
+            m.hi = (unsigned)(cells >> 32);
+        } else if (set != 0) {
+            m.lo = MARK;
+        }
+        s.move_lut[i] = m;
     }
 }
 
 #ifndef MCTSNC_C4_MAXNREG
 #define MCTSNC_C4_MAXNREG 64
 #endif
-template <bool OCP>
+template <bool OCP, bool STRAIGHT>
 __global__ void __maxnreg__(MCTSNC_C4_MAXNREG) search_kernel(const SearchParams p) {
     __shared__ Shared s;
     extern __shared__ ulonglong2 s_rng[];
@@ -823,7 +981,7 @@ __global__ void __maxnreg__(MCTSNC_C4_MAXNREG) search_kernel(const SearchParams 
         const int n_steps = (queued && rem > p.chunk) ? p.chunk : rem;
         long long t_start = 0;
         if (queued && tid == 0) t_start = global_timer_ns();
-        run_slice<OCP, 1>(p, s, s_rng, nullptr, g, n_steps, p.first != 0 && rem == p.steps);
+        run_slice<OCP, 1, STRAIGHT>(p, s, s_rng, nullptr, g, n_steps, p.first != 0 && rem == p.steps);
         if (!queued) break;
         __syncthreads();  // every thread's writes of the slice precede the fence of thread 0
         if (tid == 0) {
@@ -877,7 +1035,7 @@ __global__ void __launch_bounds__(CLUSTER_THREADS) search_cluster_kernel(const S
     extern __shared__ ulonglong2 s_rng[];
     build_move_lut(s);
     const int n_local = ((OCP ? 1 : A) * p.n_playouts) / CLUSTER_BLOCKS;   // streams this block keeps; the record cache follows
-    run_slice<OCP, CLUSTER_BLOCKS>(p, s, s_rng, reinterpret_cast<int4 *>(s_rng + n_local), (int)(blockIdx.x / CLUSTER_BLOCKS), p.steps,
+    run_slice<OCP, CLUSTER_BLOCKS, true>(p, s, s_rng, reinterpret_cast<int4 *>(s_rng + n_local), (int)(blockIdx.x / CLUSTER_BLOCKS), p.steps,
                                    p.first != 0);
 }
 

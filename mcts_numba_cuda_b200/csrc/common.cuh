@@ -16,6 +16,7 @@
 //        bit  7      terminal          (trees_terminals)
 //        bits 8..9   outcome + 1, 3 = game ongoing (trees_outcomes)
 //        bit  10     1 if the player to move is +1 (trees_turns)
+//        bits 11..13 rank of the child that select goes on to (Connect-4; the backup of a path keeps it up to date)
 //        bits 16..31 depth             (trees_depths)
 // A node is a leaf (trees_leaves) while its expanded-action set is empty.
 #pragma once
@@ -27,6 +28,8 @@ namespace mctsnc {
 constexpr int META_TERMINAL = 1 << 7;
 constexpr int META_OUTCOME_SHIFT = 8;
 constexpr int META_TURN_POS = 1 << 10;
+constexpr int META_BEST_SHIFT = 11;
+constexpr int META_BEST_MASK = 7 << META_BEST_SHIFT;
 constexpr int META_DEPTH_SHIFT = 16;
 
 constexpr int MODE_ALL_CHILDREN = -2;  // trees_actions_expanded[ti, -2] of the ACP variants
@@ -42,6 +45,7 @@ constexpr int PATH_CAP = 256;  // longest root-to-leaf path kept per tree (Conne
 
 __host__ __device__ __forceinline__ int meta_outcome(int meta) { return ((meta >> META_OUTCOME_SHIFT) & 3) - 1; }
 __host__ __device__ __forceinline__ int meta_turn(int meta) { return (meta & META_TURN_POS) ? 1 : -1; }
+__host__ __device__ __forceinline__ int meta_best(int meta) { return (meta >> META_BEST_SHIFT) & 7; }
 __host__ __device__ __forceinline__ int meta_depth(int meta) { return (meta >> META_DEPTH_SHIFT) & 0xFFFF; }
 __host__ __device__ __forceinline__ int make_meta(int mask, bool terminal, int outcome, int turn, int depth) {
     return mask | (terminal ? META_TERMINAL : 0) | ((outcome + 1) << META_OUTCOME_SHIFT) |

@@ -476,8 +476,8 @@ int c4_encode_root(const int8_t *board, const int8_t *fills, ulonglong2 *out) {
                 continue;
             }
             if (gap || (v != 1 && v != -1)) return MCTSNC_E_BAD_ROOT;  // a disc above an empty cell
-            if (v > 0) pos |= 1ULL << (7 * j + h);
-            else neg |= 1ULL << (7 * j + h);
+            if (v > 0) pos |= 1ULL << (c4::column_shift(j) + h);
+            else neg |= 1ULL << (c4::column_shift(j) + h);
             f++;
         }
         if (fills && fills[j] != f) return MCTSNC_E_BAD_ROOT;
@@ -570,11 +570,17 @@ void release(mctsnc_handle *h) {
 #endif
 constexpr int SLICE_STEPS = MCTSNC_SLICE_STEPS;  // steps a block runs of one tree before it takes the next tree from the queue
 
-const void *search_kernel_ptr(const mctsnc_config &c) {
-    return is_ocp(c) ? (const void *)c4::search_kernel<true> : (const void *)c4::search_kernel<false>;
+// A step whose games all have a thread of their own is as long as its longest game: the playouts then go straight through
+// blocks of plies (2.7 us a step against 4.6 for 32 games; with five games a thread 49 ms against 36 for a search of 2000 steps
+// that takes a block of 1024 threads, so with more games than threads a lane takes its next game at once).
+bool play_straight(const mctsnc_config &c, int threads) { return threads >= c.n_playouts * (is_ocp(c) ? 1 : c4::A); }
+
+const void *search_kernel_ptr(const mctsnc_config &c, bool straight) {
+    if (straight) return is_ocp(c) ? (const void *)c4::search_kernel<true, true> : (const void *)c4::search_kernel<false, true>;
+    return is_ocp(c) ? (const void *)c4::search_kernel<true, false> : (const void *)c4::search_kernel<false, false>;
 }
 
-// Threads of the block that grows one tree, from the games a step plays (n_playouts, times the children of a node for
+// Threads that play the games of one tree, from the games a step plays (n_playouts, times the children of a node for
 // the ACP variants) and from how many trees there are for the device.
 //   Many trees (at least two per SM): a quarter of the games, between 32 and 320; half of them when a step has at most 256
 //   games.  Measured on 256 roots: headline ACP
@@ -596,7 +602,7 @@ int choose_threads(mctsnc_handle *h, long long trees) {
     if (trees >= 2LL * h->sm_count) threads = fit(games <= 256 ? games / 2 : games / 4, 320);
     else if (trees <= h->sm_count) threads = fit(games, 1024);
     else threads = fit(games / 2, 512);
-    const void *fn = search_kernel_ptr(h->cfg);
+    const void *fn = search_kernel_ptr(h->cfg, play_straight(h->cfg, threads));
     int per_sm = 0;
     while (threads > 32 &&
            (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, h->dyn_smem) != cudaSuccess || per_sm < 1))
@@ -790,8 +796,8 @@ int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_
         attr.val.clusterDim.z = 1;
         lc.attrs = &attr;
         lc.numAttrs = 1;
-        if (is_ocp(h->cfg)) cudaFuncSetAttribute(c4::search_cluster_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024);
-        else cudaFuncSetAttribute(c4::search_cluster_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024);
+        if (is_ocp(h->cfg)) cudaFuncSetAttribute(c4::search_cluster_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        else cudaFuncSetAttribute(c4::search_cluster_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         // The first records of a tree stay in the first block's shared memory: many if every block can have an SM to itself,
         // else few.  All clusters of the launch have to be on the device at once (clusters do not spread over GPCs, so fewer
         // fit than blocks / 8): a tree whose cluster waits for another to finish would take two searches' time.
@@ -820,10 +826,14 @@ int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_
         }
         p.cache_nodes = 0;
     }
-    const int threads = h->cfg.threads_per_tree > 0 ? h->cfg.threads_per_tree : choose_threads(h, trees);
+    int threads = h->cfg.threads_per_tree > 0 ? h->cfg.threads_per_tree : choose_threads(h, trees);
     h->threads = threads;
+    // A tree that has an SM to itself gets a warp more, for the walker: it works out the counts and logarithms of the backup
+    // while the others play (one warp for 32 games and the walker: 5.9 us a step, two: 4.4).
+    if (h->cfg.threads_per_tree == 0 && trees <= h->sm_count && threads + 32 <= 1024) threads += 32;
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, search_kernel_ptr(h->cfg), threads, h->dyn_smem) != cudaSuccess || per_sm < 1)
+    const void *kernel = search_kernel_ptr(h->cfg, play_straight(h->cfg, threads));
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, h->dyn_smem) != cudaSuccess || per_sm < 1)
         return MCTSNC_E_BAD_ARGUMENT;
     h->blocks_per_sm = per_sm;
     // More trees than blocks fit on the device at once: a persistent grid takes slices of SLICE_STEPS steps from the
@@ -847,8 +857,8 @@ int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_
         }
         grid = (unsigned)resident;
     }
-    if (is_ocp(h->cfg)) c4::search_kernel<true><<<grid, threads, h->dyn_smem, stream>>>(p);
-    else c4::search_kernel<false><<<grid, threads, h->dyn_smem, stream>>>(p);
+    void *args[] = {&p};
+    CUDA_TRY(cudaLaunchKernel(kernel, dim3(grid), dim3((unsigned)threads), args, h->dyn_smem, stream));
     if (p.queue) check_queue_kernel<<<(unsigned)((trees + 255) / 256), 256, 0, stream>>>(h->remaining, h->state, (int)trees);
     return (int)cudaGetLastError();
 }
@@ -981,17 +991,21 @@ extern "C" int mctsnc_create(const mctsnc_config *cfg, mctsnc_handle **out) {
     h->dyn_smem = sizeof(ulonglong2) * (size_t)(h->rng_per_search / c.n_trees);
     if (is_gomoku(c))   // per-thread game state + per-warp templates + the tables of the exactly-five test
         h->dyn_smem = gomoku::DYN_SMEM_BYTES;
-    if (h->dyn_smem > 48 * 1024) {
-        const void *kernel = is_gomoku(c) ? (ocp ? (const void *)gomoku::playout_dynamic_kernel<true> : (const void *)gomoku::playout_dynamic_kernel<false>)
-                                          : search_kernel_ptr(c);
-        // the limit belongs to the kernel, not to the handle: never lower what another handle (or a launch) has asked for
-        cudaFuncAttributes now;
-        cudaError_t e = cudaFuncGetAttributes(&now, kernel);
-        if (e == cudaSuccess && (size_t)now.maxDynamicSharedSizeBytes < h->dyn_smem)
-            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->dyn_smem);
-        if (e != cudaSuccess) {
-            delete h;
-            return (int)e;
+    if (h->dyn_smem > 28 * 1024) {   // with the kernels' static part more than the 48 KB every launch may have
+        const void *kernels[2] = {is_gomoku(c) ? (ocp ? (const void *)gomoku::playout_dynamic_kernel<true> : (const void *)gomoku::playout_dynamic_kernel<false>)
+                                               : search_kernel_ptr(c, false),
+                                  is_gomoku(c) ? nullptr : search_kernel_ptr(c, true)};
+        for (const void *kernel : kernels) {
+            if (!kernel) continue;
+            // the limit belongs to the kernel, not to the handle: never lower what another handle (or a launch) has asked for
+            cudaFuncAttributes now;
+            cudaError_t e = cudaFuncGetAttributes(&now, kernel);
+            if (e == cudaSuccess && (size_t)now.maxDynamicSharedSizeBytes < h->dyn_smem)
+                e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h->dyn_smem);
+            if (e != cudaSuccess) {
+                delete h;
+                return (int)e;
+            }
         }
     }
     int rc = 0;
@@ -1367,7 +1381,7 @@ extern "C" int mctsnc_export(mctsnc_handle *h, int32_t search, int32_t field, vo
                 if (valid)
                     for (int j = 0; j < c4::COLS; j++)
                         for (int hgt = 0; hgt < c4::ROWS; hgt++) {
-                            const int bit = 7 * j + hgt;
+                            const int bit = c4::column_shift(j) + hgt;
                             const int v = ((brd[(size_t)i].y >> bit) & 1ULL) ? 1 : (((brd[(size_t)i].x >> bit) & 1ULL) ? -1 : 0);
                             bo[(c4::ROWS - 1 - hgt) * c4::COLS + j] = (int8_t)v;
                         }
@@ -1378,7 +1392,7 @@ extern "C" int mctsnc_export(mctsnc_handle *h, int32_t search, int32_t field, vo
                 memset(eo, 0, extra);
                 if (valid) {
                     const unsigned long long all = brd[(size_t)i].x | brd[(size_t)i].y;
-                    for (int j = 0; j < c4::COLS; j++) eo[j] = (int8_t)__builtin_popcountll((all >> (7 * j)) & 0x3FULL);
+                    for (int j = 0; j < c4::COLS; j++) eo[j] = (int8_t)__builtin_popcountll((all >> c4::column_shift(j)) & 0x3FULL);
                 }
                 break;
             }
@@ -1634,8 +1648,8 @@ extern "C" int mctsnc_search_c4_static(const int8_t *board, const int8_t *extra_
     p.ms_per_cycle = 0.f;
     p.cache_nodes = 0;
     const size_t dyn_smem = sizeof(ulonglong2) * (size_t)per_tree;   // <= 28 KB: below the 48 KB that need an opt-in
-    if (ocp) c4::search_kernel<true><<<n_trees, 256, dyn_smem, s>>>(p);
-    else c4::search_kernel<false><<<n_trees, 256, dyn_smem, s>>>(p);
+    if (ocp) c4::search_kernel<true, false><<<n_trees, 256, dyn_smem, s>>>(p);
+    else c4::search_kernel<false, false><<<n_trees, 256, dyn_smem, s>>>(p);
     CUDA_TRY(cudaGetLastError());
     long long *out = reinterpret_cast<long long *>(out_device);
     reduce_over_trees_kernel<<<1, 256, 0, s>>>(sc->rec, sc->state, CAP, n_trees, A, out, sc->flags, sc->dres);

@@ -27,6 +27,13 @@ MCTS_HD unsigned long long rng_next(unsigned long long &s0, unsigned long long &
     return result;
 }
 
+// the state before the last rng_next
+MCTS_HD void rng_back(unsigned long long &s0, unsigned long long &s1) {
+    const unsigned long long t = rotl64(s1, 28);
+    s0 = rotl64(s0 ^ t ^ (t << 14), 9);
+    s1 = t ^ s0;
+}
+
 inline void rng_seed(RngState &s, unsigned long long seed) {
     unsigned long long z = seed + 0x9E3779B97F4A7C15ULL;
     z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ULL;
