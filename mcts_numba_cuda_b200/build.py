@@ -1,13 +1,17 @@
-"""Builds ``libmctsnc_b200.so`` in-tree with nvcc for sm_100a (cross-compiles without a GPU)."""
+"""Builds ``libmctsnc_b200.so`` in-tree with nvcc for sm_100a (cross-compiles without a GPU), and ``_wave.so``, the Python
+extension through which the tree selects are launched."""
 import os
 import shutil
 import subprocess
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 LIB_PATH = os.path.join(HERE, "libmctsnc_b200.so")
+WAVE_PATH = os.path.join(HERE, "_wave.so")
+WAVE_SOURCE = os.path.join(HERE, "csrc", "wave_module.cpp")
 SOURCES = [os.path.join(HERE, "csrc", n) for n in ("mctsnc_abi.cu", "peer_exchange.cu", "puct_select.cu", "puct_select_v2.cu", "duct_select.cu")]
-HEADERS = [os.path.join(HERE, "csrc", n) for n in ("c4_search.cuh", "gomoku_search.cuh", "common.cuh", "rng.cuh")] + [
+HEADERS = [os.path.join(HERE, "csrc", n) for n in ("c4_search.cuh", "gomoku_search.cuh", "common.cuh", "rng.cuh", "select_math.cuh")] + [
     os.path.join(ROOT, "include", "mctsnc_b200.h")]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-shared",
               "-Xcompiler", "-fPIC"]
@@ -20,15 +24,21 @@ def nvcc_path():
     return path
 
 
-def is_stale():
-    if not os.path.exists(LIB_PATH):
+def is_stale(path=LIB_PATH, sources=SOURCES + HEADERS):
+    if not os.path.exists(path):
         return True
-    built = os.path.getmtime(LIB_PATH)
-    return any(os.path.exists(p) and os.path.getmtime(p) > built for p in SOURCES + HEADERS)
+    built = os.path.getmtime(path)
+    return any(os.path.exists(p) and os.path.getmtime(p) > built for p in sources)
 
 
 def build(force=False, verbose=False):
-    """Compiles the library if it is missing or older than its sources; returns its path."""
+    """Compiles the library and the extension if they are missing or older than their sources; returns the library's path."""
+    if force or is_stale(WAVE_PATH, [WAVE_SOURCE]):
+        cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-I" + sysconfig.get_paths()["include"], "-o", WAVE_PATH,
+               WAVE_SOURCE]
+        res = subprocess.run(cmd, capture_output=True, text=True)
+        if res.returncode != 0:
+            raise RuntimeError("g++ failed:\n" + res.stdout + res.stderr)
     if force or is_stale():
         cmd = [nvcc_path()] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else []) + ["-o", LIB_PATH] + SOURCES
         res = subprocess.run(cmd, capture_output=True, text=True)

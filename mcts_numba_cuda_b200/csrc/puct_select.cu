@@ -10,20 +10,25 @@
 // path entry (node << 8) | edge (:436), the packed result reason << 25 | kind << 22 | slot << 14 | node (:38-41),
 // and the rollback of every claim of the traversal when it fails (:206-217).
 //
-// What is done differently: the traversal is latency-bound (dependent loads from gigabytes of edge arrays), so a level
-// is built to cost ONE memory round trip instead of four.  Every lane keeps child / prior / W / N / inflight of its
-// edges in registers; the parent count and the arg-max both come from those registers; and as soon as the winner is
-// known, the claim (atomicCAS), the child's node record and ALL the child's edges are requested together, so that the
-// next level starts with its data already on the way.  A retry after a lost CAS reloads only `inflight`.  Sums and
-// maxima use the warp-reduce instructions (redux.sync) instead of five rounds of three shuffles; the tie-break is a
-// second redux over the lanes that hold the maximum.
+// What is done differently: a traversal is a chain of dependent loads from gigabytes of edge arrays, and a warp that is alone
+// on its scheduler takes 4 to 5 cycles for every instruction of the chain between two of them, so a level is built to cost
+// ONE memory round trip and few instructions.  Every lane keeps child / prior / W / N / inflight of its edges in
+// registers; as soon as the winner is known, the child's node record and ALL the child's edges are requested, then the claim
+// (atomicCAS) is sent; and the claim's answer is looked at only when the child's own winner has been worked out, right before
+// anything else is claimed, so that its round trip is not waited for.  A lost claim goes back to the level it was made on
+// and reads that level's edges again.  Sums, maxima and the tie-break use the warp-reduce instructions (redux.sync); the
+// edge number of the winner names the lane that holds it.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "select_math.cuh"
+
 namespace puct {
 
-constexpr unsigned FULL = 0xFFFFFFFFu;
+using namespace select_math;
+
 constexpr int NODE_TERMINAL = -1;
+constexpr int OUTSIDE = -2;   // in place of a node's record: the node does not exist
 constexpr int NODE_LIMIT = 16384, NODE_MASK = 0x3FFF, EDGE_LIMIT = 256;
 constexpr int KIND_SHIFT = 22, SLOT_SHIFT = 14, REASON_SHIFT = 25;
 enum Kind { INVALID = 0, EXPAND = 1, TERMINAL = 2, DEPTH_LIMIT = 3, BUSY = 4 };
@@ -33,25 +38,16 @@ enum Reason {
     R_INVALID_CHILD_OOB = 15, R_INVALID_UNKNOWN = 16
 };
 constexpr int MAX_EVALUATIONS = 2;
-#ifndef PUCT_SELECT_WARPS_PER_BLOCK
-#define PUCT_SELECT_WARPS_PER_BLOCK 1
-#endif
-constexpr int SELECT_WARPS_PER_BLOCK = PUCT_SELECT_WARPS_PER_BLOCK;  // traversals per thread block of the select kernel
-constexpr float LOWEST = -3.4028234663852886e38f;
 constexpr int NO_EDGE = 0x7FFFFFFF;
 
 __device__ __forceinline__ int pack(int kind, int node, int slot, int reason) {
     return (reason << REASON_SHIFT) | (kind << KIND_SHIFT) | (slot << SLOT_SHIFT) | node;
 }
 
-__device__ __forceinline__ unsigned ordered(float v) {
-    const unsigned b = __float_as_uint(v);
-    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-}
-
 // undo the claims of the first `depth` path entries of this warp
 __device__ __forceinline__ void rollback(const int *path, int depth, int lane, int *edge_inflight, long long tree_edges_base,
                                          int node_cnt, int edges, int amount) {
+    __syncwarp();   // lane 0 wrote the entries
     for (int d = lane; d < depth; d += 32) {
         const int enc = path[d];
         const int parent = enc >> 8, slot = enc & 0xFF;
@@ -60,110 +56,260 @@ __device__ __forceinline__ void rollback(const int *path, int depth, int lane, i
     }
 }
 
-// the edges of one node as seen by one lane (edge lane + 32 k in slot k)
+// The edges of one node as seen by one lane (edge lane + 32 k in slot k).  Slots beyond the array's `edges` keep harmless values.
 template <int EPL>
 struct EdgeRegs {
+    const int *child_of, *n_of;   // of this tree
+    const float *prior_of, *w_of;
+    int *inflight_of;
     float prior[EPL], w[EPL];
     int n[EPL], inflight[EPL], child[EPL];
-};
 
-// requests all `edges` slots of a node, expanded or not (the arrays are dense, so the addresses are valid): used
-// before the node's record has arrived, i.e. before the number of expanded edges is known
-template <int EPL>
-__device__ __forceinline__ void load_edges(EdgeRegs<EPL> &r, long long e0, int lane, int edges, const int *edge_child_id,
-                                           const float *edge_prior, const float *edge_W, const int *edge_N,
-                                           const int *edge_inflight) {
+    __device__ __forceinline__ void init(long long tree_edges, const int *edge_child_id, const float *edge_prior, const float *edge_W,
+                                         const int *edge_N, int *edge_inflight) {
+        child_of = edge_child_id + tree_edges;
+        prior_of = edge_prior + tree_edges;
+        w_of = edge_W + tree_edges;
+        n_of = edge_N + tree_edges;
+        inflight_of = edge_inflight + tree_edges;
 #pragma unroll
-    for (int k = 0; k < EPL; k++) {
-        const int e = lane + 32 * k;
-        r.n[k] = 0;
-        r.inflight[k] = 0;
-        r.prior[k] = 0.f;
-        r.w[k] = 0.f;
-        r.child[k] = -1;
-        if (e < edges) {
-            r.child[k] = edge_child_id[e0 + e];
-            r.n[k] = edge_N[e0 + e];
-            r.inflight[k] = *(volatile const int *)&edge_inflight[e0 + e];
-            r.prior[k] = edge_prior[e0 + e];
-            r.w[k] = edge_W[e0 + e];
+        for (int k = 0; k < EPL; k++) {
+            prior[k] = w[k] = 1.f;
+            n[k] = 1;
+            inflight[k] = 0;
+            child[k] = -1;
         }
     }
-}
 
-// EPL: edges per lane, ceil(edges / 32) rounded up to 1, 2, 4 or 8 (registers follow it)
-template <int VL_GENERAL, int EPL>
-__global__ void select_kernel(float cpuct, float c_pw, float alpha_pw, int soft_winner, const int *__restrict__ edge_child_id,
-                              const float *__restrict__ edge_prior, const float *__restrict__ edge_W,
-                              const int *__restrict__ edge_N, int *edge_inflight, int *node_expand_inflight,
-                              const int *__restrict__ node_expanded, const int *__restrict__ tree_nodes, int *out_selected_node,
-                              int *out_path_eids, int *out_path_len, int trees, int nodes, int edges, int warps,
-                              int path_depth, int virtual_loss) {
-    // Traversal i = tree * warps + w is run by warp i of the grid, in blocks of SELECT_WARPS_PER_BLOCK warps.  The reference
-    // puts the `warps` traversals of a tree into one block (src/puct/puct_gpu_v3_cpp.cu:472-473); with 8 traversals per
-    // tree most of them lose the claim at the root and leave after two evaluations, and a block of 8 warps then keeps
-    // its 6 idle warp slots until its last traversal has gone all the way down.  Small blocks give the slots back at
-    // once; the traversals of a tree still start together (their warps are neighbours in the grid).  Measured on 4096
-    // trees x 64 edges x depth 16 with 8 / 1 traversals per tree: one warp per block 0.140 / 0.054 ms, two 0.140 / 0.060,
-    // four 0.149 / 0.057, eight (the reference's shape for 8) 0.307 / 0.079; the reference kernel 0.260 / 0.081.
-    const int lane = threadIdx.x & 31;
-    const int traversal = blockIdx.x * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5);
+    // requests all `edges` slots of a node, expanded or not (the arrays are dense, so the addresses are valid): this is done
+    // before the node's record has arrived, i.e. before the number of expanded edges is known
+    __device__ __forceinline__ void request(int node, int lane, int edges) {
+        const unsigned first = (unsigned)(node * edges + lane) * 4u;   // < 2^24
+#pragma unroll
+        for (int k = 0; k < EPL; k++)
+            if (lane + 32 * k < edges) {
+                n[k] = *at(n_of, first + 128u * k);
+                inflight[k] = *(volatile const int *)at(inflight_of, first + 128u * k);
+                prior[k] = *at(prior_of, first + 128u * k);
+                w[k] = *at(w_of, first + 128u * k);
+                child[k] = *at(child_of, first + 128u * k);
+            }
+    }
+};
+
+// EPL: edges per lane, ceil(edges / 32) rounded up to 1, 2, 4 or 8 (registers follow it).
+//
+// Traversal i = tree * warps + w is block i, a single warp.  The reference puts the `warps` traversals of a tree into one block
+// (src/puct/puct_gpu_v3_cpp.cu:472-473); with 8 traversals per tree most of them lose the claim at the root and leave after
+// two evaluations, and a block of 8 warps then keeps its 6 idle warp slots until its last traversal has gone all the way
+// down.  Small blocks give the slots back at once; the traversals of a tree still start together (their blocks are
+// neighbours in the grid).  As many blocks as an SM can hold (32) with up to 64 edges.
+// WIDENING: c_pw is not zero.
+template <int EPL, bool WIDENING>
+__global__ void __launch_bounds__(32, EPL <= 2 ? 32 : (EPL == 4 ? 24 : 16))
+select_kernel(float cpuct, float c_pw, float alpha_pw, int soft_winner, const int *__restrict__ edge_child_id,
+              const float *__restrict__ edge_prior, const float *__restrict__ edge_W, const int *__restrict__ edge_N,
+              int *edge_inflight, int *node_expand_inflight, const int *__restrict__ node_expanded,
+              const int *__restrict__ tree_nodes, int *out_selected_node, int *out_path_eids, int *out_path_len, int nodes,
+              int edges, int warps, int path_depth, int vl) {
+    const int lane = threadIdx.x;
+    const int traversal = blockIdx.x;
     const int tree = traversal / warps;
     const int wid = traversal - tree * warps;
-    const int vl = VL_GENERAL ? virtual_loss : 1;
-    if (tree >= trees) return;
-    const int out_ix = traversal;
-    int *path = out_path_eids + (long long)out_ix * path_depth;
+    int *path = out_path_eids + (long long)traversal * path_depth;
+    const long long tree_nodes_base = (long long)tree * nodes;
+    const long long tree_edges_base = tree_nodes_base * edges;
     const int node_cnt = tree_nodes[tree];
     if (!(path_depth >= 1 && nodes > 0 && node_cnt > 0 && node_cnt <= nodes && node_cnt <= NODE_LIMIT && edges > 0 &&
           edges <= EDGE_LIMIT)) {
         if (lane == 0) {
-            out_selected_node[out_ix] = pack(INVALID, NODE_MASK, 0, R_INVALID_SHAPE);
-            out_path_len[out_ix] = 0;
+            out_selected_node[traversal] = pack(INVALID, NODE_MASK, 0, R_INVALID_SHAPE);
+            out_path_len[traversal] = 0;
         }
         return;
     }
-    const long long tree_nodes_base = (long long)tree * nodes;
-    const long long tree_edges_base = tree_nodes_base * edges;
-    int result = pack(INVALID, NODE_MASK, 0, R_INVALID_UNKNOWN);
-    int result_len = 0;
+    const int *expanded = node_expanded + tree_nodes_base;
+    EdgeRegs<EPL> r;
+    r.init(tree_edges_base, edge_child_id, edge_prior, edge_W, edge_N, edge_inflight);
+    int *inflight_of_tree = edge_inflight + tree_edges_base;
     int node = 0, depth = 0;
-    int info = node_expanded[tree_nodes_base];
-    EdgeRegs<EPL> cur, nxt;
-    load_edges<EPL>(cur, tree_edges_base, lane, edges, edge_child_id, edge_prior, edge_W, edge_N, edge_inflight);
-    nxt = cur;
-    for (;;) {
-        if (info == NODE_TERMINAL) {
-            result = pack(TERMINAL, node, 0, R_OK_TERMINAL);
-            result_len = depth + 1;
-            break;
+    int info = expanded[0];
+    r.request(0, lane, edges);
+    bool outside = false;      // the child that was picked does not exist
+    float sqrt_parent = 0.f;
+    int attempt = 0;           // evaluations of this level that ended with a lost claim
+    // the claim made on the level above, until its answer is needed
+    bool pending = false;
+    int up_node = 0, up_info = 0, up_edge = 0, up_attempt = 0, up_seen = 0, up_old = 0;   // the last two: the owner's lane
+    float up_sqrt = 0.f;
+    int my_seen = 0, my_child = -1;    // of the lane's best edge
+
+    // arg-max over the expanded edges (two or more); NO_EDGE: no edge has a score (NaN and -inf are none)
+    auto arg_max = [&](int n_exp) {
+        // ties go to the edge closest after `rot` = wid modulo n_exp (small numbers: the product with the reciprocal truncates
+        // right)
+        const int rot = wid - n_exp * (int)(((float)wid + 0.5f) * reciprocal((float)n_exp));
+        float score[EPL];
+        float my_best = LOWEST_INF;
+        bool plain = true;
+#pragma unroll
+        for (int k = 0; k < EPL; k++) {
+            const bool visited = r.n[k] > 0;
+            const float up = cpuct * r.prior[k] * sqrt_parent;
+            const int tries = r.n[k] + r.inflight[k] + 1;
+            const float mean = Count(visited ? r.n[k] : 1).divides(r.w[k]);
+            const float v = (visited ? mean : 0.0f) + Count(tries).divides(up);
+            plain = plain && (unsigned)((tries - 1) | r.n[k]) < (1u << 22) && Count::plain(r.w[k], up);
+            score[k] = v;
         }
-        if (info < 0 || info > edges) {
-            rollback(path, depth, lane, edge_inflight, tree_edges_base, node_cnt, edges, vl);
-            __syncwarp();
-            result = pack(INVALID, NODE_MASK, 0, R_INVALID_NODE_INFO);
-            break;
+        if (!plain) {   // counts of millions, or values no network gives
+#pragma unroll
+            for (int k = 0; k < EPL; k++) {
+                const float q = r.n[k] > 0 ? r.w[k] / (float)r.n[k] : 0.0f;
+                score[k] = q + cpuct * r.prior[k] * sqrt_parent / (float)(r.n[k] + r.inflight[k] + 1);
+            }
         }
-        if (depth >= path_depth) {
-            result = pack(DEPTH_LIMIT, node, 0, R_OK_DEPTH_LIMIT);
-            result_len = depth + 1;
-            break;
+#pragma unroll
+        for (int k = 0; k < EPL; k++) {
+            score[k] = lane + 32 * k < n_exp && score[k] >= LOWEST ? score[k] : LOWEST_INF;
+            my_best = fmaxf(my_best, score[k]);
         }
-        const int n_exp = info;
-        const long long e0 = tree_edges_base + (long long)node * edges;
-        // ---- the edges of this node are in registers already (requested while the level above was being decided)
+        const float top = max_of_warp(my_best);
+        if (top == LOWEST_INF) return NO_EDGE;
+        // the bits are compared: +0 is above -0
+        if (EPL <= 2) {
+            const unsigned low = __ballot_sync(FULL, __float_as_uint(score[0]) == __float_as_uint(top)), behind = low >> rot;   // rot < 32
+            const unsigned high = EPL == 2 ? __ballot_sync(FULL, __float_as_uint(score[EPL - 1]) == __float_as_uint(top)) : 0u;
+            const int best = behind ? rot + __ffs(behind) - 1 : (high ? 31 + __ffs(high) : __ffs(low) - 1);
+            my_seen = EPL == 2 && best >= 32 ? r.inflight[EPL - 1] : r.inflight[0];
+            my_child = EPL == 2 && best >= 32 ? r.child[EPL - 1] : r.child[0];
+            return best;
+        }
+        int my_tie = NO_EDGE;
+#pragma unroll
+        for (int k = 0; k < EPL; k++) {
+            const int e = lane + 32 * k;
+            const int tie = e >= rot ? e - rot : e - rot + n_exp;
+            if (__float_as_uint(score[k]) == __float_as_uint(top) && tie < my_tie) {
+                my_tie = tie;
+                my_seen = r.inflight[k];
+                my_child = r.child[k];
+            }
+        }
+        const int tie = (int)__reduce_min_sync(FULL, (unsigned)my_tie);
+        return tie + rot >= n_exp ? tie + rot - n_exp : tie + rot;
+    };
+    auto parent_count = [&](int n_exp) {
         int partial = 0;
-        const bool need_stats = n_exp != 1 || c_pw != 0.0f;
 #pragma unroll
         for (int k = 0; k < EPL; k++)
-            if (lane + 32 * k < n_exp) partial += cur.n[k] + cur.inflight[k];
-        int parent_eff = 1, allowed = 1;
-        if (need_stats) {
-            parent_eff = max(__reduce_add_sync(FULL, partial), 1);
-            const float quota = (alpha_pw == 0.5f) ? c_pw * sqrtf((float)parent_eff) : c_pw * powf((float)parent_eff, alpha_pw);
-            allowed = quota >= (float)edges ? edges : max(1, (int)ceilf(quota));
+            if (lane + 32 * k < n_exp) partial += r.n[k] + r.inflight[k];
+        return max(__reduce_add_sync(FULL, partial), 1);
+    };
+    auto quota_of = [&](int parent_eff) {
+        const float quota = (alpha_pw == 0.5f) ? c_pw * root_of_count(parent_eff) : c_pw * powf((float)parent_eff, alpha_pw);
+        return quota >= (float)edges ? edges : max(1, (int)ceilf(quota));
+    };
+    // (no claim made: up_old == up_seen everywhere)
+    auto claim_held = [&]() { return __any_sync(FULL, lane == (up_edge & 31) && up_old == up_seen) != 0; };
+    // claims edge `best` of `node` and goes on to its child, whose data is requested first
+    auto descend = [&](int best, bool only) {
+        const int owner = best & 31;
+        const int child = __shfl_sync(FULL, my_child, owner);
+        outside = (unsigned)child >= (unsigned)node_cnt;
+        up_info = info;
+        const int there = outside ? 0 : child;
+        info = *at(expanded, (unsigned)there * 4u);
+        r.request(there, lane, edges);
+        if (outside) info = OUTSIDE;
+        int *count = inflight_of_tree + (node * edges + best);
+        if (only) {
+            if (lane == 0) atomicAdd(count, vl);
+            up_old = up_seen;
+        } else {
+            // predicated, so that nothing behind it waits for the answer
+            up_seen = my_seen;
+            asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %4, %5;\n\t@p atom.global.cas.b32 %0, [%1], %2, %3;\n\t}"
+                         : "+r"(up_old) : "l"(count), "r"(my_seen), "r"(my_seen + vl), "r"(lane), "r"(owner) : "memory");
         }
-        if (allowed > n_exp) {
+        pending = !only;
+        up_node = node;
+        up_edge = best;
+        if (lane == 0) path[depth] = (node << 8) | best;
+        node = child;
+        depth++;
+    };
+
+    const unsigned several = edges - 1;   // info - 2 below it: two edges or more, and no more than there are
+    // A claim's answer takes longer than the next level's data out of L2: a traversal that is alone in its tree looks at it
+    // only when it is about to make the next claim.  Where others compete for the tree a lost claim is noticed before the level
+    // below is worked out for nothing.
+    const bool alone = warps == 1;
+    int result, result_len = 0;
+    for (;;) {
+        // ---- the usual level: two or more edges, no room for another, a score, and the claim of the level above held
+        if (attempt == 0) while ((unsigned)(info - 2) < several && depth < path_depth) {
+            if (!alone && !claim_held()) break;
+            const int parent_eff = parent_count(info);
+            sqrt_parent = root_of_count(parent_eff);
+            if (WIDENING && quota_of(parent_eff) > info) break;
+            const int best = arg_max(info);
+            if (best == NO_EDGE || (alone && !claim_held())) break;
+            up_attempt = 0;
+            up_sqrt = sqrt_parent;
+            descend(best, false);
+        }
+        // ---- anything else.  The claim of the level above has to hold first
+        if (pending) {
+            pending = false;
+            bool held = claim_held();
+            if (!held && up_attempt + 1 >= MAX_EVALUATIONS && soft_winner != 0) {
+                if (lane == 0) atomicAdd(inflight_of_tree + (up_node * edges + up_edge), vl);
+                held = true;
+            }
+            if (!held) {
+                // somebody else moved the winner's count
+                depth--;
+                node = up_node;
+                if (up_attempt + 1 >= MAX_EVALUATIONS) {
+                    rollback(path, depth, lane, edge_inflight, tree_edges_base, node_cnt, edges, vl);
+                    result = pack(BUSY, node, 0, R_BUSY_WINNER_RECALC);
+                    break;
+                }
+                info = up_info;
+                attempt = up_attempt + 1;
+                sqrt_parent = up_sqrt;
+                outside = false;
+                r.request(node, lane, edges);
+                continue;
+            }
+        }
+        const int n_exp = info;
+        const bool at_end = outside || info < 0 || info > edges || depth >= path_depth;
+        int allowed = 1, best = NO_EDGE;
+        if (!at_end && (n_exp != 1 || WIDENING)) {
+            const int parent_eff = parent_count(n_exp);
+            if (attempt == 0) sqrt_parent = root_of_count(parent_eff);   // another evaluation keeps the parent's count
+            if (WIDENING) allowed = quota_of(parent_eff);
+            if (n_exp > 1) best = arg_max(n_exp);
+        }
+        if (at_end) {
+            if (outside) {
+                rollback(path, depth, lane, edge_inflight, tree_edges_base, node_cnt, edges, vl);
+                result = pack(INVALID, NODE_MASK, 0, R_INVALID_CHILD_OOB);
+            } else if (info == NODE_TERMINAL) {
+                result = pack(TERMINAL, node, 0, R_OK_TERMINAL);
+                result_len = depth + 1;
+            } else if (info < 0 || info > edges) {
+                rollback(path, depth, lane, edge_inflight, tree_edges_base, node_cnt, edges, vl);
+                result = pack(INVALID, NODE_MASK, 0, R_INVALID_NODE_INFO);
+            } else {
+                result = pack(DEPTH_LIMIT, node, 0, R_OK_DEPTH_LIMIT);
+                result_len = depth + 1;
+            }
+            break;
+        }
+        if (allowed > n_exp && attempt == 0) {
             // room for a new child: take a ticket unless the tickets in flight already fill the quota
             int slot = -1;
             if (lane == 0) {
@@ -182,107 +328,28 @@ __global__ void select_kernel(float cpuct, float c_pw, float alpha_pw, int soft_
             }
             if (n_exp == 0) {
                 rollback(path, depth, lane, edge_inflight, tree_edges_base, node_cnt, edges, vl);
-                __syncwarp();
                 result = pack(BUSY, node, 0, R_BUSY_EXPAND_INFLIGHT);
-                result_len = 0;
                 break;
             }
         }
-        // ---- pick an existing child
-        // The child of every edge is in a register already, so as soon as the winner is known its node record can be
-        // requested together with the claim instead of after it: one memory round trip per level less.
-        int best = 0, held = 0, child = -1, next_info = 0;
-        if (n_exp == 1) {
-            child = __shfl_sync(FULL, cur.child[0], 0);
-            if (child >= 0 && child < node_cnt) {
-                next_info = node_expanded[tree_nodes_base + child];
-                load_edges<EPL>(nxt, tree_edges_base + (long long)child * edges, lane, edges, edge_child_id, edge_prior, edge_W,
-                                edge_N, edge_inflight);
-            }
-            if (lane == 0) atomicAdd(&edge_inflight[e0], vl);
-            held = 1;
-        } else {
-            const int rot = wid >= n_exp ? wid % n_exp : wid;  // ties go to the edge closest after `rot`
-            const float sqrt_parent = sqrtf((float)parent_eff);
-            for (int attempt = 0;; attempt++) {
-                unsigned my_key = 0;
-                int my_tie = NO_EDGE, my_seen = 0, my_child = -1;
-#pragma unroll
-                for (int k = 0; k < EPL; k++) {
-                    const int e = lane + 32 * k;
-                    if (e < n_exp) {
-                        const float q = cur.n[k] > 0 ? cur.w[k] / (float)cur.n[k] : 0.0f;
-                        const float u = cpuct * cur.prior[k] * sqrt_parent / (float)(cur.n[k] + cur.inflight[k] + 1);
-                        const float score = q + u;
-                        if (score >= LOWEST) {  // not NaN, not -inf
-                            const unsigned key = ordered(score);
-                            int tie = e - rot;
-                            if (tie < 0) tie += n_exp;
-                            if (key > my_key || (key == my_key && tie < my_tie)) {
-                                my_key = key;
-                                my_tie = tie;
-                                my_seen = cur.inflight[k];
-                                my_child = cur.child[k];
-                            }
-                        }
-                    }
-                }
-                const unsigned top = __reduce_max_sync(FULL, my_key);
-                const int tie = (int)__reduce_min_sync(FULL, (my_key == top && my_tie != NO_EDGE) ? (unsigned)my_tie : 0xFFFFFFFFu);
-                if (top == 0u || tie < 0) {
-                    best = NO_EDGE;
-                    break;
-                }
-                best = tie + rot;
-                if (best >= n_exp) best -= n_exp;
-                const int owner = __ffs(__ballot_sync(FULL, my_key == top && my_tie == tie)) - 1;
-                const int seen = __shfl_sync(FULL, my_seen, owner);
-                child = __shfl_sync(FULL, my_child, owner);
-                if (child >= 0 && child < node_cnt) {  // the next level's data travels together with the claim
-                    next_info = node_expanded[tree_nodes_base + child];
-                    load_edges<EPL>(nxt, tree_edges_base + (long long)child * edges, lane, edges, edge_child_id, edge_prior,
-                                    edge_W, edge_N, edge_inflight);
-                }
-                if (lane == 0) held = atomicCAS(&edge_inflight[e0 + best], seen, seen + vl) == seen ? 1 : 0;
-                held = __shfl_sync(FULL, held, 0);
-                if (held || attempt + 1 >= MAX_EVALUATIONS) break;
-                // somebody else moved the winner's count: look at the counts again
-#pragma unroll
-                for (int k = 0; k < EPL; k++) {
-                    const int e = lane + 32 * k;
-                    if (e < n_exp) cur.inflight[k] = *(volatile int *)&edge_inflight[e0 + e];
-                }
-            }
-            if (soft_winner != 0 && !held && best != NO_EDGE) {
-                if (lane == 0) atomicAdd(&edge_inflight[e0 + best], vl);
-                held = 1;
-            }
-        }
-        if (!held) {
-            __syncwarp();
+        // ---- go on to an existing child
+        const bool only = n_exp == 1;
+        if (only) {
+            best = 0;
+            my_child = r.child[0];
+        } else if (best == NO_EDGE) {
             rollback(path, depth, lane, edge_inflight, tree_edges_base, node_cnt, edges, vl);
-            __syncwarp();
-            result = best == NO_EDGE ? pack(INVALID, NODE_MASK, 0, R_INVALID_NO_VALID_EDGE) : pack(BUSY, node, 0, R_BUSY_WINNER_RECALC);
+            result = pack(INVALID, NODE_MASK, 0, R_INVALID_NO_VALID_EDGE);
             break;
         }
-        if (child < 0 || child >= node_cnt) {
-            if (lane == 0) atomicSub(&edge_inflight[e0 + best], vl);
-            __syncwarp();
-            rollback(path, depth, lane, edge_inflight, tree_edges_base, node_cnt, edges, vl);
-            __syncwarp();
-            result = pack(INVALID, NODE_MASK, 0, R_INVALID_CHILD_OOB);
-            break;
-        }
-        if (lane == 0) path[depth] = (node << 8) | best;
-        __syncwarp();
-        node = child;
-        info = next_info;
-        cur = nxt;
-        depth++;
+        up_attempt = attempt;
+        up_sqrt = sqrt_parent;
+        descend(best, only);
+        attempt = 0;
     }
     if (lane == 0) {
-        out_selected_node[out_ix] = result;
-        out_path_len[out_ix] = result_len;
+        out_selected_node[traversal] = result;
+        out_path_len[traversal] = result_len;
     }
 }
 
@@ -293,25 +360,25 @@ __global__ void select_kernel(float cpuct, float c_pw, float alpha_pw, int soft_
 __global__ void backup_kernel(int virtual_loss, float *edge_W, int *edge_N, int *edge_inflight, int *node_expand_inflight,
                               const int *__restrict__ tree_nodes, const int *__restrict__ out_selected_node,
                               const int *__restrict__ out_path_eids, const int *__restrict__ out_path_len,
-                              const float *__restrict__ path_edge_values, int trees, int nodes, int edges, int warps,
-                              int path_depth) {
-    const int tree = blockIdx.x;
-    const int lane = threadIdx.x & 31;
-    const int wid = threadIdx.x >> 5;
-    if (tree >= trees || wid >= min((int)(blockDim.x >> 5), warps)) return;
+                              const float *__restrict__ path_edge_values, int traversals, int nodes, int edges, int warps,
+                              int path_depth, int log2_lanes) {
+    const BackupLane at_work(traversals, log2_lanes);
+    const int out_ix = at_work.traversal;
+    if (out_ix < 0) return;
+    const int tree = out_ix / warps;
+    const int raw = out_selected_node[out_ix];
+    const int plen = out_path_len[out_ix];
     const int node_cnt = tree_nodes[tree];
     if (node_cnt <= 0 || node_cnt > nodes || node_cnt > NODE_LIMIT) return;
-    const int out_ix = tree * warps + wid;
-    const int raw = out_selected_node[out_ix];
     if (raw < 0) return;
     const int kind = (raw >> KIND_SHIFT) & 7;
     if (kind == INVALID || kind == BUSY) return;
-    const int plen = out_path_len[out_ix];
     if (plen <= 0) return;
     const long long tree_edges_base = (long long)tree * nodes * edges;
     const int *path = out_path_eids + (long long)out_ix * path_depth;
-    for (int d = lane; d < plen - 1; d += 32) {
+    for (int d = at_work.lane; d < plen - 1; d += 1 << log2_lanes) {
         const int enc = path[d];
+        const float value = path_edge_values ? path_edge_values[(long long)out_ix * path_depth + d] : 0.f;
         if (enc < 0) continue;
         const int parent = enc >> 8, slot = enc & 0xFF;
         if (parent < node_cnt && slot < edges) {
@@ -319,34 +386,38 @@ __global__ void backup_kernel(int virtual_loss, float *edge_W, int *edge_N, int 
             atomicSub(&edge_inflight[ix], virtual_loss);
             if (path_edge_values) {
                 atomicAdd(&edge_N[ix], 1);
-                atomicAdd(&edge_W[ix], path_edge_values[(long long)out_ix * path_depth + d]);
+                atomicAdd(&edge_W[ix], value);
             }
         }
     }
-    if (lane == 0 && kind == EXPAND) {
+    if (at_work.lane == 0 && kind == EXPAND) {
         const int leaf = raw & NODE_MASK;
         if (leaf < node_cnt) atomicSub(&node_expand_inflight[(long long)tree * nodes + leaf], 1);
     }
 }
 
-template <int VL>
 static int launch_select(float cpuct, float c_pw, float alpha_pw, int soft_winner, int virtual_loss, const int *edge_child_id,
                          const float *edge_prior, const float *edge_W, const int *edge_N, int *edge_inflight,
                          int *node_expand_inflight, const int *node_expanded, const int *tree_nodes, int *out_selected_node,
                          int *out_path_eids, int *out_path_len, int trees, int nodes, int edges, int warps, int path_depth,
                          cudaStream_t stream) {
-    const long long traversals = (long long)trees * warps;
-    const unsigned grid = (unsigned)((traversals + SELECT_WARPS_PER_BLOCK - 1) / SELECT_WARPS_PER_BLOCK);
-#define PUCT_LAUNCH(E)                                                                                                      \
-    select_kernel<VL, E><<<grid, SELECT_WARPS_PER_BLOCK * 32, 0, stream>>>(                                                 \
-        cpuct, c_pw, alpha_pw, soft_winner, edge_child_id, edge_prior, edge_W, edge_N, edge_inflight, node_expand_inflight, \
-        node_expanded, tree_nodes, out_selected_node, out_path_eids, out_path_len, trees, nodes, edges, warps, path_depth,  \
-        virtual_loss)
+    const unsigned grid = (unsigned)((long long)trees * warps);
+#define PUCT_LAUNCH_AS(E, W)                                                                                              \
+    select_kernel<E, W><<<grid, 32, 0, stream>>>(cpuct, c_pw, alpha_pw, soft_winner, edge_child_id, edge_prior, edge_W,     \
+                                                 edge_N, edge_inflight, node_expand_inflight, node_expanded, tree_nodes,    \
+                                                 out_selected_node, out_path_eids, out_path_len, nodes, edges, warps,       \
+                                                 path_depth, virtual_loss)
+#define PUCT_LAUNCH(E)                        \
+    do {                                      \
+        if (c_pw != 0.0f) PUCT_LAUNCH_AS(E, true); \
+        else PUCT_LAUNCH_AS(E, false);        \
+    } while (0)
     if (edges <= 32) PUCT_LAUNCH(1);
     else if (edges <= 64) PUCT_LAUNCH(2);
     else if (edges <= 128) PUCT_LAUNCH(4);
     else PUCT_LAUNCH(8);   // more than 256 edges: the kernel itself reports the invalid shape
 #undef PUCT_LAUNCH
+#undef PUCT_LAUNCH_AS
     return (int)cudaGetLastError();
 }
 
@@ -360,7 +431,7 @@ extern "C" int puct_select_winner_recalc_launch(float cpuct, float c_pw, float a
                                                 int *out_path_len, int trees, int nodes, int edges, int warps, int path_depth,
                                                 void *stream) {
     if (trees <= 0 || warps <= 0 || warps > 32) return (int)cudaErrorInvalidValue;
-    return puct::launch_select<0>(cpuct, c_pw, alpha_pw, soft_winner, 1, edge_child_id, edge_prior, edge_W, edge_N, edge_inflight,
+    return puct::launch_select(cpuct, c_pw, alpha_pw, soft_winner, 1, edge_child_id, edge_prior, edge_W, edge_N, edge_inflight,
                                   node_expand_inflight, node_expanded, tree_nodes, out_selected_node, out_path_eids,
                                   out_path_len, trees, nodes, edges, warps, path_depth, (cudaStream_t)stream);
 }
@@ -373,7 +444,7 @@ extern "C" int puct_select_virtual_loss_launch(float cpuct, float c_pw, float al
                                                int *out_path_eids, int *out_path_len, int trees, int nodes, int edges, int warps,
                                                int path_depth, void *stream) {
     if (trees <= 0 || warps <= 0 || warps > 32 || virtual_loss < 1) return (int)cudaErrorInvalidValue;
-    return puct::launch_select<1>(cpuct, c_pw, alpha_pw, soft_winner, virtual_loss, edge_child_id, edge_prior, edge_W, edge_N,
+    return puct::launch_select(cpuct, c_pw, alpha_pw, soft_winner, virtual_loss, edge_child_id, edge_prior, edge_W, edge_N,
                                   edge_inflight, node_expand_inflight, node_expanded, tree_nodes, out_selected_node,
                                   out_path_eids, out_path_len, trees, nodes, edges, warps, path_depth, (cudaStream_t)stream);
 }
@@ -385,10 +456,12 @@ extern "C" int puct_backup_launch(int virtual_loss, float *edge_W, int *edge_N, 
                                   const int *out_path_len, const float *path_edge_values, int trees, int nodes, int edges,
                                   int warps, int path_depth, void *stream) {
     if (trees <= 0 || warps <= 0 || warps > 32) return (int)cudaErrorInvalidValue;
-    puct::backup_kernel<<<trees, warps * 32, 0, (cudaStream_t)stream>>>(virtual_loss, edge_W, edge_N, edge_inflight,
-                                                                       node_expand_inflight, tree_nodes, out_selected_node,
-                                                                       out_path_eids, out_path_len, path_edge_values, trees,
-                                                                       nodes, edges, warps, path_depth);
+    if ((long long)trees * warps > 0x7FFFFFFF) return (int)cudaErrorInvalidValue;
+    const select_math::BackupGrid g(trees * warps, path_depth);
+    puct::backup_kernel<<<g.blocks, g.THREADS, 0, (cudaStream_t)stream>>>(virtual_loss, edge_W, edge_N, edge_inflight, node_expand_inflight,
+                                                                          tree_nodes, out_selected_node, out_path_eids, out_path_len,
+                                                                          path_edge_values, trees * warps, nodes, edges, warps,
+                                                                          path_depth, g.log2_lanes);
     return (int)cudaGetLastError();
 }
 

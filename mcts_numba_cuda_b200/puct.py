@@ -10,84 +10,63 @@ import ctypes
 
 from . import _abi
 
-_configured = False
+_wave = None
 
 
-def _lib():
-    global _configured
-    L = _abi.lib()
-    if not _configured:
-        vp, i32, f32 = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
-        L.puct_select_winner_recalc_launch.argtypes = [f32, f32, f32, i32] + [vp] * 11 + [i32] * 5 + [vp]
-        L.puct_select_winner_recalc_launch.restype = i32
-        L.puct_select_virtual_loss_launch.argtypes = [f32, f32, f32, i32, i32] + [vp] * 11 + [i32] * 5 + [vp]
-        L.puct_select_virtual_loss_launch.restype = i32
-        L.puct_backup_launch.argtypes = [i32] + [vp] * 9 + [i32] * 5 + [vp]
-        L.puct_backup_launch.restype = i32
-        L.puct_v2_select_launch.argtypes = [i32, f32, f32, f32] + [vp] * 11 + [i32] * 5 + [vp]
-        L.puct_v2_select_launch.restype = i32
-        L.puct_v2_backup_launch.argtypes = [i32] + [vp] * 10 + [i32] * 5 + [vp]
-        L.puct_v2_backup_launch.restype = i32
-        L.puct_cpp_cuda_error_string.argtypes = [i32]
-        L.puct_cpp_cuda_error_string.restype = ctypes.c_char_p
-        _configured = True
-    return L
+def _launcher():
+    """The extension that gathers a launch's arguments, bound to the library's launchers on first use."""
+    global _wave
+    if _wave is None:
+        try:
+            from . import _wave as module
+        except ImportError as e:
+            raise RuntimeError("mcts_numba_cuda_b200/_wave.so is missing: build it with `python -m mcts_numba_cuda_b200.build`") from e
+        L = _abi.lib()
+        module.bind(*(ctypes.cast(getattr(L, name), ctypes.c_void_p).value for name in (
+            "puct_select_winner_recalc_launch", "puct_select_virtual_loss_launch", "puct_backup_launch", "puct_v2_select_launch",
+            "puct_v2_backup_launch", "duct_select_launch", "duct_backup_launch")))
+        _wave = module
+    return _wave
 
 
-def _ptr(a):
-    if a is None:
-        return None
-    if hasattr(a, "data_ptr"):
-        return ctypes.c_void_p(a.data_ptr())
-    if hasattr(a, "__cuda_array_interface__"):
-        return ctypes.c_void_p(a.__cuda_array_interface__["data"][0])
-    raise TypeError(f"not a device array: {type(a)}")
+_raw_stream = _device_index = None
+
+
+def _current_stream():
+    """Handle of torch's current stream; 0 (the default stream) where torch or a device is missing."""
+    global _raw_stream, _device_index
+    try:
+        if _raw_stream is not None:   # without building a Stream object (0.1 instead of 1.2 us)
+            return _raw_stream(_device_index())
+        import torch
+        handle = torch.cuda.current_stream().cuda_stream
+        _device_index = getattr(torch._C, "_cuda_getDevice", None)
+        _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) if _device_index else None
+        return handle
+    except Exception:
+        return 0
 
 
 def _stream(stream):
-    if stream is not None:
-        return ctypes.c_void_p(stream)
-    try:
-        import torch
-        return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-    except Exception:
-        return ctypes.c_void_p(0)
+    return _current_stream() if stream is None else stream
 
 
-def _check(code, what):
+def _check(code, what, name="PUCT"):
     if code != 0:
-        msg = _lib().puct_cpp_cuda_error_string(code).decode("utf-8", "replace")
-        raise RuntimeError(f"PUCT {what} launch failed: {msg} ({code})")
-
-
-def _shape(d):
-    ec = d["edge_child"]
-    return int(d["trees"]), int(ec.shape[1]), int(ec.shape[2]), int(d["warps"]), int(d["out_path"].shape[2])
+        text = _abi.lib().puct_cpp_cuda_error_string
+        text.argtypes, text.restype = [ctypes.c_int], ctypes.c_char_p
+        raise RuntimeError(f"{name} {what} launch failed: {text(code).decode('utf-8', 'replace')} ({code})")
 
 
 def launch_select(d, cpuct=1.0, c_pw=1.0, alpha_pw=0.5, soft_winner=0, virtual_loss=1, stream=None):
     """One traversal per (tree, warp); results in ``d["out_selected"], d["out_path"], d["out_len"]``."""
-    trees, nodes, edges, warps, path_depth = _shape(d)
-    args = [_ptr(d[k]) for k in ("edge_child", "edge_prior", "edge_w", "edge_n", "edge_inflight", "node_expand_inflight",
-                                 "node_expanded", "node_count", "out_selected", "out_path", "out_len")]
-    if virtual_loss == 1:
-        code = _lib().puct_select_winner_recalc_launch(cpuct, c_pw, alpha_pw, int(soft_winner), *args, trees, nodes, edges,
-                                                       warps, path_depth, _stream(stream))
-    else:
-        code = _lib().puct_select_virtual_loss_launch(cpuct, c_pw, alpha_pw, int(soft_winner), int(virtual_loss), *args,
-                                                      trees, nodes, edges, warps, path_depth, _stream(stream))
-    _check(code, "select")
+    _check((_wave or _launcher()).puct_select(d, cpuct, c_pw, alpha_pw, int(soft_winner), int(virtual_loss), _stream(stream)), "select")
 
 
 def launch_backup(d, values=None, virtual_loss=1, stream=None):
     """Turns the claims of the last select into statistics (``values``: float32[trees, warps, path_depth] on the device),
     or only releases them (``values=None``)."""
-    trees, nodes, edges, warps, path_depth = _shape(d)
-    code = _lib().puct_backup_launch(int(virtual_loss), _ptr(d["edge_w"]), _ptr(d["edge_n"]), _ptr(d["edge_inflight"]),
-                                     _ptr(d["node_expand_inflight"]), _ptr(d["node_count"]), _ptr(d["out_selected"]),
-                                     _ptr(d["out_path"]), _ptr(d["out_len"]), _ptr(values), trees, nodes, edges, warps,
-                                     path_depth, _stream(stream))
-    _check(code, "backup")
+    _check((_wave or _launcher()).puct_backup(d, values, int(virtual_loss), _stream(stream)), "backup")
 
 
 def launch_release(d, virtual_loss=1, stream=None):
@@ -102,20 +81,12 @@ def launch_select_v2(d, cpuct=1.0, c_pw=1.0, alpha_pw=0.5, variant=V2_PRECLAIM, 
     visits per child node: ``d`` holds ``node_inflight`` (int32[trees, nodes]) in place of ``edge_inflight``.
     ``variant``: preclaim (every candidate is visited before it is scored, losers leave) or counter-CAS (the winner alone
     is claimed by compare-and-swap; a claim that met other visits is given back once)."""
-    trees, nodes, edges, warps, path_depth = _shape(d)
-    args = [_ptr(d[k]) for k in ("edge_child", "edge_prior", "edge_w", "edge_n", "node_inflight", "node_expand_inflight",
-                                 "node_expanded", "node_count", "out_selected", "out_path", "out_len")]
-    _check(_lib().puct_v2_select_launch(int(variant), cpuct, c_pw, alpha_pw, *args, trees, nodes, edges, warps, path_depth,
-                                        _stream(stream)), "v2 select")
+    _check((_wave or _launcher()).puct_v2_select(d, int(variant), cpuct, c_pw, alpha_pw, _stream(stream)), "v2 select")
 
 
 def launch_backup_v2(d, values=None, virtual_loss=1, stream=None):
     """``_backup_kernel_native`` of ``src/puct/puct_gpu_v2.py:847-927`` (``values=None``: release only)."""
-    trees, nodes, edges, warps, path_depth = _shape(d)
-    _check(_lib().puct_v2_backup_launch(int(virtual_loss), _ptr(d["edge_child"]), _ptr(d["edge_w"]), _ptr(d["edge_n"]),
-                                        _ptr(d["node_inflight"]), _ptr(d["node_expand_inflight"]), _ptr(d["node_count"]),
-                                        _ptr(d["out_selected"]), _ptr(d["out_path"]), _ptr(d["out_len"]), _ptr(values), trees,
-                                        nodes, edges, warps, path_depth, _stream(stream)), "v2 backup")
+    _check((_wave or _launcher()).puct_v2_backup(d, values, int(virtual_loss), _stream(stream)), "v2 backup")
 
 
 def to_device(case, device="cuda"):
