@@ -251,6 +251,8 @@ struct Shared {
     int pick;                // OCP: index (among expanded children) of the child that is played out
     int root_turn;
     int size;
+    int max_depth;           // of the nodes, and the sum of their depths
+    long long depth_sum;
     int out_neg, out_pos;
     unsigned status;
     unsigned long long plies;
@@ -418,6 +420,8 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
             board[0] = p.root_board[b];
             parent[0] = -1;
             s.size = 1;
+            s.max_depth = 0;
+            s.depth_sum = 0;
             s.root_turn = turn;
             s.status = 0;
             s.plies = 0;
@@ -426,6 +430,8 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
             s.path_len = 1;
         } else {
             s.size = st->size;
+            s.max_depth = st->max_depth;
+            s.depth_sum = st->depth_sum;
             s.root_turn = meta_turn(rec[0].w);
             s.status = st->status;
             s.plies = st->plies;
@@ -703,7 +709,11 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
             }
             __syncwarp();
             if (lane == 0) {
-                if (mode == MODE_ALL_CHILDREN) s.size += n_exp;
+                if (mode == MODE_ALL_CHILDREN) {
+                    s.size += n_exp;
+                    s.depth_sum += n_exp * (depth + 1);
+                    s.max_depth = max(s.max_depth, depth + 1);
+                }
                 s.ae[A + 1] = (short)(mode == MODE_ALL_CHILDREN ? n_exp : 1);
                 int m2 = mode;
                 if (OCP && mode == MODE_ALL_CHILDREN) m2 = thrifty ? pick : nth_set(exp_mask, pick);
@@ -916,6 +926,8 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
     if (rank != 0) return;
     if (tid == 0) {
         st->size = s.size;
+        st->max_depth = s.max_depth;
+        st->depth_sum = s.depth_sum;
         st->selected = s.selected;
         st->path_len = s.path_len;
         st->out_neg = s.out_neg;

@@ -69,7 +69,8 @@ struct TreeState {
     // SM clock (cycle counter of the SM the block ran on): select, expand, playouts, backup.  The reference times the same
     // stages with host clocks around its launches (src/mctsnc.py:606-686).
     float stage_ms[4];
-    int reserved;
+    int max_depth;       // deepest node, and
+    long long depth_sum; // the sum of the depths of all nodes
 };
 
 // Work queue of a batched launch.  A tree's search is cut into slices of `chunk` steps; the blocks of a persistent grid

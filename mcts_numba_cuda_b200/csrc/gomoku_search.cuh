@@ -185,6 +185,8 @@ __global__ void __launch_bounds__(256) tree_step_kernel(const Params p) {
             rec[0] = make_int4(0, 0, -1, g_make_meta(0, false, 2, turn, 0));
             parent[0] = -1;
             st->size = 1;
+            st->depth_sum = 0;
+            st->max_depth = 0;
             st->selected = 0;
             st->path_len = 1;
             st->status = 0;
@@ -499,7 +501,11 @@ __global__ void __launch_bounds__(256) tree_step_kernel(const Params p) {
     if (mode == MODE_TERMINAL && tid < A && !thrifty) ae[tid] = -1;
     __syncthreads();
     if (tid == 0) {
-        if (mode == MODE_ALL_CHILDREN) st->size += n_exp;
+        if (mode == MODE_ALL_CHILDREN) {
+            st->size += n_exp;
+            st->depth_sum += (long long)n_exp * (meta_depth(r.w) + 1);
+            st->max_depth = max(st->max_depth, meta_depth(r.w) + 1);
+        }
         ae[A + 1] = (short)(mode == MODE_ALL_CHILDREN ? n_exp : 1);
         int m2 = mode;
         const int pick = (OCP && mode == MODE_ALL_CHILDREN) ? s_pick : 0;

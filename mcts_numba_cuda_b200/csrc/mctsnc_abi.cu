@@ -93,7 +93,7 @@ struct mctsnc_handle {
     ulonglong2 *rng_expand_base = nullptr;
     JumpColumn *jump_cols = nullptr;      // [JUMP_LEVELS][128] matrices of the 2^64-step jump, for seeding streams on the device
     ulonglong2 *root_board = nullptr;
-    signed char *root_turn = nullptr;
+    signed char *root_turn = nullptr;     // behind the boards of the staged roots
     WorkQueues *queue = nullptr;          // Connect 4: work queue of batched launches
     QueueCell *ring = nullptr;            // [QUEUE_LEVELS][n_trees_total]
     int *remaining = nullptr;             // [n_trees_total]
@@ -110,15 +110,16 @@ struct mctsnc_handle {
     unsigned char *active_rank = nullptr;
     unsigned *root_gboard = nullptr;      // [max_batch][16]
     unsigned *h_root_gboard = nullptr;
-    long long *sums = nullptr;            // [max_batch][3A]
-    unsigned char *flags = nullptr;       // [max_batch][2A]: win flags, expanded-at-root
-    DevResult *dres = nullptr;            // [max_batch]
+    // [max_batch] results, [max_batch][3A] sums, [max_batch][2A] flags (win flags, expanded-at-root) in one piece of memory
+    DevResult *dres = nullptr;
+    long long *sums = nullptr;
+    unsigned char *flags = nullptr;
     // pinned host staging
     ulonglong2 *h_root_board = nullptr;
-    signed char *h_root_turn = nullptr;
+    DevResult *h_dres = nullptr;          // the same three in one pinned piece
     long long *h_sums = nullptr;
     unsigned char *h_flags = nullptr;
-    DevResult *h_dres = nullptr;
+    size_t result_bytes = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaEvent_t ev_staged = nullptr;  // recorded behind the host-to-device copies of the staged roots
     bool staging_in_flight = false;
@@ -176,6 +177,59 @@ __global__ void replicate_streams_kernel(ulonglong2 *dst, const ulonglong2 *base
         dst[i] = base[i % per_search];
 }
 
+// The part of the two reductions over trees that both games share.  Every load of a search's trees is independent of the others
+// (roots first, then their children; a tree's counters by a lane of the last warp): read one tree after the other they were a
+// chain of 16 to 32 memory latencies (86 us for 4 trees of 14000 nodes with the node scan for the depths, which the search
+// now keeps itself; 390 us for Gomoku).
+constexpr int REDUCE_THREADS = 256;
+__device__ __forceinline__ void load_roots(int4 *s_root, const int4 *r0, long long cap, int n_trees) {
+    for (int t = threadIdx.x; t < n_trees; t += REDUCE_THREADS) s_root[t] = r0[(long long)t * cap];
+    __syncthreads();
+}
+__device__ __forceinline__ long long warp_sum(long long v) {
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xFFFFFFFFu, v, o);
+    return v;
+}
+__device__ __forceinline__ void gather_statistics(const TreeState *state, const int4 *s_root, int n_trees, int n_root_actions, DevResult *out) {
+    if (threadIdx.x < REDUCE_THREADS - 32) return;
+    const int lane = threadIdx.x & 31;
+    long long playouts = 0, plies = 0, ub = 0, nodes = 0, depths = 0;
+    int max_size = 0, max_depth = 0;
+    unsigned status = 0;
+    float stage[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int t = lane; t < n_trees; t += 32) {
+        const TreeState ts = state[t];
+        playouts += s_root[t].x;
+        plies += (long long)ts.plies;
+        ub += (long long)ts.ub_draws;
+        nodes += ts.size;
+        depths += ts.depth_sum;
+        status |= ts.status;
+        max_size = max(max_size, ts.size);
+        max_depth = max(max_depth, ts.max_depth);
+        for (int k = 0; k < 4; k++) stage[k] += ts.stage_ms[k];
+    }
+    DevResult d;
+    d.playouts = warp_sum(playouts);
+    d.plies = warp_sum(plies);
+    d.ub_draws = warp_sum(ub);
+    d.total_nodes = warp_sum(nodes);
+    d.depth_sum = warp_sum(depths);
+    d.status = __reduce_or_sync(0xFFFFFFFFu, status);
+    d.max_size = __reduce_max_sync(0xFFFFFFFFu, max_size);
+    d.max_depth = __reduce_max_sync(0xFFFFFFFFu, max_depth);
+    for (int k = 0; k < 4; k++) {
+        for (int o = 16; o > 0; o >>= 1) stage[k] += __shfl_down_sync(0xFFFFFFFFu, stage[k], o);
+        d.stage_ms[k] = stage[k] / (float)n_trees;
+    }
+    d.best_action = -1;
+    d.best_win_flag = 0;
+    d.best_n = 0;
+    d.best_n_wins = 0;
+    d.n_root_actions = n_root_actions;
+    if (lane == 0) *out = d;
+}
+
 // _reduce_over_trees_* (src/mctsnc.py:2223-2296): per root action the sums over the trees of a search of the root
 // visit count, the child's visit count and the child's win count; win flag from tree 0.  One block per search.
 // Also gathers the statistics behind performance_info (:448-494).
@@ -184,18 +238,21 @@ __global__ void reduce_over_trees_kernel(const int4 *rec, const TreeState *state
     const int b = blockIdx.x;
     const int tid = threadIdx.x;
     const int4 *r0 = rec + (long long)b * n_trees * cap;
-    const int root_meta0 = r0[0].w;
+    __shared__ int4 s_root[512];
+    load_roots(s_root, r0, cap, n_trees);
+    const int root_meta0 = s_root[0].w;
     const int root_turn = meta_turn(root_meta0);
     const unsigned mask0 = root_meta0 & 0x7F;
     for (int a = tid; a < A; a += blockDim.x) {
-        long long s_root = 0, s_n = 0, s_w = 0;
+        long long n_root = 0, s_n = 0, s_w = 0;
         unsigned char win = 0;
         const bool expanded = (mask0 >> a) & 1u;
         if (expanded) {
+#pragma unroll 4
             for (int t = 0; t < n_trees; t++) {
                 const int4 *rt = r0 + (long long)t * cap;
-                const int4 root = rt[0];
-                s_root += root.x;
+                const int4 root = s_root[t];
+                n_root += root.x;
                 const unsigned mk = root.w & 0x7F;
                 if ((mk >> a) & 1u) {
                     const int4 c = rt[root.z + __popc(mk & ((1u << a) - 1u))];
@@ -205,67 +262,13 @@ __global__ void reduce_over_trees_kernel(const int4 *rec, const TreeState *state
                 }
             }
         }
-        sums[(long long)b * 3 * A + a] = s_root;
+        sums[(long long)b * 3 * A + a] = n_root;
         sums[(long long)b * 3 * A + A + a] = s_n;
         sums[(long long)b * 3 * A + 2 * A + a] = s_w;
         flags[(long long)b * 2 * A + a] = win;
         flags[(long long)b * 2 * A + A + a] = expanded;
     }
-    // statistics
-    __shared__ long long sh_depth[256];
-    __shared__ int sh_maxd[256];
-    long long dsum = 0;
-    int dmax = 0;
-    for (int t = 0; t < n_trees; t++) {
-        const int size = state[b * n_trees + t].size;
-        const int4 *rt = r0 + (long long)t * cap;
-        for (int i = tid; i < size; i += blockDim.x) {
-            const int d = meta_depth(rt[i].w);
-            dsum += d;
-            dmax = d > dmax ? d : dmax;
-        }
-    }
-    sh_depth[tid] = dsum;
-    sh_maxd[tid] = dmax;
-    __syncthreads();
-    for (int s = blockDim.x >> 1; s > 0; s >>= 1) {
-        if (tid < s) {
-            sh_depth[tid] += sh_depth[tid + s];
-            sh_maxd[tid] = max(sh_maxd[tid], sh_maxd[tid + s]);
-        }
-        __syncthreads();
-    }
-    if (tid == 0) {
-        DevResult d;
-        d.best_action = -1;
-        d.best_win_flag = 0;
-        d.best_n = 0;
-        d.best_n_wins = 0;
-        d.playouts = 0;
-        d.plies = 0;
-        d.ub_draws = 0;
-        d.status = 0;
-        d.max_size = 0;
-        d.total_nodes = 0;
-        for (int t = 0; t < n_trees; t++) {
-            const TreeState &ts = state[b * n_trees + t];
-            d.playouts += r0[(long long)t * cap].x;
-            d.plies += (long long)ts.plies;
-            d.ub_draws += (long long)ts.ub_draws;
-            d.status |= ts.status;
-            d.total_nodes += ts.size;
-            d.max_size = ts.size > d.max_size ? ts.size : d.max_size;
-        }
-        d.n_root_actions = __popc(mask0);
-        d.max_depth = sh_maxd[0];
-        d.depth_sum = sh_depth[0];
-        for (int k = 0; k < 4; k++) {
-            float acc = 0.f;
-            for (int t = 0; t < n_trees; t++) acc += state[b * n_trees + t].stage_ms[k];
-            d.stage_ms[k] = acc / (float)n_trees;
-        }
-        dres[b] = d;
-    }
+    gather_statistics(state + b * n_trees, s_root, n_trees, __popc(mask0), dres + b);
 }
 
 // _reduce_over_actions_* (src/mctsnc.py:2299-2375): lexicographic max/argmax over (win_flag, n, n_wins) with the
@@ -279,19 +282,25 @@ __global__ void reduce_over_actions_kernel(const long long *sums, const unsigned
     __shared__ long long s_n[512];
     __shared__ long long s_w[512];
     __shared__ short s_ord2act[512];
-    __shared__ int s_cnt;
+    __shared__ int s_expanded[16];   // expanded actions by warp
     const int b = blockIdx.x;
     const int t = threadIdx.x;
     const long long *sm = sums + (long long)b * 3 * A;
     const unsigned char *fl = flags + (long long)b * 2 * A;
-    if (t == 0) {
-        int c = 0;
-        for (int a = 0; a < A; a++)
-            if (fl[A + a]) s_ord2act[c++] = (short)a;
-        s_cnt = c;
-    }
+    // the expanded actions in ascending order: ballot and prefix over the warps (width >= A; below 32 it is a part of a warp)
+    const unsigned whole = width < 32 ? (1u << width) - 1u : 0xFFFFFFFFu;
+    const bool expanded = t < A && fl[A + t];
+    const unsigned set = __ballot_sync(whole, expanded);
+    if ((t & 31) == 0) s_expanded[t >> 5] = __popc(set);
     __syncthreads();
-    const int limit = thrifty ? s_cnt : A;
+    int n_expanded = 0, before = __popc(set & ((1u << (t & 31)) - 1u));
+    for (int w = 0; w < (width + 31) / 32; w++) {
+        if (w < (t >> 5)) before += s_expanded[w];
+        n_expanded += s_expanded[w];
+    }
+    if (expanded) s_ord2act[before] = (short)t;
+    __syncthreads();
+    const int limit = thrifty ? n_expanded : A;
     const int src = thrifty ? (t < limit ? s_ord2act[t] : 0) : t;
     s_a[t] = (short)t;
     if (t < limit) {
@@ -319,7 +328,7 @@ __global__ void reduce_over_actions_kernel(const long long *sums, const unsigned
     }
     if (t == 0) {
         int best = s_a[0];
-        if (thrifty) best = best < s_cnt ? s_ord2act[best] : 0;
+        if (thrifty) best = best < n_expanded ? s_ord2act[best] : 0;
         dres[b].best_action = best;
         dres[b].best_win_flag = s_f[0];
         dres[b].best_n = s_n[0];
@@ -338,8 +347,9 @@ __global__ void gomoku_reduce_over_trees_kernel(const int4 *rec, const unsigned 
     const unsigned *b0 = board + (long long)b * n_trees * cap * 16;   // root position (the same in every tree)
     __shared__ unsigned s_empty[8];
     __shared__ int s_prefix[9];
+    __shared__ int4 s_root[512];
     if (tid < 8) s_empty[tid] = ~(b0[tid] | b0[8 + tid]) & (tid == 7 ? 0x1u : 0xFFFFFFFFu);
-    __syncthreads();
+    load_roots(s_root, r0, cap, n_trees);
     if (tid == 0) {
         int acc = 0;
         for (int w = 0; w < 8; w++) {
@@ -349,19 +359,20 @@ __global__ void gomoku_reduce_over_trees_kernel(const int4 *rec, const unsigned 
         s_prefix[8] = acc;
     }
     __syncthreads();
-    const int root_turn = gomoku::g_turn(r0[0].w);
-    const int n_children0 = r0[0].w & gomoku::G_NCHILD_MASK;
+    const int root_turn = gomoku::g_turn(s_root[0].w);
+    const int n_children0 = s_root[0].w & gomoku::G_NCHILD_MASK;
     for (int a = tid; a < A; a += blockDim.x) {
-        long long s_root = 0, s_n = 0, s_w = 0;
+        long long n_root = 0, s_n = 0, s_w = 0;
         unsigned char win = 0;
         const int w = a >> 5, bit = a & 31;
         const int rank = s_prefix[w] + __popc(s_empty[w] & ((1u << bit) - 1u));
         const bool expanded = ((s_empty[w] >> bit) & 1u) && rank < n_children0;
         if (expanded) {
+#pragma unroll 4
             for (int t = 0; t < n_trees; t++) {
                 const int4 *rt = r0 + (long long)t * cap;
-                const int4 root = rt[0];
-                s_root += root.x;
+                const int4 root = s_root[t];
+                n_root += root.x;
                 if (rank < (root.w & gomoku::G_NCHILD_MASK)) {
                     const int4 c = rt[root.z + rank];
                     s_n += c.x;
@@ -370,66 +381,13 @@ __global__ void gomoku_reduce_over_trees_kernel(const int4 *rec, const unsigned 
                 }
             }
         }
-        sums[(long long)b * 3 * A + a] = s_root;
+        sums[(long long)b * 3 * A + a] = n_root;
         sums[(long long)b * 3 * A + A + a] = s_n;
         sums[(long long)b * 3 * A + 2 * A + a] = s_w;
         flags[(long long)b * 2 * A + a] = win;
         flags[(long long)b * 2 * A + A + a] = expanded;
     }
-    __shared__ long long sh_depth[256];
-    __shared__ int sh_maxd[256];
-    long long dsum = 0;
-    int dmax = 0;
-    for (int t = 0; t < n_trees; t++) {
-        const int size = state[b * n_trees + t].size;
-        const int4 *rt = r0 + (long long)t * cap;
-        for (int i = tid; i < size; i += blockDim.x) {
-            const int d = meta_depth(rt[i].w);
-            dsum += d;
-            dmax = d > dmax ? d : dmax;
-        }
-    }
-    sh_depth[tid] = dsum;
-    sh_maxd[tid] = dmax;
-    __syncthreads();
-    for (int s = blockDim.x >> 1; s > 0; s >>= 1) {
-        if (tid < s) {
-            sh_depth[tid] += sh_depth[tid + s];
-            sh_maxd[tid] = max(sh_maxd[tid], sh_maxd[tid + s]);
-        }
-        __syncthreads();
-    }
-    if (tid == 0) {
-        DevResult d;
-        d.best_action = -1;
-        d.best_win_flag = 0;
-        d.best_n = 0;
-        d.best_n_wins = 0;
-        d.playouts = 0;
-        d.plies = 0;
-        d.ub_draws = 0;
-        d.status = 0;
-        d.max_size = 0;
-        d.total_nodes = 0;
-        for (int t = 0; t < n_trees; t++) {
-            const TreeState &ts = state[b * n_trees + t];
-            d.playouts += r0[(long long)t * cap].x;
-            d.plies += (long long)ts.plies;
-            d.ub_draws += (long long)ts.ub_draws;
-            d.status |= ts.status;
-            d.total_nodes += ts.size;
-            d.max_size = ts.size > d.max_size ? ts.size : d.max_size;
-        }
-        d.n_root_actions = n_children0;
-        d.max_depth = sh_maxd[0];
-        d.depth_sum = sh_depth[0];
-        for (int k = 0; k < 4; k++) {
-            float acc = 0.f;
-            for (int t = 0; t < n_trees; t++) acc += state[b * n_trees + t].stage_ms[k];
-            d.stage_ms[k] = acc / (float)n_trees;
-        }
-        dres[b] = d;
-    }
+    gather_statistics(state + b * n_trees, s_root, n_trees, n_children0, dres + b);
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -529,7 +487,6 @@ void release(mctsnc_handle *h) {
     cudaFree(h->rng_expand_base);
     cudaFree(h->jump_cols);
     cudaFree(h->root_board);
-    cudaFree(h->root_turn);
     cudaFree(h->queue);
     cudaFree(h->ring);
     cudaFree(h->remaining);
@@ -545,13 +502,8 @@ void release(mctsnc_handle *h) {
     cudaFree(h->active_rank);
     cudaFree(h->root_gboard);
     cudaFreeHost(h->h_root_gboard);
-    cudaFree(h->sums);
-    cudaFree(h->flags);
     cudaFree(h->dres);
     cudaFreeHost(h->h_root_board);
-    cudaFreeHost(h->h_root_turn);
-    cudaFreeHost(h->h_sums);
-    cudaFreeHost(h->h_flags);
     cudaFreeHost(h->h_dres);
     if (h->ev0) cudaEventDestroy(h->ev0);
     if (h->ev1) cudaEventDestroy(h->ev1);
@@ -618,6 +570,15 @@ int seed_streams(mctsnc_handle *h, int batch, cudaStream_t stream) {
     return (int)cudaGetLastError();
 }
 
+// the turns of the roots lie behind the `batch` boards, so that one copy takes both
+int send_roots(mctsnc_handle *h, void *boards, const void *host_boards, size_t board_bytes, int batch, cudaStream_t stream) {
+    h->root_turn = reinterpret_cast<signed char *>(boards) + board_bytes;
+    CUDA_TRY(cudaMemcpyAsync(boards, host_boards, board_bytes + (size_t)batch, cudaMemcpyHostToDevice, stream));
+    CUDA_TRY(cudaEventRecord(h->ev_staged, stream));
+    h->staging_in_flight = true;
+    return 0;
+}
+
 int stage_roots(mctsnc_handle *h, int batch, const int8_t *boards, const int8_t *extras, const int8_t *turns,
                 cudaStream_t stream) {
     const int cells = h->cfg.board_rows * h->cfg.board_cols;
@@ -628,31 +589,25 @@ int stage_roots(mctsnc_handle *h, int batch, const int8_t *boards, const int8_t 
         CUDA_TRY(cudaEventSynchronize(h->ev_staged));
         h->staging_in_flight = false;
     }
+    signed char *host_turns = is_gomoku(h->cfg) ? reinterpret_cast<signed char *>(h->h_root_gboard + (long long)batch * 16)
+                                                : reinterpret_cast<signed char *>(h->h_root_board + batch);
     if (is_gomoku(h->cfg)) {
         for (int b = 0; b < batch; b++) {
             if (turns[b] != 1 && turns[b] != -1) return MCTSNC_E_BAD_ARGUMENT;
             const int rc = gomoku_encode_root(boards + (long long)b * cells, h->h_root_gboard + (long long)b * 16);
             if (rc) return rc;
-            h->h_root_turn[b] = turns[b];
+            host_turns[b] = turns[b];
         }
-        CUDA_TRY(cudaMemcpyAsync(h->root_gboard, h->h_root_gboard, sizeof(unsigned) * 16 * batch, cudaMemcpyHostToDevice, stream));
-        CUDA_TRY(cudaMemcpyAsync(h->root_turn, h->h_root_turn, batch, cudaMemcpyHostToDevice, stream));
-        CUDA_TRY(cudaEventRecord(h->ev_staged, stream));
-        h->staging_in_flight = true;
-        return 0;
+        return send_roots(h, h->root_gboard, h->h_root_gboard, sizeof(unsigned) * 16 * batch, batch, stream);
     }
     for (int b = 0; b < batch; b++) {
         if (turns[b] != 1 && turns[b] != -1) return MCTSNC_E_BAD_ARGUMENT;
         const int rc = c4_encode_root(boards + (long long)b * cells, extras ? extras + (long long)b * extra : nullptr,
                                       &h->h_root_board[b]);
         if (rc) return rc;
-        h->h_root_turn[b] = turns[b];
+        host_turns[b] = turns[b];
     }
-    CUDA_TRY(cudaMemcpyAsync(h->root_board, h->h_root_board, sizeof(ulonglong2) * batch, cudaMemcpyHostToDevice, stream));
-    CUDA_TRY(cudaMemcpyAsync(h->root_turn, h->h_root_turn, batch, cudaMemcpyHostToDevice, stream));
-    CUDA_TRY(cudaEventRecord(h->ev_staged, stream));
-    h->staging_in_flight = true;
-    return 0;
+    return send_roots(h, h->root_board, h->h_root_board, sizeof(ulonglong2) * batch, batch, stream);
 }
 
 // Gomoku: two launches per step (tree step, playouts) and a closing backup, all enqueued without waiting.
@@ -865,11 +820,11 @@ int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_
 
 int launch_reduce_trees(mctsnc_handle *h, int batch, long long *sums, cudaStream_t stream) {
     if (is_gomoku(h->cfg)) {
-        gomoku_reduce_over_trees_kernel<<<batch, 256, 0, stream>>>(h->rec, h->gboard, h->state, h->cfg.node_capacity,
+        gomoku_reduce_over_trees_kernel<<<batch, REDUCE_THREADS, 0, stream>>>(h->rec, h->gboard, h->state, h->cfg.node_capacity,
                                                                   h->cfg.n_trees, sums, h->flags, h->dres);
         return (int)cudaGetLastError();
     }
-    reduce_over_trees_kernel<<<batch, 256, 0, stream>>>(h->rec, h->state, h->cfg.node_capacity, h->cfg.n_trees, h->A, sums,
+    reduce_over_trees_kernel<<<batch, REDUCE_THREADS, 0, stream>>>(h->rec, h->state, h->cfg.node_capacity, h->cfg.n_trees, h->A, sums,
                                                         h->flags, h->dres);
     return (int)cudaGetLastError();
 }
@@ -880,12 +835,22 @@ int launch_reduce_actions(mctsnc_handle *h, int batch, const long long *sums, cu
     return (int)cudaGetLastError();
 }
 
-int fetch_results(mctsnc_handle *h, int batch, const long long *sums_dev, mctsnc_result *results, cudaStream_t stream) {
+// the results of `batch` searches on their way to the host: one copy where the whole handle is in use or little more is copied
+// than is needed (a copy costs about as much as 100 KB), else one for each part
+int copy_results(mctsnc_handle *h, int batch, const long long *sums_dev, cudaStream_t stream) {
     const int A = h->A;
+    const size_t per_search = h->result_bytes / h->cfg.max_batch;
+    if (sums_dev == h->sums && per_search * (size_t)(h->cfg.max_batch - batch) <= 100 * 1024)
+        return (int)cudaMemcpyAsync(h->h_dres, h->dres, h->result_bytes, cudaMemcpyDeviceToHost, stream);
     CUDA_TRY(cudaMemcpyAsync(h->h_sums, sums_dev, sizeof(long long) * 3 * A * batch, cudaMemcpyDeviceToHost, stream));
     CUDA_TRY(cudaMemcpyAsync(h->h_flags, h->flags, (size_t)2 * A * batch, cudaMemcpyDeviceToHost, stream));
     CUDA_TRY(cudaMemcpyAsync(h->h_dres, h->dres, sizeof(DevResult) * batch, cudaMemcpyDeviceToHost, stream));
-    CUDA_TRY(cudaStreamSynchronize(stream));
+    return 0;
+}
+
+// what copy_results has brought, after a synchronisation, in the form of the ABI
+void fill_results(mctsnc_handle *h, int batch, mctsnc_result *results) {
+    const int A = h->A;
     for (int b = 0; b < batch; b++) {
         mctsnc_result &r = results[b];
         const DevResult &d = h->h_dres[b];
@@ -922,7 +887,6 @@ int fetch_results(mctsnc_handle *h, int batch, const long long *sums_dev, mctsnc
             r.actions_expanded[a] = h->h_flags[(long long)b * 2 * A + A + a];
         }
     }
-    return 0;
 }
 
 }  // namespace
@@ -1019,8 +983,8 @@ extern "C" int mctsnc_create(const mctsnc_config *cfg, mctsnc_handle **out) {
     if (!rc && is_gomoku(c)) rc = dev_alloc(h, &h->child_outcome, h->n_trees_total * h->A);
     if (!rc && is_gomoku(c)) rc = dev_alloc(h, &h->child_action, h->n_trees_total * h->A);
     if (!rc && is_gomoku(c)) rc = dev_alloc(h, &h->active_rank, h->n_trees_total * h->A);
-    if (!rc && is_gomoku(c)) rc = dev_alloc(h, &h->root_gboard, (long long)c.max_batch * 16);
-    if (!rc && is_gomoku(c) && cudaMallocHost((void **)&h->h_root_gboard, sizeof(unsigned) * 16 * c.max_batch) != cudaSuccess) rc = MCTSNC_E_NO_MEMORY;
+    if (!rc && is_gomoku(c)) rc = dev_alloc(h, &h->root_gboard, (long long)c.max_batch * 17);   // boards and turns
+    if (!rc && is_gomoku(c) && cudaMallocHost((void **)&h->h_root_gboard, sizeof(unsigned) * 17 * c.max_batch) != cudaSuccess) rc = MCTSNC_E_NO_MEMORY;
     if (!rc && is_gomoku(c)) rc = (int)cudaMemset(h->gstep, 0, sizeof(gomoku::StepInfo) * h->n_trees_total);
     if (!rc && is_gomoku(c)) rc = (int)cudaMemset(h->gtpl, 0, sizeof(unsigned) * gomoku::TPL_WORDS * h->n_trees_total);
     if (!rc) rc = dev_alloc(h, &h->parent, nodes);
@@ -1034,19 +998,26 @@ extern "C" int mctsnc_create(const mctsnc_config *cfg, mctsnc_handle **out) {
     if (!rc) rc = dev_alloc(h, &h->rng_expand_base, (long long)c.n_trees);
     if (!rc) rc = dev_alloc(h, &h->jump_cols, (long long)JUMP_LEVELS * 128);
     if (!rc) rc = (int)cudaMemcpy(h->jump_cols, jump_matrix_table(), sizeof(JumpColumn) * JUMP_LEVELS * 128, cudaMemcpyHostToDevice);
-    if (!rc) rc = dev_alloc(h, &h->root_board, (long long)c.max_batch);
-    if (!rc) rc = dev_alloc(h, &h->root_turn, (long long)c.max_batch);
+    if (!rc) rc = dev_alloc(h, &h->root_board, (long long)c.max_batch * 2);   // boards and turns
     if (!rc && !is_gomoku(c)) rc = dev_alloc(h, &h->queue, 1);
     if (!rc && !is_gomoku(c)) rc = dev_alloc(h, &h->ring, h->n_trees_total * QUEUE_LEVELS);
     if (!rc && !is_gomoku(c)) rc = dev_alloc(h, &h->remaining, h->n_trees_total);
-    if (!rc) rc = dev_alloc(h, &h->sums, (long long)c.max_batch * 3 * h->A);
-    if (!rc) rc = dev_alloc(h, &h->flags, (long long)c.max_batch * 2 * h->A);
-    if (!rc) rc = dev_alloc(h, &h->dres, (long long)c.max_batch);
-    if (!rc && cudaMallocHost((void **)&h->h_root_board, sizeof(ulonglong2) * c.max_batch) != cudaSuccess) rc = MCTSNC_E_NO_MEMORY;
-    if (!rc && cudaMallocHost((void **)&h->h_root_turn, c.max_batch) != cudaSuccess) rc = MCTSNC_E_NO_MEMORY;
-    if (!rc && cudaMallocHost((void **)&h->h_sums, sizeof(long long) * 3 * h->A * c.max_batch) != cudaSuccess) rc = MCTSNC_E_NO_MEMORY;
-    if (!rc && cudaMallocHost((void **)&h->h_flags, (size_t)2 * h->A * c.max_batch) != cudaSuccess) rc = MCTSNC_E_NO_MEMORY;
-    if (!rc && cudaMallocHost((void **)&h->h_dres, sizeof(DevResult) * c.max_batch) != cudaSuccess) rc = MCTSNC_E_NO_MEMORY;
+    {
+        const size_t sums_at = sizeof(DevResult) * c.max_batch, flags_at = sums_at + sizeof(long long) * 3 * h->A * c.max_batch;
+        h->result_bytes = flags_at + (size_t)2 * h->A * c.max_batch;
+        unsigned char *dev = nullptr, *host = nullptr;
+        if (!rc) rc = dev_alloc(h, &dev, (long long)h->result_bytes);
+        if (!rc && cudaMallocHost((void **)&host, h->result_bytes) != cudaSuccess) rc = MCTSNC_E_NO_MEMORY;
+        h->dres = reinterpret_cast<DevResult *>(dev);
+        h->h_dres = reinterpret_cast<DevResult *>(host);
+        if (!rc) {
+            h->sums = reinterpret_cast<long long *>(dev + sums_at);
+            h->flags = dev + flags_at;
+            h->h_sums = reinterpret_cast<long long *>(host + sums_at);
+            h->h_flags = host + flags_at;
+        }
+    }
+    if (!rc && cudaMallocHost((void **)&h->h_root_board, sizeof(ulonglong2) * 2 * c.max_batch) != cudaSuccess) rc = MCTSNC_E_NO_MEMORY;
     if (!rc && cudaEventCreate(&h->ev0) != cudaSuccess) rc = MCTSNC_E_NO_MEMORY;
     if (!rc && cudaEventCreate(&h->ev1) != cudaSuccess) rc = MCTSNC_E_NO_MEMORY;
     if (!rc && cudaEventCreateWithFlags(&h->ev_staged, cudaEventDisableTiming) != cudaSuccess) rc = MCTSNC_E_NO_MEMORY;
@@ -1120,14 +1091,28 @@ extern "C" int mctsnc_run(mctsnc_handle *h, const int8_t *board, const int8_t *e
     int rc = stage_roots(h, 1, board, extra_info, &t8, 0);
     if (rc) return rc;
     h->staged_roots = 1;
+    // behind the last launch of the search: the reductions and the copy of the results, then one wait for everything
+    auto finish = [&]() -> int {
+        int e = launch_reduce_trees(h, 1, h->sums, 0);
+        if (e) return e;
+        CUDA_TRY(cudaEventRecord(h->ev_r0, 0));
+        e = launch_reduce_actions(h, 1, h->sums, 0);
+        if (e) return e;
+        CUDA_TRY(cudaEventRecord(h->ev_r1, 0));
+        e = copy_results(h, 1, h->sums, 0);
+        if (e) return e;
+        return (int)cudaStreamSynchronize(0);
+    };
     const auto t0 = std::chrono::steady_clock::now();
     long long done = 0;
     float total_ms = 0.f;
-    int chunk = steps_limit >= 0 && !(time_limit_s > 0) ? (int)(steps_limit > 1000000 ? 1000000 : steps_limit) : 16;
+    const bool timed = time_limit_s > 0;   // otherwise all steps in launches of at most a million
+    int chunk = timed ? 16 : (int)(steps_limit > 1000000 ? 1000000 : steps_limit);
     int first = 1;
+    bool finished = false;
     for (;;) {
         bool stop = steps_limit >= 0 && done >= steps_limit;
-        if (!stop && time_limit_s > 0) {
+        if (!stop && timed) {
             const double el = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
             stop = el >= time_limit_s;
         }
@@ -1138,14 +1123,17 @@ extern "C" int mctsnc_run(mctsnc_handle *h, const int8_t *board, const int8_t *e
         rc = launch_search(h, 1, (int)n, first, 0);
         if (rc) return rc;
         CUDA_TRY(cudaEventRecord(h->ev1, 0));
-        CUDA_TRY(cudaEventSynchronize(h->ev1));
+        finished = steps_limit >= 0 && done + n >= steps_limit;   // known to be the last launch
+        if (finished) rc = finish();
+        else rc = (int)cudaEventSynchronize(h->ev1);
+        if (rc) return rc;
         float ms = 0.f;
         CUDA_TRY(cudaEventElapsedTime(&ms, h->ev0, h->ev1));
         total_ms += ms;
         done += n;
         first = 0;
-        if (stop) break;
-        if (time_limit_s > 0 && n > 0) {
+        if (stop || finished) break;
+        if (timed && n > 0) {
             // aim at launches of about 2 ms so that the clock is read often enough
             const double per_step = ms / (double)n;
             int next = per_step > 0 ? (int)(2.0 / per_step) : chunk * 2;
@@ -1154,18 +1142,16 @@ extern "C" int mctsnc_run(mctsnc_handle *h, const int8_t *board, const int8_t *e
             chunk = next;
         }
     }
+    if (!finished) {
+        rc = finish();
+        if (rc) return rc;
+    }
     h->last_ms = total_ms;
     h->last_steps = done;
-    rc = launch_reduce_trees(h, 1, h->sums, 0);
-    if (rc) return rc;
-    CUDA_TRY(cudaEventRecord(h->ev_r0, 0));
-    rc = launch_reduce_actions(h, 1, h->sums, 0);
-    if (rc) return rc;
-    CUDA_TRY(cudaEventRecord(h->ev_r1, 0));
-    CUDA_TRY(cudaEventSynchronize(h->ev_r1));
     CUDA_TRY(cudaEventElapsedTime(&h->reduce_ms[0], h->ev1, h->ev_r0));
     CUDA_TRY(cudaEventElapsedTime(&h->reduce_ms[1], h->ev_r0, h->ev_r1));
-    return fetch_results(h, 1, h->sums, out, 0);
+    fill_results(h, 1, out);
+    return 0;
 }
 
 extern "C" int mctsnc_launch_batch_device(mctsnc_handle *h, int32_t batch, const int8_t *boards, const int8_t *extras,
@@ -1220,9 +1206,13 @@ extern "C" int mctsnc_finish_batch_device(mctsnc_handle *h, int32_t batch, const
     int rc = launch_reduce_actions(h, batch, sums, s);
     if (rc) return rc;
     if (!results) return 0;  // the caller keeps everything on the device
-    CUDA_TRY(cudaEventSynchronize(h->ev1));
+    rc = copy_results(h, batch, sums, s);
+    if (rc) return rc;
+    CUDA_TRY(cudaStreamSynchronize(s));
+    CUDA_TRY(cudaEventSynchronize(h->ev1));   // recorded on another stream, perhaps
     CUDA_TRY(cudaEventElapsedTime(&h->last_ms, h->ev0, h->ev1));
-    return fetch_results(h, batch, sums, results, s);
+    fill_results(h, batch, results);
+    return 0;
 }
 
 extern "C" int mctsnc_run_batch(mctsnc_handle *h, int32_t batch, const int8_t *boards, const int8_t *extras, const int8_t *turns,
@@ -1652,7 +1642,7 @@ extern "C" int mctsnc_search_c4_static(const int8_t *board, const int8_t *extra_
     else c4::search_kernel<false, false><<<n_trees, 256, dyn_smem, s>>>(p);
     CUDA_TRY(cudaGetLastError());
     long long *out = reinterpret_cast<long long *>(out_device);
-    reduce_over_trees_kernel<<<1, 256, 0, s>>>(sc->rec, sc->state, CAP, n_trees, A, out, sc->flags, sc->dres);
+    reduce_over_trees_kernel<<<1, REDUCE_THREADS, 0, s>>>(sc->rec, sc->state, CAP, n_trees, A, out, sc->flags, sc->dres);
     const bool thrifty = variant == MCTSNC_OCP_THRIFTY || variant == MCTSNC_ACP_THRIFTY;
     reduce_over_actions_kernel<<<1, 8, 0, s>>>(out, sc->flags, A, 8, thrifty ? 1 : 0, sc->dres);
     append_best_kernel<<<1, 32, 0, s>>>(sc->dres, out, A);

@@ -284,9 +284,9 @@ class MCTSNC:
             extra = np.ascontiguousarray(root_extra_info, dtype=np.int8)
             if extra.size != self.state_extra_info_memory:
                 raise ValueError(f"[MCTSNC.run(): root extra info of {extra.size} bytes, expected {self.state_extra_info_memory}]")
-        res = _abi.Result()
+        res = np.zeros(1, dtype=_abi.RESULT_DTYPE)
         _abi.check(_abi.lib().mctsnc_run(self._handle, board.ctypes.data, extra.ctypes.data if extra is not None else None,
-                                         int(root_turn), steps_limit, time_limit, ctypes.byref(res)))
+                                         int(root_turn), steps_limit, time_limit, res.ctypes.data))
         self._adopt_result(res)
         t2 = time.time()
         self.time_total = t2 - t1
@@ -303,53 +303,57 @@ class MCTSNC:
         print(f"MCTSNC RUN DONE. [time: {self.time_total} s; best action: {best_action_label}, best win_flag: {self.best_win_flag}, best n: {self.best_n}, best n_wins: {self.best_n_wins}, best q: {self.best_q}]")
         return self.best_action
 
+    _RESULT_SCALARS = ("best_action", "best_win_flag", "best_n", "best_n_wins", "steps", "playouts", "plies", "ub_draws", "status",
+                       "device_ms", "max_depth", "total_nodes", "depth_sum", "max_size")
+
     def _adopt_result(self, res):
+        """``res``: array of one ``mctsnc_result``."""
         A = self.state_max_actions
+        r = dict(zip(self._RESULT_SCALARS, res[list(self._RESULT_SCALARS)].item()))
+        stage_ms, reduce_ms = res["stage_ms"][0].tolist(), res["reduce_ms"][0].tolist()
         self._res = {
-            "root_ns": np.array(res.root_ns[:A], dtype=np.int64), "actions_ns": np.array(res.actions_ns[:A], dtype=np.int64),
-            "actions_ns_wins": np.array(res.actions_ns_wins[:A], dtype=np.int64),
-            "actions_win_flags": np.array(res.actions_win_flags[:A], dtype=bool),
-            "actions_expanded": np.array(res.actions_expanded[:A], dtype=bool),
-            "playouts": int(res.playouts), "plies": int(res.plies), "ub_draws": int(res.ub_draws), "status": int(res.status),
-            "max_depth": int(res.max_depth), "total_nodes": int(res.total_nodes), "depth_sum": int(res.depth_sum),
-            "max_size": int(res.max_size), "device_ms": float(res.device_ms),
-            "stage_ms": [float(x) for x in res.stage_ms], "reduce_ms": [float(x) for x in res.reduce_ms]}
-        self.best_action = np.int16(res.best_action)
-        self.best_win_flag = bool(res.best_win_flag)
-        self.best_n = np.int64(res.best_n)
-        self.best_n_wins = np.int64(res.best_n_wins)
+            "root_ns": res["root_ns"][0, :A], "actions_ns": res["actions_ns"][0, :A], "actions_ns_wins": res["actions_ns_wins"][0, :A],
+            "actions_win_flags": res["actions_win_flags"][0, :A].astype(bool),
+            "actions_expanded": res["actions_expanded"][0, :A].astype(bool),
+            "playouts": r["playouts"], "plies": r["plies"], "ub_draws": r["ub_draws"], "status": r["status"],
+            "max_depth": r["max_depth"], "total_nodes": r["total_nodes"], "depth_sum": r["depth_sum"],
+            "max_size": r["max_size"], "device_ms": r["device_ms"], "stage_ms": stage_ms, "reduce_ms": reduce_ms}
+        self.best_action = np.int16(r["best_action"])
+        self.best_win_flag = bool(r["best_win_flag"])
+        self.best_n = np.int64(r["best_n"])
+        self.best_n_wins = np.int64(r["best_n_wins"])
         self.best_q = self.best_n_wins / self.best_n if self.best_n > 0 else np.nan
-        self.steps = int(res.steps)
-        self.status = int(res.status)
-        self.ub_draws = int(res.ub_draws)
-        self.device_time = float(res.device_ms) * 1e-3
+        self.steps = int(r["steps"])
+        self.status = int(r["status"])
+        self.ub_draws = int(r["ub_draws"])
+        self.device_time = r["device_ms"] * 1e-3
         # The loop runs on the device in one piece: its CUDA-event time is the loop time.  The per-stage times of the
         # reference (host clocks around each launch, src/mctsnc.py:606-686) are here the time a tree's thread block spent in
         # each stage, counted on the device (mean over the trees, which run side by side); the two reductions are timed
         # with CUDA events.
         self.time_loop = self.device_time
-        self.time_select, self.time_expand, self.time_playout, self.time_backup = (1e-3 * float(x) for x in res.stage_ms)
-        self.time_reduce_over_trees, self.time_reduce_over_actions = (1e-3 * float(x) for x in res.reduce_ms)
+        self.time_select, self.time_expand, self.time_playout, self.time_backup = (1e-3 * x for x in stage_ms)
+        self.time_reduce_over_trees, self.time_reduce_over_actions = (1e-3 * x for x in reduce_ms)
 
     def _make_actions_info(self):
         """``actions_info`` with the keys of ``src/mctsnc.py:496-563`` (one layout for thrifty and prodigal: keyed by action)."""
         r = self._res
         actions_info = {}
         best_entry = None
-        for a in range(self.state_max_actions):
-            if not r["actions_expanded"][a]:
-                continue
-            entry = {}
-            entry["name"] = self.action_index_to_name_function(a) if self.action_index_to_name_function else str(a)
-            entry["n_root"] = int(r["root_ns"][a])
-            entry["win_flag"] = bool(r["actions_win_flags"][a])
-            entry["n"] = int(r["actions_ns"][a])
-            entry["n_wins"] = int(r["actions_ns_wins"][a])
-            entry["q"] = entry["n_wins"] / entry["n"] if entry["n"] > 0 else np.nan
-            entry["ucb"] = entry["q"] + self.ucb_c * np.sqrt(np.log(entry["n_root"]) / entry["n"]) if entry["n"] > 0 else np.inf
-            actions_info[a] = entry
+        # all entries at once: one by one the 225 of a Gomoku root took a quarter of a millisecond
+        actions = np.flatnonzero(r["actions_expanded"])
+        n_root, n, n_wins = r["root_ns"][actions], r["actions_ns"][actions], r["actions_ns_wins"][actions]
+        with np.errstate(divide="ignore", invalid="ignore"):
+            q = n_wins / n
+            ucb = q + self.ucb_c * np.sqrt(np.log(n_root) / n)
+        rows = zip(actions.tolist(), n_root.tolist(), r["actions_win_flags"][actions].tolist(), n.tolist(), n_wins.tolist(), q.tolist(), ucb)
+        name_of = self.action_index_to_name_function or str
+        for a, a_root, a_win, a_n, a_wins, a_q, a_ucb in rows:
+            if a_n <= 0:
+                a_q, a_ucb = np.nan, np.inf
+            actions_info[a] = {"name": name_of(a), "n_root": a_root, "win_flag": a_win, "n": a_n, "n_wins": a_wins, "q": a_q, "ucb": a_ucb}
             if a == self.best_action:
-                best_entry = {"index": int(a), **entry}
+                best_entry = {"index": a, **actions_info[a]}
         actions_info["best"] = best_entry
         self.actions_info = actions_info
         return actions_info
