@@ -81,11 +81,6 @@ __device__ __forceinline__ int pick_among_tied(unsigned m) {
     return 3;
 }
 
-__device__ __forceinline__ unsigned ordered_key(float v) {
-    unsigned b = __float_as_uint(v);
-    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-}
-
 // ---------------------------------------------------------------------------------------------------------------
 // Byte-for-byte emulation of one playout of the reference (src/mctsnc.py:2049-2069 with the Connect-4 functions of
 // src/mctsnc_game_mechanics.py:102-179) on int8 arrays.  Only entered when a uniform draw equals 1.0f, which makes
@@ -216,15 +211,6 @@ constexpr unsigned MARK = 0x10u;
 __host__ __device__ constexpr float move_row(unsigned set) { return MOVE_LUT_BASE + (float)(8u * (set ^ 1u)); }
 constexpr float NO_MOVES = MOVE_LUT_BASE + 8.f;   // move_row(0)
 
-// one level of the selected path, as far as the backup can know it while the games are still being played; the last entry of a
-// path: its children, which all get the same counts
-struct PathTerm {
-    double explore;      // sqrt(log N / n) of the child on the path, with the counts the backup will leave
-    double n, reciprocal;  // n (as the float32 the UCB divides by) and 1 / n
-    unsigned other_key;  // ordered key of the best UCB among the other children (0: there is none)
-    int other;           // that child's rank, and bit 8: on equal UCB the child on the path wins
-};
-
 constexpr int MAX_PATH = 48;
 
 struct Shared {
@@ -270,20 +256,6 @@ __device__ __forceinline__ int4 rec_load(const int4 *rec, const int4 *cache, int
 __device__ __forceinline__ void rec_store(int4 *rec, int4 *cache, int cache_n, int i, int4 v) {
     rec[i] = v;
     if (i < cache_n) cache[i] = v;
-}
-
-// w / n from the correctly rounded reciprocal of n: one Newton correction of w * (1 / n) with its exact remainder gives the
-// correctly rounded quotient (Markstein, "Computation of elementary functions on the IBM RISC System/6000", 1990), in three
-// dependent operations.  Both operands are whole numbers below 2^53 here, so nothing overflows or is lost.
-__device__ __forceinline__ double divide_by_reciprocal(double w, double n, double reciprocal) {
-    const double q = w * reciprocal;
-    return fma(fma(-q, n, w), reciprocal, q);
-}
-
-// UCB of a child (src/mctsnc.py:1337), evaluated in float64 (numba promotes int32/float32 and log(int32) to float64), fused
-// multiply-add as NVVM contracts it, rounded once to float32; `explore` is sqrt(log(N) / n), `n` is rounded to float32 first
-__device__ __forceinline__ float ucb_value(double c_ucb, double explore, double n, double reciprocal, int wins) {
-    return __double2float_rn(fma(c_ucb, explore, divide_by_reciprocal((double)wins, n, reciprocal)));
 }
 
 // What the backup of the selected path needs and what does not depend on how the games end: the visit counts it will leave

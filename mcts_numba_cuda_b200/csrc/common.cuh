@@ -73,6 +73,37 @@ struct TreeState {
     long long depth_sum; // the sum of the depths of all nodes
 };
 
+#if defined(__CUDACC__)
+__device__ __forceinline__ unsigned ordered_key(float v) {
+    unsigned b = __float_as_uint(v);
+    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+}
+
+// w / n from the correctly rounded reciprocal of n: one Newton correction of w * (1 / n) with its exact remainder gives the
+// correctly rounded quotient (Markstein, "Computation of elementary functions on the IBM RISC System/6000", 1990), in three
+// dependent operations.  Both operands are whole numbers below 2^53 here, so nothing overflows or is lost.
+__device__ __forceinline__ double divide_by_reciprocal(double w, double n, double reciprocal) {
+    const double q = w * reciprocal;
+    return fma(fma(-q, n, w), reciprocal, q);
+}
+
+// UCB of a child (src/mctsnc.py:1337), evaluated in float64 (numba promotes int32/float32 and log(int32) to float64), fused
+// multiply-add as NVVM contracts it, rounded once to float32; `explore` is sqrt(log(N) / n), `n` is rounded to float32 first
+__device__ __forceinline__ float ucb_value(double c_ucb, double explore, double n, double reciprocal, int wins) {
+    return __double2float_rn(fma(c_ucb, explore, divide_by_reciprocal((double)wins, n, reciprocal)));
+}
+
+#endif
+
+// one level of the selected path, as far as the backup can know it while the games are still being played; the last entry of a
+// path: its children, which all get the same counts
+struct PathTerm {
+    double explore;      // sqrt(log N / n) of the child on the path, with the counts the backup will leave
+    double n, reciprocal;  // n (as the float32 the UCB divides by) and 1 / n
+    unsigned other_key;  // ordered key of the best UCB among the other children (0: there is none)
+    int other;             // that child's rank, and bit 8: on equal UCB the child on the path wins
+};
+
 // Work queue of a batched launch.  A tree's search is cut into slices of `chunk` steps; the blocks of a persistent grid
 // take a tree from the queue, run one slice from the state the previous slice left in global memory, and put the tree
 // back while it has steps left.  A tree is sequential, so a launch cannot end before its slowest tree (the one whose

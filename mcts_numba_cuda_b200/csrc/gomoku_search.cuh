@@ -1,12 +1,14 @@
 // Gomoku (15x15, exactly five in a row wins) search kernels.
 //
-// A Gomoku tree-step plays out up to 225 children x P games of about 110 plies each: far more than one block can do
-// in reasonable time, so a step is two launches that the host enqueues without waiting:
-//   tree_step_kernel   one block per tree: backup of the previous step, then select and expand
+// A Gomoku tree-step plays out up to 225 children x P games of about 110 plies each: far more than one block can do in
+// reasonable time, so a step is two launches that the host enqueues without waiting:
+//   tree_step_kernel   one warp per tree (Walker): backup of the previous step, then select and expand
 //                      (_backup_* :2084-2220, _select :1293-1365, _expand_1_* :1368-1681, _expand_2_* :1691-1821)
 //   playout_dynamic_kernel  a persistent grid whose lanes take the step's games one by one (_playout_ocp /
 //                      _playout_acp_* :1824-2081 with the Gomoku device functions of src/mctsnc_game_mechanics.py:181-281)
-// and a last tree_step_kernel launch in backup-only mode.  (Line numbers: src/mctsnc.py of the reference.)
+// and a last tree_step_kernel launch in backup-only mode.  The OCP variants play P games a step: where every tree fits on the
+// device a block per tree does the whole search in one launch (search_block_kernel).
+// (Line numbers: src/mctsnc.py of the reference.)
 //
 // Positions are bitboards: cell (i, j) is bit i*15+j of an 8-word set per player; a node stores 16 words
 // (player -1, then player +1).  As for Connect 4 the children of a node occupy consecutive slots in ascending action
@@ -23,19 +25,25 @@ constexpr int M = 15, N = 15, A = 225;
 constexpr int WORDS = 8;  // 32-bit words of one player's stone set
 
 // meta of a Gomoku node: bits 0..7 number of children (0 = leaf), bit 8 terminal, bits 9..10 outcome + 1, bit 11 turn,
-// bits 16..31 depth
+// bits 16..23 depth, bits 24..31 rank of the child that select goes on to (the backup of a path keeps it up to date)
 constexpr int G_NCHILD_MASK = 0xFF;
 constexpr int G_TERMINAL = 1 << 8;
 constexpr int G_OUTCOME_SHIFT = 9;
 constexpr int G_TURN_POS = 1 << 11;
 __host__ __device__ __forceinline__ int g_outcome(int meta) { return ((meta >> G_OUTCOME_SHIFT) & 3) - 1; }
 __host__ __device__ __forceinline__ int g_turn(int meta) { return (meta & G_TURN_POS) ? 1 : -1; }
+constexpr int G_BEST_SHIFT = 24;
+__host__ __device__ __forceinline__ int g_best(int meta) { return (int)((unsigned)meta >> G_BEST_SHIFT); }
+__host__ __device__ __forceinline__ int g_depth(int meta) { return (meta >> META_DEPTH_SHIFT) & 0xFF; }
 __host__ __device__ __forceinline__ int g_make_meta(int n_children, bool terminal, int outcome, int turn, int depth) {
     return n_children | (terminal ? G_TERMINAL : 0) | ((outcome + 1) << G_OUTCOME_SHIFT) | (turn > 0 ? G_TURN_POS : 0) |
            (depth << META_DEPTH_SHIFT);
 }
 
-// what one step leaves for the playout kernel and for the backup that follows it
+// the side that makes the first move of a step's games
+__device__ __forceinline__ int turn_at_start(int mode, int sel_turn) { return mode == MODE_TREE_FULL ? sel_turn : -sel_turn; }
+
+// what one step leaves for the backup that follows it
 struct StepInfo {
     int selected;
     int mode;         // MODE_ALL_CHILDREN / MODE_TERMINAL / MODE_TREE_FULL
@@ -44,10 +52,12 @@ struct StepInfo {
     int sel_meta;
     int path_len;
     int pick;         // OCP: rank of the child that is played out
-    int pending;      // 1: playouts of this step have been launched, their backup is still to be done
-    int n_active;     // children that need real playouts this step (their ranks: Params::active_rank)
-    int game_counter; // next game of the step to hand out (game = active child index * P + t)
-    int n_empty;      // empty cells of the selected node's position
+    int pending;      // 1: the step has been made, its backup is still to be done
+};
+
+// the games of a step: how many, and the next one to hand out
+struct StepGames {
+    int games, taken;
 };
 
 struct Params {
@@ -57,77 +67,42 @@ struct Params {
     TreeState *state;
     StepInfo *step;           // [trees]
     int *paths;               // [trees][PATH_CAP]
-    int *path_ns;             // [trees][PATH_CAP]
-    int *path_wins;           // [trees][PATH_CAP]
+    int4 *path_rec;           // [trees][PATH_CAP]  the records of the selected path as the select read them
+    PathTerm *term;           // [trees][PATH_CAP]
     short *actions_expanded;  // [trees][A + 2]
-    int *child_out;           // [trees][A][2]   trees_playout_outcomes_children / per-child tallies of the step
+    int2 *child_out;          // [trees][A]   trees_playout_outcomes_children / per-child tallies of the step
     signed char *child_outcome;  // [trees][A]   by rank: outcome of the child (2 = ongoing)
     unsigned char *child_action; // [trees][A]   by rank: action of the child
-    unsigned char *active_rank;  // [trees][A]   ranks of the children that need real playouts, ascending
-    unsigned *tpl;               // [trees][TPL_WORDS]  the selected node's position in the form the playouts use
+    unsigned *sheet;             // [trees][SHEET_WORDS]  what the games of a step start from
     ulonglong2 *rng_playout;
     ulonglong2 *rng_expand;
     const unsigned *root_board;  // [batch][16]
     const signed char *root_turn;
+    StepGames *work;          // [trees]
     long long cap;
     long long node_limit;
     int n_trees;
     int n_playouts;
     int variant;
-    int tree_base;            // a launch works on the trees [tree_base, tree_base + its number of trees)
     int first;                // 1: reset the trees to the roots before anything else
-    int backup_only;          // 1: only the backup of the pending step
+    int tree_base;            // tree_step_kernel, playout_dynamic_kernel: the launch works on the trees from here on
+    int backup_only;          // tree_step_kernel: only the backup of the pending step
+    int steps;                // search_block_kernel
     float ucb_c;
     float ms_per_cycle;       // 1 / (nominal SM clock in kHz), for the stage times of TreeState
 };
 
 __device__ __forceinline__ unsigned bitrev8(unsigned x) { return __brev(x) >> 24; }
 
-__device__ __forceinline__ unsigned ordered_key(float v) {
-    unsigned b = __float_as_uint(v);
-    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-}
-
-// compute_outcome_gomoku (src/mctsnc_game_mechanics.py:220-272) for one direction, on a line word of the form the playouts
-// keep (see below): does the stone that `hs` (0: player -1, 16: player +1) puts at position `pos` make a line of exactly
-// five?  The reference counts at most 5 stones either way and wants a total of 4, i.e. a run of exactly five that holds
-// the stone; cells that do not exist are never set, so the ends of the board count as empty.
-__device__ __forceinline__ bool five_on_line(unsigned word, int hs, int pos) {
-    const unsigned u = ((word >> hs) & 0x7FFFu) | (1u << pos);
-    const unsigned f = u & (u >> 1) & (u >> 2) & (u >> 3) & (u >> 4);   // bit s: stones at s .. s + 4
-    const unsigned e = f & ~(u << 1) & ~(u >> 5);                        // and none at s - 1 and s + 5
-    return (e & ((0x1Fu << pos) >> 4)) != 0u;                            // runs that hold pos: s = pos - 4 .. pos
-}
-
-// block-wide max of a 32-bit key followed by min of a tie-break value among the threads that hold the max
-// (256 threads); returns the winning thread's tie value to every thread
-__device__ __forceinline__ unsigned block_argmax(unsigned key, unsigned tie, unsigned *s_red, int tid) {
-    const int lane = tid & 31, warp = tid >> 5;
-    unsigned m = __reduce_max_sync(0xFFFFFFFFu, key);
-    if (lane == 0) s_red[warp] = m;
-    __syncthreads();
-    unsigned best = s_red[0];
-#pragma unroll
-    for (int w = 1; w < 8; w++) best = max(best, s_red[w]);
-    __syncthreads();
-    unsigned t = __reduce_min_sync(0xFFFFFFFFu, key == best ? tie : 0xFFFFFFFFu);
-    if (lane == 0) s_red[warp] = t;
-    __syncthreads();
-    unsigned tbest = s_red[0];
-#pragma unroll
-    for (int w = 1; w < 8; w++) tbest = min(tbest, s_red[w]);
-    __syncthreads();
-    return tbest;
-}
-
 // ---------------------------------------------------------------------------------------------------------------
-// A game in progress, as the playouts keep it (per thread in shared memory; the same words per tree in Params::tpl for
-// the selected node, written by the tree step and copied by the playouts):
+// A game in progress, as the playouts keep it (per thread in shared memory; the same words per tree on the sheet for the
+// selected node, written by the tree step and copied by the playouts):
 //   LIST_WORDS words   the list of legal actions, one byte each, in the order the reference's swap-remove leaves them
 //                      (src/mctsnc_game_mechanics.py:209-217); the byte of cell (i, j) is i * 16 + j, row and column ready
 //                      to use;
-//   LINE_WORDS words   the stones by line, one word per line of each of the four directions, stones of -1 in bits 0..14,
-//                      stones of +1 in bits 16..30, at the bit of their position along the line:
+//   LINE_WORDS words   the stones by line, one word per line of each of the four directions, at the bit of their position
+//                      along the line: stones of the side that makes the game's first move in bits 0..14, stones of the other
+//                      side in bits 16..30, so that a ply reads and writes one halfword per direction:
 //                        row i                     (position j)
 //                        column j                  (position i)
 //                        diagonal (i - j + 14) & 15   (position j)
@@ -140,49 +115,85 @@ __device__ __forceinline__ unsigned block_argmax(unsigned key, unsigned tie, uns
 //                      0 .. a) and a + 16 (positions a + 2 .. 14).
 constexpr int LIST_WORDS = 57, LINE_WORDS = 15 + 15 + 16 + 16, THREAD_WORDS = LIST_WORDS + LINE_WORDS;
 constexpr int LINE_ROW = LIST_WORDS, LINE_COL = LINE_ROW + 15, LINE_DIAG = LINE_COL + 15, LINE_ANTI = LINE_DIAG + 16;
-// Params::tpl keeps the two parts on 16-byte boundaries, so that a playout thread copies them four words at a time
-constexpr int TPL_LIST = 0, TPL_LINES = 60, TPL_WORDS = 124;
-// Table of the exactly-five test: one byte per 11-cell window of a line (the new stone at bit 5, five cells either way; bit
-// k = the mover's stone k - 5 positions along): 1 iff the stones next to the middle add up to exactly 4, which is what the
-// reference asks for (it counts at most 5 stones either way and wants a total of 4, src/mctsnc_game_mechanics.py:220-272).
-constexpr int FIVE_BYTES = 2048;
+// The sheet of a step: the selected node's position in that form (the two parts on 16-byte boundaries, so that a thread copies them
+// four words at a time), the ranks of the children that are played out, ascending, a byte each, a few numbers, and the list
+// without its first entry
+constexpr int TPL_LIST = 0, TPL_LINES = 60, SHEET_ACTIVE = 124, SHEET_MODE = 184, SHEET_FIRST_CHILD = 185, SHEET_SELECTED = 186,
+              SHEET_FIRST_MOVER = 187, SHEET_EMPTY = 188, SHEET_OLD_FIVE = 189, SHEET_LIST_UP = 192, SHEET_WORDS = 256;
+
+// bit s: stones at s .. s + 4 (for a word of two lines, one in each half: bits 15 and 31 are empty, so no run passes over)
+__device__ __forceinline__ unsigned fives(unsigned w) {
+    const unsigned a = w & (w >> 1);
+    return a & (a >> 2) & (w >> 4);
+}
+// the bits without a neighbour: runs of exactly five (a longer one has several bits in a row)
+__device__ __forceinline__ unsigned lone_bits(unsigned f) { return f & ~(f << 1) & ~(f >> 1); }
+
+// runs of exactly five through a new stone at position `pos1` of line word u1 and `pos2` of u2 (one side's stones, 15 bits each)
+__device__ __forceinline__ bool five_on_lines(unsigned u1, int pos1, unsigned u2, int pos2) {
+    const unsigned one = lone_bits(fives((u1 | (1u << pos1)) + ((u2 | (1u << pos2)) << 16)));
+    return (one & (((0x1Fu << pos1) >> 4) | (((0x1Fu << pos2) >> 4) << 16))) != 0u;   // starts of the runs that hold the stone
+}
+
+// LOCAL: the tree stays with one block for the whole search; else it is read once in a launch, from L2
+template <bool LOCAL, typename T>
+__device__ __forceinline__ T load(const T *p) {
+    if (LOCAL) return *p;
+    return __ldcg(p);
+}
 
 // ---------------------------------------------------------------------------------------------------------------
-// one block of 256 threads per tree
-template <bool OCP>
-__global__ void __launch_bounds__(256) tree_step_kernel(const Params p) {
-    __shared__ unsigned s_board[16];
-    __shared__ unsigned s_lines[15 + 15 + 16 + 16];   // the selected node's stones by line (LINE_WORDS words, see below)
-    __shared__ int s_prefix[9];      // empty cells before word w
-    __shared__ unsigned s_red[8];
-    __shared__ int s_red_i[2][8];
-    __shared__ int4 s_rec;
-    __shared__ int s_node;
-    __shared__ int s_pick;
-    const int g = p.tree_base + (int)blockIdx.x;
-    const int tid = threadIdx.x;
-    const int lane = tid & 31, warp = tid >> 5;
-    const int P = p.n_playouts;
-    int4 *rec = p.rec + (long long)g * p.cap;
-    unsigned *board = p.board + (long long)g * p.cap * 16;
-    int *parent = p.parent + (long long)g * p.cap;
-    TreeState *st = p.state + g;
-    StepInfo *si = p.step + g;
-    int *path = p.paths + g * PATH_CAP;
-    int *path_ns = p.path_ns + g * PATH_CAP;
-    int *path_wins = p.path_wins + g * PATH_CAP;
-    short *ae = p.actions_expanded + g * (A + 2);
-    int *child_out = p.child_out + g * A * 2;
-    signed char *child_outcome = p.child_outcome + g * A;
-    unsigned char *child_action = p.child_action + g * A;
-    const bool thrifty = (p.variant == 0 || p.variant == 2);
+// One warp does a tree's step: backup of the step before, select, expand.
+//
+// As for Connect 4 a node names the child that the arg-max over its children's UCBs picks, so select is one load a level.  The
+// backup decides on every level of its path whether that child changes; all it needs for that except the games' results
+// (the best UCB among the other children, the logarithms, quotients and roots of the new counts) is worked out by `prepare`
+// while the games are being played.  A lane holds cell 32 k + lane in round k, so a round is one word of the stone sets.
+template <bool OCP, bool LOCAL>
+struct Walker {
+    const Params &p;
+    unsigned *sheet;         // shared memory, SHEET_WORDS
+    int g, lane;
+    int4 *rec, *path_rec;
+    unsigned *board;
+    int *parent, *path;
+    TreeState *st;
+    StepInfo *si;
+    PathTerm *term;
+    short *ae;
+    int2 *child_out;
+    signed char *child_outcome;
+    unsigned char *child_action;
+    ulonglong2 *rng_expand;
 
-    if (p.first) {
+    __device__ __forceinline__ Walker(const Params &params, unsigned *sheet_, int tree, int lane_) : p(params), sheet(sheet_), g(tree), lane(lane_) {
+        rec = p.rec + (long long)g * p.cap;
+        board = p.board + (long long)g * p.cap * 16;
+        parent = p.parent + (long long)g * p.cap;
+        path = p.paths + (long long)g * PATH_CAP;
+        path_rec = p.path_rec + (long long)g * PATH_CAP;
+        term = p.term + (long long)g * PATH_CAP;
+        st = p.state + g;
+        si = p.step + g;
+        ae = p.actions_expanded + g * (A + 2);
+        child_out = p.child_out + g * A;
+        child_outcome = p.child_outcome + g * A;
+        child_action = p.child_action + g * A;
+        rng_expand = OCP ? p.rng_expand + g : nullptr;
+    }
+
+    // lane l < 8: the empty cells of word l of a node's position; `mine`: word l < 16 of it
+    __device__ __forceinline__ unsigned empty_cells(int node, unsigned &mine) const {
+        mine = lane < 16 ? load<LOCAL>(&board[(long long)node * 16 + lane]) : 0u;
+        const unsigned other = __shfl_down_sync(0xFFFFFFFFu, mine, 8);
+        return lane < 8 ? ~(mine | other) & (lane == 7 ? 0x1u : 0xFFFFFFFFu) : 0u;   // 225 = 7 * 32 + 1
+    }
+
+    __device__ __forceinline__ void reset() {
         const int b = g / p.n_trees;
-        if (tid < 16) board[tid] = p.root_board[b * 16 + tid];
-        if (tid == 0) {
-            const int turn = p.root_turn[b];
-            rec[0] = make_int4(0, 0, -1, g_make_meta(0, false, 2, turn, 0));
+        if (lane < 16) board[lane] = p.root_board[b * 16 + lane];
+        if (lane == 0) {
+            rec[0] = make_int4(0, 0, -1, g_make_meta(0, false, 2, p.root_turn[b], 0));
             parent[0] = -1;
             st->size = 1;
             st->depth_sum = 0;
@@ -195,347 +206,342 @@ __global__ void __launch_bounds__(256) tree_step_kernel(const Params p) {
             for (int k = 0; k < 4; k++) st->stage_ms[k] = 0.f;
             si->pending = 0;
         }
-        __syncthreads();
+        __syncwarp();
     }
-    const int root_turn = g_turn(rec[0].w);
-    const unsigned c_begin = (unsigned)clock();   // stage times: cycle counts of thread 0 (differences modulo 2^32)
 
-    // =============================================================== backup of the step whose playouts have finished
-    if (si->pending) {
-        const int mode = si->mode, n_exp = si->n_exp, sel_meta = si->sel_meta, first_child = si->first_child;
-        const int child_turn = -g_turn(sel_meta);
-        const int pick = si->pick;
-        int my_neg = 0, my_pos = 0;
-        long long n_tot = P;
+    // _backup_* of the reference, and the choice of the next child on every level of the path
+    __device__ __forceinline__ void backup() {
+        if (load<LOCAL>(&si->pending) == 0) return;
+        const unsigned c_begin = (unsigned)clock();   // stage times: cycle counts of lane 0 (differences modulo 2^32)
+        const int P = p.n_playouts;
+        const int mode = load<LOCAL>(&si->mode), n_exp = load<LOCAL>(&si->n_exp), sel_meta = load<LOCAL>(&si->sel_meta);
+        const int first_child = load<LOCAL>(&si->first_child), plen = load<LOCAL>(&si->path_len), pick = load<LOCAL>(&si->pick);
+        const int root_turn = g_turn(load<LOCAL>(&path_rec[0].w));
+        const double c_ucb = (double)p.ucb_c;
+        int my_neg = 0, my_pos = 0, n_tot = P, leaf_best = 0;
         if (mode == MODE_ALL_CHILDREN) {
-            if (tid < n_exp) {
-                const int a = child_action[tid];
-                const int o = child_outcome[tid];
-                const bool played = !OCP || tid == pick;
-                if (played) {
-                    if (o == 2) {
-                        my_neg = child_out[a * 2 + 0];
-                        my_pos = child_out[a * 2 + 1];
-                    } else {  // terminal child: its stored outcome stands for all P playouts (:2016-2021)
-                        my_neg = o == -1 ? P : 0;
-                        my_pos = o == 1 ? P : 0;
-                        if (!OCP) {
-                            child_out[a * 2 + 0] = my_neg;
-                            child_out[a * 2 + 1] = my_pos;
-                        }
-                    }
-                }
-                const int cns = played ? P : 0;
-                const int cw = played ? (child_turn == 1 ? my_neg : my_pos) : 0;
-                rec[first_child + tid] =
-                    make_int4(cns, cw, -1, g_make_meta(0, o != 2, o, child_turn, meta_depth(sel_meta) + 1));
-            }
-            if (!OCP) n_tot = (long long)P * n_exp;
-        } else if (mode == MODE_TERMINAL) {
-            if (tid == 0) {
-                my_neg = st->out_neg;
-                my_pos = st->out_pos;
-            }
-        } else {  // the selected node itself was played out (slot of action 0)
-            if (tid == 0) {
-                my_neg = child_out[0];
-                my_pos = child_out[1];
-            }
-        }
-        int wn = __reduce_add_sync(0xFFFFFFFFu, my_neg), wp = __reduce_add_sync(0xFFFFFFFFu, my_pos);
-        if (lane == 0) {
-            s_red_i[0][warp] = wn;
-            s_red_i[1][warp] = wp;
-        }
-        __syncthreads();
-        int neg_tot = 0, pos_tot = 0;
+            const int child_turn = -g_turn(sel_meta);
+            const PathTerm *leaf = term + plen - 1;
+            const double explore = load<LOCAL>(&leaf->explore), leaf_n = load<LOCAL>(&leaf->n), reciprocal = load<LOCAL>(&leaf->reciprocal);
+            int action[8], outcome[8];
+            int2 tally[8];
 #pragma unroll
-        for (int w = 0; w < 8; w++) {
-            neg_tot += s_red_i[0][w];
-            pos_tot += s_red_i[1][w];
+            for (int k = 0; k < 8; k++) {
+                const int r = lane + 32 * k;
+                action[k] = r < n_exp ? load<LOCAL>(&child_action[r]) : 0;
+                outcome[k] = r < n_exp ? load<LOCAL>(&child_outcome[r]) : 2;
+            }
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const int r = lane + 32 * k;
+                const bool played = r < n_exp && (!OCP || r == pick);
+                tally[k] = make_int2(0, 0);
+                if (played && outcome[k] == 2) tally[k] = load<LOCAL>(&child_out[action[k]]);
+                else if (played) {   // terminal child: its stored outcome stands for all P playouts (:2016-2021)
+                    tally[k] = make_int2(outcome[k] == -1 ? P : 0, outcome[k] == 1 ? P : 0);
+                    if (!OCP) child_out[action[k]] = tally[k];
+                }
+            }
+            unsigned best = 0, tie = 0xFFFFFFFFu;   // ties: the smallest bit-reversed action (:1343-1351)
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const int r = lane + 32 * k;
+                if (r >= n_exp) continue;
+                const bool played = !OCP || r == pick;
+                my_neg += tally[k].x;
+                my_pos += tally[k].y;
+                const int wins = played ? (child_turn == 1 ? tally[k].x : tally[k].y) : 0;
+                rec[first_child + r] = make_int4(played ? P : 0, wins, -1, g_make_meta(0, outcome[k] != 2, outcome[k], child_turn, g_depth(sel_meta) + 1));
+                const unsigned key = ordered_key(played ? ucb_value(c_ucb, explore, leaf_n, reciprocal, wins) : __int_as_float(0x7f800000));
+                const unsigned t = (bitrev8((unsigned)action[k]) << 8) | (unsigned)r;
+                if (key > best || (key == best && t < tie)) {
+                    best = key;
+                    tie = t;
+                }
+            }
+            const unsigned top = __reduce_max_sync(0xFFFFFFFFu, best);
+            leaf_best = (int)(__reduce_min_sync(0xFFFFFFFFu, best == top ? tie : 0xFFFFFFFFu) & 0xFFu);
+            if (!OCP) n_tot = P * n_exp;
+        } else if (lane == 0) {
+            if (mode == MODE_TERMINAL) {
+                my_neg = load<LOCAL>(&st->out_neg);
+                my_pos = load<LOCAL>(&st->out_pos);
+            } else {   // the selected node itself was played out (slot of action 0)
+                const int2 t = load<LOCAL>(&child_out[0]);
+                my_neg = t.x;
+                my_pos = t.y;
+            }
         }
-        const int plen = si->path_len;
-        for (int e = tid; e < plen; e += 256) {
-            const int node = path[e];
+        const int neg_tot = __reduce_add_sync(0xFFFFFFFFu, my_neg), pos_tot = __reduce_add_sync(0xFFFFFFFFu, my_pos);
+        for (int e = lane; e < plen; e += 32) {
+            int4 r = load<LOCAL>(&path_rec[e]);
+            const int node = load<LOCAL>(&path[e]);
             const int turn_e = (e & 1) ? -root_turn : root_turn;
-            const int ns = path_ns[e] + (int)n_tot;
-            const int wins = path_wins[e] + (turn_e == 1 ? neg_tot : pos_tot);
-            if (e == plen - 1 && mode == MODE_ALL_CHILDREN) rec[node] = make_int4(ns, wins, first_child, sel_meta | n_exp);
-            else *reinterpret_cast<int2 *>(&rec[node]) = make_int2(ns, wins);
+            r.x += n_tot;
+            r.y += turn_e == 1 ? neg_tot : pos_tot;
+            if (e < plen - 1) {
+                const unsigned other_key = load<LOCAL>(&term[e].other_key);
+                const int other = load<LOCAL>(&term[e].other);
+                const int wins = load<LOCAL>(&path_rec[e + 1].y) + (turn_e == 1 ? pos_tot : neg_tot);
+                const unsigned key = ordered_key(ucb_value(c_ucb, load<LOCAL>(&term[e].explore), load<LOCAL>(&term[e].n),
+                                                           load<LOCAL>(&term[e].reciprocal), wins));
+                if (key < other_key || (key == other_key && !(other & 256)))
+                    r.w = (r.w & ((1 << G_BEST_SHIFT) - 1)) | (other & 255) << G_BEST_SHIFT;
+            } else if (mode == MODE_ALL_CHILDREN) {
+                r.z = first_child;
+                r.w = sel_meta | n_exp | (leaf_best << G_BEST_SHIFT);
+            }
+            rec[node] = r;
         }
-        __syncthreads();
-        if (tid == 0) {
+        if (lane == 0) {
             st->out_neg = neg_tot;
             st->out_pos = pos_tot;
             si->pending = 0;
+            st->stage_ms[3] = load<LOCAL>(&st->stage_ms[3]) + (float)((unsigned)clock() - c_begin) * p.ms_per_cycle;
         }
-        __threadfence_block();
-        __syncthreads();
-    }
-    const unsigned c_select = (unsigned)clock();
-    if (tid == 0) st->stage_ms[3] += (float)(c_select - c_begin) * p.ms_per_cycle;
-    if (p.backup_only) return;
-
-    // =============================================================== select
-    if (tid == 0) {
-        s_rec = rec[0];
-        s_node = 0;
-        path[0] = 0;
-        path_ns[0] = s_rec.x;
-        path_wins[0] = s_rec.y;
-    }
-    __syncthreads();
-    int depth = 0;
-    const double c_ucb = (double)p.ucb_c;
-    while ((s_rec.w & G_NCHILD_MASK) != 0 && depth < PATH_CAP - 2) {
-        const int4 r = s_rec;
-        const int node = s_node;
-        const int n_children = r.w & G_NCHILD_MASK;
-        if (tid < 16) s_board[tid] = board[(long long)node * 16 + tid];
-        __syncthreads();
-        if (tid == 0) {
-            int acc = 0;
-            for (int w = 0; w < WORDS; w++) {
-                s_prefix[w] = acc;
-                const unsigned valid = w == 7 ? 0x1u : 0xFFFFFFFFu;  // 225 = 7*32 + 1
-                acc += __popc(~(s_board[w] | s_board[8 + w]) & valid);
-            }
-            s_prefix[8] = acc;
-        }
-        __syncthreads();
-        unsigned key = 0;
-        int child = -1;
-        int4 cr = make_int4(0, 0, -1, 0);
-        if (tid < A) {
-            const int w = tid >> 5, bit = tid & 31;
-            const unsigned empty = ~(s_board[w] | s_board[8 + w]);
-            if ((empty >> bit) & 1u) {
-                const int rank = s_prefix[w] + __popc(empty & ((1u << bit) - 1u));
-                if (rank < n_children) {
-                    child = r.z + rank;
-                    cr = rec[child];
-                    float v;
-                    if (cr.x == 0) {
-                        v = __int_as_float(0x7f800000);
-                    } else {
-                        // src/mctsnc.py:1337: float64 arithmetic, fused multiply-add, one rounding to float32
-                        const double q = (double)cr.y / (double)__int2float_rn(cr.x);
-                        const double e = sqrt(log((double)r.x) / (double)cr.x);
-                        v = __double2float_rn(fma(c_ucb, e, q));
-                    }
-                    key = ordered_key(v);
-                }
-            }
-        }
-        // ties: the reference's stride-halving reduction keeps the left operand (:1343-1351): smallest bit-reversed index
-        const unsigned win_rev = block_argmax(child >= 0 ? key : 0u, child >= 0 ? bitrev8(tid) : 0xFFFFFFFFu, s_red, tid);
-        const int winner = (int)bitrev8(win_rev);
-        __syncthreads();
-        if (tid == winner) {
-            s_rec = cr;
-            s_node = child;
-            path[depth + 1] = child;
-            path_ns[depth + 1] = cr.x;
-            path_wins[depth + 1] = cr.y;
-        }
-        depth++;
-        __syncthreads();
+        __syncwarp();
     }
 
-    // =============================================================== expand
-    const unsigned c_expand = (unsigned)clock();
-    const int4 r = s_rec;
-    const int node = s_node;
-    const int sel_turn = g_turn(r.w);
-    int mode, n_exp = 0, first_child = -1;
-    if (r.w & G_TERMINAL) {
-        mode = MODE_TERMINAL;
-        if (tid == 0) {
-            const int o = g_outcome(r.w);
-            st->out_neg = o == -1 ? P : 0;
-            st->out_pos = o == 1 ? P : 0;
+    // select and expand; writes the sheet; returns how many children are to be played out
+    __device__ __forceinline__ int advance() {
+        const unsigned c_select = (unsigned)clock();
+        const int P = p.n_playouts;
+        const bool thrifty = (p.variant == 0 || p.variant == 2);
+        int node = 0, depth = 0;
+        int4 r = load<LOCAL>(&rec[0]);
+        const int size = load<LOCAL>(&st->size);
+        if (lane == 0) {
+            path[0] = 0;
+            path_rec[0] = r;
         }
-    } else {
-        if (tid < 16) s_board[tid] = board[(long long)node * 16 + tid];
-        __syncthreads();
-        if (tid == 0) {
-            int acc = 0;
-            for (int w = 0; w < WORDS; w++) {
-                s_prefix[w] = acc;
-                const unsigned valid = w == 7 ? 0x1u : 0xFFFFFFFFu;
-                acc += __popc(~(s_board[w] | s_board[8 + w]) & valid);
+        while ((r.w & G_NCHILD_MASK) != 0 && depth < PATH_CAP - 2) {
+            node = r.z + g_best(r.w);
+            r = load<LOCAL>(&rec[node]);
+            depth++;
+            if (lane == 0) {
+                path[depth] = node;
+                path_rec[depth] = r;
             }
-            s_prefix[8] = acc;
         }
-        __syncthreads();
-        const int n_legal = s_prefix[8];
-        {
-            // the position in the playouts' form: the list of empty cells in ascending order, the stones by line
-            unsigned *tpl = p.tpl + (long long)g * TPL_WORDS;
-            unsigned char *tpl_list = reinterpret_cast<unsigned char *>(tpl + TPL_LIST);
-            if (tid < A) {
-                const int w = tid >> 5, bit = tid & 31;
-                const unsigned empty = ~(s_board[w] | s_board[8 + w]);
-                if ((empty >> bit) & 1u)
-                    tpl_list[s_prefix[w] + __popc(empty & ((1u << bit) - 1u))] = (unsigned char)(((tid / N) << 4) | (tid % N));
-            }
-            // the line words: one (line, position) pair per thread and round, the cell's stones OR-ed into the line's word
-            if (tid < LINE_WORDS) s_lines[tid] = 0u;
-            __syncthreads();
-            for (int pair = tid; pair < LINE_WORDS * 15; pair += 256) {
-                const int lt = pair / 15, pos = pair - lt * 15;
-                const int family = lt < 15 ? 0 : (lt < 30 ? 1 : (lt < 46 ? 2 : 3));
-                const int idx = lt - (family == 0 ? 0 : (family == 1 ? 15 : (family == 2 ? 30 : 46)));
-                unsigned bits = 0;
-                for (int fold = 0; fold < 2; fold++) {   // the two lines of a folded word; rows and columns have one
-                    int i, j;
-                    if (family == 0) {
-                        i = idx;
-                        j = pos;
-                    } else if (family == 1) {
-                        i = pos;
-                        j = idx;
-                    } else if (family == 2) {
-                        j = pos;
-                        i = idx + 16 * fold - 14 + j;
-                    } else {
-                        j = pos;
-                        i = idx + 16 * fold - j;
-                    }
-                    if ((family < 2 && fold == 1) || i < 0 || i >= M) continue;
-                    const int c = i * N + j;
-                    if ((s_board[c >> 5] >> (c & 31)) & 1u) bits |= 1u << pos;
-                    if ((s_board[8 + (c >> 5)] >> (c & 31)) & 1u) bits |= 1u << (16 + pos);
-                }
-                if (bits) atomicOr(&s_lines[lt], bits);
-            }
-            __syncthreads();
-            if (tid < LINE_WORDS) tpl[TPL_LINES + tid] = s_lines[tid];
-        }
-        const int size = st->size;
-        long long room = p.node_limit - (long long)size;
-        if (room < 0) room = 0;
-        n_exp = n_legal < room ? n_legal : (int)room;
-        if (n_exp < n_legal && tid == 0) st->status |= STATUS_TREE_FULL;
-        if (n_exp > 0) {
-            mode = MODE_ALL_CHILDREN;
-            first_child = size;
-            if (OCP) {
-                if (tid == 0) {
-                    // src/mctsnc.py:1435 / :1511: float32 * int64 is a float64 product, truncated
-                    ulonglong2 es = p.rng_expand[g];
-                    const float u = rng_uniform_f32(es.x, es.y);
-                    p.rng_expand[g] = es;
-                    int pick = __double2int_rz((double)u * (double)n_exp);
-                    if (pick >= n_exp) {  // u == 1.0f: undefined in the reference, clamped
-                        pick = n_exp - 1;
-                        st->ub_draws += 1;
-                        st->status |= STATUS_UB_DRAW;
-                    }
-                    s_pick = pick;
-                }
-                __syncthreads();
-            }
-            bool plays = false;   // this thread's child needs real playouts
-            int my_rank = 0;
-            if (tid < A) {
-                const int w = tid >> 5, bit = tid & 31;
-                const unsigned empty = ~(s_board[w] | s_board[8 + w]);
-                const bool legal = (empty >> bit) & 1u;
-                const int rank = s_prefix[w] + __popc(empty & ((1u << bit) - 1u));
-                if (legal && rank < n_exp) {
-                    // _expand_2_*: the child's position and outcome (:1794-1821)
-                    const int off = sel_turn > 0 ? 8 : 0, hs = sel_turn > 0 ? 16 : 0;
-                    const int i = tid / N, j = tid - i * N;
-                    const bool win = five_on_line(s_lines[i], hs, j) || five_on_line(s_lines[15 + j], hs, i) ||
-                                     five_on_line(s_lines[30 + ((i - j + 14) & 15)], hs, j) ||
-                                     five_on_line(s_lines[46 + ((i + j) & 15)], hs, j);
-                    const int outcome = win ? sel_turn : (n_legal == 1 ? 0 : 2);
-                    uint4 *cb = reinterpret_cast<uint4 *>(board + (long long)(first_child + rank) * 16);
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {   // the parent's 16 words, the new stone in word off + w
-                        uint4 v = make_uint4(s_board[4 * q], s_board[4 * q + 1], s_board[4 * q + 2], s_board[4 * q + 3]);
-                        if (((off + w) >> 2) == q) {
-                            const unsigned stone = 1u << bit;
-                            const int k = (off + w) & 3;
-                            v.x |= k == 0 ? stone : 0u;
-                            v.y |= k == 1 ? stone : 0u;
-                            v.z |= k == 2 ? stone : 0u;
-                            v.w |= k == 3 ? stone : 0u;
-                        }
-                        cb[q] = v;
-                    }
-                    parent[first_child + rank] = node;
-                    child_action[rank] = (unsigned char)tid;
-                    child_outcome[rank] = (signed char)outcome;
-                    if (!OCP || rank == s_pick) {  // the tallies the playout block adds to
-                        child_out[tid * 2 + 0] = 0;
-                        child_out[tid * 2 + 1] = 0;
-                    }
-                    if (thrifty) ae[rank] = (short)tid;
-                    else ae[tid] = (short)tid;
-                    plays = outcome == 2 && (!OCP || rank == s_pick);
-                    my_rank = rank;
-                } else if (!thrifty) {
-                    ae[tid] = -1;
-                }
-            }
-            // the ranks of the children that are played out, ascending: position = playing children of lower rank
-            const unsigned playing_lanes = __ballot_sync(0xFFFFFFFFu, plays);
-            if (lane == 0) s_red[warp] = (unsigned)__popc(playing_lanes);
-            __syncthreads();
-            if (plays) {
-                int before = __popc(playing_lanes & ((1u << lane) - 1u));
-                for (int wb = 0; wb < warp; wb++) before += (int)s_red[wb];
-                p.active_rank[g * A + before] = (unsigned char)my_rank;
+        const unsigned c_expand = (unsigned)clock();
+        const int sel_turn = g_turn(r.w);
+        int mode = MODE_TERMINAL, n_exp = 0, first_child = -1, n_active = 0, pick = 0;
+        if (r.w & G_TERMINAL) {
+            if (lane == 0) {
+                const int o = g_outcome(r.w);
+                st->out_neg = o == -1 ? P : 0;
+                st->out_pos = o == 1 ? P : 0;
             }
         } else {
-            mode = MODE_TREE_FULL;
-            if (tid == 0) {
-                child_out[0] = 0;
-                child_out[1] = 0;
+            unsigned mine;
+            const unsigned empties = empty_cells(node, mine);
+            const int n_legal = __reduce_add_sync(0xFFFFFFFFu, __popc(empties));
+            long long room = p.node_limit - (long long)size;
+            if (room < 0) room = 0;
+            n_exp = n_legal < room ? n_legal : (int)room;
+            mode = n_exp > 0 ? MODE_ALL_CHILDREN : MODE_TREE_FULL;
+            const int first_mover = turn_at_start(mode, sel_turn);
+            // the position in the playouts' form: the list of empty cells in ascending order, the stones by line
+            __syncwarp();
+            for (int i = lane; i < LINE_WORDS; i += 32) sheet[TPL_LINES + i] = 0u;
+            __syncwarp();
+            unsigned char *list = reinterpret_cast<unsigned char *>(sheet + TPL_LIST), *list_up = reinterpret_cast<unsigned char *>(sheet + SHEET_LIST_UP);
+            unsigned words[16];
+#pragma unroll
+            for (int k = 0; k < 16; k++) words[k] = __shfl_sync(0xFFFFFFFFu, mine, k);
+            int before = 0;   // empty cells before word k
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const int cell = 32 * k + lane, i = cell / N, j = cell - i * N;
+                const unsigned empty = __shfl_sync(0xFFFFFFFFu, empties, k);
+                if ((empty >> lane) & 1u) {
+                    const int rank = before + __popc(empty & ((1u << lane) - 1u));
+                    list[rank] = (unsigned char)((i << 4) | j);
+                    if (rank > 0) list_up[rank - 1] = (unsigned char)((i << 4) | j);
+                } else if (cell < A) {
+                    const bool low = (((words[k] >> lane) & 1u) != 0u) == (first_mover < 0);   // the first mover's stones: the low halves
+                    const int hs = low ? 0 : 16;
+                    atomicOr(&sheet[TPL_LINES + i], 1u << (hs + j));
+                    atomicOr(&sheet[TPL_LINES + 15 + j], 1u << (hs + i));
+                    atomicOr(&sheet[TPL_LINES + 30 + ((i - j + 14) & 15)], 1u << (hs + j));
+                    atomicOr(&sheet[TPL_LINES + 46 + ((i + j) & 15)], 1u << (hs + j));
+                }
+                before += __popc(empty);
             }
-            if (tid < A && !thrifty) ae[tid] = -1;
+            __syncwarp();
+            const unsigned *lines = sheet + TPL_LINES;
+            const bool five = lone_bits(fives(lines[lane])) != 0u || (lane + 32 < LINE_WORDS && lone_bits(fives(lines[lane + 32])) != 0u);
+            const bool old_five = __any_sync(0xFFFFFFFFu, five);
+            if (lane == 0 && n_exp < n_legal) atomicOr(&st->status, STATUS_TREE_FULL);
+            unsigned char *active = reinterpret_cast<unsigned char *>(sheet + SHEET_ACTIVE);
+            if (mode == MODE_ALL_CHILDREN) {
+                first_child = size;
+                if (OCP) {
+                    // src/mctsnc.py:1435 / :1511: float32 * int64 is a float64 product, truncated
+                    if (lane == 0) {
+                        ulonglong2 es = load<LOCAL>(rng_expand);
+                        const float u = rng_uniform_f32(es.x, es.y);
+                        *rng_expand = es;
+                        pick = __double2int_rz((double)u * (double)n_exp);
+                        if (pick >= n_exp) {  // u == 1.0f: undefined in the reference, clamped
+                            pick = n_exp - 1;
+                            atomicAdd(&st->ub_draws, 1ULL);
+                            atomicOr(&st->status, STATUS_UB_DRAW);
+                        }
+                    }
+                    pick = __shfl_sync(0xFFFFFFFFu, pick, 0);
+                }
+                // _expand_2_*: the children's positions and outcomes (:1794-1821); the side to move here has the high halves
+                before = 0;
+#pragma unroll
+                for (int k = 0; k < 8; k++) {
+                    const int cell = 32 * k + lane, i = cell / N, j = cell - i * N;
+                    const unsigned empty = __shfl_sync(0xFFFFFFFFu, empties, k);
+                    const int rank = before + __popc(empty & ((1u << lane) - 1u));
+                    const bool child = ((empty >> lane) & 1u) && rank < n_exp;
+                    bool plays = false;
+                    if (child) {
+                        const bool win = five_on_lines(lines[i] >> 16, j, lines[15 + j] >> 16, i) ||
+                                         five_on_lines(lines[30 + ((i - j + 14) & 15)] >> 16, j, lines[46 + ((i + j) & 15)] >> 16, j);
+                        const int outcome = win ? sel_turn : (n_legal == 1 ? 0 : 2);
+                        uint4 *cb = reinterpret_cast<uint4 *>(board + (long long)(first_child + rank) * 16);
+                        const unsigned stone = 1u << lane, neg = sel_turn < 0 ? stone : 0u, pos = sel_turn < 0 ? 0u : stone;
+#pragma unroll
+                        for (int q = 0; q < 4; q++) {   // the parent's 16 words, the new stone in word k of its side
+                            const int w0 = 4 * q;
+                            cb[q] = make_uint4(words[w0] | (w0 == k ? neg : 0u) | (w0 == 8 + k ? pos : 0u),
+                                               words[w0 + 1] | (w0 + 1 == k ? neg : 0u) | (w0 + 1 == 8 + k ? pos : 0u),
+                                               words[w0 + 2] | (w0 + 2 == k ? neg : 0u) | (w0 + 2 == 8 + k ? pos : 0u),
+                                               words[w0 + 3] | (w0 + 3 == k ? neg : 0u) | (w0 + 3 == 8 + k ? pos : 0u));
+                        }
+                        parent[first_child + rank] = node;
+                        child_action[rank] = (unsigned char)cell;
+                        child_outcome[rank] = (signed char)outcome;
+                        if (!OCP || rank == pick) child_out[cell] = make_int2(0, 0);   // the tallies the games add to
+                        if (thrifty) ae[rank] = (short)cell;
+                        else ae[cell] = (short)cell;
+                        plays = outcome == 2 && (!OCP || rank == pick);
+                    } else if (!thrifty && cell < A) {
+                        ae[cell] = -1;
+                    }
+                    const unsigned playing = __ballot_sync(0xFFFFFFFFu, plays);
+                    if (plays) active[n_active + __popc(playing & ((1u << lane) - 1u))] = (unsigned char)rank;
+                    n_active += __popc(playing);
+                    before += __popc(empty);
+                }
+            } else {
+                n_active = 1;
+                if (lane == 0) {
+                    child_out[0] = make_int2(0, 0);
+                    active[0] = 0;
+                }
+            }
+            if (lane == 0) {
+                sheet[SHEET_MODE] = (unsigned)mode;
+                sheet[SHEET_FIRST_CHILD] = (unsigned)first_child;
+                sheet[SHEET_SELECTED] = (unsigned)node;
+                sheet[SHEET_FIRST_MOVER] = (unsigned)first_mover;
+                sheet[SHEET_EMPTY] = (unsigned)n_legal;
+                sheet[SHEET_OLD_FIVE] = old_five ? 1u : 0u;
+            }
         }
+        if (mode != MODE_ALL_CHILDREN && !thrifty)
+            for (int a = lane; a < A; a += 32) ae[a] = -1;
+        __syncwarp();
+        if (lane == 0) {
+            if (mode == MODE_ALL_CHILDREN) {
+                st->size = size + n_exp;
+                st->depth_sum = load<LOCAL>(&st->depth_sum) + (long long)n_exp * (depth + 1);
+                st->max_depth = max(load<LOCAL>(&st->max_depth), depth + 1);
+            }
+            ae[A + 1] = (short)(mode == MODE_ALL_CHILDREN ? n_exp : 1);
+            int m2 = mode;
+            if (OCP && mode == MODE_ALL_CHILDREN) {
+                m2 = pick;
+                if (!thrifty) {   // the pick's action, from the list (the cell's row and column)
+                    const int c = reinterpret_cast<unsigned char *>(sheet + TPL_LIST)[pick];
+                    m2 = (c >> 4) * N + (c & 15);
+                }
+            }
+            ae[A] = (short)m2;
+            if (!OCP && mode != MODE_ALL_CHILDREN) ae[0] = 0;
+            si->selected = node;
+            si->mode = mode;
+            si->n_exp = n_exp;
+            si->first_child = first_child;
+            si->sel_meta = r.w;
+            si->path_len = depth + 1;
+            si->pick = pick;
+            si->pending = 1;
+            st->selected = node;
+            st->path_len = depth + 1;
+            st->stage_ms[0] = load<LOCAL>(&st->stage_ms[0]) + (float)(c_expand - c_select) * p.ms_per_cycle;
+            st->stage_ms[1] = load<LOCAL>(&st->stage_ms[1]) + (float)((unsigned)clock() - c_expand) * p.ms_per_cycle;
+        }
+        __syncwarp();
+        return n_active;
     }
-    if (mode == MODE_TERMINAL && tid < A && !thrifty) ae[tid] = -1;
-    __syncthreads();
-    if (tid == 0) {
-        if (mode == MODE_ALL_CHILDREN) {
-            st->size += n_exp;
-            st->depth_sum += (long long)n_exp * (meta_depth(r.w) + 1);
-            st->max_depth = max(st->max_depth, meta_depth(r.w) + 1);
+
+    // for the backup of the step just made: see PathTerm
+    __device__ __forceinline__ void prepare() {
+        const int mode = load<LOCAL>(&si->mode), plen = load<LOCAL>(&si->path_len);
+        const int n_tot = p.n_playouts * (mode == MODE_ALL_CHILDREN && !OCP ? load<LOCAL>(&si->n_exp) : 1);
+        const double c_ucb = (double)p.ucb_c;
+        for (int e = 0; e < plen - 1; e++) {
+            const int4 pr = load<LOCAL>(&path_rec[e]);
+            const int node = load<LOCAL>(&path[e]);
+            const int n_path = load<LOCAL>(&path_rec[e + 1].x) + n_tot, on_path = g_best(pr.w), n_children = pr.w & G_NCHILD_MASK;
+            unsigned mine;
+            const unsigned empties = empty_cells(node, mine);
+            const double log_parent = log((double)(pr.x + n_tot));
+            unsigned best = 0, tie = 0xFFFFFFFFu, path_tie = 0;
+            int before = 0;
+#pragma unroll 2
+            for (int k = 0; k < 8; k++) {
+                const unsigned empty = __shfl_sync(0xFFFFFFFFu, empties, k);
+                const int rank = before + __popc(empty & ((1u << lane) - 1u));
+                const unsigned t = (bitrev8((unsigned)(32 * k + lane)) << 8) | (unsigned)rank;
+                if (((empty >> lane) & 1u) && rank < n_children) {
+                    if (rank == on_path) {
+                        path_tie = t;
+                    } else {
+                        const int4 c = load<LOCAL>(&rec[pr.z + rank]);
+                        const double n_f = (double)__int2float_rn(c.x);
+                        const unsigned key = ordered_key(c.x == 0 ? __int_as_float(0x7f800000)
+                                                                  : ucb_value(c_ucb, sqrt(log_parent / (double)c.x), n_f, 1.0 / n_f, c.y));
+                        if (key > best || (key == best && t < tie)) {
+                            best = key;
+                            tie = t;
+                        }
+                    }
+                }
+                before += __popc(empty);
+            }
+            const unsigned top = __reduce_max_sync(0xFFFFFFFFu, best);
+            const unsigned other = __reduce_min_sync(0xFFFFFFFFu, best == top && best != 0u ? tie : 0xFFFFFFFFu);
+            path_tie = __reduce_max_sync(0xFFFFFFFFu, path_tie);
+            if (lane == 0) {
+                PathTerm t;
+                t.explore = sqrt(log_parent / (double)n_path);
+                t.n = (double)__int2float_rn(n_path);
+                t.reciprocal = 1.0 / t.n;
+                t.other_key = top;
+                t.other = (int)(other & 255u) | (path_tie < other ? 256 : 0);
+                term[e] = t;
+            }
         }
-        ae[A + 1] = (short)(mode == MODE_ALL_CHILDREN ? n_exp : 1);
-        int m2 = mode;
-        const int pick = (OCP && mode == MODE_ALL_CHILDREN) ? s_pick : 0;
-        if (OCP && mode == MODE_ALL_CHILDREN) m2 = thrifty ? pick : child_action[pick];
-        ae[A] = (short)m2;
-        if (!OCP && mode != MODE_ALL_CHILDREN) ae[0] = 0;
-        si->selected = node;
-        si->mode = mode;
-        si->n_exp = n_exp;
-        si->first_child = first_child;
-        si->sel_meta = r.w;
-        si->path_len = depth + 1;
-        si->pick = pick;
-        int n_active = 0;
-        if (mode == MODE_ALL_CHILDREN) {
-            for (int wb = 0; wb < 8; wb++) n_active += (int)s_red[wb];
-        } else if (mode == MODE_TREE_FULL) {
-            p.active_rank[g * A] = 0;
-            n_active = 1;
+        if (mode == MODE_ALL_CHILDREN && lane == 0) {
+            PathTerm t;
+            t.n = (double)p.n_playouts;   // at most 512: the same as a float32
+            t.explore = sqrt(log((double)(load<LOCAL>(&path_rec[plen - 1].x) + n_tot)) / t.n);
+            t.reciprocal = 1.0 / t.n;
+            t.other_key = 0u;
+            t.other = 0;
+            term[plen - 1] = t;
         }
-        si->n_active = n_active;
-        si->n_empty = mode == MODE_TERMINAL ? 0 : s_prefix[8];
-        si->game_counter = 0;
-        si->pending = 1;
-        st->selected = node;
-        st->path_len = depth + 1;
-        st->stage_ms[0] += (float)(c_expand - c_select) * p.ms_per_cycle;
-        st->stage_ms[1] += (float)((unsigned)clock() - c_expand) * p.ms_per_cycle;
+        __syncwarp();
     }
-}
+};
 
 // ---------------------------------------------------------------------------------------------------------------
 // Byte-for-byte emulation of one Gomoku playout of the reference on int8 / int16 local arrays (see the Connect-4
@@ -563,7 +569,7 @@ __device__ __noinline__ EmuResult playout_emulated(const unsigned *start /* 16 w
     short legal[513];
     unsigned err = 0;
     for (int c = 0; c < A; c++) {
-        const bool neg = (start[c >> 5] >> (c & 31)) & 1u, pos = (start[8 + (c >> 5)] >> (c & 31)) & 1u;
+        const bool neg = (__ldcg(start + (c >> 5)) >> (c & 31)) & 1u, pos = (__ldcg(start + 8 + (c >> 5)) >> (c & 31)) & 1u;
         bd[c] = pos ? 1 : (neg ? -1 : 0);
     }
     for (int k = 0; k < 513; k++) legal[k] = 0;
@@ -633,25 +639,218 @@ __device__ __noinline__ EmuResult playout_emulated(const unsigned *start /* 16 w
     return r;
 }
 
-__device__ __forceinline__ int turn_at_start(int mode, int sel_turn) { return mode == MODE_TREE_FULL ? sel_turn : -sel_turn; }
+// ---------------------------------------------------------------------------------------------------------------
+// A game in progress: one per thread, list and lines in the thread's column of shared memory (STRIDE threads side by side).
+//   * The four words of a new stone hold a run of five iff the AND of the word with itself shifted by 1 to 4 has a bit, and one of
+//     exactly five (which the reference wants: it counts at most 5 stones either way and asks for a total of 4,
+//     src/mctsnc_game_mechanics.py:220-272) iff that bit has no neighbour.  Two lines are tested in the halves of a word.  A run
+//     of exactly five that does not go through the new stone would have ended the game before, unless the starting position
+//     has one: then (`careful`) the place of the run is looked at too.
+//   * The draw of a ply and the two list entries it reads are fetched one ply ahead.
+//   * The plies of a block depend on no branch, so that they overlap; a game that has been won plays on to the end of the block,
+//     which is put right when it is closed.  A draw of exactly 1.0f is noticed at the end of the block too (the largest draw is
+//     kept); until then the lane plays on with a list entry it should not have, inside its own column.
+template <int STRIDE>
+struct Game {
+    unsigned char *list;      // the thread's column
+    bool playing;             // the game is going on
+    bool careful;
+    int left, left_at_start, left_at_end;   // empty cells: now, before the first move, after the last one
+    int winner;               // of a game that is over: 1 first mover, 2 the other side, 0 a draw
+    float left_2m64;          // left * 2^-64, the factor of the draws scaled by 2^64
+    float draw, largest;      // the draw of the ply to come and the largest of those before it, times 2^64
+    int at;                   // byte offset in the column of the list entry that the ply to come takes
+    int next_cell, next_last; // that entry and the last one of the list
+    unsigned long long s0, s1;
+
+    // byte offset of list entry q: byte q & 3 of word q >> 2, words STRIDE apart; (q >> 2) * 4 * STRIDE + (q & 3) written as one
+    // shift and one multiply-add
+    static __device__ __forceinline__ int list_byte(int q) { return (q >> 2) * (4 * STRIDE - 4) + q; }
+
+    // The position a game starts from, out of a sheet in shared memory: the parent's with `count` empty cells, less the child's own
+    // cell, which is at position `skip` of the list (child_cell < 0: the parent itself, skip = NO_SKIP).
+    // The list: four words at a time, from the list in front of `skip` and from the list without its first entry behind it; the four
+    // words around `skip` are put right afterwards.  Words past the last entry are never read; up to three words past the list
+    // are written and then covered by the lines.
+    static constexpr int NO_SKIP = 1 << 30;
+    __device__ __forceinline__ void copy_position(const unsigned *sheet, int count, int skip, int child_cell) {
+        unsigned *my = reinterpret_cast<unsigned *>(list);
+        const int skip_word = skip >> 2, skip_chunk = skip >> 4;
+        const int chunks = (count + 15) >> 4;
+        const uint4 *list4 = reinterpret_cast<const uint4 *>(sheet + TPL_LIST), *up4 = reinterpret_cast<const uint4 *>(sheet + SHEET_LIST_UP);
+        for (int c = 0; c < chunks; c++) {
+            const uint4 v = (c < skip_chunk ? list4 : up4)[c];
+            unsigned *dst = my + 4 * c * STRIDE;
+            dst[0 * STRIDE] = v.x;
+            dst[1 * STRIDE] = v.y;
+            dst[2 * STRIDE] = v.z;
+            dst[3 * STRIDE] = v.w;
+        }
+        if (skip_chunk < chunks) {
+            const uint4 v = list4[skip_chunk], u = up4[skip_chunk];
+            const unsigned keep = (1u << (8 * (skip & 3))) - 1u;   // the bytes in front of `skip` in its word
+            unsigned *dst = my + 4 * skip_chunk * STRIDE;
+            const int k = skip_word & 3;
+            dst[0 * STRIDE] = k > 0 ? v.x : (v.x & keep) | (u.x & ~keep);
+            dst[1 * STRIDE] = k > 1 ? v.y : (k == 1 ? (v.y & keep) | (u.y & ~keep) : u.y);
+            dst[2 * STRIDE] = k > 2 ? v.z : (k == 2 ? (v.z & keep) | (u.z & ~keep) : u.z);
+            dst[3 * STRIDE] = k == 3 ? (v.w & keep) | (u.w & ~keep) : u.w;
+        }
+        const uint4 *lines4 = reinterpret_cast<const uint4 *>(sheet + TPL_LINES);
+#pragma unroll
+        for (int c = 0; c < LINE_WORDS / 4; c++) {
+            const uint4 l = lines4[c];
+            unsigned *dst = my + (LIST_WORDS + 4 * c) * STRIDE;
+            dst[0 * STRIDE] = l.x;
+            dst[1 * STRIDE] = l.y;
+            dst[2 * STRIDE] = l.z;
+            dst[3 * STRIDE] = l.w;
+        }
+        static_assert(LINE_WORDS % 4 == 2, "the last two line words");
+        my[(LIST_WORDS + LINE_WORDS - 2) * STRIDE] = sheet[TPL_LINES + LINE_WORDS - 2];
+        my[(LIST_WORDS + LINE_WORDS - 1) * STRIDE] = sheet[TPL_LINES + LINE_WORDS - 1];
+        if (child_cell >= 0) {   // the child's own stone, put down by the side that is second to move in the game
+            const int i = child_cell >> 4, j = child_cell & 15;
+            my[(LINE_ROW + i) * STRIDE] |= 0x10000u << j;
+            my[(LINE_COL + j) * STRIDE] |= 0x10000u << i;
+            my[(LINE_DIAG + ((i - j + 14) & 15)) * STRIDE] |= 0x10000u << j;
+            my[(LINE_ANTI + ((i + j) & 15)) * STRIDE] |= 0x10000u << j;
+        }
+    }
+
+    // list and lines are in place
+    __device__ __forceinline__ void begin(int empty, bool old_five, ulonglong2 stream) {
+        left = left_at_start = empty;
+        left_2m64 = (float)empty * RNG_2M64;
+        careful = old_five;
+        s0 = stream.x;
+        s1 = stream.y;
+        largest = 0.f;
+        winner = 0;
+        left_at_end = 0;
+        playing = true;
+        next_draw();
+    }
+
+    // float32 u * int16 count -> float32 (src/mctsnc.py:2061); here (u * 2^64) * (count * 2^-64): the same product, rounded once.
+    // Added to 2^23 with rounding towards zero it leaves the position in the low bits; position <= left <= 225.
+    __device__ __forceinline__ void next_draw() {
+        draw = rng_uniform_times_2p64(s0, s1);
+        const int q = (int)(__float_as_uint(__fadd_rz(__fmul_rn(draw, left_2m64), 8388608.f)) & 0xFFu);
+        at = list_byte(q);
+        next_last = list[list_byte(max(left - 1, 0))];
+        next_cell = list[at];
+    }
+
+    // One ply (src/mctsnc.py:2059-2064): last_action = legal[ord]; legal[ord] = legal[count - 1]; count -= 1 (:2062, :215-217), byte
+    // loads and stores, no read-modify-write of words; then the stone.  Returns whether it makes a run of exactly five.
+    template <bool CAREFUL>
+    __device__ __forceinline__ bool ply(int rep) {
+        const int cell = next_cell;
+        list[at] = (unsigned char)next_last;
+        left--;
+        left_2m64 -= RNG_2M64;   // exact: small integers times 2^-64
+        largest = fmaxf(largest, draw);
+        next_draw();
+        const int i = cell >> 4, j = cell & 15;
+        const unsigned bit_j = 1u << j, bit_i = 1u << i;
+        // the mover's halfwords of the stone's row, column, diagonal and anti-diagonal
+        unsigned char *half = list + 2 * (rep & 1);
+        unsigned short *row = reinterpret_cast<unsigned short *>(half + (LINE_ROW + i) * (4 * STRIDE));
+        unsigned short *col = reinterpret_cast<unsigned short *>(half + (LINE_COL + j) * (4 * STRIDE));
+        unsigned short *diag = reinterpret_cast<unsigned short *>(half + (LINE_DIAG + ((i - cell + 14) & 15)) * (4 * STRIDE));
+        unsigned short *anti = reinterpret_cast<unsigned short *>(half + (LINE_ANTI + ((i + cell) & 15)) * (4 * STRIDE));
+        const unsigned wr = *row | bit_j, wc = *col | bit_i, wd = *diag | bit_j, wa = *anti | bit_j;
+        *row = (unsigned short)wr;
+        *col = (unsigned short)wc;
+        *diag = (unsigned short)wd;
+        *anti = (unsigned short)wa;
+        const unsigned one = lone_bits(fives(wr + (wc << 16))), two = lone_bits(fives(wd + (wa << 16)));
+        if (!CAREFUL) return (one | two) != 0u;
+        const unsigned through_j = (0x1Fu << j) >> 4, through_i = (0x1Fu << i) >> 4;   // starts of the runs that hold the stone
+        return ((one & (through_j | (through_i << 16))) | (two & (through_j | (through_j << 16)))) != 0u;
+    }
+
+    // PLIES plies, or as many as there are
+    template <int PLIES>
+    __device__ __forceinline__ void play() {
+        static_assert(PLIES % 2 == 0 && PLIES <= 32, "the sides take turns with the plies of a block");
+        if (left >= PLIES && !careful) {
+            unsigned wins = 0u;
+#pragma unroll
+            for (int rep = 0; rep < PLIES; rep++)
+                if (ply<false>(rep)) wins |= 1u << rep;
+            if (wins != 0u) {
+                const int rep = __ffs(wins) - 1;
+                winner = 1 + (rep & 1);
+                left_at_end = left + PLIES - 1 - rep;
+                playing = false;
+            }
+        } else {
+#pragma unroll 1
+            for (int rep = 0; rep < PLIES && playing && left > 0; rep++)
+                if (ply<true>(rep)) {
+                    winner = 1 + (rep & 1);
+                    left_at_end = left;
+                    playing = false;
+                }
+        }
+        if (left == 0 || largest >= RNG_2P64) playing = false;
+    }
+
+    // The game is over: its outcome, number of plies and the stream as it left it.  `board` is the position it began from, `start`
+    // where its stream began.
+    template <bool LOCAL>
+    __device__ __forceinline__ int close(const unsigned *board, int first_mover, const ulonglong2 *start, TreeState *st, int &plies) {
+        if (largest >= RNG_2P64) {
+            // u == 1.0f in the game or in the plies behind its end: played again by the byte-level emulation of the reference
+            const ulonglong2 stream = load<LOCAL>(start);
+            const EmuResult er = playout_emulated(board, first_mover, stream.x, stream.y);
+            s0 = er.s0;
+            s1 = er.s1;
+            plies = (int)er.plies;
+            if (er.ub) {
+                atomicAdd(&st->ub_draws, (unsigned long long)er.ub);
+                atomicOr(&st->status, STATUS_UB_DRAW);
+            }
+            if (er.err) atomicOr(&st->status, STATUS_INTERNAL);
+            return er.outcome;
+        }
+        for (int k = left_at_end - left; k >= 0; k--) rng_back(s0, s1);   // one draw ahead, and the plies behind the end
+        plies = left_at_start - left_at_end;
+        return winner == 0 ? 0 : (winner == 1 ? first_mover : -first_mover);
+    }
+};
 
 // ---------------------------------------------------------------------------------------------------------------
-// The playouts, with games handed out to lanes one by one: a persistent grid of DYN_THREADS-thread blocks; every warp
-// works through the games of one tree's step (game = active child * P + t, taken with one atomicAdd per refill by
-// the warp's idle lanes together), then moves on to the next tree that still has games.  A lane that finishes its game
-// waits until at least REFILL_MIN lanes of its warp are idle (a refill costs a few hundred instructions, mostly the copy
-// of the legal-action list; doing it for several lanes at once keeps it a small fraction of the playing).  Which lane
-// plays a game does not matter: game (child, t) draws from the stream of the reference's thread (tree, action, t).
-// Per warp a copy of the parent position (Params::tpl) sits in shared memory; a child's list is the parent's without the
-// child's own cell (the reference builds it by scanning the child's board in ascending order).
+// ACP variants (and OCP with more trees than fit on the device as blocks): a step is two launches that the host enqueues
+// without waiting.
+template <bool OCP>
+__global__ void __launch_bounds__(32) tree_step_kernel(const __grid_constant__ Params p) {
+    __shared__ __align__(16) unsigned sheet[SHEET_WORDS];
+    const int lane = threadIdx.x, tree = p.tree_base + (int)blockIdx.x;
+    Walker<OCP, false> w(p, sheet, tree, lane);
+    if (p.first != 0) w.reset();
+    w.backup();
+    if (p.backup_only != 0) return;
+    const int n_active = w.advance();
+    unsigned *out = p.sheet + (long long)tree * SHEET_WORDS;
+    for (int i = lane; i < SHEET_WORDS; i += 32) out[i] = sheet[i];
+    if (lane == 0) {
+        p.work[tree].games = n_active * p.n_playouts;
+        p.work[tree].taken = 0;
+    }
+}
+
+// The games of a step, handed out to lanes one by one: every warp works through the games of one tree's step (game = active child * P
+// + t, taken by the warp's idle lanes together), then moves on to the next tree that still has games.  Game (child, t) draws
+// from the stream of the reference's thread (tree, action, t) whichever lane plays it.  A lane that finishes its game waits
+// until at least REFILL_MIN lanes of its warp are idle: closing games and taking new ones costs a few hundred instructions,
+// for one lane or for many.
 //
 // Per-thread game state lives in shared memory, laid out so that every thread owns one bank column: word k of thread t
-// is s_mem[k * DYN_THREADS + t].  That state (476 bytes) decides how many games an SM plays at once: two blocks of 224
-// threads.  With so few warps the kernel is bound by the latency of a warp's own instruction chain, not by issue
-// slots, which is what the choices below answer (Gomoku 15x15 acp_prodigal 4 x 256, 500 steps, one / eight searches,
-// M playouts/s): a look at idle lanes after every ply 765 / 769, every 2nd 941 / 980, 4th 1004 / 1058, 8th 1053 / 1129
-// (a lane whose game has ended sits out the plies up to the next look); refills for at least 4 idle lanes 1156 / 1429,
-// 6: 1164 / 1485, 8: 1170 / 1500, 12: 1167 / 1478; blocks of 448 threads 1163 / 1434, of 128 threads (three per SM) slower.
+// is s_mem[k * DYN_THREADS + t].  That state (476 bytes) decides how many games an SM plays at once: 14 warps, so what counts is
+// the length of a ply: its instructions and their chain (see Game).
 #ifndef MCTSNC_GOMOKU_REFILL_MIN
 #define MCTSNC_GOMOKU_REFILL_MIN 8
 #endif
@@ -660,169 +859,94 @@ constexpr int REFILL_MIN = MCTSNC_GOMOKU_REFILL_MIN;
 #define MCTSNC_GOMOKU_PLIES_PER_LOOK 8
 #endif
 constexpr int PLIES_PER_LOOK = MCTSNC_GOMOKU_PLIES_PER_LOOK;   // plies between two looks at whether lanes are idle
-#ifndef MCTSNC_GOMOKU_UNROLL
-#define MCTSNC_GOMOKU_UNROLL 8
-#endif
-constexpr int PLY_COPIES = MCTSNC_GOMOKU_UNROLL;   // copies of the ply's code in the loop between two looks
 #ifndef MCTSNC_GOMOKU_THREADS
 #define MCTSNC_GOMOKU_THREADS 224
 #endif
 constexpr int DYN_THREADS = MCTSNC_GOMOKU_THREADS;
-// per warp: the parent position and, behind it, the ranks of the children that are played out (one byte each)
-constexpr int WARP_ACTIVE = TPL_WORDS, WARP_WORDS = TPL_WORDS + 60;
-constexpr size_t DYN_SMEM_BYTES = sizeof(unsigned) * ((size_t)THREAD_WORDS * DYN_THREADS + (size_t)WARP_WORDS * (DYN_THREADS / 32)) + FIVE_BYTES;
-static_assert((THREAD_WORDS * DYN_THREADS) % 4 == 0 && WARP_WORDS % 4 == 0 && TPL_LINES % 4 == 0, "16-byte loads of the warp's copy");
-
-// byte offset of list entry q of a thread from the thread's word 0: byte q & 3 of word q >> 2, words DYN_THREADS apart;
-// (q >> 2) * 4 * DYN_THREADS + (q & 3) written as one shift and one multiply-add
-__device__ __forceinline__ int list_byte(int q) { return (q >> 2) * (4 * DYN_THREADS - 4) + q; }
+constexpr size_t DYN_SMEM_BYTES = sizeof(unsigned) * ((size_t)THREAD_WORDS * DYN_THREADS + (size_t)SHEET_WORDS * (DYN_THREADS / 32));
+static_assert((THREAD_WORDS * DYN_THREADS) % 4 == 0 && SHEET_WORDS % 4 == 0 && TPL_LINES % 4 == 0, "16-byte loads of the sheet");
 
 template <bool OCP>
-__global__ void __launch_bounds__(DYN_THREADS) playout_dynamic_kernel(const Params p, int total_trees) {
+__global__ void __launch_bounds__(DYN_THREADS) playout_dynamic_kernel(const __grid_constant__ Params p, int total_trees) {
     extern __shared__ __align__(16) unsigned s_mem[];
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
     const int P = p.n_playouts;
     int log2p = 0;
     while ((1 << log2p) < P) log2p++;
-    unsigned *my = s_mem + tid;                                                     // word k of this thread: my[k * DYN_THREADS]
-    unsigned *tpl = s_mem + THREAD_WORDS * DYN_THREADS + warp * WARP_WORDS;         // this warp's copy of the parent position
-    const unsigned char *tpl_bytes = reinterpret_cast<const unsigned char *>(tpl + TPL_LIST);
-    unsigned char *act_bytes = reinterpret_cast<unsigned char *>(tpl + WARP_ACTIVE);
-    unsigned char *s_five = reinterpret_cast<unsigned char *>(s_mem + THREAD_WORDS * DYN_THREADS + WARP_WORDS * (DYN_THREADS / 32));
-    for (int window = tid; window < FIVE_BYTES; window += DYN_THREADS) {
-        int above = 0, below = 0;
-        while (above < 5 && ((window >> (6 + above)) & 1)) above++;
-        while (below < 5 && ((window >> (4 - below)) & 1)) below++;
-        s_five[window] = above + below == 4 ? 1 : 0;
-    }
-    __syncthreads();
+    unsigned *sheet = s_mem + THREAD_WORDS * DYN_THREADS + warp * SHEET_WORDS;   // this warp's copy of a tree's sheet
+    const unsigned char *list_bytes = reinterpret_cast<const unsigned char *>(sheet + TPL_LIST);
+    const unsigned char *active = reinterpret_cast<const unsigned char *>(sheet + SHEET_ACTIVE);
+    // what the backup of the step needs and the games do not wait for
+    if (warp == 0)
+        for (int t = blockIdx.x; t < total_trees; t += gridDim.x) Walker<OCP, false>(p, nullptr, p.tree_base + t, lane).prepare();
     int tree = p.tree_base + (int)(((long long)blockIdx.x * (DYN_THREADS / 32) + warp) % total_trees);
     int tried = 0;
-    bool have_tpl = false, exhausted = false;
-    // warp-uniform description of the current tree's step
-    int n_items = 0, mode = 0, sel_turn = 0, count0 = 0, first_child = 0, selected = 0;
+    bool have_sheet = false, exhausted = false;
+    int n_items = 0;          // games of the current tree's step
     // per-lane game (a lane may still be playing a game of an earlier tree after the warp has moved on)
-    bool playing = false;
-    int count = 0, turn = 0, action = 0, node = 0, my_tree = 0, my_start_turn = 0;
-    int ord = 0;              // the draw of the ply to come, already turned into a position of the list
-    int next_cell = 0, next_last = 0;   // list entries at that position and at the end of the list
-    float count_2m64 = 0.f;   // count * 2^-64, the factor of the draws scaled by 2^64
+    Game<DYN_THREADS> game;
+    game.list = reinterpret_cast<unsigned char *>(s_mem + tid);
+    game.playing = false;
+    bool has_game = false;    // going on, or over and not closed yet
+    int first_mover = 0, action = 0, node = 0, my_tree = 0;
     long long rng_idx = 0;
-    unsigned long long s0 = 0, s1 = 0, start0 = 0, start1 = 0;
-    unsigned plies = 0;
     for (;;) {
-        if (!have_tpl) {
-            // ---- describe the tree's step; fetch the parent position
-            const StepInfo si = p.step[tree];
-            mode = si.mode;
-            n_items = si.n_active << log2p;
-            selected = si.selected;
-            first_child = si.first_child;
-            sel_turn = g_turn(si.sel_meta);
-            count0 = si.n_empty;
+        if (!have_sheet) {
             int taken = 0;   // read by one lane, so that the whole warp sees the same value
-            if (lane == 0) taken = *(volatile int *)&p.step[tree].game_counter;
+            n_items = p.work[tree].games;
+            if (lane == 0) taken = *(volatile int *)&p.work[tree].taken;
             taken = __shfl_sync(0xFFFFFFFFu, taken, 0);
-            exhausted = n_items == 0 || taken >= n_items;
+            exhausted = taken >= n_items;
             if (!exhausted) {
                 __syncwarp();   // lanes of an earlier refill are done with the copy
-                const unsigned *src = p.tpl + (long long)tree * TPL_WORDS;
-                for (int w = lane; w < TPL_WORDS; w += 32) tpl[w] = src[w];
-                const unsigned char *ranks = p.active_rank + tree * A;
-                for (int k = lane; k < si.n_active; k += 32) act_bytes[k] = ranks[k];
+                const unsigned *src = p.sheet + (long long)tree * SHEET_WORDS;
+#pragma unroll
+                for (int i = 0; i < SHEET_WORDS; i += 32) sheet[i + lane] = src[i + lane];
                 __syncwarp();
             }
-            have_tpl = true;
+            have_sheet = true;
+        }
+        // ---- a look
+        const unsigned idle = __ballot_sync(0xFFFFFFFFu, !game.playing);
+        const int n_idle = __popc(idle);
+        if (has_game && !game.playing && (exhausted || n_idle >= REFILL_MIN || idle == 0xFFFFFFFFu)) {
+            has_game = false;
+            int plies;
+            const int outcome = game.template close<false>(p.board + ((long long)my_tree * p.cap + node) * 16, first_mover, p.rng_playout + rng_idx,
+                                                           p.state + my_tree, plies);
+            p.rng_playout[rng_idx] = make_ulonglong2(game.s0, game.s1);
+            if (outcome != 0) atomicAdd(outcome > 0 ? &p.child_out[my_tree * A + action].y : &p.child_out[my_tree * A + action].x, 1);
+            atomicAdd(&p.state[my_tree].plies, (unsigned long long)plies);
         }
         // ---- refill: idle lanes take games together
-        const unsigned idle = __ballot_sync(0xFFFFFFFFu, !playing);
-        const int n_idle = __popc(idle);
-        if (!exhausted && (n_idle >= REFILL_MIN || idle == 0xFFFFFFFFu) && n_idle > 0) {
+        if (!exhausted && (n_idle >= REFILL_MIN || idle == 0xFFFFFFFFu)) {
             int base = 0;
             const int leader = __ffs(idle) - 1;
-            if (lane == leader) base = atomicAdd(&p.step[tree].game_counter, n_idle);
+            if (lane == leader) base = atomicAdd(&p.work[tree].taken, n_idle);
             base = __shfl_sync(0xFFFFFFFFu, base, leader);
             if (base + n_idle >= n_items) exhausted = true;
             const int item = base + __popc(idle & ((1u << lane) - 1u));
-            if (!playing && item < n_items) {
+            if (!game.playing && item < n_items) {
                 const int t = item & (P - 1);
-                int skip = 1 << 30;   // position of the parent's list that the child's list leaves out
-                int cell = 0;
-                if (mode == MODE_ALL_CHILDREN) {
-                    const int rank = act_bytes[item >> log2p];
-                    cell = tpl_bytes[rank];              // children are the first empty cells in ascending order
+                const bool child = (int)sheet[SHEET_MODE] == MODE_ALL_CHILDREN;
+                const int empty = (int)sheet[SHEET_EMPTY];
+                int skip = Game<DYN_THREADS>::NO_SKIP, cell = -1;
+                action = 0;   // the selected node itself is played out with the streams of action 0
+                node = (int)sheet[SHEET_SELECTED];
+                if (child) {
+                    skip = active[item >> log2p];   // rank of the child: children are the first empty cells in ascending order
+                    cell = list_bytes[skip];
                     action = (cell >> 4) * N + (cell & 15);
-                    skip = rank;
-                    node = first_child + rank;
-                    count = count0 - 1;
-                    turn = -sel_turn;
-                } else {   // the selected node itself is played out, with the streams of action 0
-                    action = 0;
-                    node = selected;
-                    count = count0;
-                    turn = sel_turn;
+                    node = (int)sheet[SHEET_FIRST_CHILD] + skip;
                 }
+                first_mover = (int)sheet[SHEET_FIRST_MOVER];
                 rng_idx = OCP ? ((long long)tree * P + t) : (((long long)tree * A + action) * P + t);
                 const ulonglong2 rs = p.rng_playout[rng_idx];   // on its way while the position is copied
-                // the child's list: the parent's without position `skip`.  Four words at a time; a word behind the one that
-                // holds `skip` takes its bytes one position further up (a funnel shift by 0 or 8 bits), the word that holds
-                // it is put right afterwards.  Words past the last entry are never read; up to three words past the list
-                // are written and then covered by the lines.
-                const int skip_word = skip >> 2;
-                const int chunks = (count0 + 15) >> 4;
-                const uint4 *tpl_list4 = reinterpret_cast<const uint4 *>(tpl + TPL_LIST);
-                uint4 v = tpl_list4[0];
-                for (int c = 0; c < chunks; c++) {
-                    const uint4 nx = tpl_list4[c + 1];   // c + 1 <= 15: the lines follow the list in the warp's copy
-                    const int d = skip_word - 4 * c;
-                    unsigned *dst = my + 4 * c * DYN_THREADS;
-                    dst[0 * DYN_THREADS] = __funnelshift_r(v.x, v.y, d < 0 ? 8 : 0);
-                    dst[1 * DYN_THREADS] = __funnelshift_r(v.y, v.z, d < 1 ? 8 : 0);
-                    dst[2 * DYN_THREADS] = __funnelshift_r(v.z, v.w, d < 2 ? 8 : 0);
-                    dst[3 * DYN_THREADS] = __funnelshift_r(v.w, nx.x, d < 3 ? 8 : 0);
-                    v = nx;
-                }
-                if (skip_word < LIST_WORDS) {
-                    const unsigned prev = tpl[TPL_LIST + skip_word], next = tpl[TPL_LIST + skip_word + 1];
-                    const unsigned keep = (1u << (8 * (skip & 3))) - 1u;
-                    my[skip_word * DYN_THREADS] = (prev & keep) | (__funnelshift_r(prev, next, 8) & ~keep);
-                }
-                const uint4 *tpl_lines4 = reinterpret_cast<const uint4 *>(tpl + TPL_LINES);
-#pragma unroll
-                for (int c = 0; c < LINE_WORDS / 4; c++) {
-                    const uint4 l = tpl_lines4[c];
-                    unsigned *dst = my + (LIST_WORDS + 4 * c) * DYN_THREADS;
-                    dst[0 * DYN_THREADS] = l.x;
-                    dst[1 * DYN_THREADS] = l.y;
-                    dst[2 * DYN_THREADS] = l.z;
-                    dst[3 * DYN_THREADS] = l.w;
-                }
-                static_assert(LINE_WORDS % 4 == 2, "the last two line words");
-                my[(LIST_WORDS + LINE_WORDS - 2) * DYN_THREADS] = tpl[TPL_LINES + LINE_WORDS - 2];
-                my[(LIST_WORDS + LINE_WORDS - 1) * DYN_THREADS] = tpl[TPL_LINES + LINE_WORDS - 1];
-                if (mode == MODE_ALL_CHILDREN) {   // the child's own stone, put down by the side to move at the parent
-                    const int i = cell >> 4, j = cell & 15;
-                    const int hs = sel_turn > 0 ? 16 : 0;
-                    my[(LINE_ROW + i) * DYN_THREADS] |= 1u << (hs + j);
-                    my[(LINE_COL + j) * DYN_THREADS] |= 1u << (hs + i);
-                    my[(LINE_DIAG + ((i - j + 14) & 15)) * DYN_THREADS] |= 1u << (hs + j);
-                    my[(LINE_ANTI + ((i + j) & 15)) * DYN_THREADS] |= 1u << (hs + j);
-                }
-                count_2m64 = (float)count * RNG_2M64;
+                game.copy_position(sheet, empty, skip, cell);
+                game.begin(child ? empty - 1 : empty, sheet[SHEET_OLD_FIVE] != 0u, rs);
                 my_tree = tree;
-                my_start_turn = turn;
-                s0 = start0 = rs.x;
-                s1 = start1 = rs.y;
-                ord = __float2int_rz(__fmul_rn(rng_uniform_times_2p64(s0, s1), count_2m64));   // the draw of the first ply
-                {
-                    const unsigned char *list = reinterpret_cast<const unsigned char *>(my);
-                    const int q_last = max(count - 1, 0);
-                    next_last = list[list_byte(q_last)];
-                    next_cell = list[list_byte(ord)];
-                }
-                plies = 0;
-                playing = true;
+                has_game = true;
             }
         }
         if (exhausted) {
@@ -832,81 +956,108 @@ __global__ void __launch_bounds__(DYN_THREADS) playout_dynamic_kernel(const Para
             if (tried + 1 < total_trees) {
                 tried++;
                 tree = tree + 1 == p.tree_base + total_trees ? p.tree_base : tree + 1;
-                have_tpl = false;
+                have_sheet = false;
                 continue;
             }
-            if (__ballot_sync(0xFFFFFFFFu, playing) == 0u) break;
+            if (__ballot_sync(0xFFFFFFFFu, has_game) == 0u) break;
         }
-#pragma unroll(PLY_COPIES)
-        for (int rep = 0; rep < PLIES_PER_LOOK; rep++) {
-          if (playing) {
-            // ---- one ply (src/mctsnc.py:2059-2064).  float32 u * int16 count -> float32 (:2061); here (u * 2^64) * (count * 2^-64):
-            // the same product, rounded once.  u == 1.0f gives ord == count.  The draw of a ply is made one ply ahead, next to
-            // the work of the ply before it, so that the chain of dependent steps of a ply starts at the list; if the game ends
-            // with this ply, the stream is stored as it was before the draw for the next one.
-            const int this_ord = ord;
-            unsigned long long end0 = s0, end1 = s1;   // the stream after the draw of this ply
-            ord = __float2int_rz(__fmul_rn(rng_uniform_times_2p64(s0, s1), count_2m64 - RNG_2M64));
-            int outcome = 2;
-            if (this_ord >= count) {
-                // u == 1.0f: replay this game through the byte-level emulation of the reference
-                const EmuResult er = playout_emulated(p.board + ((long long)my_tree * p.cap + node) * 16, my_start_turn, start0, start1);
-                end0 = er.s0;
-                end1 = er.s1;
-                outcome = er.outcome;
-                plies = er.plies;
-                TreeState *st = p.state + my_tree;
-                atomicAdd(&st->ub_draws, (unsigned long long)er.ub);
-                atomicOr(&st->status, STATUS_UB_DRAW | (er.err ? STATUS_INTERNAL : 0u));
-            } else {
-                // last_action = legal[ord]; legal[ord] = legal[count - 1]; count -= 1   (:2062, :215-217).  List entry q of this
-                // thread is byte q & 3 of its word q >> 2: byte loads and stores, no read-modify-write of words.  The two
-                // entries a ply reads were fetched at the end of the ply before (after its store); here the two of the next
-                // ply are fetched, so that they arrive while this ply's stone is tested.
-                unsigned char *list = reinterpret_cast<unsigned char *>(my);
-                const int cell = next_cell;
-                list[list_byte(this_ord)] = (unsigned char)next_last;
-                count--;
-                count_2m64 -= RNG_2M64;   // exact: small integers times 2^-64
-                const int q_last = max(count - 1, 0);
-                next_last = list[list_byte(q_last)];
-                next_cell = list[list_byte(ord)];   // ord <= count <= 225: inside the list words
-                const int i = cell >> 4, j = cell & 15;
-                const int hs = turn > 0 ? 16 : 0;
-                plies++;
-                // compute_outcome_gomoku (src/mctsnc_game_mechanics.py:220-272) without loops: the stone goes into the word of
-                // its row, column, diagonal and anti-diagonal; of each word the mover's half is rotated so that the new
-                // stone sits at bit 5, and the 11 bits around it index the table.  The bits of the half never wrap into the
-                // window: rotating right by s = hs + pos - 5, a bit b < s lands at 32 - s + b >= 23 (low half: s <= 9; high
-                // half: b >= 16, s <= 25), and a negative s is a shift of the low half to the left by at most 5.
-                const unsigned half = 0x7FFFu << hs;
-                const unsigned bit_j = 1u << (hs + j), bit_i = 1u << (hs + i);
-                const int rot_j = hs + j - 5, rot_i = hs + i - 5;   // the funnel shift takes them modulo 32
-                unsigned *row_w = my + (LINE_ROW + i) * DYN_THREADS;
-                unsigned *col_w = my + (LINE_COL + j) * DYN_THREADS;
-                unsigned *diag_w = my + (LINE_DIAG + ((i - j + 14) & 15)) * DYN_THREADS;
-                unsigned *anti_w = my + (LINE_ANTI + ((i + j) & 15)) * DYN_THREADS;
-                const unsigned wr = *row_w | bit_j, wc = *col_w | bit_i, wd = *diag_w | bit_j, wa = *anti_w | bit_j;
-                *row_w = wr;
-                *col_w = wc;
-                *diag_w = wd;
-                *anti_w = wa;
-                const unsigned tr = wr & half, tc = wc & half, td = wd & half, ta = wa & half;
-                const unsigned win = s_five[__funnelshift_r(tr, tr, rot_j) & 0x7FFu] | s_five[__funnelshift_r(tc, tc, rot_i) & 0x7FFu] |
-                                     s_five[__funnelshift_r(td, td, rot_j) & 0x7FFu] | s_five[__funnelshift_r(ta, ta, rot_j) & 0x7FFu];
-                if (win) outcome = turn;
-                else if (count == 0) outcome = 0;
-                turn = -turn;
-            }
-            if (outcome != 2) {
-                p.rng_playout[rng_idx] = make_ulonglong2(end0, end1);
-                if (outcome != 0) atomicAdd(&p.child_out[(my_tree * A + action) * 2 + (outcome > 0 ? 1 : 0)], 1);
-                atomicAdd(&p.state[my_tree].plies, (unsigned long long)plies);
-                playing = false;
-            }
-          }
-        }
+        if (game.playing) game.template play<PLIES_PER_LOOK>();
     }
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// The whole search of one tree in one block, for the OCP variants (one child played out per step: P games) where every tree has
+// room on the device at once: a step is as long as its longest game (about 180 plies).  Warp 0 walks, the other STRIDE threads
+// play; what a step hands over stays in shared memory, as do the random streams.
+// One search, 8 trees x 128 playouts, 300 steps: 19.0 ms with two launches a step (63 us, 31 of them the games), 5.9 ms so.
+#ifndef MCTSNC_GOMOKU_BLOCK_PLIES
+#define MCTSNC_GOMOKU_BLOCK_PLIES 8
+#endif
+constexpr int BLOCK_PLIES = MCTSNC_GOMOKU_BLOCK_PLIES;
+template <int STRIDE>
+struct BlockMemory {
+    unsigned sheet[SHEET_WORDS];
+    ulonglong2 streams[512];
+    int2 tally;               // of the child that is played out
+    int n_active, pad;
+    unsigned long long plies;
+    unsigned columns[THREAD_WORDS * STRIDE];
+};
+
+// blocks that shared memory lets on an SM (registers follow)
+constexpr int blocks_per_sm(int stride) { return stride == 32 ? 8 : (stride == 64 ? 5 : (stride == 128 ? 3 : 1)); }
+
+template <int STRIDE>
+__global__ void __launch_bounds__(STRIDE + 32, blocks_per_sm(STRIDE)) search_block_kernel(const __grid_constant__ Params p) {
+    extern __shared__ __align__(16) unsigned s_mem[];
+    BlockMemory<STRIDE> &b = *reinterpret_cast<BlockMemory<STRIDE> *>(s_mem);
+    const int lane = (int)threadIdx.x & 31;
+    const int player = (int)threadIdx.x - 32;   // < 0: the walker
+    const int g = (int)blockIdx.x;
+    const int P = p.n_playouts;
+    for (int i = threadIdx.x; i < P; i += STRIDE + 32) b.streams[i] = p.rng_playout[(long long)g * P + i];
+    for (int i = threadIdx.x; i < SHEET_WORDS; i += STRIDE + 32) b.sheet[i] = 0u;
+    if (threadIdx.x == 0) b.plies = 0;
+    __syncthreads();
+    Walker<true, true> w(p, b.sheet, g, lane);
+    Game<STRIDE> game;
+    game.list = reinterpret_cast<unsigned char *>(b.columns + (player < 0 ? 0 : player));
+    unsigned my_plies = 0;
+    int left = p.steps;
+    if (player < 0 && p.first != 0) w.reset();
+    for (;;) {
+        if (player < 0) {
+            int n_active = 0;
+            for (;;) {
+                w.backup();
+                if (left == 0) break;
+                n_active = w.advance();
+                left--;
+                if (n_active > 0) break;
+                w.prepare();   // nothing to play: the backup follows at once
+            }
+            if (lane == 0) {
+                b.n_active = n_active;
+                b.tally = make_int2(0, 0);
+            }
+        }
+        __syncthreads();
+        if (b.n_active == 0) break;
+        const bool child = (int)b.sheet[SHEET_MODE] == MODE_ALL_CHILDREN;
+        const int skip = child ? reinterpret_cast<const unsigned char *>(b.sheet + SHEET_ACTIVE)[0] : Game<STRIDE>::NO_SKIP;
+        const int cell = child ? reinterpret_cast<const unsigned char *>(b.sheet + TPL_LIST)[skip] : -1;
+        if (player < 0) {
+            w.prepare();
+        } else {
+            const int first_mover = (int)b.sheet[SHEET_FIRST_MOVER], empty = (int)b.sheet[SHEET_EMPTY];
+            const int node = child ? (int)b.sheet[SHEET_FIRST_CHILD] + skip : (int)b.sheet[SHEET_SELECTED];
+            for (int base = 0; base < P; base += STRIDE) {
+                // the games of a warp are played to their ends together and closed together
+                const int item = base + player;
+                if (item < P) {
+                    game.copy_position(b.sheet, empty, skip, cell);
+                    game.begin(child ? empty - 1 : empty, b.sheet[SHEET_OLD_FIVE] != 0u, b.streams[item]);
+                    while (game.playing) game.template play<BLOCK_PLIES>();
+                }
+                __syncwarp();
+                if (item < P) {
+                    int plies;
+                    const int outcome = game.template close<true>(p.board + ((long long)g * p.cap + node) * 16, first_mover, &b.streams[item],
+                                                                  p.state + g, plies);
+                    b.streams[item] = make_ulonglong2(game.s0, game.s1);
+                    if (outcome != 0) atomicAdd(outcome > 0 ? &b.tally.y : &b.tally.x, 1);
+                    my_plies += (unsigned)plies;
+                }
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) p.child_out[(long long)g * A + (child ? (cell >> 4) * N + (cell & 15) : 0)] = b.tally;
+        __syncwarp();
+    }
+    if (my_plies) atomicAdd(&b.plies, (unsigned long long)my_plies);
+    __syncthreads();
+    for (int i = threadIdx.x; i < P; i += STRIDE + 32) p.rng_playout[(long long)g * P + i] = b.streams[i];
+    if (threadIdx.x == 0) p.state[g].plies += b.plies;
 }
 
 }  // namespace gomoku

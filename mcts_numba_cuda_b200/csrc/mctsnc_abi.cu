@@ -22,6 +22,7 @@ using namespace mctsnc;
 
 namespace {
 
+constexpr int GOMOKU_STREAMS = 8;     // tree groups of a Gomoku search launch that run out of step with each other
 constexpr int MAX_TREE_DEPTH = 2048;  // src/mctsnc.py:197
 #ifndef MCTSNC_C4_CLUSTER_MIN_GAMES
 #define MCTSNC_C4_CLUSTER_MIN_GAMES 256    // Connect 4: clusters only for steps with more games than this
@@ -32,8 +33,6 @@ constexpr int MAX_TREE_DEPTH = 2048;  // src/mctsnc.py:197
 #ifndef MCTSNC_C4_CLUSTER_SM_SHARE
 #define MCTSNC_C4_CLUSTER_SM_SHARE 4   // Connect 4: clusters of blocks per tree while they make at most this many blocks per SM
 #endif
-constexpr int GOMOKU_STREAMS = 8;     // tree groups of a Gomoku search launch that run out of step with each other
-
 #define CUDA_TRY(expr)                        \
     do {                                      \
         cudaError_t _e = (expr);              \
@@ -103,11 +102,12 @@ struct mctsnc_handle {
     // Gomoku only
     unsigned *gboard = nullptr;           // [trees][cap][16]
     gomoku::StepInfo *gstep = nullptr;    // [trees]
-    unsigned *gtpl = nullptr;             // [trees][gomoku::TPL_WORDS]
-    int *path_ns = nullptr, *path_wins = nullptr;
+    unsigned *gsheet = nullptr;           // [trees][gomoku::SHEET_WORDS]
+    int4 *path_rec = nullptr;             // [trees][PATH_CAP]
+    PathTerm *path_term = nullptr;        // [trees][PATH_CAP]
     signed char *child_outcome = nullptr;
     unsigned char *child_action = nullptr;
-    unsigned char *active_rank = nullptr;
+    gomoku::StepGames *gwork = nullptr;   // [trees]
     unsigned *root_gboard = nullptr;      // [max_batch][16]
     unsigned *h_root_gboard = nullptr;
     // [max_batch] results, [max_batch][3A] sums, [max_batch][2A] flags (win flags, expanded-at-root) in one piece of memory
@@ -494,12 +494,12 @@ void release(mctsnc_handle *h) {
     cudaFree(h->trace_count);
     cudaFree(h->gboard);
     cudaFree(h->gstep);
-    cudaFree(h->gtpl);
-    cudaFree(h->path_ns);
-    cudaFree(h->path_wins);
+    cudaFree(h->gsheet);
+    cudaFree(h->path_rec);
+    cudaFree(h->path_term);
+    cudaFree(h->gwork);
     cudaFree(h->child_outcome);
     cudaFree(h->child_action);
-    cudaFree(h->active_rank);
     cudaFree(h->root_gboard);
     cudaFreeHost(h->h_root_gboard);
     cudaFree(h->dres);
@@ -610,14 +610,29 @@ int stage_roots(mctsnc_handle *h, int batch, const int8_t *boards, const int8_t 
     return send_roots(h, h->root_board, h->h_root_board, sizeof(ulonglong2) * batch, batch, stream);
 }
 
-// Gomoku: two launches per step (tree step, playouts) and a closing backup, all enqueued without waiting.
-//
-// The trees are split into groups, each with a stream of its own: a tree's next step only needs that tree's games to be
-// over, so the groups run out of step with each other and the lanes one tree leaves idle while its longest games finish
-// (up to ~170 plies against a mean of ~85) play the games of the others.  Every playout launch asks for enough blocks
-// for all its games at once; blocks whose warps find no game left return at once and make room for the blocks of the
-// other groups' launches, so the device is shared by whatever games exist at the moment.  No kernel waits for another:
-// the order inside a group is stream order, the groups are forked from and joined to the caller's stream with events.
+// The kernel that runs an OCP search of Gomoku with a block per tree, its threads and dynamic shared memory: a player for every
+// game of a step up to 256
+const void *gomoku_block_kernel(int playouts, int *threads, size_t *smem) {
+    if (playouts <= 32) {
+        *threads = 32 + 32;
+        *smem = sizeof(gomoku::BlockMemory<32>);
+        return (const void *)gomoku::search_block_kernel<32>;
+    }
+    if (playouts <= 64) {
+        *threads = 64 + 32;
+        *smem = sizeof(gomoku::BlockMemory<64>);
+        return (const void *)gomoku::search_block_kernel<64>;
+    }
+    if (playouts <= 128) {
+        *threads = 128 + 32;
+        *smem = sizeof(gomoku::BlockMemory<128>);
+        return (const void *)gomoku::search_block_kernel<128>;
+    }
+    *threads = 256 + 32;
+    *smem = sizeof(gomoku::BlockMemory<256>);
+    return (const void *)gomoku::search_block_kernel<256>;
+}
+
 int launch_search_gomoku(mctsnc_handle *h, int batch, int steps, int first, cudaStream_t stream) {
     gomoku::Params p;
     p.rec = h->rec;
@@ -626,28 +641,51 @@ int launch_search_gomoku(mctsnc_handle *h, int batch, int steps, int first, cuda
     p.state = h->state;
     p.step = h->gstep;
     p.paths = h->paths;
-    p.path_ns = h->path_ns;
-    p.path_wins = h->path_wins;
+    p.path_rec = h->path_rec;
+    p.term = h->path_term;
     p.actions_expanded = h->actions_expanded;
-    p.child_out = h->child_out;
+    p.child_out = reinterpret_cast<int2 *>(h->child_out);
     p.child_outcome = h->child_outcome;
     p.child_action = h->child_action;
-    p.active_rank = h->active_rank;
-    p.tpl = h->gtpl;
+    p.sheet = h->gsheet;
     p.rng_playout = h->rng_playout;
     p.rng_expand = h->rng_expand;
     p.root_board = h->root_gboard;
     p.root_turn = h->root_turn;
+    p.work = h->gwork;
     p.cap = h->cfg.node_capacity;
     p.node_limit = h->cfg.max_tree_size < h->cfg.node_capacity ? h->cfg.max_tree_size : h->cfg.node_capacity;
     p.n_trees = h->cfg.n_trees;
     p.n_playouts = h->cfg.n_playouts;
     p.variant = h->cfg.variant;
+    p.first = first;
+    p.steps = steps;
     p.ucb_c = h->cfg.ucb_c;
     p.ms_per_cycle = h->ms_per_cycle;
     const int trees = (int)((long long)batch * h->cfg.n_trees);
+    p.tree_base = 0;
+    p.backup_only = 0;
     const bool ocp = is_ocp(h->cfg);
-    // resident playout blocks: three per SM (limited by shared memory)
+    void *args[] = {&p};
+    if (ocp) {
+        // a block per tree while all of them are on the device at once
+        int threads = 0, fit = 0;
+        size_t smem = 0;
+        const void *kernel = gomoku_block_kernel(p.n_playouts, &threads, &smem);
+        CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kernel, threads, smem) == cudaSuccess &&
+            trees <= (long long)fit * h->sm_count) {
+            h->threads = threads;
+            h->blocks_per_sm = fit;
+            return (int)cudaLaunchKernel(kernel, dim3((unsigned)trees), dim3((unsigned)threads), args, smem, stream);
+        }
+    }
+    // Else two launches per step (tree step, playouts) and a closing backup, all enqueued without waiting.
+    //
+    // The trees are split into groups, each with a stream of its own: a tree's next step only needs that tree's games to be
+    // over, so the groups run out of step with each other and the lanes one tree leaves idle while its longest games finish
+    // (up to ~170 plies against a mean of ~85) play the games of the others.  No kernel waits for another: the order inside a
+    // group is stream order, the groups are forked from and joined to the caller's stream with events.
     int per_sm = 0;
     const void *pk = ocp ? (const void *)gomoku::playout_dynamic_kernel<true> : (const void *)gomoku::playout_dynamic_kernel<false>;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pk, gomoku::DYN_THREADS, h->dyn_smem) != cudaSuccess || per_sm < 1) per_sm = 1;
@@ -665,15 +703,13 @@ int launch_search_gomoku(mctsnc_handle *h, int batch, int steps, int first, cuda
             const int n = t1 - t0;
             p.tree_base = t0;
             cudaStream_t gs = h->g_stream[g];
-            if (ocp) gomoku::tree_step_kernel<true><<<n, 256, 0, gs>>>(p);
-            else gomoku::tree_step_kernel<false><<<n, 256, 0, gs>>>(p);
+            if (ocp) gomoku::tree_step_kernel<true><<<n, 32, 0, gs>>>(p);
+            else gomoku::tree_step_kernel<false><<<n, 32, 0, gs>>>(p);
             if (s == steps) continue;
             // Blocks of the launch.  A lane for every game while that does not oversubscribe the device much (OCP: one child
             // per tree); otherwise 1.5 to 2 times the group's share of the blocks that fit on the device at once, so that a
             // lane plays several games one after the other and its warp stays full, and blocks are waiting to start
-            // where another group's launch is running out of games (a step is as long as its longest chain of games, mean
-            // ~85 plies, longest ~170).  Measured, 4 x 256 acp_prodigal, 500 steps, one search (4 groups) / eight searches
-            // (8 groups): 1.0 times the share 90.9 / 597 ms, 1.25: 86.4 / 541, 1.5: 85.3 / 525, 2: 87.7 / 515.
+            // where another group's launch is running out of games.
             const long long games = (long long)n * h->cfg.n_playouts * (ocp ? 1 : h->A);
             const long long enough = (games + gomoku::DYN_THREADS - 1) / gomoku::DYN_THREADS;
             long long blocks = enough;
@@ -977,16 +1013,15 @@ extern "C" int mctsnc_create(const mctsnc_config *cfg, mctsnc_handle **out) {
     if (!rc && !is_gomoku(c)) rc = dev_alloc(h, &h->board, nodes);
     if (!rc && is_gomoku(c)) rc = dev_alloc(h, &h->gboard, nodes * 16);
     if (!rc && is_gomoku(c)) rc = dev_alloc(h, &h->gstep, h->n_trees_total);
-    if (!rc && is_gomoku(c)) rc = dev_alloc(h, &h->gtpl, h->n_trees_total * gomoku::TPL_WORDS);
-    if (!rc && is_gomoku(c)) rc = dev_alloc(h, &h->path_ns, h->n_trees_total * PATH_CAP);
-    if (!rc && is_gomoku(c)) rc = dev_alloc(h, &h->path_wins, h->n_trees_total * PATH_CAP);
+    if (!rc && is_gomoku(c)) rc = dev_alloc(h, &h->gsheet, h->n_trees_total * gomoku::SHEET_WORDS);
+    if (!rc && is_gomoku(c)) rc = dev_alloc(h, &h->path_rec, h->n_trees_total * PATH_CAP);
+    if (!rc && is_gomoku(c)) rc = dev_alloc(h, &h->path_term, h->n_trees_total * PATH_CAP);
+    if (!rc && is_gomoku(c)) rc = dev_alloc(h, &h->gwork, h->n_trees_total);
     if (!rc && is_gomoku(c)) rc = dev_alloc(h, &h->child_outcome, h->n_trees_total * h->A);
     if (!rc && is_gomoku(c)) rc = dev_alloc(h, &h->child_action, h->n_trees_total * h->A);
-    if (!rc && is_gomoku(c)) rc = dev_alloc(h, &h->active_rank, h->n_trees_total * h->A);
     if (!rc && is_gomoku(c)) rc = dev_alloc(h, &h->root_gboard, (long long)c.max_batch * 17);   // boards and turns
     if (!rc && is_gomoku(c) && cudaMallocHost((void **)&h->h_root_gboard, sizeof(unsigned) * 17 * c.max_batch) != cudaSuccess) rc = MCTSNC_E_NO_MEMORY;
     if (!rc && is_gomoku(c)) rc = (int)cudaMemset(h->gstep, 0, sizeof(gomoku::StepInfo) * h->n_trees_total);
-    if (!rc && is_gomoku(c)) rc = (int)cudaMemset(h->gtpl, 0, sizeof(unsigned) * gomoku::TPL_WORDS * h->n_trees_total);
     if (!rc) rc = dev_alloc(h, &h->parent, nodes);
     if (!rc) rc = dev_alloc(h, &h->state, h->n_trees_total);
     if (!rc) rc = dev_alloc(h, &h->paths, h->n_trees_total * PATH_CAP);
@@ -1263,7 +1298,7 @@ static int export_nodes_gomoku(mctsnc_handle *h, const std::vector<TreeState> &s
                 }
                 break;
             }
-            case MCTSNC_F_DEPTHS: ((int16_t *)dst)[o] = valid ? (int16_t)meta_depth(r.w) : 0; break;
+            case MCTSNC_F_DEPTHS: ((int16_t *)dst)[o] = valid ? (int16_t)gomoku::g_depth(r.w) : 0; break;
             case MCTSNC_F_TURNS: ((int8_t *)dst)[o] = valid ? (int8_t)gomoku::g_turn(r.w) : 0; break;
             case MCTSNC_F_LEAVES: ((uint8_t *)dst)[o] = valid ? ((r.w & gomoku::G_NCHILD_MASK) == 0) : 0; break;
             case MCTSNC_F_TERMINALS: ((uint8_t *)dst)[o] = valid ? ((r.w & gomoku::G_TERMINAL) != 0) : 0; break;
