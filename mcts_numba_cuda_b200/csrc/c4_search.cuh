@@ -357,9 +357,9 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
                                           const int n_steps, const bool first) {
     namespace cg = cooperative_groups;
     const int cache_n = CL > 1 ? p.cache_nodes : 0;
-    static_assert(CL == 1 || CL == 2 || CL == 4 || CL == 8, "cluster sizes");
+    static_assert(CL == 1 || CL == 8 || CL == 16, "cluster sizes");
     constexpr int PLIES = STRAIGHT ? STRAIGHT_PLIES : PLIES_PER_CHECK;
-    constexpr int LOG_CL = CL == 8 ? 3 : (CL == 4 ? 2 : (CL == 2 ? 1 : 0));
+    constexpr int LOG_CL = CL == 16 ? 4 : (CL == 8 ? 3 : 0);
     const int tid = threadIdx.x;
     const int nt = blockDim.x;
     const int lane = tid & 31;
@@ -1012,26 +1012,23 @@ __global__ void __maxnreg__(MCTSNC_C4_MAXNREG) search_kernel(const SearchParams 
     }
 }
 
-// A cluster of CLUSTER_BLOCKS blocks per tree: launches with few trees (one search), where a step of a tree is bound by what one
-// SM can play.  Launched with the cluster dimension as a launch attribute; cluster c grows tree c for the whole launch.
-#ifndef MCTSNC_C4_CLUSTER_BLOCKS
-#define MCTSNC_C4_CLUSTER_BLOCKS 8
-#endif
-#ifndef MCTSNC_C4_CLUSTER_THREADS
-#define MCTSNC_C4_CLUSTER_THREADS 256
-#endif
-constexpr int CLUSTER_BLOCKS = MCTSNC_C4_CLUSTER_BLOCKS;
-constexpr int CLUSTER_THREADS = MCTSNC_C4_CLUSTER_THREADS;
-
-template <bool OCP>
-__global__ void __launch_bounds__(CLUSTER_THREADS) search_cluster_kernel(const SearchParams p) {
+// A cluster of CL blocks per tree: launches with few trees (one search), where a step of a tree is bound by what one SM can play.
+// Launched with the cluster dimension as a launch attribute; cluster c grows tree c for the whole launch.  THREADS: of a block.
+template <bool OCP, int CL, int THREADS>
+__global__ void __launch_bounds__(THREADS) search_cluster_kernel(const SearchParams p) {
     __shared__ Shared s;
     extern __shared__ ulonglong2 s_rng[];
     build_move_lut(s);
-    const int n_local = ((OCP ? 1 : A) * p.n_playouts) / CLUSTER_BLOCKS;   // streams this block keeps; the record cache follows
-    run_slice<OCP, CLUSTER_BLOCKS, true>(p, s, s_rng, reinterpret_cast<int4 *>(s_rng + n_local), (int)(blockIdx.x / CLUSTER_BLOCKS), p.steps,
-                                   p.first != 0);
+    const int n_local = ((OCP ? 1 : A) * p.n_playouts) / CL;   // streams this block keeps; the record cache follows
+    run_slice<OCP, CL, true>(p, s, s_rng, reinterpret_cast<int4 *>(s_rng + n_local), (int)(blockIdx.x / CL), p.steps, p.first != 0);
 }
+
+// Clusters of 8 blocks of 256 threads, or -- for steps with more games than those blocks can play one to a thread while a warp
+// walks -- of 16 blocks of 128 and a warp for the walk: a scheduler has one warp of games then instead of two.  4 trees, ACP 64 /
+// 128 / 256 / 512 playouts, us a step: 5.6 / 5.6 / 7.2 / 9.9 with 8 blocks, 6.0 / 6.0 / 6.8 / 8.4 with 16 (the barriers of the larger
+// cluster cost more).
+constexpr int CLUSTER_BLOCKS = 8, CLUSTER_THREADS = 256;
+constexpr int WIDE_CLUSTER_BLOCKS = 16, WIDE_CLUSTER_THREADS = 160, WIDE_CLUSTER_MIN_GAMES = CLUSTER_BLOCKS * (CLUSTER_THREADS - 32);
 
 }  // namespace c4
 }  // namespace mctsnc

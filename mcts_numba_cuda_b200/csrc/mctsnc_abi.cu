@@ -72,7 +72,7 @@ struct mctsnc_handle {
     int tpb_roa = 0;
     int sm_count = 0;
     bool cluster_ok = false;      // thread-block clusters can be launched (and MCTSNC_B200_NO_CLUSTER is not set)
-    int cluster_fit[2] = {0, 0};  // clusters that fit on the device at once, by record-cache size (0: not asked yet, -1: unknown)
+    int cluster_fit[2][2] = {};   // clusters that fit on the device at once, [wide][small record cache] (0: not asked yet, -1: unknown)
     int threads = 0;
     int blocks_per_sm = 0;
     long long bytes = 0;
@@ -776,44 +776,56 @@ int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_
     if (h->cfg.threads_per_tree == 0 && h->cluster_ok && h->cfg.n_playouts >= c4::CLUSTER_BLOCKS &&
         (long long)(is_ocp(h->cfg) ? 1 : h->A) * h->cfg.n_playouts > MCTSNC_C4_CLUSTER_MIN_GAMES &&
         trees * c4::CLUSTER_BLOCKS <= (long long)MCTSNC_C4_CLUSTER_SM_SHARE * h->sm_count) {
-        cudaLaunchConfig_t lc = {};
-        lc.gridDim = dim3((unsigned)(trees * c4::CLUSTER_BLOCKS));
-        lc.blockDim = dim3(c4::CLUSTER_THREADS);
-        lc.stream = stream;
-        cudaLaunchAttribute attr;
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = c4::CLUSTER_BLOCKS;
-        attr.val.clusterDim.y = 1;
-        attr.val.clusterDim.z = 1;
-        lc.attrs = &attr;
-        lc.numAttrs = 1;
-        if (is_ocp(h->cfg)) cudaFuncSetAttribute(c4::search_cluster_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        else cudaFuncSetAttribute(c4::search_cluster_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        // The first records of a tree stay in the first block's shared memory: many if every block can have an SM to itself,
-        // else few.  All clusters of the launch have to be on the device at once (clusters do not spread over GPCs, so fewer
-        // fit than blocks / 8): a tree whose cluster waits for another to finish would take two searches' time.
-        bool fits = false;
-        for (int small = trees * c4::CLUSTER_BLOCKS <= h->sm_count ? 0 : 1; small < 2 && !fits; small++) {
-            p.cache_nodes = small ? 2048 : MCTSNC_C4_CACHE_NODES;
-            lc.dynamicSmemBytes = h->dyn_smem / c4::CLUSTER_BLOCKS + sizeof(int4) * (size_t)p.cache_nodes;
-            int &fit = h->cluster_fit[small];
-            if (fit == 0) {
-                int n = 0;
-                const cudaError_t q = is_ocp(h->cfg) ? cudaOccupancyMaxActiveClusters(&n, c4::search_cluster_kernel<true>, &lc)
-                                                     : cudaOccupancyMaxActiveClusters(&n, c4::search_cluster_kernel<false>, &lc);
-                if (q != cudaSuccess) cudaGetLastError();
-                fit = q == cudaSuccess && n > 0 ? n : -1;
+        const bool ocp = is_ocp(h->cfg);
+        // the wide cluster first where a step has games for it, the other one if those do not fit on the device
+        for (int wide = (ocp ? 1 : h->A) * h->cfg.n_playouts >= c4::WIDE_CLUSTER_MIN_GAMES ? 1 : 0; wide >= 0; wide--) {
+            const int blocks = wide ? c4::WIDE_CLUSTER_BLOCKS : c4::CLUSTER_BLOCKS;
+            const void *kernel = wide ? (ocp ? (const void *)c4::search_cluster_kernel<true, c4::WIDE_CLUSTER_BLOCKS, c4::WIDE_CLUSTER_THREADS>
+                                             : (const void *)c4::search_cluster_kernel<false, c4::WIDE_CLUSTER_BLOCKS, c4::WIDE_CLUSTER_THREADS>)
+                                      : (ocp ? (const void *)c4::search_cluster_kernel<true, c4::CLUSTER_BLOCKS, c4::CLUSTER_THREADS>
+                                             : (const void *)c4::search_cluster_kernel<false, c4::CLUSTER_BLOCKS, c4::CLUSTER_THREADS>);
+            if (wide && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+                cudaGetLastError();
+                continue;
             }
-            fits = fit >= trees;
-        }
-        if (fits) {
-            h->threads = c4::CLUSTER_THREADS * c4::CLUSTER_BLOCKS;
+            cudaLaunchConfig_t lc = {};
+            lc.gridDim = dim3((unsigned)(trees * blocks));
+            lc.blockDim = dim3(wide ? c4::WIDE_CLUSTER_THREADS : c4::CLUSTER_THREADS);
+            lc.stream = stream;
+            cudaLaunchAttribute attr;
+            attr.id = cudaLaunchAttributeClusterDimension;
+            attr.val.clusterDim.x = (unsigned)blocks;
+            attr.val.clusterDim.y = 1;
+            attr.val.clusterDim.z = 1;
+            lc.attrs = &attr;
+            lc.numAttrs = 1;
+            CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+            // The first records of a tree stay in the first block's shared memory: many if every block can have an SM to itself,
+            // else few.  All clusters of the launch have to be on the device at once (clusters do not spread over GPCs, so fewer
+            // fit than blocks / 8): a tree whose cluster waits for another to finish would take two searches' time.  A wide cluster
+            // is for blocks that have an SM each.
+            bool fits = false;
+            const bool own_sm = trees * blocks <= h->sm_count;
+            for (int small = own_sm ? 0 : 1; small < (wide ? 1 : 2) && !fits; small++) {
+                p.cache_nodes = small ? 2048 : MCTSNC_C4_CACHE_NODES;
+                lc.dynamicSmemBytes = h->dyn_smem / blocks + sizeof(int4) * (size_t)p.cache_nodes;
+                int &fit = h->cluster_fit[wide][small];
+                if (fit == 0) {
+                    int n = 0;
+                    const cudaError_t q = cudaOccupancyMaxActiveClusters(&n, kernel, &lc);
+                    if (q != cudaSuccess) cudaGetLastError();
+                    fit = q == cudaSuccess && n > 0 ? n : -1;
+                }
+                fits = fit >= trees;
+            }
+            if (!fits) continue;
+            h->threads = wide ? (c4::WIDE_CLUSTER_THREADS - 32) * blocks : c4::CLUSTER_THREADS * blocks;
             h->blocks_per_sm = 1;
-            const cudaError_t e = is_ocp(h->cfg) ? cudaLaunchKernelEx(&lc, c4::search_cluster_kernel<true>, p)
-                                                 : cudaLaunchKernelEx(&lc, c4::search_cluster_kernel<false>, p);
-            if (e == cudaSuccess) return 0;
+            void *args[] = {&p};
+            if (cudaLaunchKernelExC(&lc, kernel, args) == cudaSuccess) return 0;
             cudaGetLastError();      // the launch was refused (nothing ran): one block per tree from now on
             h->cluster_ok = false;
+            break;
         }
         p.cache_nodes = 0;
     }

@@ -31,7 +31,8 @@ def late_root(empty, seed):
 @pytest.mark.parametrize("variant,n_playouts,threads,empty", [
     ("ocp_prodigal", 32, 0, 9), ("ocp_thrifty", 8, 32, 3), ("ocp_thrifty", 64, 64, 14), ("ocp_prodigal", 64, 32, 14),
     ("acp_prodigal", 8, 0, 5), ("acp_thrifty", 32, 224, 12), ("acp_prodigal", 32, 96, 12), ("acp_thrifty", 64, 0, 8),
-    ("acp_prodigal", 256, 0, 20), ("acp_prodigal", 256, 320, 20), ("acp_thrifty", 1, 0, 30)])
+    ("acp_prodigal", 256, 0, 20), ("acp_prodigal", 256, 320, 20), ("acp_thrifty", 1, 0, 30),
+    ("acp_thrifty", 512, 0, 18), ("acp_prodigal", 256, 0, 2), ("acp_prodigal", 128, 0, 22)])
 def test_late_positions_match_oracle_whatever_thread_plays_a_game(variant, n_playouts, threads, empty):
     steps, trees = 70, 2
     board, fills, turn = late_root(empty, seed=empty)
