@@ -99,7 +99,8 @@ __device__ __forceinline__ unsigned bitrev8(unsigned x) { return __brev(x) >> 24
 // selected node, written by the tree step and copied by the playouts):
 //   LIST_WORDS words   the list of legal actions, one byte each, in the order the reference's swap-remove leaves them
 //                      (src/mctsnc_game_mechanics.py:209-217); the byte of cell (i, j) is i * 16 + j, row and column ready
-//                      to use;
+//                      to use.  `pad` bytes (0 to 7) lie in front of it, so that the list of a game ends on a multiple of 8 and
+//                      the plies of a block find its last entry at places known at compile time;
 //   LINE_WORDS words   the stones by line, one word per line of each of the four directions, at the bit of their position
 //                      along the line: stones of the side that makes the game's first move in bits 0..14, stones of the other
 //                      side in bits 16..30, so that a ply reads and writes one halfword per direction:
@@ -113,26 +114,26 @@ __device__ __forceinline__ unsigned bitrev8(unsigned x) { return __brev(x) >> 24
 //                      0 .. 12 - d, with position 13 - d between them always empty: a run of stones cannot pass from one to
 //                      the other and finds the empty position where the board ends.  Likewise i + j = a <= 12 (positions
 //                      0 .. a) and a + 16 (positions a + 2 .. 14).
-constexpr int LIST_WORDS = 57, LINE_WORDS = 15 + 15 + 16 + 16, THREAD_WORDS = LIST_WORDS + LINE_WORDS;
+constexpr int LIST_WORDS = 58, LINE_WORDS = 15 + 15 + 16 + 16, THREAD_WORDS = LIST_WORDS + LINE_WORDS;
 constexpr int LINE_ROW = LIST_WORDS, LINE_COL = LINE_ROW + 15, LINE_DIAG = LINE_COL + 15, LINE_ANTI = LINE_DIAG + 16;
 // The sheet of a step: the selected node's position in that form (the two parts on 16-byte boundaries, so that a thread copies them
 // four words at a time), the ranks of the children that are played out, ascending, a byte each, a few numbers, and the list
 // without its first entry
 constexpr int TPL_LIST = 0, TPL_LINES = 60, SHEET_ACTIVE = 124, SHEET_MODE = 184, SHEET_FIRST_CHILD = 185, SHEET_SELECTED = 186,
-              SHEET_FIRST_MOVER = 187, SHEET_EMPTY = 188, SHEET_OLD_FIVE = 189, SHEET_LIST_UP = 192, SHEET_WORDS = 256;
+              SHEET_FIRST_MOVER = 187, SHEET_EMPTY = 188, SHEET_OLD_FIVE = 189, SHEET_PAD = 190, SHEET_LIST_UP = 192, SHEET_WORDS = 256;
 
-// bit s: stones at s .. s + 4 (for a word of two lines, one in each half: bits 15 and 31 are empty, so no run passes over)
-__device__ __forceinline__ unsigned fives(unsigned w) {
-    const unsigned a = w & (w >> 1);
-    return a & (a >> 2) & (w >> 4);
+// bit p: a run of exactly five stones at p - 5 .. p - 1 (for a word of two lines, one in each half: bits 15 and 31 are empty, so no
+// run passes over).  Shifts to the left only: those the multiply-add pipe can do too, and the logic pipe is the busier one.
+__device__ __forceinline__ unsigned exact_fives(unsigned u) {
+    const unsigned x = u << 1, two = x & (x << 1), four = two & (two << 2);
+    return four & (x << 4) & ~(x << 5) & ~u;
 }
-// the bits without a neighbour: runs of exactly five (a longer one has several bits in a row)
-__device__ __forceinline__ unsigned lone_bits(unsigned f) { return f & ~(f << 1) & ~(f >> 1); }
+// where the bit of a run that holds a stone at `pos` can be
+__device__ __forceinline__ unsigned runs_through(int pos) { return (0x3Eu << pos) & 0xFFFFu; }
 
 // runs of exactly five through a new stone at position `pos1` of line word u1 and `pos2` of u2 (one side's stones, 15 bits each)
 __device__ __forceinline__ bool five_on_lines(unsigned u1, int pos1, unsigned u2, int pos2) {
-    const unsigned one = lone_bits(fives((u1 | (1u << pos1)) + ((u2 | (1u << pos2)) << 16)));
-    return (one & (((0x1Fu << pos1) >> 4) | (((0x1Fu << pos2) >> 4) << 16))) != 0u;   // starts of the runs that hold the stone
+    return (exact_fives((u1 | (1u << pos1)) + ((u2 | (1u << pos2)) << 16)) & (runs_through(pos1) | (runs_through(pos2) << 16))) != 0u;
 }
 
 // LOCAL: the tree stays with one block for the whole search; else it is read once in a launch, from L2
@@ -346,6 +347,9 @@ struct Walker {
             for (int i = lane; i < LINE_WORDS; i += 32) sheet[TPL_LINES + i] = 0u;
             __syncwarp();
             unsigned char *list = reinterpret_cast<unsigned char *>(sheet + TPL_LIST), *list_up = reinterpret_cast<unsigned char *>(sheet + SHEET_LIST_UP);
+            const int pad = -(mode == MODE_ALL_CHILDREN ? n_legal - 1 : n_legal) & 7;   // a child's games have one cell less
+            list += pad;
+            list_up += pad;
             unsigned words[16];
 #pragma unroll
             for (int k = 0; k < 16; k++) words[k] = __shfl_sync(0xFFFFFFFFu, mine, k);
@@ -370,7 +374,7 @@ struct Walker {
             }
             __syncwarp();
             const unsigned *lines = sheet + TPL_LINES;
-            const bool five = lone_bits(fives(lines[lane])) != 0u || (lane + 32 < LINE_WORDS && lone_bits(fives(lines[lane + 32])) != 0u);
+            const bool five = exact_fives(lines[lane]) != 0u || (lane + 32 < LINE_WORDS && exact_fives(lines[lane + 32]) != 0u);
             const bool old_five = __any_sync(0xFFFFFFFFu, five);
             if (lane == 0 && n_exp < n_legal) atomicOr(&st->status, STATUS_TREE_FULL);
             unsigned char *active = reinterpret_cast<unsigned char *>(sheet + SHEET_ACTIVE);
@@ -443,6 +447,7 @@ struct Walker {
                 sheet[SHEET_FIRST_MOVER] = (unsigned)first_mover;
                 sheet[SHEET_EMPTY] = (unsigned)n_legal;
                 sheet[SHEET_OLD_FIVE] = old_five ? 1u : 0u;
+                sheet[SHEET_PAD] = (unsigned)pad;
             }
         }
         if (mode != MODE_ALL_CHILDREN && !thrifty)
@@ -459,7 +464,7 @@ struct Walker {
             if (OCP && mode == MODE_ALL_CHILDREN) {
                 m2 = pick;
                 if (!thrifty) {   // the pick's action, from the list (the cell's row and column)
-                    const int c = reinterpret_cast<unsigned char *>(sheet + TPL_LIST)[pick];
+                    const int c = reinterpret_cast<unsigned char *>(sheet + TPL_LIST)[sheet[SHEET_PAD] + pick];
                     m2 = (c >> 4) * N + (c & 15);
                 }
             }
@@ -641,12 +646,14 @@ __device__ __noinline__ EmuResult playout_emulated(const unsigned *start /* 16 w
 
 // ---------------------------------------------------------------------------------------------------------------
 // A game in progress: one per thread, list and lines in the thread's column of shared memory (STRIDE threads side by side).
-//   * The four words of a new stone hold a run of five iff the AND of the word with itself shifted by 1 to 4 has a bit, and one of
-//     exactly five (which the reference wants: it counts at most 5 stones either way and asks for a total of 4,
-//     src/mctsnc_game_mechanics.py:220-272) iff that bit has no neighbour.  Two lines are tested in the halves of a word.  A run
-//     of exactly five that does not go through the new stone would have ended the game before, unless the starting position
-//     has one: then (`careful`) the place of the run is looked at too.
-//   * The draw of a ply and the two list entries it reads are fetched one ply ahead.
+//   * The four words of a new stone are tested for a run of exactly five (the reference counts at most 5 stones either way and asks
+//     for a total of 4, src/mctsnc_game_mechanics.py:220-272), two lines in the halves of a word.  A run of exactly five that
+//     does not go through the new stone would have ended the game before, unless the starting position has one: then
+//     (`careful`) the place of the run is looked at too.
+//   * The draw of a ply and the two list entries it reads are fetched one ply ahead; where the last entry is does not have to be
+//     worked out ply by ply (`pad`).
+// Where the SM is full (eight searches, 14 warps) the logic pipe binds: 169.8 ms with shifts to the right and a test for lone bits,
+// 162.5 with exact_fives, 159.5 with the padded list; where a step waits for its longest game: 5.89, 5.75, 5.66 ms.
 //   * The plies of a block depend on no branch, so that they overlap; a game that has been won plays on to the end of the block,
 //     which is put right when it is closed.  A draw of exactly 1.0f is noticed at the end of the block too (the largest draw is
 //     kept); until then the lane plays on with a list entry it should not have, inside its own column.
@@ -659,24 +666,28 @@ struct Game {
     int winner;               // of a game that is over: 1 first mover, 2 the other side, 0 a draw
     float left_2m64;          // left * 2^-64, the factor of the draws scaled by 2^64
     float draw, largest;      // the draw of the ply to come and the largest of those before it, times 2^64
+    int pad;                  // bytes in front of the list
+    float magic;              // 2^23 + pad
     int at;                   // byte offset in the column of the list entry that the ply to come takes
     int next_cell, next_last; // that entry and the last one of the list
     unsigned long long s0, s1;
 
-    // byte offset of list entry q: byte q & 3 of word q >> 2, words STRIDE apart; (q >> 2) * 4 * STRIDE + (q & 3) written as one
+    // byte offset of the list's byte b: byte b & 3 of word b >> 2, words STRIDE apart; (b >> 2) * 4 * STRIDE + (b & 3) written as one
     // shift and one multiply-add
-    static __device__ __forceinline__ int list_byte(int q) { return (q >> 2) * (4 * STRIDE - 4) + q; }
+    static __device__ __forceinline__ unsigned list_byte(unsigned b) { return (b >> 2) * (4 * STRIDE - 4) + b; }
+    __device__ __forceinline__ int last_entry() const { return (int)list_byte((unsigned)(max(left - 1, 0) + pad)); }
 
     // The position a game starts from, out of a sheet in shared memory: the parent's with `count` empty cells, less the child's own
-    // cell, which is at position `skip` of the list (child_cell < 0: the parent itself, skip = NO_SKIP).
+    // cell, which is at byte `skip` of the padded list (child_cell < 0: the parent itself, skip = NO_SKIP).
     // The list: four words at a time, from the list in front of `skip` and from the list without its first entry behind it; the four
     // words around `skip` are put right afterwards.  Words past the last entry are never read; up to three words past the list
     // are written and then covered by the lines.
     static constexpr int NO_SKIP = 1 << 30;
     __device__ __forceinline__ void copy_position(const unsigned *sheet, int count, int skip, int child_cell) {
+        pad = (int)sheet[SHEET_PAD];
         unsigned *my = reinterpret_cast<unsigned *>(list);
         const int skip_word = skip >> 2, skip_chunk = skip >> 4;
-        const int chunks = (count + 15) >> 4;
+        const int chunks = (count + pad + 15) >> 4;
         const uint4 *list4 = reinterpret_cast<const uint4 *>(sheet + TPL_LIST), *up4 = reinterpret_cast<const uint4 *>(sheet + SHEET_LIST_UP);
         for (int c = 0; c < chunks; c++) {
             const uint4 v = (c < skip_chunk ? list4 : up4)[c];
@@ -729,29 +740,30 @@ struct Game {
         winner = 0;
         left_at_end = 0;
         playing = true;
-        next_draw();
+        magic = 8388608.f + (float)pad;
+        next_draw(last_entry());
     }
 
     // float32 u * int16 count -> float32 (src/mctsnc.py:2061); here (u * 2^64) * (count * 2^-64): the same product, rounded once.
-    // Added to 2^23 with rounding towards zero it leaves the position in the low bits; position <= left <= 225.
-    __device__ __forceinline__ void next_draw() {
+    // Added to 2^23 + pad with rounding towards zero it leaves the place in the padded list in the low bits (below them the bits of
+    // 2^23, whose share of the byte offset is taken off again).  `last`: byte offset of the last entry.
+    __device__ __forceinline__ void next_draw(int last) {
         draw = rng_uniform_times_2p64(s0, s1);
-        const int q = (int)(__float_as_uint(__fadd_rz(__fmul_rn(draw, left_2m64), 8388608.f)) & 0xFFu);
-        at = list_byte(q);
-        next_last = list[list_byte(max(left - 1, 0))];
+        at = (int)(list_byte(__float_as_uint(__fadd_rz(__fmul_rn(draw, left_2m64), magic))) - list_byte(0x4B000000u));
+        next_last = list[last];
         next_cell = list[at];
     }
 
     // One ply (src/mctsnc.py:2059-2064): last_action = legal[ord]; legal[ord] = legal[count - 1]; count -= 1 (:2062, :215-217), byte
-    // loads and stores, no read-modify-write of words; then the stone.  Returns whether it makes a run of exactly five.
+    // loads and stores, no read-modify-write of words; then the stone.  Returns whether it makes a run of exactly five.  `last`: byte
+    // offset of the last entry after this ply.
     template <bool CAREFUL>
-    __device__ __forceinline__ bool ply(int rep) {
+    __device__ __forceinline__ bool ply(int rep, int last) {
         const int cell = next_cell;
         list[at] = (unsigned char)next_last;
-        left--;
         left_2m64 -= RNG_2M64;   // exact: small integers times 2^-64
         largest = fmaxf(largest, draw);
-        next_draw();
+        next_draw(last);
         const int i = cell >> 4, j = cell & 15;
         const unsigned bit_j = 1u << j, bit_i = 1u << i;
         // the mover's halfwords of the stone's row, column, diagonal and anti-diagonal
@@ -765,21 +777,27 @@ struct Game {
         *col = (unsigned short)wc;
         *diag = (unsigned short)wd;
         *anti = (unsigned short)wa;
-        const unsigned one = lone_bits(fives(wr + (wc << 16))), two = lone_bits(fives(wd + (wa << 16)));
+        const unsigned one = exact_fives(wr + (wc << 16)), two = exact_fives(wd + (wa << 16));
         if (!CAREFUL) return (one | two) != 0u;
-        const unsigned through_j = (0x1Fu << j) >> 4, through_i = (0x1Fu << i) >> 4;   // starts of the runs that hold the stone
+        const unsigned through_j = runs_through(j), through_i = runs_through(i);
         return ((one & (through_j | (through_i << 16))) | (two & (through_j | (through_j << 16)))) != 0u;
     }
 
     // PLIES plies, or as many as there are
     template <int PLIES>
     __device__ __forceinline__ void play() {
-        static_assert(PLIES % 2 == 0 && PLIES <= 32, "the sides take turns with the plies of a block");
+        static_assert(PLIES == 8, "what `pad` rounds a list up to");
         if (left >= PLIES && !careful) {
             unsigned wins = 0u;
+            const int end = (left + pad) * STRIDE;   // byte offset of the word behind the list: left + pad is a multiple of 8
 #pragma unroll
-            for (int rep = 0; rep < PLIES; rep++)
-                if (ply<false>(rep)) wins |= 1u << rep;
+            for (int rep = 0; rep < PLIES; rep++) {
+                const int e = rep + 2;   // the last entry after this ply is the e-th from the end
+                int last = end - 4 * STRIDE * ((e + 3) / 4) + ((-e) & 3);
+                if (rep == PLIES - 1) last = max(last, 0);   // after the last ply of a game without pad there is none
+                if (ply<false>(rep, last)) wins |= 1u << rep;
+            }
+            left -= PLIES;
             if (wins != 0u) {
                 const int rep = __ffs(wins) - 1;
                 winner = 1 + (rep & 1);
@@ -788,12 +806,14 @@ struct Game {
             }
         } else {
 #pragma unroll 1
-            for (int rep = 0; rep < PLIES && playing && left > 0; rep++)
-                if (ply<true>(rep)) {
+            for (int rep = 0; rep < PLIES && playing && left > 0; rep++) {
+                left--;
+                if (ply<true>(rep, last_entry())) {
                     winner = 1 + (rep & 1);
                     left_at_end = left;
                     playing = false;
                 }
+            }
         }
         if (left == 0 || largest >= RNG_2P64) playing = false;
     }
@@ -849,7 +869,7 @@ __global__ void __launch_bounds__(32) tree_step_kernel(const __grid_constant__ P
 // for one lane or for many.
 //
 // Per-thread game state lives in shared memory, laid out so that every thread owns one bank column: word k of thread t
-// is s_mem[k * DYN_THREADS + t].  That state (476 bytes) decides how many games an SM plays at once: 14 warps, so what counts is
+// is s_mem[k * DYN_THREADS + t].  That state (480 bytes) decides how many games an SM plays at once: 14 warps, so what counts is
 // the length of a ply: its instructions and their chain (see Game).
 #ifndef MCTSNC_GOMOKU_REFILL_MIN
 #define MCTSNC_GOMOKU_REFILL_MIN 8
@@ -935,10 +955,11 @@ __global__ void __launch_bounds__(DYN_THREADS) playout_dynamic_kernel(const __gr
                 action = 0;   // the selected node itself is played out with the streams of action 0
                 node = (int)sheet[SHEET_SELECTED];
                 if (child) {
-                    skip = active[item >> log2p];   // rank of the child: children are the first empty cells in ascending order
+                    const int rank = active[item >> log2p];   // children are the first empty cells in ascending order
+                    skip = (int)sheet[SHEET_PAD] + rank;
                     cell = list_bytes[skip];
                     action = (cell >> 4) * N + (cell & 15);
-                    node = (int)sheet[SHEET_FIRST_CHILD] + skip;
+                    node = (int)sheet[SHEET_FIRST_CHILD] + rank;
                 }
                 first_mover = (int)sheet[SHEET_FIRST_MOVER];
                 rng_idx = OCP ? ((long long)tree * P + t) : (((long long)tree * A + action) * P + t);
@@ -1024,13 +1045,14 @@ __global__ void __launch_bounds__(STRIDE + 32, blocks_per_sm(STRIDE)) search_blo
         __syncthreads();
         if (b.n_active == 0) break;
         const bool child = (int)b.sheet[SHEET_MODE] == MODE_ALL_CHILDREN;
-        const int skip = child ? reinterpret_cast<const unsigned char *>(b.sheet + SHEET_ACTIVE)[0] : Game<STRIDE>::NO_SKIP;
+        const int rank = child ? reinterpret_cast<const unsigned char *>(b.sheet + SHEET_ACTIVE)[0] : 0;
+        const int skip = child ? (int)b.sheet[SHEET_PAD] + rank : Game<STRIDE>::NO_SKIP;
         const int cell = child ? reinterpret_cast<const unsigned char *>(b.sheet + TPL_LIST)[skip] : -1;
         if (player < 0) {
             w.prepare();
         } else {
             const int first_mover = (int)b.sheet[SHEET_FIRST_MOVER], empty = (int)b.sheet[SHEET_EMPTY];
-            const int node = child ? (int)b.sheet[SHEET_FIRST_CHILD] + skip : (int)b.sheet[SHEET_SELECTED];
+            const int node = child ? (int)b.sheet[SHEET_FIRST_CHILD] + rank : (int)b.sheet[SHEET_SELECTED];
             for (int base = 0; base < P; base += STRIDE) {
                 // the games of a warp are played to their ends together and closed together
                 const int item = base + player;
