@@ -549,96 +549,83 @@ struct Walker {
 };
 
 // ---------------------------------------------------------------------------------------------------------------
-// Byte-for-byte emulation of one Gomoku playout of the reference on int8 / int16 local arrays (see the Connect-4
-// counterpart): entered only after a uniform draw equal to 1.0f, which makes the reference read the slot one past its
-// list of legal actions.  The per-thread list starts as zeros, negative indices wrap once (numba), and the loop gives
-// up after 4096 plies (list and board can get out of step for good; the reference would then never return).
+// One Gomoku playout as the reference plays it, entered only after a uniform draw equal to 1.0f, which makes the reference read the
+// slot one past its list of legal actions: an entry left by an earlier ply, or 0 where none was (the per-thread list starts as
+// zeros).  From then on a stone may fall on another one and replace it, and list and board may part: the list is made anew from
+// the board when it runs out before the board is full, and the loop gives up after 4096 plies (the reference might never
+// return).  Replayed from the first ply in the thread's own column, so that the slots hold what they would hold.
+// One lane plays while its warp waits, in about one of eight steps of a 4 x 256 search, which the replay then decides the length
+// of: on byte arrays in local memory, with a look at all cells after every ply, it took 270 us (73.8 ms a search of 500 steps; 71.2 so).
 struct EmuResult {
     int outcome;
     unsigned plies, ub, err;
     unsigned long long s0, s1;
 };
 
-__device__ __forceinline__ int emu_wrap(int i, int len, unsigned &err) {
-    if (i < 0) i += len;
-    if (i < 0 || i >= len) {
-        err = 1;
-        i = i < 0 ? 0 : len - 1;
+template <int STRIDE>
+__device__ __noinline__ EmuResult replay(unsigned char *list, const unsigned *start /* 16 words */, int first_mover,
+                                         unsigned long long s0, unsigned long long s1) {
+    auto word = [&](int w) -> unsigned & { return reinterpret_cast<unsigned *>(list)[w * STRIDE]; };
+    auto entry = [&](int q) -> unsigned char & { return list[(q >> 2) * (4 * STRIDE) + (q & 3)]; };
+    for (int w = 0; w < THREAD_WORDS; w++) word(w) = 0u;
+    int count = 0;
+    for (int k = 0; k < 8; k++) {
+        const unsigned neg = __ldcg(start + k), pos = __ldcg(start + 8 + k);
+        const unsigned low = first_mover < 0 ? neg : pos;   // the first mover's stones: the low halves of the lines
+        for (unsigned todo = ~(neg | pos) & (k < 7 ? 0xFFFFFFFFu : (1u << (A - 224)) - 1u); todo != 0u; todo &= todo - 1u) {
+            const int cell = 32 * k + __ffs(todo) - 1;
+            entry(count++) = (unsigned char)(cell + cell / N);   // 16 i + j
+        }
+        for (unsigned todo = neg | pos; todo != 0u; todo &= todo - 1u) {
+            const int bit = __ffs(todo) - 1, cell = 32 * k + bit, i = cell / N, j = cell - i * N, hs = (low >> bit) & 1u ? 0 : 16;
+            word(LINE_ROW + i) |= 1u << (hs + j);
+            word(LINE_COL + j) |= 1u << (hs + i);
+            word(LINE_DIAG + ((i - j + 14) & 15)) |= 1u << (hs + j);
+            word(LINE_ANTI + ((i + j) & 15)) |= 1u << (hs + j);
+        }
     }
-    return i;
-}
-
-__device__ __noinline__ EmuResult playout_emulated(const unsigned *start /* 16 words */, int turn, unsigned long long s0,
-                                                   unsigned long long s1) {
-    signed char bd[A];
-    short legal[513];
-    unsigned err = 0;
-    for (int c = 0; c < A; c++) {
-        const bool neg = (__ldcg(start + (c >> 5)) >> (c & 31)) & 1u, pos = (__ldcg(start + 8 + (c >> 5)) >> (c & 31)) & 1u;
-        bd[c] = pos ? 1 : (neg ? -1 : 0);
-    }
-    for (int k = 0; k < 513; k++) legal[k] = 0;
+    int empty = count;   // cells of the board
     EmuResult r = {0, 0u, 0u, 0u, 0ULL, 0ULL};
-    int outcome = 2;
-    for (;;) {
+    for (;; r.plies++) {
         if (r.plies >= 4096u) {
-            err = 1;
-            outcome = 0;
+            r.err = 1u;
+            break;
         }
-        if (outcome != 2) break;
-        if (legal[512] == 0) {  // legal_actions_playout_gomoku :196-207
-            int count = 0;
-            for (int c = 0; c < A; c++)
-                if (bd[c] == 0) legal[count++] = (short)c;
-            legal[512] = (short)count;
-        }
-        const int count = legal[512];
+        if (count == 0)   // legal_actions_playout_gomoku :196-207
+            for (int i = 0; i < M; i++) {
+                const unsigned both = word(LINE_ROW + i);
+                for (unsigned todo = ~(both | (both >> 16)) & 0x7FFFu; todo != 0u; todo &= todo - 1u)
+                    entry(count++) = (unsigned char)(16 * i + __ffs(todo) - 1);
+            }
         const float u = rng_uniform_f32(s0, s1);
-        const int ord = (int)(short)__float2int_rz(__fmul_rn(u, (float)count));
+        const int q = __float2int_rz(__fmul_rn(u, (float)count));   // count where u is 1.0f
         if (u >= 1.0f) r.ub++;
-        int action = legal[emu_wrap(ord, 513, err)];
         // take_action_playout_gomoku :210-217
-        int i, j;
-        if (action < 0) {
-            err = 1;
-            action = 0;
+        const int cell = entry(q), i = cell >> 4, j = cell & 15, last = entry(count - 1);
+        entry(q) = (unsigned char)last;
+        count--;
+        const int hs = (r.plies & 1u) ? 16 : 0;   // the mover's halves; the stone replaces one of the other side
+        unsigned &row = word(LINE_ROW + i), &col = word(LINE_COL + j), &diag = word(LINE_DIAG + ((i - j + 14) & 15)), &anti = word(LINE_ANTI + ((i + j) & 15));
+        const unsigned at_j = 0x10001u << j, at_i = 0x10001u << i;
+        const unsigned wr = row, wc = col, wd = diag, wa = anti;
+        if ((wr & at_j) == 0u) empty--;
+        const unsigned nr = (wr & ~at_j) | (1u << (hs + j)), nc = (wc & ~at_i) | (1u << (hs + i)), nd = (wd & ~at_j) | (1u << (hs + j)),
+                       na = (wa & ~at_j) | (1u << (hs + j));
+        row = nr;
+        col = nc;
+        diag = nd;
+        anti = na;
+        // compute_outcome_gomoku :220-281
+        if (five_on_lines((nr >> hs) & 0x7FFFu, j, (nc >> hs) & 0x7FFFu, i) || five_on_lines((nd >> hs) & 0x7FFFu, j, (na >> hs) & 0x7FFFu, j)) {
+            r.outcome = hs == 0 ? first_mover : -first_mover;
+            r.plies++;
+            break;
         }
-        i = action / N;
-        j = action % N;
-        bd[emu_wrap(i, M, err) * N + emu_wrap(j, N, err)] = (signed char)turn;
-        const int cnt = legal[512];
-        const short last = legal[emu_wrap(cnt - 1, 513, err)];
-        legal[emu_wrap(ord, 513, err)] = last;
-        legal[512] = (short)(legal[512] - 1);
-        turn = -turn;
-        r.plies++;
-        // compute_outcome_gomoku :220-281 (last_token = the stone just placed)
-        const int token = -turn;
-        const int di[4] = {1, 0, 1, 1}, dj[4] = {0, 1, 1, -1};
-        outcome = 2;
-        for (int d = 0; d < 4 && outcome == 2; d++) {
-            int total = 0;
-            for (int k = 1; k < 6; k++) {
-                const int ii = i + k * di[d], jj = j + k * dj[d];
-                if (ii < 0 || ii >= M || jj < 0 || jj >= N || bd[ii * N + jj] != token) break;
-                total++;
-            }
-            for (int k = 1; k < 6; k++) {
-                const int ii = i - k * di[d], jj = j - k * dj[d];
-                if (ii < 0 || ii >= M || jj < 0 || jj >= N || bd[ii * N + jj] != token) break;
-                total++;
-            }
-            if (total == 4) outcome = token;
-        }
-        if (outcome == 2) {
-            bool draw = true;
-            for (int c = 0; c < A; c++)
-                if (bd[c] == 0) draw = false;
-            if (draw) outcome = 0;
+        if (empty == 0) {
+            r.plies++;
+            break;
         }
     }
-    r.outcome = outcome;
-    r.err = err;
     r.s0 = s0;
     r.s1 = s1;
     return r;
@@ -823,9 +810,9 @@ struct Game {
     template <bool LOCAL>
     __device__ __forceinline__ int close(const unsigned *board, int first_mover, const ulonglong2 *start, TreeState *st, int &plies) {
         if (largest >= RNG_2P64) {
-            // u == 1.0f in the game or in the plies behind its end: played again by the byte-level emulation of the reference
+            // u == 1.0f in the game or in the plies behind its end: played again as the reference does
             const ulonglong2 stream = load<LOCAL>(start);
-            const EmuResult er = playout_emulated(board, first_mover, stream.x, stream.y);
+            const EmuResult er = replay<STRIDE>(list, board, first_mover, stream.x, stream.y);
             s0 = er.s0;
             s1 = er.s1;
             plies = (int)er.plies;
