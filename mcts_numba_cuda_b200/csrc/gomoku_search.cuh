@@ -6,7 +6,8 @@
 //                      (_backup_* :2084-2220, _select :1293-1365, _expand_1_* :1368-1681, _expand_2_* :1691-1821)
 //   playout_dynamic_kernel  a persistent grid whose lanes take the step's games one by one (_playout_ocp /
 //                      _playout_acp_* :1824-2081 with the Gomoku device functions of src/mctsnc_game_mechanics.py:181-281)
-// and a last tree_step_kernel launch in backup-only mode.  The OCP variants play P games a step: where every tree fits on the
+// and a last tree_step_kernel launch in backup-only mode.  Where a launch has the games of one tree only, its last warp makes the
+// tree's next step, and there is one launch per step.  The OCP variants play P games a step: where every tree fits on the
 // device a block per tree does the whole search in one launch (search_block_kernel).
 // (Line numbers: src/mctsnc.py of the reference.)
 //
@@ -55,9 +56,9 @@ struct StepInfo {
     int pending;      // 1: the step has been made, its backup is still to be done
 };
 
-// the games of a step: how many, and the next one to hand out
+// the games of a step: how many, the next one to hand out, and the warps that are through with them
 struct StepGames {
-    int games, taken;
+    int games, taken, done;
 };
 
 struct Params {
@@ -833,9 +834,7 @@ struct Game {
 // ACP variants (and OCP with more trees than fit on the device as blocks): a step is two launches that the host enqueues
 // without waiting.
 template <bool OCP>
-__global__ void __launch_bounds__(32) tree_step_kernel(const __grid_constant__ Params p) {
-    __shared__ __align__(16) unsigned sheet[SHEET_WORDS];
-    const int lane = threadIdx.x, tree = p.tree_base + (int)blockIdx.x;
+__device__ __forceinline__ void tree_step(const Params &p, unsigned *sheet, int tree, int lane) {
     Walker<OCP, false> w(p, sheet, tree, lane);
     if (p.first != 0) w.reset();
     w.backup();
@@ -846,26 +845,30 @@ __global__ void __launch_bounds__(32) tree_step_kernel(const __grid_constant__ P
     if (lane == 0) {
         p.work[tree].games = n_active * p.n_playouts;
         p.work[tree].taken = 0;
+        p.work[tree].done = 0;
     }
+}
+
+template <bool OCP>
+__global__ void __launch_bounds__(32) tree_step_kernel(const __grid_constant__ Params p) {
+    __shared__ __align__(16) unsigned sheet[SHEET_WORDS];
+    tree_step<OCP>(p, sheet, p.tree_base + (int)blockIdx.x, (int)threadIdx.x);
 }
 
 // The games of a step, handed out to lanes one by one: every warp works through the games of one tree's step (game = active child * P
 // + t, taken by the warp's idle lanes together), then moves on to the next tree that still has games.  Game (child, t) draws
 // from the stream of the reference's thread (tree, action, t) whichever lane plays it.  A lane that finishes its game waits
-// until at least REFILL_MIN lanes of its warp are idle: closing games and taking new ones costs a few hundred instructions,
-// for one lane or for many.
+// until enough lanes of its warp are idle: closing games and taking new ones costs a few hundred instructions, for one lane or
+// for many.  Eight searches: 159.7 / 153.7 / 150.3 / 153.0 ms at 6 / 8 / 12 / 16 lanes; one search, where the length of a step
+// counts: 65.2 / 65.4 / 65.8 / 66.4 ms.
+//
+// ONE_TREE: the launch has the games of one tree.  The warp that is through last makes the tree's next step at once: a launch of its
+// own waited 10 to 20 us of a step's 140 for its turn among the other trees' blocks (one search 71.2 -> 65.3 ms).
 //
 // Per-thread game state lives in shared memory, laid out so that every thread owns one bank column: word k of thread t
 // is s_mem[k * DYN_THREADS + t].  That state (480 bytes) decides how many games an SM plays at once: 14 warps, so what counts is
 // the length of a ply: its instructions and their chain (see Game).
-#ifndef MCTSNC_GOMOKU_REFILL_MIN
-#define MCTSNC_GOMOKU_REFILL_MIN 8
-#endif
-constexpr int REFILL_MIN = MCTSNC_GOMOKU_REFILL_MIN;
-#ifndef MCTSNC_GOMOKU_PLIES_PER_LOOK
-#define MCTSNC_GOMOKU_PLIES_PER_LOOK 8
-#endif
-constexpr int PLIES_PER_LOOK = MCTSNC_GOMOKU_PLIES_PER_LOOK;   // plies between two looks at whether lanes are idle
+constexpr int PLIES_PER_LOOK = 8;   // plies between two looks at whether lanes are idle
 #ifndef MCTSNC_GOMOKU_THREADS
 #define MCTSNC_GOMOKU_THREADS 224
 #endif
@@ -873,8 +876,9 @@ constexpr int DYN_THREADS = MCTSNC_GOMOKU_THREADS;
 constexpr size_t DYN_SMEM_BYTES = sizeof(unsigned) * ((size_t)THREAD_WORDS * DYN_THREADS + (size_t)SHEET_WORDS * (DYN_THREADS / 32));
 static_assert((THREAD_WORDS * DYN_THREADS) % 4 == 0 && SHEET_WORDS % 4 == 0 && TPL_LINES % 4 == 0, "16-byte loads of the sheet");
 
-template <bool OCP>
+template <bool OCP, bool ONE_TREE>
 __global__ void __launch_bounds__(DYN_THREADS) playout_dynamic_kernel(const __grid_constant__ Params p, int total_trees) {
+    constexpr int REFILL_MIN = ONE_TREE ? 8 : 12;
     extern __shared__ __align__(16) unsigned s_mem[];
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
@@ -971,6 +975,18 @@ __global__ void __launch_bounds__(DYN_THREADS) playout_dynamic_kernel(const __gr
         }
         if (game.playing) game.template play<PLIES_PER_LOOK>();
     }
+    if (ONE_TREE) {
+        // what this warp's lanes have written comes before its arrival, and the step after all arrivals
+        __threadfence();
+        __syncwarp();
+        int arrived = 0;
+        if (lane == 0) arrived = atomicAdd(&p.work[p.tree_base].done, 1);
+        arrived = __shfl_sync(0xFFFFFFFFu, arrived, 0);
+        if (arrived == (int)gridDim.x * (DYN_THREADS / 32) - 1) {
+            __threadfence();
+            tree_step<OCP>(p, sheet, p.tree_base, lane);
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -978,10 +994,7 @@ __global__ void __launch_bounds__(DYN_THREADS) playout_dynamic_kernel(const __gr
 // room on the device at once: a step is as long as its longest game (about 180 plies).  Warp 0 walks, the other STRIDE threads
 // play; what a step hands over stays in shared memory, as do the random streams.
 // One search, 8 trees x 128 playouts, 300 steps: 19.0 ms with two launches a step (63 us, 31 of them the games), 5.9 ms so.
-#ifndef MCTSNC_GOMOKU_BLOCK_PLIES
-#define MCTSNC_GOMOKU_BLOCK_PLIES 8
-#endif
-constexpr int BLOCK_PLIES = MCTSNC_GOMOKU_BLOCK_PLIES;
+constexpr int BLOCK_PLIES = 8;
 template <int STRIDE>
 struct BlockMemory {
     unsigned sheet[SHEET_WORDS];

@@ -610,6 +610,11 @@ int stage_roots(mctsnc_handle *h, int batch, const int8_t *boards, const int8_t 
     return send_roots(h, h->root_board, h->h_root_board, sizeof(ulonglong2) * batch, batch, stream);
 }
 
+const void *gomoku_playout_kernel(bool ocp, bool one_tree) {
+    if (ocp) return one_tree ? (const void *)gomoku::playout_dynamic_kernel<true, true> : (const void *)gomoku::playout_dynamic_kernel<true, false>;
+    return one_tree ? (const void *)gomoku::playout_dynamic_kernel<false, true> : (const void *)gomoku::playout_dynamic_kernel<false, false>;
+}
+
 // The kernel that runs an OCP search of Gomoku with a block per tree, its threads and dynamic shared memory: a player for every
 // game of a step up to 256
 const void *gomoku_block_kernel(int playouts, int *threads, size_t *smem) {
@@ -680,32 +685,38 @@ int launch_search_gomoku(mctsnc_handle *h, int batch, int steps, int first, cuda
             return (int)cudaLaunchKernel(kernel, dim3((unsigned)trees), dim3((unsigned)threads), args, smem, stream);
         }
     }
-    // Else two launches per step (tree step, playouts) and a closing backup, all enqueued without waiting.
+    // Else two launches per step (tree step, playouts) and a closing backup, or, where a group is one tree, one launch per step after
+    // the first tree step; all enqueued without waiting.
     //
     // The trees are split into groups, each with a stream of its own: a tree's next step only needs that tree's games to be
     // over, so the groups run out of step with each other and the lanes one tree leaves idle while its longest games finish
     // (up to ~170 plies against a mean of ~85) play the games of the others.  No kernel waits for another: the order inside a
     // group is stream order, the groups are forked from and joined to the caller's stream with events.
     int per_sm = 0;
-    const void *pk = ocp ? (const void *)gomoku::playout_dynamic_kernel<true> : (const void *)gomoku::playout_dynamic_kernel<false>;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pk, gomoku::DYN_THREADS, h->dyn_smem) != cudaSuccess || per_sm < 1) per_sm = 1;
+    const int groups = trees < GOMOKU_STREAMS ? trees : GOMOKU_STREAMS;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gomoku_playout_kernel(ocp, trees == groups), gomoku::DYN_THREADS, h->dyn_smem) != cudaSuccess ||
+        per_sm < 1)
+        per_sm = 1;
     const long long resident = (long long)per_sm * h->sm_count;
     h->threads = gomoku::DYN_THREADS;
     h->blocks_per_sm = per_sm;
-    const int groups = trees < GOMOKU_STREAMS ? trees : GOMOKU_STREAMS;
     CUDA_TRY(cudaEventRecord(h->g_fork, stream));
     for (int g = 0; g < groups; g++) CUDA_TRY(cudaStreamWaitEvent(h->g_stream[g], h->g_fork, 0));
     for (int s = 0; s <= steps; s++) {
-        p.first = (first && s == 0) ? 1 : 0;
-        p.backup_only = s == steps ? 1 : 0;
         for (int g = 0; g < groups; g++) {
             const int t0 = (int)((long long)trees * g / groups), t1 = (int)((long long)trees * (g + 1) / groups);
             const int n = t1 - t0;
             p.tree_base = t0;
             cudaStream_t gs = h->g_stream[g];
-            if (ocp) gomoku::tree_step_kernel<true><<<n, 32, 0, gs>>>(p);
-            else gomoku::tree_step_kernel<false><<<n, 32, 0, gs>>>(p);
+            if (s == 0 || n > 1) {   // the playouts of one tree make the tree's step that follows them
+                p.first = (first && s == 0) ? 1 : 0;
+                p.backup_only = s == steps ? 1 : 0;
+                if (ocp) gomoku::tree_step_kernel<true><<<n, 32, 0, gs>>>(p);
+                else gomoku::tree_step_kernel<false><<<n, 32, 0, gs>>>(p);
+            }
             if (s == steps) continue;
+            p.first = 0;
+            p.backup_only = s + 1 == steps ? 1 : 0;
             // Blocks of the launch.  A lane for every game while that does not oversubscribe the device much (OCP: one child
             // per tree); otherwise 1.5 to 2 times the group's share of the blocks that fit on the device at once, so that a
             // lane plays several games one after the other and its warp stays full, and blocks are waiting to start
@@ -718,8 +729,9 @@ int launch_search_gomoku(mctsnc_handle *h, int batch, int steps, int first, cuda
             if (blocks > enough) blocks = enough;
             if (blocks > resident) blocks = resident;
             if (blocks < 1) blocks = 1;
-            if (ocp) gomoku::playout_dynamic_kernel<true><<<(unsigned)blocks, gomoku::DYN_THREADS, h->dyn_smem, gs>>>(p, n);
-            else gomoku::playout_dynamic_kernel<false><<<(unsigned)blocks, gomoku::DYN_THREADS, h->dyn_smem, gs>>>(p, n);
+            int count = n;
+            void *play_args[] = {&p, &count};
+            CUDA_TRY(cudaLaunchKernel(gomoku_playout_kernel(ocp, n == 1), dim3((unsigned)blocks), dim3(gomoku::DYN_THREADS), play_args, h->dyn_smem, gs));
         }
     }
     for (int g = 0; g < groups; g++) {
@@ -1001,14 +1013,12 @@ extern "C" int mctsnc_create(const mctsnc_config *cfg, mctsnc_handle **out) {
     const bool ocp = is_ocp(c);
     h->rng_per_search = ocp ? (long long)c.n_trees * c.n_playouts : (long long)c.n_trees * h->A * c.n_playouts;
     h->dyn_smem = sizeof(ulonglong2) * (size_t)(h->rng_per_search / c.n_trees);
-    if (is_gomoku(c))   // per-thread game state + per-warp templates + the tables of the exactly-five test
+    if (is_gomoku(c))   // per-thread game state + per-warp sheets
         h->dyn_smem = gomoku::DYN_SMEM_BYTES;
     if (h->dyn_smem > 28 * 1024) {   // with the kernels' static part more than the 48 KB every launch may have
-        const void *kernels[2] = {is_gomoku(c) ? (ocp ? (const void *)gomoku::playout_dynamic_kernel<true> : (const void *)gomoku::playout_dynamic_kernel<false>)
-                                               : search_kernel_ptr(c, false),
-                                  is_gomoku(c) ? nullptr : search_kernel_ptr(c, true)};
+        const void *kernels[2] = {is_gomoku(c) ? gomoku_playout_kernel(ocp, false) : search_kernel_ptr(c, false),
+                                  is_gomoku(c) ? gomoku_playout_kernel(ocp, true) : search_kernel_ptr(c, true)};
         for (const void *kernel : kernels) {
-            if (!kernel) continue;
             // the limit belongs to the kernel, not to the handle: never lower what another handle (or a launch) has asked for
             cudaFuncAttributes now;
             cudaError_t e = cudaFuncGetAttributes(&now, kernel);

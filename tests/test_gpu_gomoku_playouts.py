@@ -56,3 +56,15 @@ def test_a_line_of_five_on_the_root_is_not_a_win_of_later_stones(variant):
         orc.run(board, None, turn, 6)
         compare(ai, orc)
         assert int(best) == orc.best_action and ai._res["plies"] == orc.plies
+
+
+@pytest.mark.parametrize("seed,stones", [(10, 0), (7, 20), (12, 20)])
+def test_a_draw_of_one_is_replayed_like_the_oracle(seed, stones):
+    steps = 6
+    ai, orc = make_pair("acp_prodigal", 1, 64, steps, seed=seed)
+    board = spread_root(7, stones)
+    best = ai.run(board, None, 1)
+    orc.run(board, None, 1, steps)
+    compare(ai, orc)
+    assert orc.ub_draws > 0 and ai._res["ub_draws"] == orc.ub_draws
+    assert int(best) == orc.best_action and ai._res["plies"] == orc.plies
