@@ -85,3 +85,19 @@ def test_widening_tickets_are_unique_under_contention(variant):
         slots = [pv.decode(x)[1] for x in h["out_selected"][t] if pv.decode(x)[0] == pv.EXPAND]
         assert sorted(slots) == [1, 2, 3, 4]
     assert (h["node_expand_inflight"][:, 0] == 4).all()
+
+
+@pytest.mark.parametrize("variant", VARIANTS)
+@pytest.mark.parametrize("edges,c_pw", [(64, 0.0), (64, 0.02), (256, 0.0), (40, 0.0)])
+def test_edges_that_lead_to_the_same_child_count_its_visits_once_each(variant, edges, c_pw):
+    """The counters are per child node, so a node met by several edges gives each of them the visits it had before the level.
+    Edges e and e + 32 share their child: one lane visits it twice, in that order."""
+    base = pv.from_v3_case(po.layered_case(trees=60, edges=edges, depth=4, warps=1, seed=edges, nodes_per_level=32))
+    rng = np.random.default_rng(edges)
+    base["edge_n"] = rng.integers(0, 3, base["edge_n"].shape).astype(np.int32)     # counts that the visits weigh against
+    base["edge_w"] = (base["edge_n"] * rng.uniform(-1, 1, base["edge_n"].shape)).astype(np.float32)
+    base["node_inflight"] = rng.integers(0, 3, base["node_inflight"].shape).astype(np.int32)
+    want = pv.select(copy.deepcopy(base), cpuct=1.5, c_pw=c_pw, variant=variant)
+    _, got = run_select(copy.deepcopy(base), variant, cpuct=1.5, c_pw=c_pw)
+    for key in ("out_selected", "out_path", "out_len", "node_inflight", "node_expand_inflight"):
+        assert np.array_equal(got[key], want[key]), key
