@@ -42,6 +42,9 @@ __device__ __forceinline__ unsigned ordered(float v) {
     return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
 }
 
+// a counter that can take a visit: not a corrupt (negative) one, nor one at its largest value (:328-347)
+__device__ __forceinline__ bool claimable(int count) { return (unsigned)count < 0x7FFFFFFFu; }
+
 // give back the visit of every child on the first `depth` path entries (:291-311)
 __device__ __forceinline__ void rollback(const int *path, int depth, int lane, const int *edge_child_id, int *node_inflight,
                                          long long tree_nodes_base, long long tree_edges_base, int node_cnt, int edges) {
@@ -215,11 +218,11 @@ select_kernel(float cpuct, float c_pw, float alpha_pw, const int *__restrict__ e
             int claim = 0;   // bit 0: held, bit 1: conflict
             if (lane == (up_best & 31)) {
                 int *counter = node_inflight + up_child;
-                bool can_claim = true, got = up_seen >= 0 && up_old == up_seen;
+                bool can_claim = true, got = claimable(up_seen) && up_old == up_seen;
                 int old = up_old;
                 if (got) old = up_seen;
                 for (int t = 1; t < MAX_CLAIM_RETRY && !got; t++) {
-                    if (old < 0 || old >= 0x7FFFFFFF) {
+                    if (!claimable(old)) {
                         can_claim = false;
                         break;
                     }
@@ -356,9 +359,9 @@ select_kernel(float cpuct, float c_pw, float alpha_pw, const int *__restrict__ e
         } else if (child >= 0) {
             next_info = expanded[child];
             r.request(child, lane, edges);
-            // predicated, so that nothing behind it waits for the answer; a corrupt (negative) count is only read
+            // predicated, so that nothing behind it waits for the answer; a count that cannot take a visit is only read
             asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %4, %5;\n\t@p atom.global.cas.b32 %0, [%1], %2, %3;\n\t}"
-                         : "+r"(up_old) : "l"(node_inflight + child), "r"(my_seen), "r"(my_seen >= 0 ? my_seen + 1 : my_seen), "r"(lane),
+                         : "+r"(up_old) : "l"(node_inflight + child), "r"(my_seen), "r"(claimable(my_seen) ? my_seen + 1 : my_seen), "r"(lane),
                            "r"(best & 31) : "memory");
             pending = true;
             up_node = node;

@@ -101,3 +101,18 @@ def test_edges_that_lead_to_the_same_child_count_its_visits_once_each(variant, e
     _, got = run_select(copy.deepcopy(base), variant, cpuct=1.5, c_pw=c_pw)
     for key in ("out_selected", "out_path", "out_len", "node_inflight", "node_expand_inflight"):
         assert np.array_equal(got[key], want[key]), key
+
+
+@pytest.mark.parametrize("visits", [0x7FFFFFFE, 0x7FFFFFFF, -1])
+def test_a_counter_that_cannot_take_a_visit_is_left_alone(visits):
+    """Counter-CAS refuses a child whose counter is negative or at its largest value."""
+    base = pv.make_case(trees=2, nodes=3, actions=4, path_depth=4)
+    base["node_expanded"][:, 0] = 1
+    base["node_expanded"][:, 1] = pv.NODE_TERMINAL
+    base["edge_child"][:, 0, 0] = 1
+    base["node_inflight"][:, 1] = visits
+    with np.errstate(all="ignore"):
+        want = pv.select(copy.deepcopy(base), cpuct=1.5, c_pw=0.0, variant=puct.V2_COUNTER_CAS)
+    _, got = run_select(copy.deepcopy(base), puct.V2_COUNTER_CAS, cpuct=1.5, c_pw=0.0)
+    for key in ("out_selected", "out_len", "node_inflight"):
+        assert np.array_equal(got[key], want[key]), key
