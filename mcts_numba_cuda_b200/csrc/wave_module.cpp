@@ -153,6 +153,12 @@ bool count_is(Py_ssize_t got, Py_ssize_t want) {
     return false;
 }
 
+// the arguments of a launch: as many as there should be, and launchers to hand them to
+bool ready(Py_ssize_t got, Py_ssize_t want) {
+    if (!fn.duct_backup) PyErr_SetString(PyExc_RuntimeError, "no launchers: bind() has not been called");
+    return fn.duct_backup && count_is(got, want);
+}
+
 // the launch itself: other Python threads may run meanwhile (it waits where the device's queue is full)
 template <typename Launch>
 PyObject *launched(Launch launch) {
@@ -168,7 +174,7 @@ int whole(PyObject *o) { return (int)PyLong_AsLong(o); }
 
 // puct_select(d, cpuct, c_pw, alpha_pw, soft_winner, virtual_loss, stream) -> error code
 PyObject *puct_select(PyObject *, PyObject *const *a, Py_ssize_t n) {
-    if (!count_is(n, 7)) return nullptr;
+    if (!ready(n, 7)) return nullptr;
     const float cpuct = real(a[1]), c_pw = real(a[2]), alpha = real(a[3]);
     const int soft = whole(a[4]), vl = whole(a[5]);
     void *stream = PyLong_AsVoidPtr(a[6]), *p[11];
@@ -189,7 +195,7 @@ PyObject *puct_select(PyObject *, PyObject *const *a, Py_ssize_t n) {
 
 // puct_backup(d, values, virtual_loss, stream) -> error code
 PyObject *puct_backup(PyObject *, PyObject *const *a, Py_ssize_t n) {
-    if (!count_is(n, 4)) return nullptr;
+    if (!ready(n, 4)) return nullptr;
     const int vl = whole(a[2]);
     void *stream = PyLong_AsVoidPtr(a[3]), *values, *p[8];
     Shape s;
@@ -201,7 +207,7 @@ PyObject *puct_backup(PyObject *, PyObject *const *a, Py_ssize_t n) {
 
 // puct_v2_select(d, variant, cpuct, c_pw, alpha_pw, stream) -> error code
 PyObject *puct_v2_select(PyObject *, PyObject *const *a, Py_ssize_t n) {
-    if (!count_is(n, 6)) return nullptr;
+    if (!ready(n, 6)) return nullptr;
     const int variant = whole(a[1]);
     const float cpuct = real(a[2]), c_pw = real(a[3]), alpha = real(a[4]);
     void *stream = PyLong_AsVoidPtr(a[5]), *p[11];
@@ -216,7 +222,7 @@ PyObject *puct_v2_select(PyObject *, PyObject *const *a, Py_ssize_t n) {
 
 // puct_v2_backup(d, values, virtual_loss, stream) -> error code
 PyObject *puct_v2_backup(PyObject *, PyObject *const *a, Py_ssize_t n) {
-    if (!count_is(n, 4)) return nullptr;
+    if (!ready(n, 4)) return nullptr;
     const int vl = whole(a[2]);
     void *stream = PyLong_AsVoidPtr(a[3]), *values, *p[9];
     Shape s;
@@ -228,7 +234,7 @@ PyObject *puct_v2_backup(PyObject *, PyObject *const *a, Py_ssize_t n) {
 
 // duct_select(d, cpuct, virtual_loss, stream) -> error code
 PyObject *duct_select(PyObject *, PyObject *const *a, Py_ssize_t n) {
-    if (!count_is(n, 4)) return nullptr;
+    if (!ready(n, 4)) return nullptr;
     const float cpuct = real(a[1]);
     const int vl = whole(a[2]);
     void *stream = PyLong_AsVoidPtr(a[3]), *p[10];
@@ -242,7 +248,7 @@ PyObject *duct_select(PyObject *, PyObject *const *a, Py_ssize_t n) {
 
 // duct_backup(d, values, new_child, virtual_loss, stream) -> error code
 PyObject *duct_backup(PyObject *, PyObject *const *a, Py_ssize_t n) {
-    if (!count_is(n, 5)) return nullptr;
+    if (!ready(n, 5)) return nullptr;
     const int vl = whole(a[3]);
     void *stream = PyLong_AsVoidPtr(a[4]), *values, *new_child, *p[7];
     Shape s;
@@ -258,8 +264,14 @@ PyObject *duct_backup(PyObject *, PyObject *const *a, Py_ssize_t n) {
 PyObject *bind(PyObject *, PyObject *const *a, Py_ssize_t n) {
     if (!count_is(n, 7)) return nullptr;
     void *p[7];
-    for (int i = 0; i < 7; i++) p[i] = PyLong_AsVoidPtr(a[i]);
-    if (PyErr_Occurred()) return nullptr;
+    for (int i = 0; i < 7; i++) {
+        p[i] = PyLong_AsVoidPtr(a[i]);
+        if (PyErr_Occurred()) return nullptr;
+        if (!p[i]) {
+            PyErr_Format(PyExc_ValueError, "bind: launcher %d has no address", i);
+            return nullptr;
+        }
+    }
     fn.puct_select = (PuctSelect)p[0];
     fn.puct_select_vl = (PuctSelectVl)p[1];
     fn.puct_backup = (PuctBackup)p[2];

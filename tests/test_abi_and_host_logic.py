@@ -3,6 +3,8 @@ follows the reference (validation messages, memory model, tpb table, budget rule
 import ctypes
 import os
 import re
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -159,3 +161,28 @@ def test_drop_in_import_as_top_level_module():
             "ai = MCTSNC((6, 7), 7, 7, verbose_info=False); print(type(ai).__module__, ai.variant)" % pkg)
     out = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, check=True).stdout.split()
     assert out == ["mctsnc", "acp_prodigal"]
+
+
+def test_the_wave_extension_refuses_to_launch_before_it_has_the_launchers():
+    """In a process of its own: an extension without the library's addresses, and one handed a null address."""
+    code = ("from mcts_numba_cuda_b200 import _wave\n"
+            "class Array:\n"
+            "    shape = (1, 1, 1, 1)\n"
+            "    def data_ptr(self): return 0\n"
+            "class Arrays(dict):\n"
+            "    def __missing__(self, key): return Array()\n"
+            "d = Arrays(trees=1, warps=1)\n"
+            "calls = [lambda: _wave.puct_select(d, 1.0, 0.0, 0.5, 0, 1, 0), lambda: _wave.puct_select(d, 1.0, 0.0, 0.5, 0, 3, 0),\n"
+            "         lambda: _wave.puct_backup(d, None, 1, 0), lambda: _wave.puct_v2_select(d, 0, 1.0, 0.0, 0.5, 0),\n"
+            "         lambda: _wave.puct_v2_backup(d, None, 1, 0), lambda: _wave.duct_select(d, 1.0, 1, 0),\n"
+            "         lambda: _wave.duct_backup(d, None, None, 1, 0)]\n"
+            "for unbound in (lambda: None, lambda: _wave.bind(1, 1, 1, 0, 1, 1, 1)):\n"
+            "    try: unbound()\n"
+            "    except ValueError: pass\n"
+            "    for call in calls:\n"
+            "        try: call()\n"
+            "        except RuntimeError as e: assert 'bind' in str(e)\n"
+            "        else: raise SystemExit('launched')\n"
+            "print('refused')\n")
+    res = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=120)
+    assert res.returncode == 0 and res.stdout.strip() == "refused", (res.returncode, res.stdout, res.stderr)
