@@ -11,8 +11,9 @@ LIB_PATH = os.path.join(HERE, "libmctsnc_b200.so")
 WAVE_PATH = os.path.join(HERE, "_wave.so")
 WAVE_SOURCE = os.path.join(HERE, "csrc", "wave_module.cpp")
 SOURCES = [os.path.join(HERE, "csrc", n) for n in ("mctsnc_abi.cu", "peer_exchange.cu", "puct_select.cu", "puct_select_v2.cu", "duct_select.cu")]
-HEADERS = [os.path.join(HERE, "csrc", n) for n in ("c4_search.cuh", "gomoku_search.cuh", "common.cuh", "rng.cuh", "select_math.cuh")] + [
-    os.path.join(ROOT, "include", "mctsnc_b200.h")]
+HEADERS = [os.path.join(HERE, "csrc", n) for n in ("c4_search.cuh", "gomoku_search.cuh", "common.cuh", "rng.cuh", "select_math.cuh")]
+WAVE_HEADERS = [os.path.join(ROOT, "include", n) for n in ("puct_b200.h", "duct_b200.h")]
+HEADERS += WAVE_HEADERS + [os.path.join(ROOT, "include", "mctsnc_b200.h")]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-shared",
               "-Xcompiler", "-fPIC"]
 
@@ -33,7 +34,7 @@ def is_stale(path=LIB_PATH, sources=SOURCES + HEADERS):
 
 def build(force=False, verbose=False):
     """Compiles the library and the extension if they are missing or older than their sources; returns the library's path."""
-    if force or is_stale(WAVE_PATH, [WAVE_SOURCE]):
+    if force or is_stale(WAVE_PATH, [WAVE_SOURCE] + WAVE_HEADERS):
         cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-I" + sysconfig.get_paths()["include"], "-o", WAVE_PATH,
                WAVE_SOURCE]
         res = subprocess.run(cmd, capture_output=True, text=True)

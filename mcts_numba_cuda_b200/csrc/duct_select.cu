@@ -15,6 +15,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "../../include/duct_b200.h"
 #include "select_math.cuh"
 
 namespace duct {

@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "../../include/puct_b200.h"
 #include "select_math.cuh"
 
 namespace puct_v2 {

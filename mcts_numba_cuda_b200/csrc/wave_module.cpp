@@ -6,31 +6,20 @@
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
+#include "../../include/duct_b200.h"
+#include "../../include/puct_b200.h"
+
 namespace {
 
-typedef int (*PuctSelect)(float, float, float, int, const int *, const float *, const float *, const int *, int *, int *, const int *,
-                          const int *, int *, int *, int *, int, int, int, int, int, void *);
-typedef int (*PuctSelectVl)(float, float, float, int, int, const int *, const float *, const float *, const int *, int *, int *,
-                            const int *, const int *, int *, int *, int *, int, int, int, int, int, void *);
-typedef int (*PuctBackup)(int, float *, int *, int *, int *, const int *, const int *, const int *, const int *, const float *, int, int,
-                          int, int, int, void *);
-typedef int (*PuctV2Select)(int, float, float, float, const int *, const float *, const float *, const int *, int *, int *, const int *,
-                            const int *, int *, int *, int *, int, int, int, int, int, void *);
-typedef int (*PuctV2Backup)(int, const int *, float *, int *, int *, int *, const int *, const int *, const int *, const int *,
-                            const float *, int, int, int, int, int, void *);
-typedef int (*DuctSelect)(float, int, int *, const float *, const float *, const int *, int *, const int *, const int *, int *, int *,
-                          int *, int, int, int, int, int, void *);
-typedef int (*DuctBackup)(int, int *, float *, int *, int *, const int *, const int *, const int *, const float *, const int *, int, int,
-                          int, int, int, void *);
-
+// the launchers' types are those of the public headers: a launcher whose arguments change does not compile here
 struct {
-    PuctSelect puct_select;
-    PuctSelectVl puct_select_vl;
-    PuctBackup puct_backup;
-    PuctV2Select puct_v2_select;
-    PuctV2Backup puct_v2_backup;
-    DuctSelect duct_select;
-    DuctBackup duct_backup;
+    decltype(&puct_select_winner_recalc_launch) puct_select;
+    decltype(&puct_select_virtual_loss_launch) puct_select_vl;
+    decltype(&puct_backup_launch) puct_backup;
+    decltype(&puct_v2_select_launch) puct_v2_select;
+    decltype(&puct_v2_backup_launch) puct_v2_backup;
+    decltype(&duct_select_launch) duct_select;
+    decltype(&duct_backup_launch) duct_backup;
 } fn;
 
 enum Key { EDGE_CHILD, EDGE_PRIOR, EDGE_W, EDGE_N, EDGE_INFLIGHT, NODE_INFLIGHT, NODE_EXPAND_INFLIGHT, NODE_EXPANDED, NODE_COUNT,
@@ -272,13 +261,13 @@ PyObject *bind(PyObject *, PyObject *const *a, Py_ssize_t n) {
             return nullptr;
         }
     }
-    fn.puct_select = (PuctSelect)p[0];
-    fn.puct_select_vl = (PuctSelectVl)p[1];
-    fn.puct_backup = (PuctBackup)p[2];
-    fn.puct_v2_select = (PuctV2Select)p[3];
-    fn.puct_v2_backup = (PuctV2Backup)p[4];
-    fn.duct_select = (DuctSelect)p[5];
-    fn.duct_backup = (DuctBackup)p[6];
+    fn.puct_select = (decltype(fn.puct_select))p[0];
+    fn.puct_select_vl = (decltype(fn.puct_select_vl))p[1];
+    fn.puct_backup = (decltype(fn.puct_backup))p[2];
+    fn.puct_v2_select = (decltype(fn.puct_v2_select))p[3];
+    fn.puct_v2_backup = (decltype(fn.puct_v2_backup))p[4];
+    fn.duct_select = (decltype(fn.duct_select))p[5];
+    fn.duct_backup = (decltype(fn.duct_backup))p[6];
     Py_RETURN_NONE;
 }
 
