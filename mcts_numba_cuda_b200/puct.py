@@ -20,7 +20,7 @@ def _launcher():
         try:
             from . import _wave as module
         except ImportError as e:
-            raise RuntimeError("mcts_numba_cuda_b200/_wave.so is missing: build it with `python -m mcts_numba_cuda_b200.build`") from e
+            raise RuntimeError("the extension mcts_numba_cuda_b200/_wave is missing: build it with `python -m mcts_numba_cuda_b200.build`") from e
         L = _abi.lib()
         module.bind(*(ctypes.cast(getattr(L, name), ctypes.c_void_p).value for name in (
             "puct_select_winner_recalc_launch", "puct_select_virtual_loss_launch", "puct_backup_launch", "puct_v2_select_launch",

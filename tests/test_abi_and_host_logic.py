@@ -1,15 +1,17 @@
 """CPU-side checks: the C-ABI library loads and exports what the header declares, the host logic of the drop-in class
 follows the reference (validation messages, memory model, tpb table, budget rule), and nothing computes without a GPU."""
 import ctypes
+import importlib
 import os
 import re
 import subprocess
 import sys
+import sysconfig
 
 import numpy as np
 import pytest
 
-from mcts_numba_cuda_b200 import MCTSNC, _abi
+from mcts_numba_cuda_b200 import MCTSNC, _abi, build
 from mcts_numba_cuda_b200.distributed import reduce_over_actions_host, shard_trees
 from mcts_numba_cuda_b200.roots import c4_random_roots
 
@@ -186,3 +188,28 @@ def test_the_wave_extension_refuses_to_launch_before_it_has_the_launchers():
             "print('refused')\n")
     res = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=120)
     assert res.returncode == 0 and res.stdout.strip() == "refused", (res.returncode, res.stdout, res.stderr)
+
+
+@pytest.mark.parametrize("missing", [False, True])
+def test_a_failing_extension_build_leaves_the_library_built(monkeypatch, missing):
+    """A machine with nvcc but without a C++ compiler on the path, or without Python.h, still gets the library."""
+    commands = []
+
+    def run(cmd, **kw):
+        commands.append(cmd)
+        if "wave_module.cpp" in cmd[-1]:
+            if missing:
+                raise FileNotFoundError(cmd[0])
+            return subprocess.CompletedProcess(cmd, 1, "", "Python.h: No such file or directory")
+        return subprocess.CompletedProcess(cmd, 0, "", "")
+
+    monkeypatch.setattr(build.subprocess, "run", run)
+    with pytest.warns(RuntimeWarning, match="extension"):
+        assert build.build(force=True) == build.LIB_PATH
+    assert any(build.LIB_PATH in cmd for cmd in commands)
+
+
+def test_the_extension_is_named_for_its_interpreter():
+    """Another interpreter on the same checkout finds it stale and builds its own."""
+    assert build.WAVE_PATH == os.path.join(build.HERE, "_wave" + sysconfig.get_config_var("EXT_SUFFIX"))
+    assert os.path.samefile(importlib.import_module("mcts_numba_cuda_b200._wave").__file__, build.WAVE_PATH)
