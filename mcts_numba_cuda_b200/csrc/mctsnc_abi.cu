@@ -610,8 +610,9 @@ int stage_roots(mctsnc_handle *h, int batch, const int8_t *boards, const int8_t 
     return send_roots(h, h->root_board, h->h_root_board, sizeof(ulonglong2) * batch, batch, stream);
 }
 
+// one_tree: acp only (ocp searches of few trees run in gomoku_block_kernel)
 const void *gomoku_playout_kernel(bool ocp, bool one_tree) {
-    if (ocp) return one_tree ? (const void *)gomoku::playout_dynamic_kernel<true, true> : (const void *)gomoku::playout_dynamic_kernel<true, false>;
+    if (ocp) return (const void *)gomoku::playout_dynamic_kernel<true, false>;
     return one_tree ? (const void *)gomoku::playout_dynamic_kernel<false, true> : (const void *)gomoku::playout_dynamic_kernel<false, false>;
 }
 
@@ -685,8 +686,8 @@ int launch_search_gomoku(mctsnc_handle *h, int batch, int steps, int first, cuda
             return (int)cudaLaunchKernel(kernel, dim3((unsigned)trees), dim3((unsigned)threads), args, smem, stream);
         }
     }
-    // Else two launches per step (tree step, playouts) and a closing backup, or, where a group is one tree, one launch per step after
-    // the first tree step; all enqueued without waiting.
+    // Else two launches per step (tree step, playouts) and a closing backup, or, where a group of an acp search is one tree, one launch
+    // per step after the first tree step; all enqueued without waiting.
     //
     // The trees are split into groups, each with a stream of its own: a tree's next step only needs that tree's games to be
     // over, so the groups run out of step with each other and the lanes one tree leaves idle while its longest games finish
@@ -706,9 +707,10 @@ int launch_search_gomoku(mctsnc_handle *h, int batch, int steps, int first, cuda
         for (int g = 0; g < groups; g++) {
             const int t0 = (int)((long long)trees * g / groups), t1 = (int)((long long)trees * (g + 1) / groups);
             const int n = t1 - t0;
+            const bool one_tree = !ocp && n == 1;
             p.tree_base = t0;
             cudaStream_t gs = h->g_stream[g];
-            if (s == 0 || n > 1) {   // the playouts of one tree make the tree's step that follows them
+            if (s == 0 || !one_tree) {   // the playouts of one tree make the tree's step that follows them
                 p.first = (first && s == 0) ? 1 : 0;
                 p.backup_only = s == steps ? 1 : 0;
                 if (ocp) gomoku::tree_step_kernel<true><<<n, 32, 0, gs>>>(p);
@@ -731,7 +733,7 @@ int launch_search_gomoku(mctsnc_handle *h, int batch, int steps, int first, cuda
             if (blocks < 1) blocks = 1;
             int count = n;
             void *play_args[] = {&p, &count};
-            CUDA_TRY(cudaLaunchKernel(gomoku_playout_kernel(ocp, n == 1), dim3((unsigned)blocks), dim3(gomoku::DYN_THREADS), play_args, h->dyn_smem, gs));
+            CUDA_TRY(cudaLaunchKernel(gomoku_playout_kernel(ocp, one_tree), dim3((unsigned)blocks), dim3(gomoku::DYN_THREADS), play_args, h->dyn_smem, gs));
         }
     }
     for (int g = 0; g < groups; g++) {
@@ -789,13 +791,13 @@ int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_
         (long long)(is_ocp(h->cfg) ? 1 : h->A) * h->cfg.n_playouts > MCTSNC_C4_CLUSTER_MIN_GAMES &&
         trees * c4::CLUSTER_BLOCKS <= (long long)MCTSNC_C4_CLUSTER_SM_SHARE * h->sm_count) {
         const bool ocp = is_ocp(h->cfg);
-        // the wide cluster first where a step has games for it, the other one if those do not fit on the device
-        for (int wide = (ocp ? 1 : h->A) * h->cfg.n_playouts >= c4::WIDE_CLUSTER_MIN_GAMES ? 1 : 0; wide >= 0; wide--) {
+        // the wide cluster first where a step has games for it (an ocp step never has: 512 at most), the other one if those do not fit
+        // on the device
+        for (int wide = !ocp && h->A * h->cfg.n_playouts >= c4::WIDE_CLUSTER_MIN_GAMES ? 1 : 0; wide >= 0; wide--) {
             const int blocks = wide ? c4::WIDE_CLUSTER_BLOCKS : c4::CLUSTER_BLOCKS;
-            const void *kernel = wide ? (ocp ? (const void *)c4::search_cluster_kernel<true, c4::WIDE_CLUSTER_BLOCKS, c4::WIDE_CLUSTER_THREADS>
-                                             : (const void *)c4::search_cluster_kernel<false, c4::WIDE_CLUSTER_BLOCKS, c4::WIDE_CLUSTER_THREADS>)
-                                      : (ocp ? (const void *)c4::search_cluster_kernel<true, c4::CLUSTER_BLOCKS, c4::CLUSTER_THREADS>
-                                             : (const void *)c4::search_cluster_kernel<false, c4::CLUSTER_BLOCKS, c4::CLUSTER_THREADS>);
+            const void *kernel = wide  ? (const void *)c4::search_cluster_kernel<false, c4::WIDE_CLUSTER_BLOCKS, c4::WIDE_CLUSTER_THREADS>
+                                 : ocp ? (const void *)c4::search_cluster_kernel<true, c4::CLUSTER_BLOCKS, c4::CLUSTER_THREADS>
+                                       : (const void *)c4::search_cluster_kernel<false, c4::CLUSTER_BLOCKS, c4::CLUSTER_THREADS>;
             if (wide && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
                 cudaGetLastError();
                 continue;
