@@ -1016,8 +1016,8 @@ __global__ void __maxnreg__(MCTSNC_C4_MAXNREG) search_kernel(const SearchParams 
 
 // A cluster of CL blocks per tree: launches with few trees (one search), where a step of a tree is bound by what one SM can play.
 // Launched with the cluster dimension as a launch attribute; cluster c grows tree c for the whole launch.  THREADS: of a block.
-template <bool OCP, int CL, int THREADS>
-__global__ void __launch_bounds__(THREADS) search_cluster_kernel(const SearchParams p) {
+template <bool OCP, int CL>
+__device__ __forceinline__ void run_cluster(const SearchParams &p) {
     __shared__ Shared s;
     extern __shared__ ulonglong2 s_rng[];
     build_move_lut(s);
@@ -1025,12 +1025,23 @@ __global__ void __launch_bounds__(THREADS) search_cluster_kernel(const SearchPar
     run_slice<OCP, CL, true>(p, s, s_rng, reinterpret_cast<int4 *>(s_rng + n_local), (int)(blockIdx.x / CL), p.steps, p.first != 0);
 }
 
+template <bool OCP, int CL, int THREADS>
+__global__ void __launch_bounds__(THREADS) search_cluster_kernel(const SearchParams p) { run_cluster<OCP, CL>(p); }
+
 // Clusters of 8 blocks of 256 threads, or -- for steps with more games than those blocks can play one to a thread while a warp
 // walks -- of 16 blocks of 128 and a warp for the walk: a scheduler has one warp of games then instead of two.  4 trees, ACP 64 /
 // 128 / 256 / 512 playouts, us a step: 5.6 / 5.6 / 7.2 / 9.9 with 8 blocks, 6.0 / 6.0 / 6.8 / 8.4 with 16 (the barriers of the larger
 // cluster cost more).
 constexpr int CLUSTER_BLOCKS = 8, CLUSTER_THREADS = 256;
 constexpr int WIDE_CLUSTER_BLOCKS = 16, WIDE_CLUSTER_THREADS = 160, WIDE_CLUSTER_MIN_GAMES = CLUSTER_BLOCKS * (CLUSTER_THREADS - 32);
+
+// The same with the registers capped so that four blocks share an SM, for trees whose clusters do not fit otherwise (33 to 64 trees
+// on 148 SMs, 64 registers instead of 128): 4 x 256 acp, 500 steps, 9 / 12 / 16 searches in one launch 4.97 / 5.58 / 6.99 ms against
+// 11.14 with a block per tree.  Where both fit the cap costs: 1 / 8 searches of 4 x 64 acp 3.16 / 3.57 ms against 2.91 / 3.24.
+template <bool OCP>
+__global__ void __launch_bounds__(CLUSTER_THREADS, 4) search_packed_cluster_kernel(const SearchParams p) {
+    run_cluster<OCP, CLUSTER_BLOCKS>(p);
+}
 
 }  // namespace c4
 }  // namespace mctsnc

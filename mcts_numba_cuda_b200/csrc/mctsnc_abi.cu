@@ -72,7 +72,7 @@ struct mctsnc_handle {
     int tpb_roa = 0;
     int sm_count = 0;
     bool cluster_ok = false;      // thread-block clusters can be launched (and MCTSNC_B200_NO_CLUSTER is not set)
-    int cluster_fit[2][2] = {};   // clusters that fit on the device at once, [wide][small record cache] (0: not asked yet, -1: unknown)
+    int cluster_fit[3][2] = {};   // clusters that fit on the device at once, [ClusterForm][small record cache] (0: not asked yet, -1: unknown)
     int threads = 0;
     int blocks_per_sm = 0;
     long long bytes = 0;
@@ -743,6 +743,16 @@ int launch_search_gomoku(mctsnc_handle *h, int batch, int steps, int first, cuda
     return (int)cudaGetLastError();
 }
 
+// the forms a cluster per tree comes in, in the order they are tried
+enum ClusterForm { WIDE, PLAIN, PACKED };
+
+const void *cluster_kernel_ptr(bool ocp, int form) {
+    if (form == WIDE) return (const void *)c4::search_cluster_kernel<false, c4::WIDE_CLUSTER_BLOCKS, c4::WIDE_CLUSTER_THREADS>;   // acp only
+    if (form == PACKED) return ocp ? (const void *)c4::search_packed_cluster_kernel<true> : (const void *)c4::search_packed_cluster_kernel<false>;
+    return ocp ? (const void *)c4::search_cluster_kernel<true, c4::CLUSTER_BLOCKS, c4::CLUSTER_THREADS>
+               : (const void *)c4::search_cluster_kernel<false, c4::CLUSTER_BLOCKS, c4::CLUSTER_THREADS>;
+}
+
 int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_t stream) {
     if (is_gomoku(h->cfg)) return launch_search_gomoku(h, batch, steps, first, stream);
     SearchParams p;
@@ -791,13 +801,12 @@ int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_
         (long long)(is_ocp(h->cfg) ? 1 : h->A) * h->cfg.n_playouts > MCTSNC_C4_CLUSTER_MIN_GAMES &&
         trees * c4::CLUSTER_BLOCKS <= (long long)MCTSNC_C4_CLUSTER_SM_SHARE * h->sm_count) {
         const bool ocp = is_ocp(h->cfg);
-        // the wide cluster first where a step has games for it (an ocp step never has: 512 at most), the other one if those do not fit
+        // the wide cluster first where a step has games for it (an ocp step never has: 512 at most); then the first form that fits
         // on the device
-        for (int wide = !ocp && h->A * h->cfg.n_playouts >= c4::WIDE_CLUSTER_MIN_GAMES ? 1 : 0; wide >= 0; wide--) {
+        for (int form = !ocp && h->A * h->cfg.n_playouts >= c4::WIDE_CLUSTER_MIN_GAMES ? WIDE : PLAIN; form <= PACKED; form++) {
+            const bool wide = form == WIDE;
             const int blocks = wide ? c4::WIDE_CLUSTER_BLOCKS : c4::CLUSTER_BLOCKS;
-            const void *kernel = wide  ? (const void *)c4::search_cluster_kernel<false, c4::WIDE_CLUSTER_BLOCKS, c4::WIDE_CLUSTER_THREADS>
-                                 : ocp ? (const void *)c4::search_cluster_kernel<true, c4::CLUSTER_BLOCKS, c4::CLUSTER_THREADS>
-                                       : (const void *)c4::search_cluster_kernel<false, c4::CLUSTER_BLOCKS, c4::CLUSTER_THREADS>;
+            const void *kernel = cluster_kernel_ptr(ocp, form);
             if (wide && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
                 cudaGetLastError();
                 continue;
@@ -817,13 +826,13 @@ int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_
             // The first records of a tree stay in the first block's shared memory: many if every block can have an SM to itself,
             // else few.  All clusters of the launch have to be on the device at once (clusters do not spread over GPCs, so fewer
             // fit than blocks / 8): a tree whose cluster waits for another to finish would take two searches' time.  A wide cluster
-            // is for blocks that have an SM each.
+            // is for blocks that have an SM each, a packed one for blocks that share it.
             bool fits = false;
             const bool own_sm = trees * blocks <= h->sm_count;
-            for (int small = own_sm ? 0 : 1; small < (wide ? 1 : 2) && !fits; small++) {
+            for (int small = own_sm && form != PACKED ? 0 : 1; small < (wide ? 1 : 2) && !fits; small++) {
                 p.cache_nodes = small ? 2048 : MCTSNC_C4_CACHE_NODES;
                 lc.dynamicSmemBytes = h->dyn_smem / blocks + sizeof(int4) * (size_t)p.cache_nodes;
-                int &fit = h->cluster_fit[wide][small];
+                int &fit = h->cluster_fit[form][small];
                 if (fit == 0) {
                     int n = 0;
                     const cudaError_t q = cudaOccupancyMaxActiveClusters(&n, kernel, &lc);

@@ -373,3 +373,20 @@ def test_slice_trace_accounts_for_every_step_of_every_tree():
     assert len(ai.read_slices()) == 0
     for name in ("best_action", "best_n", "best_n_wins", "actions_ns"):
         assert np.array_equal(plain[name], again[name]), name
+
+
+@pytest.mark.parametrize("variant,n_playouts,roots", [("acp_prodigal", 256, 9), ("acp_thrifty", 512, 16), ("acp_prodigal", 64, 12), ("ocp_prodigal", 512, 14)])
+def test_clusters_that_share_their_sms_match_the_oracle(variant, n_playouts, roots):
+    """36 to 64 trees: four blocks of a cluster on an SM, in place of a block per tree, which is up to twice as slow."""
+    steps, T = 40, 4
+    boards, fills, turns = c4_random_roots(roots, 20, seed=roots)
+    ai = MCTSNC((6, 7), 7, 7, search_time_limit=np.inf, search_steps_limit=steps, n_trees=T, n_playouts=n_playouts, variant=variant, seed=8,
+                verbose_info=False, max_batch=roots)
+    ai.init_device_side_arrays()
+    out = ai.run_batch(boards, fills, turns, steps=steps, reseed=True)
+    assert ai.launch_geometry()["threads_per_tree"] == 8 * 256
+    for b in (0, roots // 2, roots - 1):
+        orc = OracleMCTSNC((6, 7), 7, 7, n_trees=T, n_playouts=n_playouts, variant=variant, seed=8, node_capacity=steps * 7 + 8)
+        orc.run(boards[b], fills[b], int(turns[b]), steps)
+        compare_trees(ai, orc, search=b)
+        assert out["best_action"][b] == orc.best_action and out["plies"][b] == orc.plies
