@@ -114,10 +114,14 @@ struct PathTerm {
 //
 // Each ring is a bounded multi-producer multi-consumer queue with a sequence number per cell (cell i is free for the
 // push with ticket t when seq == t, holds the data of that push when seq == t + 1, and is handed to ticket t + cap by
-// the pop).  `nonempty` has one bit per ring, set after a push and cleared by a pop that found the ring empty and, after
-// clearing, still sees it empty.  Every loop is bounded and no call waits for another block: a pop that finds nothing
-// (or gives up) returns -1 and the block leaves, which is safe because a tree is always either in a ring or held by a
-// block that will publish it and pop again.
+// the pop).  Tickets are taken by additions that never have to be tried again: a push takes one of `tail`, a pop first takes one of
+// the `ready` trees (and puts it back where there is none) and then a ticket of `head`.  (With compare-and-swap loops on head and
+// tail the 2368 one- and two-warp blocks of a full device took turns failing, and the launch waited for the queue: 2380 trees of 4 x 128
+// ocp, 150 steps, 11.8 ms where 2360, which need no queue, take 4.4.)  `nonempty` has one bit per ring, set after a push and cleared by
+// a pop that found the ring empty and, after clearing, still sees it empty.  Every loop is bounded.  A call waits only for the few
+// instructions another block needs between taking an earlier ticket and using it (a running block, which itself waits for earlier
+// tickets alone); a pop that finds nothing (or gives up) returns -1 and the block leaves, which is safe because a tree is always
+// either in a ring or held by a block that will publish it and pop again.
 constexpr int QUEUE_LEVELS = 64;
 constexpr float QUEUE_LEVELS_PER_OCTAVE = 6.f;  // bands are logarithmic: the estimate's error grows with the time left
 struct QueueCell {
@@ -129,6 +133,8 @@ struct WorkQueue {
     int pad0[31];
     int tail;
     int pad1[31];
+    int ready;       // trees that are in the ring and not promised to a pop
+    int pad2[31];
 };
 struct WorkQueues {
     WorkQueue level[QUEUE_LEVELS];
@@ -137,48 +143,42 @@ struct WorkQueues {
     int pad[29];
 };
 
-constexpr int QUEUE_RETRIES = 1 << 16;  // attempts of a push or pop under contention before it reports failure
+constexpr int QUEUE_POLLS = 1 << 16;  // looks at a cell's number before a push or pop reports failure
 
 #if defined(__CUDACC__)
-__device__ __forceinline__ bool ring_push(WorkQueue *q, QueueCell *ring, int cap, int tree) {
-    for (int attempt = 0; attempt < QUEUE_RETRIES; attempt++) {
-        const int pos = *(volatile int *)&q->tail;
-        QueueCell *cell = ring + (pos % cap);
-        const int dif = *(volatile int *)&cell->seq - pos;
-        if (dif == 0) {
-            if (atomicCAS(&q->tail, pos, pos + 1) == pos) {
-                *(volatile int *)&cell->tree = tree;
-                __threadfence();
-                *(volatile int *)&cell->seq = pos + 1;
-                return true;
-            }
-        } else if (dif < 0) {
-            return false;  // ring full: cannot happen while cap >= number of trees
-        }
-    }
+__device__ __forceinline__ bool cell_is(const QueueCell *cell, int seq) {
+    for (int poll = 0; poll < QUEUE_POLLS; poll++)
+        if (*(volatile const int *)&cell->seq == seq) return true;
     return false;
 }
 
-// -1: nothing published (or QUEUE_RETRIES lost races in a row)
+__device__ __forceinline__ bool ring_push(WorkQueue *q, QueueCell *ring, int cap, int tree) {
+    const int pos = atomicAdd(&q->tail, 1);
+    QueueCell *cell = ring + (pos % cap);
+    if (!cell_is(cell, pos)) return false;   // the pop that held the cell before has not left it
+    *(volatile int *)&cell->tree = tree;
+    __threadfence();
+    *(volatile int *)&cell->seq = pos + 1;
+    __threadfence();
+    atomicAdd(&q->ready, 1);
+    return true;
+}
+
+// -1: nothing published (or the push of the ticket never finished: its tree keeps its steps, which the launch reports)
 __device__ __forceinline__ int ring_pop(WorkQueue *q, QueueCell *ring, int cap) {
-    for (int attempt = 0; attempt < QUEUE_RETRIES; attempt++) {
-        const int pos = *(volatile int *)&q->head;
-        QueueCell *cell = ring + (pos % cap);
-        const int dif = *(volatile int *)&cell->seq - (pos + 1);
-        if (dif == 0) {
-            if (atomicCAS(&q->head, pos, pos + 1) == pos) {
-                __threadfence();
-                const int tree = *(volatile int *)&cell->tree;
-                __threadfence();
-                *(volatile int *)&cell->seq = pos + cap;
-                return tree;
-            }
-        } else if (dif < 0) {
-            // no ticket beyond the head: empty.  Otherwise a push holds the ticket and is about to publish: look again.
-            if (*(volatile int *)&q->tail - pos <= 0) return -1;
-        }
+    if (*(volatile int *)&q->ready <= 0) return -1;
+    if (atomicSub(&q->ready, 1) <= 0) {
+        atomicAdd(&q->ready, 1);
+        return -1;
     }
-    return -1;
+    const int pos = atomicAdd(&q->head, 1);
+    QueueCell *cell = ring + (pos % cap);
+    if (!cell_is(cell, pos + 1)) return -1;
+    __threadfence();
+    const int tree = *(volatile int *)&cell->tree;
+    __threadfence();
+    *(volatile int *)&cell->seq = pos + cap;
+    return tree;
 }
 
 // the caller made the tree's state visible (block barrier after the writes, then this thread's fence) before the push

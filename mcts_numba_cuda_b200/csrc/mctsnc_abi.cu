@@ -155,7 +155,7 @@ __global__ void init_queue_kernel(WorkQueues *q, QueueCell *rings, int *remainin
     for (int i = gid; i < trees; i += gsz) remaining[i] = steps;
     if (gid < QUEUE_LEVELS) {  // blocks have 256 threads
         q->level[gid].head = 0;
-        q->level[gid].tail = gid == QUEUE_LEVELS - 1 ? trees : 0;
+        q->level[gid].tail = q->level[gid].ready = gid == QUEUE_LEVELS - 1 ? trees : 0;
     }
     if (gid == 0) {
         q->nonempty = 1ULL << (QUEUE_LEVELS - 1);

@@ -390,3 +390,28 @@ def test_clusters_that_share_their_sms_match_the_oracle(variant, n_playouts, roo
         orc.run(boards[b], fills[b], int(turns[b]), steps)
         compare_trees(ai, orc, search=b)
         assert out["best_action"][b] == orc.best_action and out["plies"][b] == orc.plies
+
+
+def test_a_few_more_trees_than_fit_take_a_little_longer():
+    """One tree too many for the device and the launch goes through the work queue: thousands of small blocks take their trees from
+    it, and its cost must not show (with retried compare-and-swaps it took 2.7 times as long)."""
+    T, P, steps = 4, 128, 150
+    boards, fills, turns = c4_random_roots(700, 10, seed=0)
+
+    def batch(roots):
+        ai = MCTSNC((6, 7), 7, 7, search_time_limit=np.inf, search_steps_limit=steps, n_trees=T, n_playouts=P, variant="ocp_prodigal",
+                    seed=0, verbose_info=False, max_batch=roots)
+        ai.init_device_side_arrays()
+        outs = [ai.run_batch(boards[:roots], fills[:roots], turns[:roots], steps=steps, reseed=True) for _ in range(4)]
+        geo = ai.launch_geometry()
+        assert all((o["status"] & _abi.STATUS_INTERNAL == 0).all() for o in outs)
+        return min(float(o["device_ms"][0]) for o in outs), outs[0], geo["blocks_per_sm"] * geo["sm_count"]
+
+    fitting = batch(512)[2] // T                   # searches whose trees all have a block
+    assert 512 <= fitting <= 690
+    ms, out, blocks = batch(fitting)
+    ms_more, out_more, blocks_more = batch(fitting + 8)
+    assert fitting * T <= blocks and (fitting + 8) * T > blocks_more
+    for name in ("actions_ns", "actions_ns_wins", "plies"):
+        assert np.array_equal(out[name], out_more[name][:fitting]), name
+    assert ms_more < 1.5 * ms, (ms, ms_more)
