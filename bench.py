@@ -37,11 +37,12 @@ GAMES = {"c4": {"shape": (6, 7), "extra": 7, "actions": 7, "inst_per_ply": 65.0,
 # move pick and placement ~18, line test through the new stone 16 (Connect 4) / ~55 (Gomoku), draw test and loop ~6.
 # It is the yardstick of the issue roofline, not a count of the compiled code.
 
-KERNEL_SOURCES = {"c4": ("c4_search.cuh", "common.cuh", "rng.cuh"), "gomoku": ("gomoku_search.cuh", "common.cuh", "rng.cuh")}
+KERNEL_SOURCES = {"c4": ("c4_search.cuh", "common.cuh", "rng.cuh"), "gomoku": ("gomoku_search.cuh", "common.cuh", "rng.cuh"),
+                  "puct": ("puct_select.cu", "select_math.cuh"), "duct": ("duct_select.cu", "select_math.cuh")}
 
 
 def kernel_source_sha(game):
-    """Identifies the kernel a profile was taken on: hash of the sources the search kernel of `game` is compiled from."""
+    """Identifies the kernel a profile was taken on: hash of the sources the kernel of `game` (or select) is compiled from."""
     import hashlib
     h = hashlib.sha256()
     for name in KERNEL_SOURCES[game]:
@@ -375,19 +376,20 @@ def run_puct(args):
             e1.record()
             torch.cuda.synchronize()
             valid = int((((d["out_selected"] >> 22) & 7) != 4).sum())
+            levels = int(d["out_len"].sum())
             puct.launch_release(d, virtual_loss=release_vl[0])
             torch.cuda.synchronize()
             if i >= args.warmup:
                 times.append(e0.elapsed_time(e1))
         assert int(d["edge_inflight"].abs().sum()) == 0
-        return float(np.mean(times)), valid
+        return float(np.mean(times)), valid, levels
 
     release_vl = [vl]
     sampler = ClockSampler(0)
     sampler.start()
-    ms, valid = timed(lambda: puct.launch_select(d, cpuct=1.5, c_pw=0.0, virtual_loss=vl))
+    ms, valid, levels = timed(lambda: puct.launch_select(d, cpuct=1.5, c_pw=0.0, virtual_loss=vl))
     release_vl[0] = 1
-    ms_vl1, valid1 = timed(lambda: puct.launch_select(d, cpuct=1.5, c_pw=0.0, virtual_loss=1))
+    ms_vl1, valid1, _ = timed(lambda: puct.launch_select(d, cpuct=1.5, c_pw=0.0, virtual_loss=1))
     ref_ms = None
     ref_path = os.path.join(ROOT, "oracle", "_ref", "libpuct_ref_sm100a.so")
     if os.path.exists(ref_path):
@@ -398,12 +400,15 @@ def run_puct(args):
                                                             "node_expand_inflight", "node_expanded", "node_count",
                                                             "out_selected", "out_path", "out_len")]
         nodes = d["edge_child"].shape[1]
-        ref_ms, _ = timed(lambda: lib.puct_select_winner_recalc_launch(1.5, 0.0, 0.5, 0, *ptrs, T, nodes, E, Wp, D,
+        ref_ms, _, _ = timed(lambda: lib.puct_select_winner_recalc_launch(1.5, 0.0, 0.5, 0, *ptrs, T, nodes, E, Wp, D,
                                                                        ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
     clocks = sampler.stop()
     sel = T * Wp
-    bytes_per_sel = D * (16 * E + 16)          # prior, W, N, inflight per edge + node record, child id, path entry, ticket
-    achieved = sel * bytes_per_sel / (ms * 1e-3) / 1e9
+    # prior, W, N, inflight per edge + node record, child id, path entry, ticket, for every level of the finished traversals
+    # (the others lost their claims and read a node or two)
+    bytes_per_level = 16 * E + 16
+    achieved = levels * bytes_per_level / (ms * 1e-3) / 1e9
+    prof = profiler_readings("puct", f"{E},{D},{Wp}")
     line = {"metric": "PUCT selections/sec (select kernel only, CUDA events)", "value": sel / (ms * 1e-3), "unit": "selections/s",
             "n_gpus": 1, "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic",
@@ -414,8 +419,9 @@ def run_puct(args):
             "reference_kernel": None if ref_ms is None else {"value": sel / (ref_ms * 1e-3), "ms": ref_ms,
                                                              "what": "src/puct/puct_gpu_v3_cpp.cu built for sm_100a, virtual loss 1"},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": pk["hbm_gbs"], "unit": "GB/s",
-                         "frac": achieved / pk["hbm_gbs"], "traffic": None, "peak_source": pk["source"],
-                         "kernel": "puct::select_kernel", "bytes_per_selection": bytes_per_sel},
+                         "frac": achieved / pk["hbm_gbs"], "traffic": None if prof is None else T * prof["dram_bytes_per_tree"],
+                         "traffic_unit": "bytes per launch, scaled by trees from an ncu capture of a smaller case", "peak_source": pk["source"],
+                         "kernel": "puct::select_kernel", "bytes_per_level": bytes_per_level, "levels": levels},
             "gpu_launches": 2 * (args.steps + args.warmup) * 2, "clocks": clocks}
     return line
 
@@ -495,6 +501,7 @@ def run_duct(args):
         dt = time.perf_counter() - t0
         cpu = {"value": sample * Wp / dt, "unit": "selections/s", "cores": 1, "kind": "port",
                "sample": f"{sample} of the {T} trees x {Wp} warps, sequential numpy restatement, {dt:.1f} s"}
+    prof = profiler_readings("duct", f"{A},{D},{Wp}")
     bytes_per_sel = mean_len * (2 * A * 16 + A * A * 4 + 4) + 16
     achieved = sel * bytes_per_sel / (ms * 1e-3) / 1e9
     line = {"metric": "DUCT selections/sec (select kernel only, CUDA events)", "value": sel / (ms * 1e-3), "unit": "selections/s",
@@ -508,11 +515,24 @@ def run_duct(args):
                     "note": "trees live on the device; a select has no host input"},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": pk["hbm_gbs"], "unit": "GB/s",
                          "frac": achieved / pk["hbm_gbs"],
-                         "traffic": sel * 10584.0 if (A, D, Wp) == (8, 16, 8) else None,
-                         "traffic_unit": "bytes per launch, scaled by traversals from an ncu capture of 1024 trees (10.6 KB each)",
+                         "traffic": None if prof is None else T * prof["dram_bytes_per_tree"],
+                         "traffic_unit": "bytes per launch, scaled by trees from an ncu capture of a smaller case",
                          "peak_source": pk["source"], "kernel": "duct::select_kernel", "bytes_per_selection": bytes_per_sel},
             "cpu_baseline": cpu, "gpu_launches": 2 * (args.steps + args.warmup), "clocks": clocks}
     return line
+
+
+def launches_per_pass(args, geo, queued):
+    """Launches of the library's own kernels in one pass: the streams (two arrays for ocp), the search, two reductions."""
+    ocp, trees, steps = "ocp" in args.variant, args.roots * args.trees, args.search_steps
+    around = 3 + ocp
+    if args.game == "c4":
+        return around + (3 if queued else 1)
+    if geo["threads_per_tree"] != 224:      # ocp, a block per tree
+        return around + 1
+    groups = min(trees, 8)
+    sizes = [trees * (g + 1) // groups - trees * g // groups for g in range(groups)]
+    return around + sum(1 + steps if n == 1 and not ocp else 1 + 2 * steps for n in sizes)
 
 
 def timed_search(game, variant, trees, playouts, steps, roots, max_plies, passes, device):
@@ -721,14 +741,15 @@ def main():
     inst_achieved = plies_per_launch * G["inst_per_ply"] / (kernel_ms * 1e-3)
     workload_key = f"{args.variant},{args.trees},{args.playouts},{args.search_steps},{B}"
     prof = profiler_readings(args.game, workload_key)
-    kernel_name = "c4::search_kernel" if args.game == "c4" else "gomoku::playout_dynamic_kernel (+ tree_step_kernel)"
+    kernel_name = "c4::search_kernel" if args.game == "c4" else ("gomoku::search_block_kernel" if geo["threads_per_tree"] != 224 else
+                                                                 "gomoku::playout_dynamic_kernel (+ tree_step_kernel)")
     line = {
         "metric": "playouts/sec", "value": value, "unit": "playouts/s", "n_gpus": n_gpus, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": dev_ms / args.steps, "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "int32", "data": "synthetic", "config": config_dict(args, n_gpus),
         "e2e": {"value": e2e_value, "unit": "playouts/s", "h2d_bytes_per_step": int(B * (17 if args.game == "c4" else 65)),
                 "d2h_bytes_per_step": int(B * (3 * A * 8 + 2 * A + 80)), "ms_per_step": e2e_ms / args.steps},
-        "gpu_launches": args.steps * ((6 if queued else 4) if args.game == "c4" else 4 + 2 * args.search_steps),
+        "gpu_launches": args.steps * launches_per_pass(args, geo, queued),
         "roofline": {"bound": "issue", "achieved": inst_achieved / 1e12, "peak": peak_inst / 1e12, "unit": "T thread-inst/s",
                      "frac": inst_achieved / peak_inst, "peak_source": f"{sm_count} SMs x 4 schedulers x 32 lanes x {pk['sm_max_mhz']:.0f} MHz ({pk['source']} clock)",
                      "traffic": None if prof is None else prof.get("dram_bytes_per_launch"),

@@ -17,7 +17,7 @@ extern "C" {
 #endif
 
 /* Replaces puct_select_winner_recalc_launch, src/puct/puct_gpu_v3_cpp.cu:450-481 (kernel :277-448; numba twin
-   src/puct/puct_gpu_v3.py:426-630): one warp per traversal, grid = trees, block = warps * 32, on `stream`. */
+   src/puct/puct_gpu_v3.py:426-630): one warp per traversal, each a block of its own, on `stream`. */
 int puct_select_winner_recalc_launch(float cpuct, float c_pw, float alpha_pw, int soft_winner, const int *edge_child_id,
                                      const float *edge_prior, const float *edge_W, const int *edge_N, int *edge_inflight,
                                      int *node_expand_inflight, const int *node_expanded, const int *tree_nodes,

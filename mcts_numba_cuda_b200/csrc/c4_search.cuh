@@ -974,8 +974,8 @@ __global__ void __maxnreg__(MCTSNC_C4_MAXNREG) search_kernel(const SearchParams 
                 // Where a quarter more trees than blocks share the queue, the next tree is taken before the last one is put back, so that
                 // trees go round the SMs: a tree with slow neighbours on its SM falls behind, has the most time left, and would be what
                 // its own block takes next (256 x 4 x 256 acp, 300 steps, 20.7 instead of 22.4 ms; 256 x 8 x 256 ocp, 500 steps,
-                // 16.9 instead of 18.2).  Where hardly any tree waits that order exchanges the trees with the most time left for those with the least
-                // at every slice (600 x 4 x 128 ocp, 1000 steps, 2400 trees on 2368 blocks: 32.8 instead of 24.7 ms).
+                // 16.9 instead of 18.2).  Where hardly any tree waits that order exchanges the trees with the most time left for those
+                // with the least at every slice (600 x 4 x 128 ocp, 1000 steps, 2400 trees on 2368 blocks: 32.8 instead of 24.7 ms).
                 int next = -1;
                 const int held = s.held;
                 if (held < 0 || 4 * p.ring_cap >= 5 * (int)gridDim.x) next = queue_pop(p.queue, p.ring, p.ring_cap);
@@ -1044,8 +1044,8 @@ __device__ __forceinline__ void run_cluster(const SearchParams &p) {
 template <bool OCP, int CL, int THREADS>
 __global__ void __launch_bounds__(THREADS) search_cluster_kernel(const SearchParams p) { run_cluster<OCP, CL>(p); }
 
-// Clusters of 8 blocks of 256 threads, or -- for steps with more games than those blocks can play one to a thread while a warp
-// walks -- of 16 blocks of 128 and a warp for the walk: a scheduler has one warp of games then instead of two.  4 trees, ACP 64 /
+// Clusters of 8 blocks of 256 threads, or -- from as many games a step as those blocks have threads beside the walking warp (1792) -- of
+// 16 blocks of 128 and a warp for the walk: a scheduler has one warp of games then instead of two.  4 trees, ACP 64 /
 // 128 / 256 / 512 playouts, us a step: 5.6 / 5.6 / 7.2 / 9.9 with 8 blocks, 6.0 / 6.0 / 6.8 / 8.4 with 16 (the barriers of the larger
 // cluster cost more).
 constexpr int CLUSTER_BLOCKS = 8, CLUSTER_THREADS = 256;

@@ -2,9 +2,8 @@
 // per joint action.  NO COUNTERPART IN THE REFERENCE: src/puct holds only the single-agent PUCT select; the benchmark
 // configuration "DUCT 2 x 8 joint actions" names a variant the reference does not implement, so the semantics below are
 // this library's own (stated in include/duct_b200.h and restated on the CPU in oracle/duct_oracle.py) and parity is
-// unpinned by construction.  The conventions of the PUCT select are kept where they apply: one warp per traversal,
-// grid = trees, block = warps * 32, path entries (node << 8) | slot, packed results
-// reason << 25 | kind << 22 | slot << 14 | node, virtual loss claimed on the way down and returned by the backup.
+// unpinned by construction.  The conventions of the PUCT select are kept where they apply: path entries (node << 8) | slot,
+// packed results reason << 25 | kind << 22 | slot << 14 | node, virtual loss claimed on the way down and returned by the backup.
 //
 // A level costs one memory round trip: the lanes of a traversal hold the statistics of one action each and, next to them,
 // their share of the node's A*A child ids, all requested together with the node's terminal flag; when both players have

@@ -525,6 +525,7 @@ constexpr int SLICE_STEPS = MCTSNC_SLICE_STEPS;  // steps a block runs of one tr
 // A step whose games all have a thread of their own is as long as its longest game: the playouts then go straight through
 // blocks of plies (2.7 us a step against 4.6 for 32 games; with five games a thread 49 ms against 36 for a search of 2000 steps
 // that takes a block of 1024 threads, so with more games than threads a lane takes its next game at once).
+// mctsnc_search_c4_static does not ask: it has the kernel for more games than threads whatever the sizes.
 bool play_straight(const mctsnc_config &c, int threads) { return threads >= c.n_playouts * (is_ocp(c) ? 1 : c4::A); }
 
 const void *search_kernel_ptr(const mctsnc_config &c, bool straight) {
@@ -535,15 +536,17 @@ const void *search_kernel_ptr(const mctsnc_config &c, bool straight) {
 // Threads that play the games of one tree, from the games a step plays (n_playouts, times the children of a node for
 // the ACP variants) and from how many trees there are for the device.
 //   Many trees (at least two per SM): a quarter of the games, between 32 and 320; half of them when a step has at most 256
-//   games.  Measured on 256 roots: headline ACP
-//   4 x 256 (1792 games a step) 16.9 / 18.2 / 17.3 / 15.8 / 15.7 G playouts/s at 256 / 320 / 384 / 448 / 512 threads (three
-//   blocks per SM up to 384; a thread of a smaller block plays more games per step, so less of a step is spent waiting for
-//   its last games); OCP 8 trees x 1000 steps with 32 / 128 / 512 playouts: 4.2 / 8.2 / 17.7 G/s at 32 / 64 / 128 threads
-//   against 1.4 / 5.0 / 12.8 at 384 (small blocks put more trees on an SM, which hides the latency of the
-//   select/expand/backup warp); with 8 x 1000 steps and 64 / 128 / 256 / 512 playouts, threads = playouts / 4, / 2, / 1:
-//   - / 6.3 / 5.9, 8.3 / 8.6 / 7.7, 11.3 / 13.0 / 10.5, 18.6 / 15.7 / 10.7 G/s.
-//   Few trees (a tree has an SM to itself): one thread per game, at most 1024; measured on one 4-tree ACP search of
-//   2000 steps: 94.7 ms with 256 threads, 69.3 ms with 512, 67.5 ms with 1024.  In between: half the games, at most 512.
+//   games.  Measured on 256 roots, G playouts/s: ACP 4 x 256 (1792 games a step), 500 steps, 18.2 / 20.3 / 20.2 / 18.7 / 19.0 / 19.0 at 256 /
+//   288 / 320 / 352 / 384 / 512 threads (a thread of a smaller block plays more games per step, so less of a step is spent
+//   waiting for its last games); OCP 8 trees x 1000 steps (small blocks put more trees on an SM, which hides the latency of
+//   the select/expand/backup warp) with 128 playouts 9.4 / 10.7 / 8.4 at 32 / 64 / 128 threads, with 256 13.8 / 15.0 / 13.7 at 64 / 128 /
+//   256, with 512 22.6 / 20.6 / 19.0 / 14.3 at 128 / 192 / 256 / 512.  The rule misses the best count where a step has 224 to 448 games
+//   (ACP 4 x 32 8.5 against 9.4 and 4 x 64 11.0 against 13.3 at 224 threads), with 64 playouts of OCP (7.0 against 8.4 at 64) and with 512
+//   of ACP (20.5 against 22.3 at 512).
+//   Few trees (a tree has an SM to itself): one thread per game, at most 1024: 132 trees of ACP 4 x 256, 1000 steps, 27.6 / 23.1 / 21.1 / 20.5 /
+//   21.7 ms at 256 / 384 / 512 / 768 / 1024 threads; of OCP 4 x 128 17.9 / 11.6 / 6.5 / 5.0 at 32 / 64 / 128 / 160.
+//   In between: half the games, at most 512: 200 trees of ACP 4 x 256 29.8 / 26.0 / 27.0 / 21.9 / 23.4 ms at 256 / 384 / 512 / 768 / 1024
+//   threads, of OCP 4 x 128 11.7 / 7.0 / 5.4 at 64 / 128 / 160: a block of more threads would pay there too.
 int choose_threads(mctsnc_handle *h, long long trees) {
     const int games = h->cfg.n_playouts * (is_ocp(h->cfg) ? 1 : h->A);
     auto fit = [](int want, int most) {
@@ -790,13 +793,13 @@ int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_
     p.trace_count = nullptr;
     p.trace_cap = 0;
     // Few trees (one search, a few searches): a cluster of blocks per tree, so that the games of a step are played on
-    // several SMs at once.  Measured, 4 x 256 acp_prodigal, 2000 steps, 4 / 8 / 16 / 32 searches in one launch: 31.4 / 37.2 /
-    // 40.4 / 63.2 ms with clusters against 57.3 / 57.3 / 57.3 / 57.4 ms with a block of 1024 threads per tree -- up to four
-    // cluster blocks per SM pay.
+    // several SMs at once.  Measured, 4 x 256 acp_prodigal, 2000 steps, 1 / 4 / 8 searches in one launch: 13.7 / 14.4 / 20.6 ms with
+    // clusters against 42.2 with a block of 1024 threads per tree; 500 steps, 9 / 12 / 16 searches: 5.0 / 5.6 / 7.0 against 11.1 --
+    // up to four cluster blocks per SM pay, and more do not fit.
     // Only where a step has more than 256 games (ACP with 64 playouts or more, OCP with 512).  One search of 2000 steps, 4
-    // trees, with a block / with clusters: ACP 8 / 16 / 32 / 64 / 128 / 256 / 512 playouts 19.6 / 20.2 / 22.8 / 27.6 / 38.1 /
-    // 57.2 / - ms against 20.7 / 22.0 / 23.5 / 24.2 / 25.0 / 28.3 / 36.3 ms; OCP 32 / 128 / 512 playouts 19.8 / 20.7 / 28.9
-    // against 20.7 / 23.4 / 25.3 ms: with few games the two cluster barriers of a step cost more than the games take.
+    // trees, with a block / with clusters: ACP 8 / 16 / 32 / 64 / 128 / 256 / 512 playouts 9.1 / 9.3 / 11.7 / 16.6 / 25.4 / 42.2 / 64.5 ms
+    // against 11.2 / 11.4 / 11.8 / 12.0 / 12.5 / 13.7 / 18.2; OCP 128 / 256 / 512 playouts 10.1 / 12.3 / 17.6 against 12.2 / 12.4 / 12.7: with few
+    // games the two cluster barriers of a step cost more than the games take.
     if (h->cfg.threads_per_tree == 0 && h->cluster_ok && h->cfg.n_playouts >= c4::CLUSTER_BLOCKS &&
         (long long)(is_ocp(h->cfg) ? 1 : h->A) * h->cfg.n_playouts > MCTSNC_C4_CLUSTER_MIN_GAMES &&
         trees * c4::CLUSTER_BLOCKS <= (long long)MCTSNC_C4_CLUSTER_SM_SHARE * h->sm_count) {
@@ -864,8 +867,8 @@ int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_
     h->blocks_per_sm = per_sm;
     // More trees than blocks fit on the device at once: a persistent grid takes slices of SLICE_STEPS steps from the
     // work queue, so that trees with long games do not keep a few SMs busy after the others have run out of work
-    // (measured on 1024 trees of 2000 steps, 4 x 256 acp_prodigal: 249 ms with one block per tree, 192 ms with the queue,
-    // before the later changes to the playout loop).  Otherwise block b grows tree b for the whole launch.
+    // (1024 trees of 2000 steps, 4 x 256 acp_prodigal: 156 ms with one block per tree, 115 with the queue; 3200 trees of 4 x 128
+    // ocp_prodigal, 1000 steps: 37.3 and 29.0).  Otherwise block b grows tree b for the whole launch.
     const long long resident = (long long)per_sm * h->sm_count;
     unsigned grid = (unsigned)trees;
     if (trees > resident && steps > SLICE_STEPS) {
@@ -943,8 +946,8 @@ void fill_results(mctsnc_handle *h, int batch, mctsnc_result *results) {
         r.max_size = d.max_size;
         for (int k = 0; k < 4; k++) r.stage_ms[k] = d.stage_ms[k];
         if (is_gomoku(h->cfg)) {
-            // the playouts of a Gomoku step run in a kernel of their own, shared by all trees: their time is what is left of
-            // the loop after the per-tree stages
+            // the playouts of a Gomoku step are not a tree's own (a kernel that all trees share), or run beside the walk (the block
+            // kernel): their time is what is left of the loop after the per-tree stages
             const float rest = h->last_ms - (d.stage_ms[0] + d.stage_ms[1] + d.stage_ms[3]);
             r.stage_ms[2] = rest > 0.f ? rest : 0.f;
         }
@@ -1706,6 +1709,7 @@ extern "C" int mctsnc_search_c4_static(const int8_t *board, const int8_t *extra_
     p.ms_per_cycle = 0.f;
     p.cache_nodes = 0;
     const size_t dyn_smem = sizeof(ulonglong2) * (size_t)per_tree;   // <= 28 KB: below the 48 KB that need an opt-in
+    // 256 threads and the kernel for more games than threads at every size
     if (ocp) c4::search_kernel<true, false><<<n_trees, 256, dyn_smem, s>>>(p);
     else c4::search_kernel<false, false><<<n_trees, 256, dyn_smem, s>>>(p);
     CUDA_TRY(cudaGetLastError());
