@@ -376,7 +376,7 @@ def run_puct(args):
             e1.record()
             torch.cuda.synchronize()
             valid = int((((d["out_selected"] >> 22) & 7) != 4).sum())
-            levels = int(d["out_len"].sum())
+            levels = int((d["out_len"] - 1).clamp_min(0).sum())   # the last entry of a length is the node it ends at
             puct.launch_release(d, virtual_loss=release_vl[0])
             torch.cuda.synchronize()
             if i >= args.warmup:
