@@ -11,10 +11,9 @@
 // each other once per step, not once per game.
 //
 // Position encoding: column c of the 6x7 board owns byte c + 1 of a 64-bit word: bits 8c + 8 .. 8c + 13 (bottom cell first) and
-// two guard bits that stay 0, so that shifts by 1, 7, 8, 9 test the four line directions without wrapping between columns;
-// byte 0 holds no cell.  Four columns are exactly the high 32-bit word: a horizontal or diagonal four ends in one of them,
-// so its test needs one funnel shift per stone and word-wide ANDs of the high word only, and the column of a stone is one
-// byte permute away.
+// two guard bits that stay 0; byte 0 holds no cell.  Four columns are exactly the high 32-bit word: a horizontal or diagonal
+// four ends in one of them, so its test works on four words of four columns each (see fours_across), and the column of a
+// stone is one byte permute away.
 #pragma once
 #include <cooperative_groups.h>
 
@@ -27,24 +26,24 @@ namespace c4 {
 constexpr int ROWS = 6, COLS = 7, A = 7;
 __host__ __device__ constexpr int column_shift(int c) { return 8 * c + 8; }
 // plies of a playout between two looks at whether the game is over
-#ifndef MCTSNC_PLIES_PER_CHECK
-#define MCTSNC_PLIES_PER_CHECK 4
-#endif
-#ifndef MCTSNC_STRAIGHT_PLIES
-#define MCTSNC_STRAIGHT_PLIES 4
-#endif
-constexpr int PLIES_PER_CHECK = MCTSNC_PLIES_PER_CHECK, STRAIGHT_PLIES = MCTSNC_STRAIGHT_PLIES;
+constexpr int PLIES_PER_CHECK = 4, STRAIGHT_PLIES = 4;
 constexpr unsigned long long BOTTOM_ROW = 0x0101010101010100ULL;
 constexpr unsigned long long FULL_BOARD = BOTTOM_ROW * 0x3FULL;
 constexpr unsigned BOTTOM_LO = 0x01010100u, BOTTOM_HI = 0x01010101u;   // of the columns 0..2 and 3..6
 constexpr unsigned TOP_LO = 0x20202000u, TOP_HI = 0x20202020u;
 
-// four in a row that end in the high word's columns (horizontal and both diagonals) of the stone set (lo, hi)
-__host__ __device__ __forceinline__ unsigned fours_across(unsigned lo, unsigned hi) {
-    const unsigned long long p = ((unsigned long long)hi << 32) | lo;   // the high word of p << k is the low word of p >> (32 - k)
-    unsigned r = hi & (unsigned)(p >> 24) & (unsigned)(p >> 16) & (unsigned)(p >> 8);
-    r |= hi & (unsigned)(p >> 23) & (unsigned)(p >> 14) & (unsigned)(p >> 5);
-    r |= hi & (unsigned)(p >> 25) & (unsigned)(p >> 18) & (unsigned)(p >> 11);
+// Four in a row that end in the high word's columns (horizontal and both diagonals) of the stone set (lo, hi), added to `r`.
+// x1, x2, x3: the columns one, two and three to the left of each, so the stones of a diagonal meet after shifts within the
+// columns.  All of those go to the left (a shift to the left can be done by the multiply-add pipe, the logic pipe is the
+// busy one): the falling diagonal is lifted by three rows.  Shifts by up to three rows leave a column across its two guard bits
+// only where the word shifted by one or two rows holds a guard bit, so nothing is found there.  (Nine funnel shifts of
+// the pair, one for every word and direction: a fifth of the headline batch 20.3 ms, 19.1 so.)
+__host__ __device__ __forceinline__ unsigned fours_across(unsigned lo, unsigned hi, unsigned r = 0u) {
+    const unsigned long long p = ((unsigned long long)hi << 32) | lo;
+    const unsigned x1 = (unsigned)(p >> 24), x2 = (unsigned)(p >> 16), x3 = (unsigned)(p >> 8);
+    r |= hi & x1 & x2 & x3;
+    r |= hi & (x1 << 1) & (x2 << 2) & (x3 << 3);
+    r |= (hi << 3) & (x1 << 2) & (x2 << 1) & x3;
     return r;
 }
 
@@ -213,22 +212,16 @@ constexpr float NO_MOVES = MOVE_LUT_BASE + 8.f;   // move_row(0)
 
 constexpr int MAX_PATH = 48;
 
-struct Shared {
-    GameSlot slot[A];        // children that need real playouts, in expansion order
+// What the walker of a tree keeps between the stages of a step.
+struct Walk {
     int4 path_rec[MAX_PATH]; // the records of the selected path as the select read them
     PathTerm term[MAX_PATH];
-    MoveEntry move_lut[128 * 8];
-    int tally[A][2];         // per slot: games won by -1, by +1 (of the games this block played)
-    int gather[A][2];        // cluster of blocks per tree: the sums over the blocks, kept by the first block
     int path[MAX_PATH];
     int child_outcome[A];    // per expanded child (expansion order): its outcome (2 = ongoing)
     int child_slot[A];       // and its slot (-1: no playouts: terminal, or not picked in OCP)
     int child_out[A][2];     // trees_playout_outcomes_children (persists over steps)
     short ae[A + 2];         // trees_actions_expanded row (persists over steps)
-    int job;                 // tree of the slice being run (-1: none left)
-    int held, held_level;    // tree of the slice before if it has steps left (-1: it has none), and its ring
     int n_slots;
-    int next_item;           // next game to hand out in the playout phase
     int mode;
     int first_child;
     int exp_mask;
@@ -244,8 +237,18 @@ struct Shared {
     unsigned status;
     unsigned long long plies;
     unsigned long long ub;
-    unsigned long long stage_cycles[4];  // cycles of this slice spent in select, expand, playouts, backup (thread 0 keeps them)
+    unsigned long long stage_cycles[4];  // cycles of this slice spent in select, expand, playouts, backup
     unsigned stage_mark;        // cycle counter when the playouts of the current step began
+};
+
+struct Shared : Walk {
+    GameSlot slot[A];        // children that need real playouts, in expansion order
+    MoveEntry move_lut[128 * 8];
+    int tally[A][2];         // per slot: games won by -1, by +1 (of the games this block played)
+    int gather[A][2];        // cluster of blocks per tree: the sums over the blocks, kept by the first block
+    int job;                 // tree of the slice being run (-1: none left)
+    int held, held_level;    // tree of the slice before if it has steps left (-1: it has none), and its ring
+    int next_item;           // next game to hand out in the playout phase
 };
 
 // Node records through the copy the walker keeps of a tree's first `cache_n` records (cluster kernel: the walk down the tree
@@ -263,7 +266,7 @@ __device__ __forceinline__ void rec_store(int4 *rec, int4 *cache, int cache_n, i
 // are known as soon as the leaf is, so every logarithm, division and square root of the UCBs can be done while the games
 // are being played.  Eight lanes per level (lane = action), four levels at a time.
 template <bool OCP>
-__device__ __forceinline__ void prepare_backup(Shared &s, const int4 *rec, const int4 *cache, int cache_n, double c_ucb, int lane,
+__device__ __forceinline__ void prepare_backup(Walk &s, const int4 *rec, const int4 *cache, int cache_n, double c_ucb, int lane,
                                                int plen, int n_tot, int leaf_playouts) {
     const int a = lane & 7, shift = lane & 24;
     for (int base = 0; base < plen - 1; base += 4) {
@@ -311,10 +314,338 @@ __device__ __forceinline__ void prepare_backup(Shared &s, const int4 *rec, const
     }
 }
 
+// The state a tree has in global memory, or that of a tree of its root alone.  One thread.
+__device__ __forceinline__ void load_tree(const SearchParams &p, Walk &s, int g, bool first, int4 *cache, int cache_n) {
+    int4 *rec = p.rec + (long long)g * p.cap;
+    TreeState *st = p.state + g;
+    const int b = g / p.n_trees;
+    if (first) {
+        const int turn = p.root_turn[b];
+        rec_store(rec, cache, cache_n, 0, make_int4(0, 0, -1, make_meta(0, false, 2, turn, 0)));
+        p.board[(long long)g * p.cap] = p.root_board[b];
+        p.parent[(long long)g * p.cap] = -1;
+        s.size = 1;
+        s.max_depth = 0;
+        s.depth_sum = 0;
+        s.root_turn = turn;
+        s.status = 0;
+        s.plies = 0;
+        s.ub = 0;
+        s.selected = 0;
+        s.path_len = 1;
+    } else {
+        s.size = st->size;
+        s.max_depth = st->max_depth;
+        s.depth_sum = st->depth_sum;
+        s.root_turn = meta_turn(rec[0].w);
+        s.status = st->status;
+        s.plies = st->plies;
+        s.ub = st->ub_draws;
+        s.selected = st->selected;
+        s.path_len = st->path_len;
+    }
+    for (int k = 0; k < 4; k++) s.stage_cycles[k] = 0;
+    // the "last step" arrays of the reference live as long as the instance: a new search starts from what the
+    // previous one left in them (trees_actions_expanded keeps stale entries in the thrifty layout)
+    s.out_neg = st->out_neg;
+    s.out_pos = st->out_pos;
+    for (int a = 0; a < A; a++) {
+        s.child_out[a][0] = p.child_out[(g * A + a) * 2 + 0];
+        s.child_out[a][1] = p.child_out[(g * A + a) * 2 + 1];
+    }
+    for (int a = 0; a < A + 2; a++) s.ae[a] = p.actions_expanded[g * (A + 2) + a];
+}
+
+// and back.  One thread.
+__device__ __forceinline__ void store_tree(const SearchParams &p, const Walk &s, int g, bool first) {
+    TreeState *st = p.state + g;
+    st->size = s.size;
+    st->max_depth = s.max_depth;
+    st->depth_sum = s.depth_sum;
+    st->selected = s.selected;
+    st->path_len = s.path_len;
+    st->out_neg = s.out_neg;
+    st->out_pos = s.out_pos;
+    st->status = s.status;
+    st->plies = s.plies;
+    st->ub_draws = s.ub;
+    for (int k = 0; k < 4; k++) st->stage_ms[k] = (first ? 0.f : st->stage_ms[k]) + (float)s.stage_cycles[k] * p.ms_per_cycle;
+    for (int a = 0; a < A; a++) {
+        p.child_out[(g * A + a) * 2 + 0] = s.child_out[a][0];
+        p.child_out[(g * A + a) * 2 + 1] = s.child_out[a][1];
+    }
+    for (int a = 0; a < A + 2; a++) p.actions_expanded[g * (A + 2) + a] = s.ae[a];
+    for (int e = 0; e < s.path_len; e++) p.paths[g * PATH_CAP + e] = s.path[e];
+}
+
+// Backup of a step (_backup_* of the reference) by one warp, after prepare_backup; wins(j): games of slot j won by -1 and by +1.
+template <bool OCP, class Wins>
+__device__ __forceinline__ void backup(Walk &s, int4 *rec, int4 *cache, int cache_n, double c_ucb, int P, int lane, Wins wins) {
+    __syncwarp();
+    const unsigned c_backup = (unsigned)clock();
+    const int mode = s.mode;
+    const int exp_mask = s.exp_mask;
+    const int sel_meta = s.sel_meta;
+    const int child_turn = -meta_turn(sel_meta);
+    const int plen = s.path_len;
+    // Lanes 0..6: the children of the expanded node (lane = action).  The other lanes: the levels of the path.
+    int neg_tot = 0, pos_tot = 0;
+    int n_tot = P;
+    int my_neg = 0, my_pos = 0;
+    const int k = __popc(exp_mask & ((1 << lane) - 1));
+    const bool child = mode == MODE_ALL_CHILDREN && lane < A && ((exp_mask >> lane) & 1);
+    bool played = false;
+    int outcome = 2;
+    if (child) {
+        outcome = s.child_outcome[k];
+        const int j = s.child_slot[k];
+        played = !OCP || k == s.pick;
+        if (j >= 0) {
+            const int2 won = wins(j);
+            my_neg = won.x;
+            my_pos = won.y;
+        } else if (played) {
+            // a terminal child: its stored outcome stands for all P playouts (src/mctsnc.py:2016-2021)
+            my_neg = outcome == -1 ? P : 0;
+            my_pos = outcome == 1 ? P : 0;
+        }
+        if (!OCP) {
+            s.child_out[lane][0] = my_neg;
+            s.child_out[lane][1] = my_pos;
+        }
+    }
+    if (mode == MODE_ALL_CHILDREN) {
+        // the sums of the children's games, both in one reduction (at most 7 * 512 games a side)
+        const int both = __reduce_add_sync(0xFFFFFFFFu, my_neg | (my_pos << 16));
+        neg_tot = both & 0xFFFF;
+        pos_tot = both >> 16;
+        if (!OCP) n_tot = P * __popc(exp_mask);
+    } else if (mode == MODE_TERMINAL) {
+        neg_tot = s.out_neg;
+        pos_tot = s.out_pos;
+    } else {
+        const int2 won = wins(0);
+        neg_tot = won.x;
+        pos_tot = won.y;
+        if (!OCP && lane == 0) {
+            s.child_out[0][0] = neg_tot;
+            s.child_out[0][1] = pos_tot;
+        }
+    }
+    // The counts and wins of the path change the UCBs of its own nodes' children only, so this is where the child
+    // that the next select goes on to is decided: on every level of the path the child on the path against the
+    // best of the others, at its end the best of the new children.
+    constexpr int LEVEL_LANES = 32 - 8;
+    const int root_turn = s.root_turn;
+    for (int base = 0; base < plen; base += LEVEL_LANES) {
+        const int e = lane < 8 ? plen - 1 : base + lane - 8;
+        const bool level = lane >= 8 && e < plen - 1;
+        const int turn_e = (e & 1) ? -root_turn : root_turn;
+        int wins_n = turn_e == 1 ? pos_tot : neg_tot;   // of the child on the path: the other side's
+        if (level) wins_n += s.path_rec[e + 1].y;
+        else wins_n = turn_e == 1 ? my_pos : my_neg;
+        const PathTerm t = s.term[min(e, plen - 1)];
+        const bool evaluate = level || (child && played);
+        unsigned key = evaluate ? ordered_key(ucb_value(c_ucb, t.explore, t.n, t.reciprocal, wins_n)) : 0u;
+        if (child && !played) key = ordered_key(__int_as_float(0x7f800000));
+        int leaf_best = 0;
+        if (base == 0 && mode == MODE_ALL_CHILDREN) {
+            const unsigned leaf_key = lane < 8 ? key : 0u;
+            const unsigned best = __reduce_max_sync(0xFFFFFFFFu, leaf_key);
+            const int a = pick_among_tied(__ballot_sync(0xFFFFFFFFu, leaf_key != 0u && leaf_key == best));
+            leaf_best = __popc(exp_mask & ((1 << a) - 1));
+            // children start from ns = ns_wins = 0 (src/mctsnc.py:1819-1820), then _backup_1_acp_* / the
+            // thread-0 part of _backup_ocp credit them (:2172-2177, :2104-2114)
+            if (child)
+                rec_store(rec, cache, cache_n, s.first_child + k,
+                          make_int4(played ? P : 0, played ? wins_n : 0, -1,
+                                    make_meta(0, outcome != 2, outcome, child_turn, meta_depth(sel_meta) + 1)));
+        }
+        if (level || (lane == 7 && base == 0)) {   // lane 7: the end of the path
+            int4 r = s.path_rec[e];
+            r.x += n_tot;
+            r.y += turn_e == 1 ? neg_tot : pos_tot;
+            if (level) {
+                if (key < t.other_key || (key == t.other_key && !(t.other & 256)))
+                    r.w = (r.w & ~META_BEST_MASK) | ((t.other & 7) << META_BEST_SHIFT);
+            } else if (mode == MODE_ALL_CHILDREN) {
+                r.z = s.first_child;
+                r.w |= exp_mask | (leaf_best << META_BEST_SHIFT);
+            }
+            rec_store(rec, cache, cache_n, s.path[e], r);
+        }
+    }
+    __syncwarp();
+    if (lane == 0) {
+        s.out_neg = neg_tot;
+        s.out_pos = pos_tot;
+        s.stage_cycles[2] += c_backup - s.stage_mark;
+        s.stage_cycles[3] += (unsigned)clock() - c_backup;
+    }
+    __syncwarp();
+}
+
+struct Selected {
+    int mode, n_slots, depth, meta;
+};
+
+// Select and expand of a step by one warp.  put(j, slot, mover) takes slot j (`mover`: the side to move there) and empties its
+// tally.
+template <bool OCP, class Put>
+__device__ __forceinline__ Selected select_expand(const SearchParams &p, Walk &s, int4 *rec, ulonglong2 *board, int *parent, int4 *cache,
+                                                  int cache_n, ulonglong2 &pick_stream, int lane, Put put) {
+    const int P = p.n_playouts;
+    const bool thrifty = (p.variant == 0 || p.variant == 2);
+    // A node names the child that the arg-max over its children's UCBs picks (the backup of every path keeps that up to
+    // date), so the walk is one dependent load per level.
+    const unsigned c_step = (unsigned)clock();   // 32-bit cycle counts: differences are right modulo 2^32
+    int node = 0;
+    int4 r = rec_load(rec, cache, cache_n, 0);
+    int depth = 0;
+    if (lane == 0) {
+        s.path[0] = 0;
+        s.path_rec[0] = r;
+    }
+    while ((r.w & 0x7F) != 0 && depth < MAX_PATH - 2) {
+        node = r.z + meta_best(r.w);
+        r = rec_load(rec, cache, cache_n, node);
+        depth++;
+        if (lane == 0) {
+            s.path[depth] = node;
+            s.path_rec[depth] = r;
+        }
+    }
+    // ------------------------------------------------------- expand (_expand_1_* and _expand_2_*)
+    const unsigned c_expand = (unsigned)clock();
+    const int sel_turn = meta_turn(r.w);
+    int mode, n_exp = 0, exp_mask = 0, first_child = -1, pick = 0, n_slots = 0;
+    if (r.w & META_TERMINAL) {
+        mode = MODE_TERMINAL;
+        if (lane == 0) {
+            const int o = meta_outcome(r.w);
+            s.out_neg = o == -1 ? P : 0;
+            s.out_pos = o == 1 ? P : 0;
+        }
+    } else {
+        const ulonglong2 bb = board[node];  // x: stones of -1, y: stones of +1
+        const unsigned long long all = bb.x | bb.y;
+        const unsigned legal = legal_columns(all);
+        const int n_legal = __popc(legal);
+        long long room = p.node_limit - (long long)s.size;
+        if (room < 0) room = 0;
+        n_exp = n_legal < room ? n_legal : (int)room;
+        exp_mask = (int)legal;
+        for (int drop = n_legal - n_exp; drop > 0; drop--)  // keep the n_exp lowest legal actions
+            exp_mask &= ~(1 << (31 - __clz(exp_mask)));
+        if (n_exp < n_legal && lane == 0) s.status |= STATUS_TREE_FULL;
+        if (n_exp > 0) {
+            mode = MODE_ALL_CHILDREN;
+            first_child = s.size;
+            if (OCP) {
+                // src/mctsnc.py:1435 / :1511 -- float32 * int64 is a float64 product, truncated
+                if (lane == 0) {
+                    const float u = rng_uniform_f32(pick_stream.x, pick_stream.y);
+                    pick = __double2int_rz((double)u * (double)n_exp);
+                    if (pick >= n_exp) {  // u == 1.0f: undefined in the reference, clamped
+                        pick = n_exp - 1;
+                        s.ub++;
+                        s.status |= STATUS_UB_DRAW;
+                    }
+                }
+                pick = __shfl_sync(0xFFFFFFFFu, pick, 0);
+            }
+            const bool has_child = lane < A && ((exp_mask >> lane) & 1);
+            const int k = __popc(exp_mask & ((1 << lane) - 1));
+            unsigned long long cneg = bb.x, cpos = bb.y, call = all;
+            int outcome = 2;
+            if (has_child) {
+                const unsigned long long move = (all + (1ULL << column_shift(lane))) & (0x3FULL << column_shift(lane));
+                if (sel_turn > 0) cpos |= move;
+                else cneg |= move;
+                call = all | move;
+                const bool win = has_four(sel_turn > 0 ? cpos : cneg);
+                outcome = win ? sel_turn : (call == FULL_BOARD ? 0 : 2);
+                board[first_child + k] = make_ulonglong2(cneg, cpos);
+                parent[first_child + k] = node;
+            }
+            const bool plays = has_child && outcome == 2 && (!OCP || k == pick);
+            const unsigned play_mask = __ballot_sync(0xFFFFFFFFu, plays);
+            n_slots = __popc(play_mask);
+            if (has_child) {
+                const int j = plays ? __popc(play_mask & ((1u << lane) - 1u)) : -1;
+                s.child_outcome[k] = outcome;
+                s.child_slot[k] = j;
+                if (plays) {
+                    GameSlot gs;
+                    const unsigned open = legal_columns(call);
+                    gs.cur = sel_turn > 0 ? cneg : cpos;  // the child is to be moved in by the other side
+                    gs.other = sel_turn > 0 ? cpos : cneg;
+                    gs.row = move_row(open);
+                    gs.count = (float)__popc(open) * RNG_2M64;
+                    gs.rng_base = OCP ? 0 : lane * P;
+                    gs.stones = __popcll(call);
+                    put(j, gs, -sel_turn);
+                }
+            }
+        } else {
+            // no room for a single child: the selected node itself is played out
+            mode = MODE_TREE_FULL;
+            n_slots = 1;
+            if (lane == 0) {
+                GameSlot gs;
+                gs.cur = sel_turn > 0 ? bb.y : bb.x;
+                gs.other = sel_turn > 0 ? bb.x : bb.y;
+                gs.row = move_row(legal);
+                gs.count = (float)n_legal * RNG_2M64;
+                gs.rng_base = 0;
+                gs.stones = __popcll(all);
+                put(0, gs, sel_turn);
+            }
+        }
+    }
+    // trees_actions_expanded in the layout of the variant (src/mctsnc.py:1430-1454, :1509-1531, :1583-1604,
+    // :1656-1681)
+    if (lane < A) {
+        if (thrifty) {
+            if (mode == MODE_ALL_CHILDREN && ((exp_mask >> lane) & 1))
+                s.ae[__popc(exp_mask & ((1 << lane) - 1))] = (short)lane;
+        } else {
+            if (mode == MODE_ALL_CHILDREN) s.ae[lane] = ((exp_mask >> lane) & 1) ? (short)lane : (short)-1;
+            else s.ae[lane] = -1;
+        }
+    }
+    __syncwarp();
+    if (lane == 0) {
+        if (mode == MODE_ALL_CHILDREN) {
+            s.size += n_exp;
+            s.depth_sum += n_exp * (depth + 1);
+            s.max_depth = max(s.max_depth, depth + 1);
+        }
+        s.ae[A + 1] = (short)(mode == MODE_ALL_CHILDREN ? n_exp : 1);
+        int m2 = mode;
+        if (OCP && mode == MODE_ALL_CHILDREN) m2 = thrifty ? pick : nth_set(exp_mask, pick);
+        s.ae[A] = (short)m2;
+        if (!OCP && mode != MODE_ALL_CHILDREN) s.ae[0] = 0;
+        s.n_slots = n_slots;
+        s.pick = pick;
+        s.mode = mode;
+        s.exp_mask = exp_mask;
+        s.first_child = first_child;
+        s.selected = node;
+        s.sel_meta = r.w;
+        s.path_len = depth + 1;
+        const unsigned c_play = (unsigned)clock();
+        s.stage_cycles[0] += c_expand - c_step;
+        s.stage_cycles[1] += c_play - c_expand;
+        s.stage_mark = c_play;
+    }
+    return {mode, n_slots, depth, r.w};
+}
+
 // Shared-memory address of the table less the offset of the float exponent: address of entry i = base + 8 * (bits of the
 // float 2^23 + i), modulo 2^32
-__device__ __forceinline__ unsigned move_lut_base(const Shared &s) {
-    return (unsigned)__cvta_generic_to_shared(s.move_lut) - MOVE_LUT_BASE_BITS * (unsigned)sizeof(MoveEntry);
+__device__ __forceinline__ unsigned move_lut_base(const MoveEntry *move_lut) {
+    return (unsigned)__cvta_generic_to_shared(move_lut) - MOVE_LUT_BASE_BITS * (unsigned)sizeof(MoveEntry);
 }
 __device__ __forceinline__ MoveEntry load_move(unsigned base, unsigned float_bits) {
     MoveEntry m;
@@ -326,22 +657,114 @@ __device__ __forceinline__ MoveEntry load_move(unsigned base, unsigned float_bit
 // two whose exponent is the column's byte number in the entry's low bits (the shift's other bits fall out, but for the
 // bottom cell of column 0, which flips the sign: that is why the set's bit 0 is kept inverted).  Two predicated additions:
 // the branch the compiler makes of it cost the warp its resolving on every ply.
-__device__ __forceinline__ void close_column(unsigned filled, float &row, float &count, unsigned entry_lo) {
-    const unsigned drop = entry_lo * (1u << 23) + (0x80000000u + (129u << 23));
+__device__ __forceinline__ void close_column(unsigned filled, float &row, float &count, unsigned entry_lo, unsigned times2p23) {
+    const unsigned drop = entry_lo * times2p23 + (0x80000000u + (129u << 23));
     asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p add.rn.f32 %0, %0, %3;\n\t@p add.rn.f32 %1, %1, %4;\n\t}"
         : "+f"(row), "+f"(count) : "r"(filled), "f"(__uint_as_float(drop)), "f"(-RNG_2M64));
 }
 
 // fours of the side that has just put a stone into the column of entry `entry_lo`: a new vertical four can only be in that
-// column, whose byte is tested alone (20 logic operations in all; the four directions over the whole board take 32)
+// column, whose byte is tested alone
 // (the permute takes the entry as it is: its other selectors name byte 0 or columns that hold no four)
 // (shifts to the left: the multiply-add pipe can do those too, and the logic pipe is the busy one; 118.4 -> 115 ms on the headline
 // batch, 23.1 -> 22.5 ms on the ocp batch)
-__device__ __forceinline__ unsigned fours_with(unsigned lo, unsigned hi, unsigned entry_lo) {
+__device__ __forceinline__ unsigned fours_with(unsigned lo, unsigned hi, unsigned entry_lo, unsigned before, unsigned two, unsigned four) {
     unsigned v = __byte_perm(lo, hi, entry_lo);
-    v &= v << 1;
-    return fours_across(lo, hi) | (v & (v << 2));
+    v &= v * two;
+    return fours_across(lo, hi, before) | (v & (v * four));
 }
+
+// A game in progress: three pairs of words -- the stones of the side that moves at the even plies of a block of PLIES plies (a
+// game starts at ply 0 of a block, so that is the side to move in the game's first position), the stones of the other side, and
+// `top`, one bit per column at its lowest empty cell (the guard bit once the column is full; top = all stones + bottom row).
+// A move in a column with room is then top & (six cells of the column), and top + move puts the marker one cell up; columns
+// are bytes, so the two words never carry.
+//
+// A block has no branch: a game that has been won plays on to its end, and what it does then is not looked at, but its generator
+// must stop where the game did.
+//   STRAIGHT (one game per thread, where a ply's latency counts): the generator does not wait for the four tests and goes back
+//   when the game is closed, so that a ply's chain is only the one from the table to the next index.
+//   Otherwise (several games per thread, where instructions count): its step is predicated on the tests of the plies before.  (With
+//   a branch behind every ply, 65 instructions a ply: moves where the paths meet.)
+__device__ __forceinline__ unsigned top_low(unsigned occupied_lo) { return occupied_lo + BOTTOM_LO + MARK; }
+__device__ __forceinline__ unsigned top_high(unsigned occupied_hi) { return occupied_hi + BOTTOM_HI; }
+
+template <bool STRAIGHT>
+struct Game {
+    static constexpr int PLIES = STRAIGHT ? STRAIGHT_PLIES : PLIES_PER_CHECK;
+    static_assert(PLIES % 2 == 0, "the two sides alternate by the parity of the ply within a block; the way back takes a power of two");
+    unsigned even_lo = 0, even_hi = 0, odd_lo = 0, odd_hi = 0, top_lo = 0, top_hi = 0;
+    unsigned long long s0 = 0, s1 = 0;
+    float row = 0.f, count = 0.f;
+    int stones = 0;
+    int drawn = 0;        // draws of the game, those behind its end too where STRAIGHT
+    unsigned fours = 0;   // of the last block (STRAIGHT: bit k for ply k)
+
+    __device__ __forceinline__ void start(const GameSlot &gs, unsigned first_top_lo, unsigned first_top_hi, const ulonglong2 &stream) {
+        even_lo = (unsigned)gs.cur;
+        even_hi = (unsigned)(gs.cur >> 32);
+        odd_lo = (unsigned)gs.other;
+        odd_hi = (unsigned)(gs.other >> 32);
+        top_lo = first_top_lo;
+        top_hi = first_top_hi;
+        row = gs.row;
+        count = gs.count;
+        stones = gs.stones;
+        s0 = stream.x;
+        s1 = stream.y;
+        drawn = -(stones & ~255);
+    }
+    __device__ __forceinline__ void play_block(unsigned lut_base, const SearchParams &p) {
+        fours = 0u;
+        if (STRAIGHT) drawn += PLIES;
+        // (a warp that is alone on its scheduler has no pipe to spare and is better off with the shifts)
+        const unsigned two = STRAIGHT ? 2u : p.times2, four = STRAIGHT ? 4u : p.times4, two23 = STRAIGHT ? 1u << 23 : p.times2p23;
+#pragma unroll
+        for (int k = 0; k < PLIES; k++) {
+            // ---- one ply (src/mctsnc.py:2059-2064, :2069)
+            // float32 u * int16 count -> float32 (:2061); here (u * 2^64) * (count * 2^-64): the same product
+            float f;
+            if (STRAIGHT || k == 0) {
+                f = rng_uniform_times_2p64(s0, s1);
+                if (!STRAIGHT) drawn++;
+            } else {
+                f = rng_uniform_times_2p64_unless(fours, s0, s1, drawn);
+            }
+            const MoveEntry m = load_move(lut_base, __float_as_uint(__fadd_rz(__fmul_rn(f, count), row)));
+            const unsigned move_lo = top_lo & m.lo, move_hi = top_hi & m.hi;
+            top_lo += move_lo;
+            top_hi += move_hi;
+            // The sides take turns with the plies of the unrolled block: no swap of "mine" and "theirs".  The cell was empty, so the
+            // stone is added (an addition can go to the multiply-add pipe, an OR cannot; 25.1 -> 24.4 ms on a fifth of the headline batch).
+            const unsigned before = STRAIGHT ? 0u : fours;
+            unsigned made;
+            if (k & 1) {
+                odd_lo += move_lo;
+                odd_hi += move_hi;
+                made = fours_with(odd_lo, odd_hi, m.lo, before, two, four);
+            } else {
+                even_lo += move_lo;
+                even_hi += move_hi;
+                made = fours_with(even_lo, even_hi, m.lo, before, two, four);
+            }
+            if (!STRAIGHT) fours = made;
+            else if (made != 0u) fours |= 1u << k;
+            close_column((move_lo & TOP_LO) | (move_hi & TOP_HI), row, count, m.lo, two23);
+        }
+    }
+    __device__ __forceinline__ bool marked() const { return ((even_lo | odd_lo) & MARK) != 0u; }   // a draw of 1.0f, see MoveEntry
+    __device__ __forceinline__ bool over() const { return fours != 0u || marked() || row == NO_MOVES; }
+    // Plies of the game that has just ended (the last one was made by the first mover iff they are odd), less any multiple of 256
+    // that was added to the `stones` of its slot; the generator goes back to where the game left it.
+    __device__ __forceinline__ int finish() {
+        int n = drawn;
+        if (fours == 0u) n = __popc(even_lo | odd_lo) + __popc(even_hi | odd_hi) - stones;   // the board is full
+        else if (STRAIGHT) n = drawn - PLIES + __ffs(fours);
+        if (STRAIGHT || fours == 0u)
+            for (int k = drawn - n; k > 0; k--) rng_back(s0, s1);
+        return n;
+    }
+};
 
 // `n_steps` steps of tree g by the whole block, from the state the tree has in global memory and back to it.
 // The random streams of the tree (ACP: 7*P, OCP: P states of 16 B) stay in dynamic shared memory meanwhile: they are
@@ -361,7 +784,6 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
     namespace cg = cooperative_groups;
     const int cache_n = CL > 1 ? p.cache_nodes : 0;
     static_assert(CL == 1 || CL == 8 || CL == 16, "cluster sizes");
-    constexpr int PLIES = STRAIGHT ? STRAIGHT_PLIES : PLIES_PER_CHECK;
     constexpr int LOG_CL = CL == 16 ? 4 : (CL == 8 ? 3 : 0);
     const int tid = threadIdx.x;
     const int nt = blockDim.x;
@@ -374,12 +796,10 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
     int4 *rec = p.rec + (long long)g * p.cap;
     ulonglong2 *board = p.board + (long long)g * p.cap;
     int *parent = p.parent + (long long)g * p.cap;
-    TreeState *st = p.state + g;
-    const bool thrifty = (p.variant == 0 || p.variant == 2);
     const bool walker = warp == 0 && rank == 0;   // the warp that selects, expands and backs up
     // threads whose first game of a step is fixed by their number: all, but for the walker where it is not the only warp
     const int first_free_item = rank == 0 && nt > 32 ? nt - 32 : nt;
-    const unsigned lut_base = move_lut_base(s);
+    const unsigned lut_base = move_lut_base(s.move_lut);
 
     const int n_streams = OCP ? P : A * P;
     ulonglong2 *g_rng = p.rng_playout + (long long)g * n_streams;
@@ -388,42 +808,7 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
         s_rng[i] = g_rng[((i >> log2_local) << p.log2_playouts) + rank * P_local + (i & (P_local - 1))];
     if (CL > 1 && tid < 2 * A) s.tally[tid >> 1][tid & 1] = 0;
     if (tid == 0 && rank == 0) {
-        const int b = g / p.n_trees;
-        if (first) {
-            const int turn = p.root_turn[b];
-            rec_store(rec, cache, cache_n, 0, make_int4(0, 0, -1, make_meta(0, false, 2, turn, 0)));
-            board[0] = p.root_board[b];
-            parent[0] = -1;
-            s.size = 1;
-            s.max_depth = 0;
-            s.depth_sum = 0;
-            s.root_turn = turn;
-            s.status = 0;
-            s.plies = 0;
-            s.ub = 0;
-            s.selected = 0;
-            s.path_len = 1;
-        } else {
-            s.size = st->size;
-            s.max_depth = st->max_depth;
-            s.depth_sum = st->depth_sum;
-            s.root_turn = meta_turn(rec[0].w);
-            s.status = st->status;
-            s.plies = st->plies;
-            s.ub = st->ub_draws;
-            s.selected = st->selected;
-            s.path_len = st->path_len;
-        }
-        for (int k = 0; k < 4; k++) s.stage_cycles[k] = 0;
-        // the "last step" arrays of the reference live as long as the instance: a new search starts from what the
-        // previous one left in them (trees_actions_expanded keeps stale entries in the thrifty layout)
-        s.out_neg = st->out_neg;
-        s.out_pos = st->out_pos;
-        for (int a = 0; a < A; a++) {
-            s.child_out[a][0] = p.child_out[(g * A + a) * 2 + 0];
-            s.child_out[a][1] = p.child_out[(g * A + a) * 2 + 1];
-        }
-        for (int a = 0; a < A + 2; a++) s.ae[a] = p.actions_expanded[g * (A + 2) + a];
+        load_tree(p, s, g, first, cache, cache_n);
     }
     if (CL > 1) cg::this_cluster().sync();
     else __syncthreads();
@@ -446,108 +831,8 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
         // =========================================================== backup of the step before, select + expand (warp 0)
         if (walker) for (;;) {
             if (backup_due) {
-                // ======================================================= backup (_backup_* of the reference)
-                __syncwarp();
-                const unsigned c_backup = (unsigned)clock();
                 const int (*tally)[2] = CL > 1 ? s.gather : s.tally;
-                const int mode = s.mode;
-                const int exp_mask = s.exp_mask;
-                const int sel_meta = s.sel_meta;
-                const int child_turn = -meta_turn(sel_meta);
-                const int plen = s.path_len;
-                // Lanes 0..6: the children of the expanded node (lane = action).  The other lanes: the levels of the path.
-                int neg_tot = 0, pos_tot = 0;
-                int n_tot = P;
-                int my_neg = 0, my_pos = 0;
-                const int k = __popc(exp_mask & ((1 << lane) - 1));
-                const bool child = mode == MODE_ALL_CHILDREN && lane < A && ((exp_mask >> lane) & 1);
-                bool played = false;
-                int outcome = 2;
-                if (child) {
-                    outcome = s.child_outcome[k];
-                    const int j = s.child_slot[k];
-                    played = !OCP || k == s.pick;
-                    if (j >= 0) {
-                        my_neg = tally[j][0];
-                        my_pos = tally[j][1];
-                    } else if (played) {
-                        // a terminal child: its stored outcome stands for all P playouts (src/mctsnc.py:2016-2021)
-                        my_neg = outcome == -1 ? P : 0;
-                        my_pos = outcome == 1 ? P : 0;
-                    }
-                    if (!OCP) {
-                        s.child_out[lane][0] = my_neg;
-                        s.child_out[lane][1] = my_pos;
-                    }
-                }
-                if (mode == MODE_ALL_CHILDREN) {
-                    // the sums of the children's games, both in one reduction (at most 7 * 512 games a side)
-                    const int both = __reduce_add_sync(0xFFFFFFFFu, my_neg | (my_pos << 16));
-                    neg_tot = both & 0xFFFF;
-                    pos_tot = both >> 16;
-                    if (!OCP) n_tot = P * __popc(exp_mask);
-                } else if (mode == MODE_TERMINAL) {
-                    neg_tot = s.out_neg;
-                    pos_tot = s.out_pos;
-                } else {
-                    neg_tot = tally[0][0];
-                    pos_tot = tally[0][1];
-                    if (!OCP && lane == 0) {
-                        s.child_out[0][0] = neg_tot;
-                        s.child_out[0][1] = pos_tot;
-                    }
-                }
-                // The counts and wins of the path change the UCBs of its own nodes' children only, so this is where the child
-                // that the next select goes on to is decided: on every level of the path the child on the path against the
-                // best of the others, at its end the best of the new children.
-                constexpr int LEVEL_LANES = 32 - 8;
-                const int root_turn = s.root_turn;
-                for (int base = 0; base < plen; base += LEVEL_LANES) {
-                    const int e = lane < 8 ? plen - 1 : base + lane - 8;
-                    const bool level = lane >= 8 && e < plen - 1;
-                    const int turn_e = (e & 1) ? -root_turn : root_turn;
-                    int wins_n = turn_e == 1 ? pos_tot : neg_tot;   // of the child on the path: the other side's
-                    if (level) wins_n += s.path_rec[e + 1].y;
-                    else wins_n = turn_e == 1 ? my_pos : my_neg;
-                    const PathTerm t = s.term[min(e, plen - 1)];
-                    const bool evaluate = level || (child && played);
-                    unsigned key = evaluate ? ordered_key(ucb_value(c_ucb, t.explore, t.n, t.reciprocal, wins_n)) : 0u;
-                    if (child && !played) key = ordered_key(__int_as_float(0x7f800000));
-                    int leaf_best = 0;
-                    if (base == 0 && mode == MODE_ALL_CHILDREN) {
-                        const unsigned leaf_key = lane < 8 ? key : 0u;
-                        const unsigned best = __reduce_max_sync(0xFFFFFFFFu, leaf_key);
-                        const int a = pick_among_tied(__ballot_sync(0xFFFFFFFFu, leaf_key != 0u && leaf_key == best));
-                        leaf_best = __popc(exp_mask & ((1 << a) - 1));
-                        // children start from ns = ns_wins = 0 (src/mctsnc.py:1819-1820), then _backup_1_acp_* / the
-                        // thread-0 part of _backup_ocp credit them (:2172-2177, :2104-2114)
-                        if (child)
-                            rec_store(rec, cache, cache_n, s.first_child + k,
-                                      make_int4(played ? P : 0, played ? wins_n : 0, -1,
-                                                make_meta(0, outcome != 2, outcome, child_turn, meta_depth(sel_meta) + 1)));
-                    }
-                    if (level || (lane == 7 && base == 0)) {   // lane 7: the end of the path
-                        int4 r = s.path_rec[e];
-                        r.x += n_tot;
-                        r.y += turn_e == 1 ? neg_tot : pos_tot;
-                        if (level) {
-                            if (key < t.other_key || (key == t.other_key && !(t.other & 256)))
-                                r.w = (r.w & ~META_BEST_MASK) | ((t.other & 7) << META_BEST_SHIFT);
-                        } else if (mode == MODE_ALL_CHILDREN) {
-                            r.z = s.first_child;
-                            r.w |= exp_mask | (leaf_best << META_BEST_SHIFT);
-                        }
-                        rec_store(rec, cache, cache_n, s.path[e], r);
-                    }
-                }
-                __syncwarp();
-                if (lane == 0) {
-                    s.out_neg = neg_tot;
-                    s.out_pos = pos_tot;
-                    s.stage_cycles[2] += c_backup - s.stage_mark;
-                    s.stage_cycles[3] += (unsigned)clock() - c_backup;
-                }
-                __syncwarp();
+                backup<OCP>(s, rec, cache, cache_n, c_ucb, P, lane, [&](int j) { return make_int2(tally[j][0], tally[j][1]); });
                 backup_due = false;
             }
             if (step == n_steps) {
@@ -555,164 +840,19 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
                 if (CL > 1 && lane > 0 && lane < CL) cg::this_cluster().map_shared_rank(&s, lane)->mode = MODE_DONE;
                 break;
             }
-            // =========================================================== select
-            // A node names the child that the arg-max over its children's UCBs picks (the backup of every path keeps that up to
-            // date), so the walk is one dependent load per level.
-            const unsigned c_step = (unsigned)clock();   // 32-bit cycle counts: differences are right modulo 2^32
-            int node = 0;
-            int4 r = rec_load(rec, cache, cache_n, 0);
-            int depth = 0;
-            if (lane == 0) {
-                s.path[0] = 0;
-                s.path_rec[0] = r;
-            }
-            while ((r.w & 0x7F) != 0 && depth < MAX_PATH - 2) {
-                node = r.z + meta_best(r.w);
-                r = rec_load(rec, cache, cache_n, node);
-                depth++;
-                if (lane == 0) {
-                    s.path[depth] = node;
-                    s.path_rec[depth] = r;
-                }
-            }
-            // ------------------------------------------------------- expand (_expand_1_* and _expand_2_*)
-            const unsigned c_expand = (unsigned)clock();
-            const int sel_turn = meta_turn(r.w);
-            int mode, n_exp = 0, exp_mask = 0, first_child = -1, pick = 0, n_slots = 0;
-            if (r.w & META_TERMINAL) {
-                mode = MODE_TERMINAL;
-                if (lane == 0) {
-                    const int o = meta_outcome(r.w);
-                    s.out_neg = o == -1 ? P : 0;
-                    s.out_pos = o == 1 ? P : 0;
-                }
-            } else {
-                const ulonglong2 bb = board[node];  // x: stones of -1, y: stones of +1
-                const unsigned long long all = bb.x | bb.y;
-                const unsigned legal = legal_columns(all);
-                const int n_legal = __popc(legal);
-                long long room = p.node_limit - (long long)s.size;
-                if (room < 0) room = 0;
-                n_exp = n_legal < room ? n_legal : (int)room;
-                exp_mask = (int)legal;
-                for (int drop = n_legal - n_exp; drop > 0; drop--)  // keep the n_exp lowest legal actions
-                    exp_mask &= ~(1 << (31 - __clz(exp_mask)));
-                if (n_exp < n_legal && lane == 0) s.status |= STATUS_TREE_FULL;
-                if (n_exp > 0) {
-                    mode = MODE_ALL_CHILDREN;
-                    first_child = s.size;
-                    if (OCP) {
-                        // src/mctsnc.py:1435 / :1511 -- float32 * int64 is a float64 product, truncated
-                        if (lane == 0) {
-                            const float u = rng_uniform_f32(pick_stream.x, pick_stream.y);
-                            pick = __double2int_rz((double)u * (double)n_exp);
-                            if (pick >= n_exp) {  // u == 1.0f: undefined in the reference, clamped
-                                pick = n_exp - 1;
-                                s.ub++;
-                                s.status |= STATUS_UB_DRAW;
-                            }
-                        }
-                        pick = __shfl_sync(0xFFFFFFFFu, pick, 0);
-                    }
-                    const bool has_child = lane < A && ((exp_mask >> lane) & 1);
-                    const int k = __popc(exp_mask & ((1 << lane) - 1));
-                    unsigned long long cneg = bb.x, cpos = bb.y, call = all;
-                    int outcome = 2;
-                    if (has_child) {
-                        const unsigned long long move = (all + (1ULL << column_shift(lane))) & (0x3FULL << column_shift(lane));
-                        if (sel_turn > 0) cpos |= move;
-                        else cneg |= move;
-                        call = all | move;
-                        const bool win = has_four(sel_turn > 0 ? cpos : cneg);
-                        outcome = win ? sel_turn : (call == FULL_BOARD ? 0 : 2);
-                        board[first_child + k] = make_ulonglong2(cneg, cpos);
-                        parent[first_child + k] = node;
-                    }
-                    const bool plays = has_child && outcome == 2 && (!OCP || k == pick);
-                    const unsigned play_mask = __ballot_sync(0xFFFFFFFFu, plays);
-                    n_slots = __popc(play_mask);
-                    if (has_child) {
-                        const int j = plays ? __popc(play_mask & ((1u << lane) - 1u)) : -1;
-                        s.child_outcome[k] = outcome;
-                        s.child_slot[k] = j;
-                        if (plays) {
-                            GameSlot gs;
-                            const unsigned open = legal_columns(call);
-                            gs.cur = sel_turn > 0 ? cneg : cpos;  // the child is to be moved in by the other side
-                            gs.other = sel_turn > 0 ? cpos : cneg;
-                            gs.row = move_row(open);
-                            gs.count = (float)__popc(open) * RNG_2M64;
-                            gs.rng_base = OCP ? 0 : lane * P;
-                            gs.stones = __popcll(call);
-                            s.slot[j] = gs;
-                            s.tally[j][0] = 0;
-                            s.tally[j][1] = 0;
-                            s.gather[j][0] = 0;
-                            s.gather[j][1] = 0;
-                        }
-                    }
-                } else {
-                    // no room for a single child: the selected node itself is played out
-                    mode = MODE_TREE_FULL;
-                    n_slots = 1;
-                    if (lane == 0) {
-                        GameSlot gs;
-                        gs.cur = sel_turn > 0 ? bb.y : bb.x;
-                        gs.other = sel_turn > 0 ? bb.x : bb.y;
-                        gs.row = move_row(legal);
-                        gs.count = (float)n_legal * RNG_2M64;
-                        gs.rng_base = 0;
-                        gs.stones = __popcll(all);
-                        s.slot[0] = gs;
-                        s.tally[0][0] = 0;
-                        s.tally[0][1] = 0;
-                        s.gather[0][0] = 0;
-                        s.gather[0][1] = 0;
-                    }
-                }
-            }
-            // trees_actions_expanded in the layout of the variant (src/mctsnc.py:1430-1454, :1509-1531, :1583-1604,
-            // :1656-1681)
-            if (lane < A) {
-                if (thrifty) {
-                    if (mode == MODE_ALL_CHILDREN && ((exp_mask >> lane) & 1))
-                        s.ae[__popc(exp_mask & ((1 << lane) - 1))] = (short)lane;
-                } else {
-                    if (mode == MODE_ALL_CHILDREN) s.ae[lane] = ((exp_mask >> lane) & 1) ? (short)lane : (short)-1;
-                    else s.ae[lane] = -1;
-                }
-            }
-            __syncwarp();
-            if (lane == 0) {
-                if (mode == MODE_ALL_CHILDREN) {
-                    s.size += n_exp;
-                    s.depth_sum += n_exp * (depth + 1);
-                    s.max_depth = max(s.max_depth, depth + 1);
-                }
-                s.ae[A + 1] = (short)(mode == MODE_ALL_CHILDREN ? n_exp : 1);
-                int m2 = mode;
-                if (OCP && mode == MODE_ALL_CHILDREN) m2 = thrifty ? pick : nth_set(exp_mask, pick);
-                s.ae[A] = (short)m2;
-                if (!OCP && mode != MODE_ALL_CHILDREN) s.ae[0] = 0;
-                s.next_item = first_free_item;
-                s.n_slots = n_slots;
-                s.pick = pick;
-                s.mode = mode;
-                s.exp_mask = exp_mask;
-                s.first_child = first_child;
-                s.selected = node;
-                s.sel_meta = r.w;
-                s.path_len = depth + 1;
-                const unsigned c_play = (unsigned)clock();
-                s.stage_cycles[0] += c_expand - c_step;
-                s.stage_cycles[1] += c_play - c_expand;
-                s.stage_mark = c_play;
-            }
+            const Selected leaf = select_expand<OCP>(p, s, rec, board, parent, cache, cache_n, pick_stream, lane, [&](int j, const GameSlot &gs, int) {
+                s.slot[j] = gs;
+                s.tally[j][0] = 0;
+                s.tally[j][1] = 0;
+                s.gather[j][0] = 0;
+                s.gather[j][1] = 0;
+            });
+            if (lane == 0) s.next_item = first_free_item;
             step++;
             backup_due = true;
-            if (mode == MODE_TERMINAL) {
+            if (leaf.mode == MODE_TERMINAL) {
                 __syncwarp();
-                prepare_backup<OCP>(s, rec, cache, cache_n, c_ucb, lane, depth + 1, P, 0);
+                prepare_backup<OCP>(s, rec, cache, cache_n, c_ucb, lane, leaf.depth + 1, P, 0);
                 continue;
             }
             if (CL > 1) {
@@ -721,11 +861,11 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
                 __syncwarp();
                 for (int other = 1; other < CL; other++) {
                     Shared *rs = cg::this_cluster().map_shared_rank(&s, other);
-                    if (lane < n_slots) rs->slot[lane] = s.slot[lane];
+                    if (lane < leaf.n_slots) rs->slot[lane] = s.slot[lane];
                     if (lane == 0) {
-                        rs->n_slots = n_slots;
-                        rs->mode = mode;
-                        rs->sel_meta = r.w;
+                        rs->n_slots = leaf.n_slots;
+                        rs->mode = leaf.mode;
+                        rs->sel_meta = leaf.meta;
                         rs->next_item = nt;
                     }
                 }
@@ -744,22 +884,13 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
         //
         // The first game of every thread is its own number.  The walker has the counts and logarithms of the backup to work
         // out first and takes what games are left after that.
-        //
-        // The board of a game in progress is three pairs of words: the stones of the side that moves at the even plies of a
-        // block of PLIES plies (a game starts at ply 0 of a block, so that is the side to move in the game's first
-        // position), the stones of the other side, and `top`, one bit per column at its lowest empty cell (the guard bit
-        // once the column is full; top = all stones + bottom row).  A move in a column with room is then top & (six cells
-        // of the column), and top + move puts the marker one cell up; columns are bytes, so the two words never carry.
         {
             const int n_items = s.n_slots << log2_local;
             // the side to move in the played-out positions: the other side than at the selected node, unless the
             // selected node itself is played out
             const int first_mover = (s.mode == MODE_TREE_FULL) ? meta_turn(s.sel_meta) : -meta_turn(s.sel_meta);
-            unsigned even_lo = 0, even_hi = 0, odd_lo = 0, odd_hi = 0, top_lo = 0, top_hi = 0;
-            unsigned long long s0 = 0, s1 = 0;
-            float row = 0.f, count = 0.f;
-            int rng_idx = 0, stones = 0, j = 0;
-            int drawn = 0;     // STRAIGHT: draws of the game
+            Game<STRAIGHT> game;
+            int rng_idx = 0, j = 0;
             int item = tid - (nt - first_free_item);
             if (walker) {
                 const int sel_n = s.mode == MODE_ALL_CHILDREN && !OCP ? P * __popc(s.exp_mask) : P;
@@ -769,82 +900,28 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
             auto start_game = [&]() {
                 j = item >> log2_local;
                 const GameSlot gs = s.slot[j];
-                even_lo = (unsigned)gs.cur;
-                even_hi = (unsigned)(gs.cur >> 32);
-                odd_lo = (unsigned)gs.other;
-                odd_hi = (unsigned)(gs.other >> 32);
-                top_lo = (even_lo | odd_lo) + BOTTOM_LO + MARK;
-                top_hi = (even_hi | odd_hi) + BOTTOM_HI;
-                row = gs.row;
-                count = gs.count;
-                stones = gs.stones;
                 rng_idx = (gs.rng_base >> LOG_CL) + (item & (P_local - 1));
-                const ulonglong2 rs = s_rng[rng_idx];
-                s0 = rs.x;
-                s1 = rs.y;
-                drawn = 0;
+                const unsigned long long occupied = gs.cur | gs.other;
+                game.start(gs, top_low((unsigned)occupied), top_high((unsigned)(occupied >> 32)), s_rng[rng_idx]);
             };
-            // PLIES plies.  STRAIGHT: no branch, and nothing waits for the four tests: a game that has been won plays on to the end of
-            // the block, which is put right when it is closed.  So the generator runs ahead of the moves and the tests behind
-            // them, and a ply's chain is only the one from the table to the next index (`fours`: bit k for ply k).  (Several
-            // games per thread: 135 against 118 ms on the headline batch, the way back costs more than the branches.)
-            unsigned fours = 0u;
-            auto play_block = [&]() {
-                fours = 0u;
-                drawn += PLIES;
-                static_assert(PLIES % 2 == 0, "the two sides alternate by the parity of the ply within a block");
-#pragma unroll
-                for (int k = 0; k < PLIES; k++) {
-                    if (!STRAIGHT && fours != 0u) continue;
-                    // ---- one ply (src/mctsnc.py:2059-2064, :2069)
-                    // float32 u * int16 count -> float32 (:2061); here (u * 2^64) * (count * 2^-64): the same product
-                    const float f = rng_uniform_times_2p64(s0, s1);
-                    const MoveEntry m = load_move(lut_base, __float_as_uint(__fadd_rz(__fmul_rn(f, count), row)));
-                    const unsigned move_lo = top_lo & m.lo, move_hi = top_hi & m.hi;
-                    top_lo += move_lo;
-                    top_hi += move_hi;
-                    // the sides take turns with the plies of the unrolled block: no swap of "mine" and "theirs"
-                    unsigned made;
-                    if (k & 1) {
-                        odd_lo |= move_lo;
-                        odd_hi |= move_hi;
-                        made = fours_with(odd_lo, odd_hi, m.lo);
-                    } else {
-                        even_lo |= move_lo;
-                        even_hi |= move_hi;
-                        made = fours_with(even_lo, even_hi, m.lo);
-                    }
-                    if (!STRAIGHT) fours |= made;
-                    else if (made != 0u) fours |= 1u << k;
-                    close_column((move_lo & TOP_LO) | (move_hi & TOP_HI), row, count, m.lo);
-                }
-            };
-            auto marked = [&]() { return ((even_lo | odd_lo) & MARK) != 0u; };   // a draw of 1.0f, see MoveEntry
-            auto over = [&]() { return fours != 0u || marked() || row == NO_MOVES; };
             auto close_game = [&]() {
-                int n = __popc(even_lo | odd_lo) + __popc(even_hi | odd_hi) - stones;  // plies of this game; the last one was made
-                if (STRAIGHT && fours != 0u) n = drawn - PLIES + __ffs(fours);         // by the first mover iff n is odd
+                int n = game.finish();
                 int winner = 0;
-                if (fours != 0u) winner = (n & 1) ? first_mover : -first_mover;
-                if (STRAIGHT) {
-                    for (int k = drawn - n; k > 0; k--) rng_back(s0, s1);
-                } else if (fours == 0u) {
-                    for (int k = n % PLIES; k != 0 && k < PLIES; k++) rng_back(s0, s1);
-                }
-                if (marked()) {
+                if (game.fours != 0u) winner = (n & 1) ? first_mover : -first_mover;
+                if (game.marked()) {
                     // u == 1.0f somewhere in this game: replay it through the byte-level emulation of the reference
                     const GameSlot gs = s.slot[j];
                     const ulonglong2 rs = s_rng[rng_idx];
                     const EmuResult er = playout_emulated(first_mover > 0 ? gs.other : gs.cur, first_mover > 0 ? gs.cur : gs.other,
                                                           first_mover, rs.x, rs.y);
-                    s0 = er.s0;
-                    s1 = er.s1;
+                    game.s0 = er.s0;
+                    game.s1 = er.s1;
                     winner = er.outcome == 2 ? 0 : er.outcome;
                     n = (int)er.plies;
                     my_ub += er.ub;
                     my_err |= er.err;
                 }
-                s_rng[rng_idx] = make_ulonglong2(s0, s1);
+                s_rng[rng_idx] = make_ulonglong2(game.s0, game.s1);
                 my_plies += n;
                 if (winner != 0) atomicAdd(&s.tally[j][winner > 0 ? 1 : 0], 1);
                 item = atomicAdd(&s.next_item, 1);
@@ -856,8 +933,8 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
                 while (__any_sync(0xFFFFFFFFu, item < n_items)) {
                     if (item < n_items) {
                         start_game();
-                        do play_block();
-                        while (!over());
+                        do game.play_block(lut_base, p);
+                        while (!game.over());
                     }
                     __syncwarp();
                     if (item < n_items) close_game();
@@ -869,8 +946,8 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
                 // after every ply it ran in nearly every iteration.
                 if (item < n_items) start_game();
                 while (item < n_items) {
-                    play_block();
-                    if (over()) {
+                    game.play_block(lut_base, p);
+                    if (game.over()) {
                         close_game();
                         if (item < n_items) start_game();
                     }
@@ -910,23 +987,7 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
         g_rng[((i >> log2_local) << p.log2_playouts) + rank * P_local + (i & (P_local - 1))] = s_rng[i];
     if (rank != 0) return;
     if (tid == 0) {
-        st->size = s.size;
-        st->max_depth = s.max_depth;
-        st->depth_sum = s.depth_sum;
-        st->selected = s.selected;
-        st->path_len = s.path_len;
-        st->out_neg = s.out_neg;
-        st->out_pos = s.out_pos;
-        st->status = s.status;
-        st->plies = s.plies;
-        st->ub_draws = s.ub;
-        for (int k = 0; k < 4; k++) st->stage_ms[k] = (first ? 0.f : st->stage_ms[k]) + (float)s.stage_cycles[k] * p.ms_per_cycle;
-        for (int a = 0; a < A; a++) {
-            p.child_out[(g * A + a) * 2 + 0] = s.child_out[a][0];
-            p.child_out[(g * A + a) * 2 + 1] = s.child_out[a][1];
-        }
-        for (int a = 0; a < A + 2; a++) p.actions_expanded[g * (A + 2) + a] = s.ae[a];
-        for (int e = 0; e < s.path_len; e++) p.paths[g * PATH_CAP + e] = s.path[e];
+        store_tree(p, s, g, first);
     }
 }
 
@@ -939,7 +1000,39 @@ __device__ __forceinline__ long long global_timer_ns() {
     return t;
 }
 
-__device__ __forceinline__ void build_move_lut(Shared &s) {
+// A slice of a queued launch is over (its writes precede, by a barrier): its record, and the ring in which the tree waits for its
+// next one (-1: the tree has no steps left).  One thread.
+__device__ __forceinline__ int finish_slice(const SearchParams &p, int g, int rem, int n_steps, long long t_start) {
+    if (p.trace) {
+        const int k = atomicAdd(p.trace_count, 1);
+        if (k < p.trace_cap) {
+            unsigned sm;
+            asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
+            p.trace[4 * k] = g;
+            p.trace[4 * k + 1] = t_start;
+            p.trace[4 * k + 2] = global_timer_ns();
+            p.trace[4 * k + 3] = ((long long)sm << 32) | (unsigned)n_steps;
+        }
+    }
+    const int left = rem - n_steps;
+    p.remaining[g] = left;
+    __threadfence();
+    if (left <= 0) return -1;
+    // band of the time the tree still needs at the pace of this slice, counted down from the longest whole
+    // search seen so far in this launch
+    // the pace of a tree changes from slice to slice (its tree deepens, its neighbours on the SM change): half
+    // the weight goes to the slices before (worth 1-2 % on the headline batch: 16.7-17.2 G playouts/s against
+    // 16.6-16.8 with the last slice alone)
+    float us_per_step = (float)(global_timer_ns() - t_start) * 1e-3f / (float)n_steps;
+    if (rem != p.steps) us_per_step = 0.5f * us_per_step + 0.5f * p.state[g].us_per_step;
+    p.state[g].us_per_step = us_per_step;
+    const int whole = (int)fminf(us_per_step * (float)p.steps, 2e9f);
+    const int longest = max(atomicMax(&p.queue->longest_us, whole), max(whole, 1));
+    const float below = QUEUE_LEVELS_PER_OCTAVE * log2f((float)longest / fmaxf(us_per_step * (float)left, 1e-3f));
+    return max(0, QUEUE_LEVELS - 1 - (int)fminf(fmaxf(below, 0.f), (float)QUEUE_LEVELS));
+}
+
+__device__ __forceinline__ void build_move_lut(MoveEntry *move_lut) {
     for (int i = threadIdx.x; i < 128 * 8; i += blockDim.x) {
         const int set = (i >> 3) ^ 1, ord = i & 7;
         MoveEntry m;
@@ -952,7 +1045,7 @@ __device__ __forceinline__ void build_move_lut(Shared &s) {
         } else if (set != 0) {
             m.lo = MARK;
         }
-        s.move_lut[i] = m;
+        move_lut[i] = m;
     }
 }
 
@@ -964,7 +1057,7 @@ __global__ void __maxnreg__(MCTSNC_C4_MAXNREG) search_kernel(const SearchParams 
     __shared__ Shared s;
     extern __shared__ ulonglong2 s_rng[];
     const int tid = threadIdx.x;
-    build_move_lut(s);
+    build_move_lut(s.move_lut);
     const bool queued = p.queue != nullptr;
     if (queued && tid == 0) s.held = -1;
     for (;;) {
@@ -997,35 +1090,8 @@ __global__ void __maxnreg__(MCTSNC_C4_MAXNREG) search_kernel(const SearchParams 
         if (!queued) break;
         __syncthreads();  // every thread's writes of the slice precede the fence of thread 0
         if (tid == 0) {
-            if (p.trace) {
-                const int k = atomicAdd(p.trace_count, 1);
-                if (k < p.trace_cap) {
-                    unsigned sm;
-                    asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
-                    p.trace[4 * k] = g;
-                    p.trace[4 * k + 1] = t_start;
-                    p.trace[4 * k + 2] = global_timer_ns();
-                    p.trace[4 * k + 3] = ((long long)sm << 32) | (unsigned)n_steps;
-                }
-            }
-            const int left = rem - n_steps;
-            p.remaining[g] = left;
-            __threadfence();
-            s.held = left > 0 ? g : -1;
-            if (left > 0) {
-                // band of the time the tree still needs at the pace of this slice, counted down from the longest whole
-                // search seen so far in this launch
-                // the pace of a tree changes from slice to slice (its tree deepens, its neighbours on the SM change): half
-                // the weight goes to the slices before (worth 1-2 % on the headline batch: 16.7-17.2 G playouts/s against
-                // 16.6-16.8 with the last slice alone)
-                float us_per_step = (float)(global_timer_ns() - t_start) * 1e-3f / (float)n_steps;
-                if (rem != p.steps) us_per_step = 0.5f * us_per_step + 0.5f * p.state[g].us_per_step;
-                p.state[g].us_per_step = us_per_step;
-                const int whole = (int)fminf(us_per_step * (float)p.steps, 2e9f);
-                const int longest = max(atomicMax(&p.queue->longest_us, whole), max(whole, 1));
-                const float below = QUEUE_LEVELS_PER_OCTAVE * log2f((float)longest / fmaxf(us_per_step * (float)left, 1e-3f));
-                s.held_level = max(0, QUEUE_LEVELS - 1 - (int)fminf(fmaxf(below, 0.f), (float)QUEUE_LEVELS));
-            }
+            s.held_level = finish_slice(p, g, rem, n_steps, t_start);
+            s.held = s.held_level >= 0 ? g : -1;
         }
     }
 }
@@ -1036,13 +1102,13 @@ template <bool OCP, int CL>
 __device__ __forceinline__ void run_cluster(const SearchParams &p) {
     __shared__ Shared s;
     extern __shared__ ulonglong2 s_rng[];
-    build_move_lut(s);
+    build_move_lut(s.move_lut);
     const int n_local = ((OCP ? 1 : A) * p.n_playouts) / CL;   // streams this block keeps; the record cache follows
     run_slice<OCP, CL, true>(p, s, s_rng, reinterpret_cast<int4 *>(s_rng + n_local), (int)(blockIdx.x / CL), p.steps, p.first != 0);
 }
 
 template <bool OCP, int CL, int THREADS>
-__global__ void __launch_bounds__(THREADS) search_cluster_kernel(const SearchParams p) { run_cluster<OCP, CL>(p); }
+__global__ void __launch_bounds__(THREADS, 2) search_cluster_kernel(const SearchParams p) { run_cluster<OCP, CL>(p); }
 
 // Clusters of 8 blocks of 256 threads, or -- from as many games a step as those blocks have threads beside the walking warp (1792) -- of
 // 16 blocks of 128 and a warp for the walk: a scheduler has one warp of games then instead of two.  4 trees, ACP 64 /

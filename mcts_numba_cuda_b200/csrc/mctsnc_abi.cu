@@ -792,6 +792,9 @@ int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_
     p.trace = nullptr;
     p.trace_count = nullptr;
     p.trace_cap = 0;
+    p.times2 = 2u;
+    p.times4 = 4u;
+    p.times2p23 = 1u << 23;
     // Few trees (one search, a few searches): a cluster of blocks per tree, so that the games of a step are played on
     // several SMs at once.  Measured, 4 x 256 acp_prodigal, 2000 steps, 1 / 4 / 8 searches in one launch: 13.7 / 14.4 / 20.6 ms with
     // clusters against 42.2 with a block of 1024 threads per tree; 500 steps, 9 / 12 / 16 searches: 5.0 / 5.6 / 7.0 against 11.1 --
@@ -1708,6 +1711,9 @@ extern "C" int mctsnc_search_c4_static(const int8_t *board, const int8_t *extra_
     p.trace_cap = 0;
     p.ms_per_cycle = 0.f;
     p.cache_nodes = 0;
+    p.times2 = 2u;
+    p.times4 = 4u;
+    p.times2p23 = 1u << 23;
     const size_t dyn_smem = sizeof(ulonglong2) * (size_t)per_tree;   // <= 28 KB: below the 48 KB that need an opt-in
     // 256 threads and the kernel for more games than threads at every size
     if (ocp) c4::search_kernel<true, false><<<n_trees, 256, dyn_smem, s>>>(p);

@@ -130,6 +130,30 @@ constexpr float RNG_2M64 = 5.421010862427522e-20f;
 __device__ __forceinline__ float rng_uniform_times_2p64(unsigned long long &s0, unsigned long long &s1) {
     return __ull2float_rn(rng_next(s0, s1) & ~0x7FFULL);
 }
+
+// The same where the generator stays where it is, and `steps` too, if `stop` is not 0: its step is predicated, in place.
+__device__ __forceinline__ float rng_uniform_times_2p64_unless(unsigned stop, unsigned long long &s0, unsigned long long &s1, int &steps) {
+    const unsigned long long x = s0 + s1;
+    unsigned a = (unsigned)s0, b = (unsigned)(s0 >> 32), c = (unsigned)s1, d = (unsigned)(s1 >> 32);
+    asm("{\n\t.reg .pred p;\n\t.reg .b32 t0, t1, u0, u1;\n\t"
+        "setp.eq.u32 p, %5, 0;\n\t"
+        "@p xor.b32 %2, %2, %0;\n\t"
+        "@p xor.b32 %3, %3, %1;\n\t"
+        "shf.r.wrap.b32 t0, %0, %1, 9;\n\t"
+        "shf.r.wrap.b32 t1, %1, %0, 9;\n\t"
+        "shl.b32 u0, %2, 14;\n\t"
+        "shf.l.wrap.b32 u1, %2, %3, 14;\n\t"
+        "@p lop3.b32 %0, t0, %2, u0, 0x96;\n\t"
+        "@p lop3.b32 %1, t1, %3, u1, 0x96;\n\t"
+        "shf.l.wrap.b32 t0, %2, %3, 4;\n\t"
+        "@p shf.l.wrap.b32 %3, %3, %2, 4;\n\t"
+        "@p mov.b32 %2, t0;\n\t"
+        "@p add.s32 %4, %4, 1;\n\t}"
+        : "+r"(a), "+r"(b), "+r"(c), "+r"(d), "+r"(steps) : "r"(stop));
+    s0 = ((unsigned long long)b << 32) | a;
+    s1 = ((unsigned long long)d << 32) | c;
+    return __ull2float_rn(x & ~0x7FFULL);
+}
 #endif
 
 }  // namespace mctsnc
