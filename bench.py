@@ -37,7 +37,7 @@ GAMES = {"c4": {"shape": (6, 7), "extra": 7, "actions": 7, "inst_per_ply": 65.0,
 # move pick and placement ~18, line test through the new stone 16 (Connect 4) / ~55 (Gomoku), draw test and loop ~6.
 # It is the yardstick of the issue roofline, not a count of the compiled code.
 
-KERNEL_SOURCES = {"c4": ("c4_search.cuh", "common.cuh", "rng.cuh"), "gomoku": ("gomoku_search.cuh", "common.cuh", "rng.cuh"),
+KERNEL_SOURCES = {"c4": ("c4_search.cuh", "c4_pool.cuh", "common.cuh", "rng.cuh"), "gomoku": ("gomoku_search.cuh", "common.cuh", "rng.cuh"),
                   "puct": ("puct_select.cu", "select_math.cuh"), "duct": ("duct_select.cu", "select_math.cuh")}
 
 
@@ -741,8 +741,11 @@ def main():
     inst_achieved = plies_per_launch * G["inst_per_ply"] / (kernel_ms * 1e-3)
     workload_key = f"{args.variant},{args.trees},{args.playouts},{args.search_steps},{B}"
     prof = profiler_readings(args.game, workload_key)
-    kernel_name = "c4::search_kernel" if args.game == "c4" else ("gomoku::search_block_kernel" if geo["threads_per_tree"] != 224 else
-                                                                 "gomoku::playout_dynamic_kernel (+ tree_step_kernel)")
+    pooled = B * args.trees > sm_count and args.playouts * (A if "acp" in args.variant else 1) > 32 and args.search_steps > 32
+    if args.game == "c4":
+        kernel_name = "c4::pool_kernel" if pooled else "c4::search_kernel"
+    else:
+        kernel_name = "gomoku::search_block_kernel" if geo["threads_per_tree"] != 224 else "gomoku::playout_dynamic_kernel (+ tree_step_kernel)"
     line = {
         "metric": "playouts/sec", "value": value, "unit": "playouts/s", "n_gpus": n_gpus, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": dev_ms / args.steps, "higher_is_better": True, "scaling": "weak",

@@ -179,8 +179,8 @@ int mctsnc_export(mctsnc_handle *h, int32_t search, int32_t field, void *dst, in
    child-pick streams (one per tree).  For tests of the generator (numba create_xoroshiro128p_states). */
 int mctsnc_export_rng(mctsnc_handle *h, int32_t search, int32_t which, uint64_t *dst, int64_t n);
 
-/* Launch shape and memory the library chose (threads per tree -- all blocks of a tree's cluster together --, blocks
-   resident per SM, bytes allocated). */
+/* Launch shape and memory the library chose (threads per tree -- all blocks of a tree's cluster together, or its share of a
+   block that grows several trees --, blocks resident per SM or, with such a block, the trees of an SM, bytes allocated). */
 int mctsnc_query(mctsnc_handle *h, int32_t *threads_per_tree, int32_t *blocks_per_sm, int32_t *sm_count,
                  int64_t *bytes_allocated);
 

@@ -13,7 +13,7 @@ LIB_PATH = os.path.join(HERE, "libmctsnc_b200.so")
 WAVE_PATH = os.path.join(HERE, "_wave" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 WAVE_SOURCE = os.path.join(HERE, "csrc", "wave_module.cpp")
 SOURCES = [os.path.join(HERE, "csrc", n) for n in ("mctsnc_abi.cu", "peer_exchange.cu", "puct_select.cu", "puct_select_v2.cu", "duct_select.cu")]
-HEADERS = [os.path.join(HERE, "csrc", n) for n in ("c4_search.cuh", "gomoku_search.cuh", "common.cuh", "rng.cuh", "select_math.cuh")]
+HEADERS = [os.path.join(HERE, "csrc", n) for n in ("c4_search.cuh", "c4_pool.cuh", "gomoku_search.cuh", "common.cuh", "rng.cuh", "select_math.cuh")]
 WAVE_HEADERS = [os.path.join(ROOT, "include", n) for n in ("puct_b200.h", "duct_b200.h")]
 HEADERS += WAVE_HEADERS + [os.path.join(ROOT, "include", "mctsnc_b200.h")]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-shared",

@@ -1071,7 +1071,7 @@ __global__ void __maxnreg__(MCTSNC_C4_MAXNREG) search_kernel(const SearchParams 
                 // with the least at every slice (600 x 4 x 128 ocp, 1000 steps, 2400 trees on 2368 blocks: 32.8 instead of 24.7 ms).
                 int next = -1;
                 const int held = s.held;
-                if (held < 0 || 4 * p.ring_cap >= 5 * (int)gridDim.x) next = queue_pop(p.queue, p.ring, p.ring_cap);
+                if (held < 0 || 4 * p.ring_cap >= 5 * p.places) next = queue_pop(p.queue, p.ring, p.ring_cap);
                 if (held >= 0) {
                     if (!queue_push(p.queue, p.ring, p.ring_cap, s.held_level, held)) atomicOr(&p.state[held].status, STATUS_INTERNAL);
                     if (next < 0) next = queue_pop(p.queue, p.ring, p.ring_cap);

@@ -241,6 +241,9 @@ struct SearchParams {
     int *trace_count;
     int trace_cap;
     float ms_per_cycle;      // 1 / (nominal SM clock in kHz): converts cycle counts into the stage times of TreeState
+    int n_trees_launched;    // trees of the launch
+    int places;              // trees that are on the device at once
+    int pool_trees, pool_walkers;  // pool kernel: trees a block grows, warps that walk
     // 2, 4 and 2^23 as factors that the compiler does not know: products with them go to the multiply-add pipe, where shifts
     // would add to the load of the logic pipe
     unsigned times2, times4, times2p23;

@@ -8,11 +8,13 @@
 #include <chrono>
 #include <cstdio>
 #include <mutex>
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <new>
 #include <vector>
 
+#include "c4_pool.cuh"
 #include "c4_search.cuh"
 #include "common.cuh"
 #include "gomoku_search.cuh"
@@ -533,7 +535,7 @@ const void *search_kernel_ptr(const mctsnc_config &c, bool straight) {
     return is_ocp(c) ? (const void *)c4::search_kernel<true, false> : (const void *)c4::search_kernel<false, false>;
 }
 
-// Threads that play the games of one tree, from the games a step plays (n_playouts, times the children of a node for
+// Threads that play the games of one tree in a block of its own (choose_pool has looked at the launch before), from the games a step plays (n_playouts, times the children of a node for
 // the ACP variants) and from how many trees there are for the device.
 //   Many trees (at least two per SM): a quarter of the games, between 32 and 320; half of them when a step has at most 256
 //   games.  Measured on 256 roots, G playouts/s: ACP 4 x 256 (1792 games a step), 500 steps, 18.2 / 20.3 / 20.2 / 18.7 / 19.0 / 19.0 at 256 /
@@ -563,6 +565,73 @@ int choose_threads(mctsnc_handle *h, long long trees) {
            (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, h->dyn_smem) != cudaSuccess || per_sm < 1))
         threads -= 32;
     return threads;
+}
+
+// The block per SM of c4_pool.cuh: the trees it grows side by side, its walking warps and its threads
+struct PoolShape {
+    int trees, walkers, threads;
+};
+constexpr int POOL_SMEM_LIMIT = 226 * 1024;
+
+const void *pool_kernel_ptr(bool ocp) { return ocp ? (const void *)c4::pool_kernel<true> : (const void *)c4::pool_kernel<false>; }
+
+// Whether the trees of a launch grow in a block per SM that plays the games of all its trees together, and that block's shape.
+// Everything is chosen by the games of a step (`games`) and the trees there are for an SM; 200 steps from random positions,
+// ms with a block per tree / with the pool:
+//   games a step                      56          128         224         256         448         512         896         1792
+//   184 trees                     1.95/1.32   2.11/1.51   1.91/1.71   2.16/1.82   2.45/2.23   2.69/2.41   3.73/3.03   5.92/4.18
+//   300 trees                     1.97/1.34   2.14/1.51   1.96/1.70   2.26/1.83   2.90/2.25   3.38/2.47   4.41/3.15   7.43/4.98
+//   600 trees                     2.04/1.49   2.35/1.83   2.53/2.03   2.86/2.21   3.84/2.77   4.43/3.06   5.97/3.90   (120 steps) 5.89/4.20
+//   1024 trees                    2.22/1.67   2.89/2.15   3.64/2.46   4.10/2.82   5.69/3.56   6.52/3.92   7.18/5.57   7.83/6.22
+//   2048 trees                    2.76/2.05   4.34/3.16   4.69/3.67   5.37/4.25   7.45/5.81   (120 steps) 5.68/4.16   7.89/6.38   14.3/12.1
+// Up to 32 games a step a block of one warp has a lane for every game and no queue to go through (1024 trees 1.53 against 1.90).  A tree
+// for every SM or fewer: nothing to share; with 896 games or more a tree and an SM the block per tree is also faster while few SMs
+// have two (160 trees of 1792 games 3.82 against 4.10).
+// Trees at once: all of an SM's while their games are few, since a tree that waits for a place stands still; where the games
+// of fewer trees fill the lanes, fewer, so that the work queue can even out the SMs.
+// Walkers: one for two trees, more where the games are few and the walk is most of a step.  Players: enough lanes, but a lane
+// of a smaller block plays its ply sooner.
+// Launches of up to SLICE_STEPS steps keep the block per tree.
+bool choose_pool(const mctsnc_handle *h, long long trees, int steps, PoolShape *shape) {
+    const int games = h->cfg.n_playouts * (is_ocp(h->cfg) ? 1 : h->A);
+    const bool large = games >= 896;
+    if (h->cfg.threads_per_tree > 0 || steps <= SLICE_STEPS || games <= 32 || trees <= (large ? h->sm_count + h->sm_count / 6 : h->sm_count)) return false;
+    const long long need = (trees + h->sm_count - 1) / h->sm_count;
+    const long long most = (long long)ceilf(150.f / sqrtf((float)games));   // 4 trees of 1792 games, 10 of 256, 14 of 128
+    long long k = need;
+    if (large) k = (long long)(0.72f * (float)trees / (float)h->sm_count + 0.6f);
+    else if (need > 3 && games > 128 && need * games > 2048) k = need * 18 / 25 < 3 ? 3 : need * 18 / 25;
+    if (k > most) k = most;
+    if (k < 1) k = 1;
+    if (k > c4::POOL_MAX_TREES) k = c4::POOL_MAX_TREES;
+    while (k > 1 && c4::pool_bytes((int)k, (int)(h->rng_per_search / h->cfg.n_trees)) > (size_t)POOL_SMEM_LIMIT) k--;
+    shape->trees = (int)k;
+    shape->walkers = (int)(k + 1) / 2;
+    if (games <= 512 && shape->walkers < 5) shape->walkers = k < 5 ? (int)k : 5;
+    const float side_by_side = (float)(k * games);
+    float lanes = (k <= 3 && games >= 224 ? 10.f : 8.f) * sqrtf(side_by_side);
+    if (side_by_side > 1024.f) lanes = fminf(lanes + 0.08f * (side_by_side - 1024.f), 12.f * sqrtf(side_by_side));
+    int players = (int)lanes / 32;
+    if (players < 1) players = 1;
+    if (players > 32 - shape->walkers) players = 32 - shape->walkers;
+    shape->threads = 32 * (shape->walkers + players);
+    return true;
+}
+
+// the launch takes its trees from the work queue, SLICE_STEPS steps at a time
+void use_queue(mctsnc_handle *h, SearchParams &p, long long trees, int steps, cudaStream_t stream) {
+    init_queue_kernel<<<(unsigned)((trees + 255) / 256), 256, 0, stream>>>(h->queue, h->ring, h->remaining, (int)trees, steps);
+    p.queue = h->queue;
+    p.ring = h->ring;
+    p.remaining = h->remaining;
+    p.ring_cap = (int)trees;
+    p.chunk = SLICE_STEPS;
+    if (h->trace) {
+        cudaMemsetAsync(h->trace_count, 0, sizeof(int), stream);
+        p.trace = h->trace;
+        p.trace_count = h->trace_count;
+        p.trace_cap = h->trace_cap;
+    }
 }
 
 int seed_streams(mctsnc_handle *h, int batch, cudaStream_t stream) {
@@ -792,6 +861,9 @@ int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_
     p.trace = nullptr;
     p.trace_count = nullptr;
     p.trace_cap = 0;
+    p.n_trees_launched = (int)trees;
+    p.places = (int)trees;
+    p.pool_trees = p.pool_walkers = 0;
     p.times2 = 2u;
     p.times4 = 4u;
     p.times2p23 = 1u << 23;
@@ -858,6 +930,23 @@ int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_
         }
         p.cache_nodes = 0;
     }
+    PoolShape pool;
+    if (choose_pool(h, trees, steps, &pool)) {
+        const void *kernel = pool_kernel_ptr(is_ocp(h->cfg));
+        CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, POOL_SMEM_LIMIT));
+        const unsigned grid = (unsigned)(trees < h->sm_count ? trees : h->sm_count);
+        p.pool_trees = pool.trees;
+        p.pool_walkers = pool.walkers;
+        p.places = pool.trees * (int)grid;
+        if (trees > p.places) use_queue(h, p, trees, steps, stream);
+        h->threads = pool.threads / pool.trees;
+        h->blocks_per_sm = pool.trees;
+        void *args[] = {&p};
+        CUDA_TRY(cudaLaunchKernel(kernel, dim3(grid), dim3((unsigned)pool.threads), args,
+                                  c4::pool_bytes(pool.trees, (int)(h->rng_per_search / h->cfg.n_trees)), stream));
+        if (p.queue) check_queue_kernel<<<(unsigned)((trees + 255) / 256), 256, 0, stream>>>(h->remaining, h->state, (int)trees);
+        return (int)cudaGetLastError();
+    }
     int threads = h->cfg.threads_per_tree > 0 ? h->cfg.threads_per_tree : choose_threads(h, trees);
     h->threads = threads;
     // A tree that has an SM to itself gets a warp more, for the walker: it works out the counts and logarithms of the backup
@@ -875,19 +964,9 @@ int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_
     const long long resident = (long long)per_sm * h->sm_count;
     unsigned grid = (unsigned)trees;
     if (trees > resident && steps > SLICE_STEPS) {
-        init_queue_kernel<<<(unsigned)((trees + 255) / 256), 256, 0, stream>>>(h->queue, h->ring, h->remaining, (int)trees, steps);
-        p.queue = h->queue;
-        p.ring = h->ring;
-        p.remaining = h->remaining;
-        p.ring_cap = (int)trees;
-        p.chunk = SLICE_STEPS;
-        if (h->trace) {
-            cudaMemsetAsync(h->trace_count, 0, sizeof(int), stream);
-            p.trace = h->trace;
-            p.trace_count = h->trace_count;
-            p.trace_cap = h->trace_cap;
-        }
+        use_queue(h, p, trees, steps, stream);
         grid = (unsigned)resident;
+        p.places = (int)resident;
     }
     void *args[] = {&p};
     CUDA_TRY(cudaLaunchKernel(kernel, dim3(grid), dim3((unsigned)threads), args, h->dyn_smem, stream));
@@ -1711,6 +1790,8 @@ extern "C" int mctsnc_search_c4_static(const int8_t *board, const int8_t *extra_
     p.trace_cap = 0;
     p.ms_per_cycle = 0.f;
     p.cache_nodes = 0;
+    p.n_trees_launched = p.places = n_trees;
+    p.pool_trees = p.pool_walkers = 0;
     p.times2 = 2u;
     p.times4 = 4u;
     p.times2p23 = 1u << 23;

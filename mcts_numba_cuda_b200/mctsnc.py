@@ -422,8 +422,8 @@ class MCTSNC:
     SLICE_STEPS = 32  # steps a block runs of one tree before it takes another from the work queue (batched launches)
 
     def launch_geometry(self):
-        """Geometry of the last search launch: threads per tree, resident blocks per SM, SMs of the device and the bytes
-        of device memory the handle holds.  A Connect-4 batch with more trees than ``blocks_per_sm * sm_count`` and more
+        """Geometry of the last search launch: threads per tree, resident blocks per SM (where a block grows several trees: the trees of
+        an SM), SMs of the device and the bytes of device memory the handle holds.  A Connect-4 batch with more trees than ``blocks_per_sm * sm_count`` and more
         than ``SLICE_STEPS`` steps runs as a persistent grid fed by the work queue."""
         if self._handle is None:
             raise RuntimeError("[MCTSNC: init_device_side_arrays() has to be called first]")

@@ -1,0 +1,63 @@
+"""Connect-4 batches in which a block grows several trees and plays the games of all of them from one queue, against the oracle,
+where that can go wrong: few and many games a step, all trees at once and through the work queue, one tree a block, more
+entries than the queue has cells, positions about to end, full trees."""
+import numpy as np
+import pytest
+
+from mcts_numba_cuda_b200 import MCTSNC, _abi
+from mcts_numba_cuda_b200.roots import c4_random_roots
+from oracle.oracle import OracleMCTSNC
+from tests.test_gpu_c4_playouts import late_root
+from tests.test_gpu_parity_c4 import compare_trees
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("variant,n_trees,n_playouts,roots,steps,at_once", [
+    ("ocp_prodigal", 3, 64, 50, 40, 2),         # 150 trees: two places on an SM, some of them empty
+    ("ocp_thrifty", 8, 128, 40, 70, 3),
+    ("ocp_prodigal", 8, 512, 100, 40, 4),       # work queue
+    ("acp_thrifty", 4, 8, 128, 100, 4),         # 56 games a step: entries of eight games
+    ("acp_prodigal", 6, 8, 560, 70, 21),        # 3360 trees, work queue: the walkers run far apart
+    ("acp_thrifty", 4, 64, 150, 50, 3),
+    ("acp_prodigal", 4, 256, 46, 40, 1),        # 184 trees take turns with a place on an SM
+    ("acp_prodigal", 1, 512, 300, 34, 2),
+])
+def test_pooled_trees_match_the_oracle(variant, n_trees, n_playouts, roots, steps, at_once):
+    boards, fills, turns = c4_random_roots(roots, 20, seed=roots)
+    for b, empty in ((0, 2), (1, 7), (2, 12)):        # full boards, one column left, steps without a game
+        boards[b], fills[b], turns[b] = late_root(empty, seed=empty)
+    ai = MCTSNC((6, 7), 7, 7, search_time_limit=np.inf, search_steps_limit=steps, n_trees=n_trees, n_playouts=n_playouts, variant=variant,
+                seed=3, verbose_info=False, max_batch=roots)
+    ai.init_device_side_arrays()
+    outs = [ai.run_batch(boards, fills, turns, steps=steps, reseed=first) for first in (True, False)]   # the streams run on
+    assert ai.launch_geometry()["blocks_per_sm"] == at_once
+    assert (outs[1]["status"] & _abi.STATUS_INTERNAL == 0).all()
+    for b in (0, 1, 2, roots // 2, roots - 1):
+        orc = OracleMCTSNC((6, 7), 7, 7, n_trees=n_trees, n_playouts=n_playouts, variant=variant, seed=3, node_capacity=steps * 7 + 8)
+        for out in outs:
+            orc.run(boards[b], fills[b], int(turns[b]), steps)
+            assert (out["playouts"][b], out["plies"][b], out["best_action"][b]) == (orc.playouts, orc.plies, orc.best_action)
+        compare_trees(ai, orc, search=b)
+
+
+@pytest.mark.parametrize("variant", MCTSNC.VARIANTS)
+def test_pooled_trees_that_fill_up_equal_a_block_per_tree(variant):
+    """A memory budget for about 150 nodes a tree (src/mctsnc.py:350-358): the leaf itself is played out from then on."""
+    roots, n_trees, steps = 60, 5, 60
+    boards, fills, turns = c4_random_roots(roots, 20, seed=1)
+    outs, handles = [], []
+    for threads in (0, 160):
+        ai = MCTSNC((6, 7), 7, 7, search_time_limit=np.inf, search_steps_limit=steps, n_trees=n_trees, n_playouts=64, variant=variant, seed=3,
+                    verbose_info=False, max_batch=roots, device_memory=n_trees * (8300 + 150 * 95) / 2 ** 30, threads_per_tree=threads)
+        ai.init_device_side_arrays()
+        assert 100 < ai.max_tree_size < 200
+        outs.append(ai.run_batch(boards, fills, turns, steps=steps))
+        handles.append(ai)
+    assert handles[0].launch_geometry()["blocks_per_sm"] == 3       # trees of a block
+    assert (outs[0]["status"] & _abi.STATUS_TREE_FULL).any()
+    for name in ("playouts", "plies", "best_action", "actions_ns", "actions_ns_wins", "status", "max_size", "depth_sum"):
+        assert np.array_equal(outs[0][name], outs[1][name]), name
+    for b in (0, roots - 1):
+        for name in ("trees_ns", "trees_ns_wins", "trees_playout_outcomes", "trees_actions_expanded"):
+            assert np.array_equal(*(ai.export(name, b) for ai in handles)), name
