@@ -5,7 +5,7 @@
  * selects joint actions.  The entry points below implement this library's own specification of the benchmark
  * configuration "DUCT, 2 players x 8 actions"; oracle/duct_oracle.py restates it on the CPU.  Conventions shared with
  * puct_b200.h: device pointers, row-major arrays, `warps` traversals per tree (they share warps of the device: one to
- * four in each, by the number of actions), path entries (node << 8) | slot, packed results reason << 25 | kind << 22 | slot << 14 | node with
+ * eight in each, by the number of actions and of traversals), path entries (node << 8) | slot, packed results reason << 25 | kind << 22 | slot << 14 | node with
  * kind 1 = expand, 2 = terminal, 3 = depth limit, 4 = busy, 0 = invalid.
  *
  * Arrays (A = actions per player <= 16, joint action of (a0, a1) = a0 * A + a1):

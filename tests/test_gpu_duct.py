@@ -116,6 +116,57 @@ def test_many_warps_keep_the_claim_protocol(warps, virtual_loss):
         assert np.array_equal(h[k], clean[k]), k
 
 
+@pytest.mark.parametrize("actions,warps,copies,skew", [(8, 8, 60, 0), (5, 2, 210, 0), (7, 3, 150, 0), (8, 5, 90, 1), (16, 8, 30, 0), (16, 4, 60, 1),
+                                                       (9, 7, 35, 0), (3, 8, 120, 0), (2, 6, 150, 1)])
+def test_traversals_of_a_tree_in_step(actions, warps, copies, skew):
+    """So many traversals that those of a tree share a warp: the claim protocol, the first of a tree as if it were alone, equal trees
+    treated equally (the order of the claims is fixed).  `skew`: rows that start where no vector load may."""
+    import torch
+    T = 24
+    case = do.grow_case(T, actions=actions, nodes=128, rounds=40, terminal_depth=4, warps=warps, seed=actions + warps, virtual_loss=2)
+    many = {k: np.tile(v, (copies,) + (1,) * (v.ndim - 1)) if isinstance(v, np.ndarray) else v for k, v in case.items()}
+    many["trees"] = T * copies
+    assert T * copies * warps > (4 if actions <= 4 else 2 if actions <= 8 else 1) * 32 * 148     # more than select_kernel holds at once
+    d = to_device(many)
+    if skew:
+        for k in ("node_prior", "node_w", "node_n", "node_inflight"):
+            flat = torch.empty(d[k].numel() + 1, dtype=d[k].dtype, device="cuda")
+            flat[1:].copy_(d[k].reshape(-1))
+            d[k] = flat[1:].view(d[k].shape)
+    duct.launch_select(d, cpuct=1.5, virtual_loss=2)
+    torch.cuda.synchronize()
+    h = to_host(d)
+    for k in STATE_KEYS:
+        first = h[k].reshape((copies, T) + h[k].shape[1:])
+        assert (first == first[:1]).all(), k
+    kind, node, joint, reason = do.decode(h["out_selected"][:T])
+    lens, paths, child = h["out_len"][:T], h["out_path"][:T], h["child"][:T]
+    ref = do.copy_case(case)
+    do.select(ref, cpuct=1.5, virtual_loss=2)
+    assert np.array_equal(h["out_selected"][:T, 0], ref["out_selected"][:, 0]) and np.array_equal(lens[:, 0], ref["out_len"][:, 0])
+    assert np.isin(kind, (do.KIND_EXPAND, do.KIND_TERMINAL, do.KIND_DEPTH_LIMIT, do.KIND_BUSY)).all()
+    assert (lens[kind == do.KIND_BUSY] == 0).all() and (kind == do.KIND_EXPAND).sum() >= T
+    claims = np.zeros_like(case["node_inflight"])
+    for t in range(T):
+        assert np.array_equal(paths[t, 0, :lens[t, 0]], ref["out_path"][t, 0, :lens[t, 0]])
+        slots = [(int(node[t, w]), int(joint[t, w])) for w in range(warps) if kind[t, w] == do.KIND_EXPAND]
+        assert len(slots) == len(set(slots)) and (child[t] == do.CHILD_CLAIMED).sum() == len(slots)
+        for w in range(warps):
+            for e in range(lens[t, w]):
+                at, j = int(paths[t, w, e]) >> 8, int(paths[t, w, e]) & 0xFF
+                claims[t, at, 0, j // actions] += 2
+                claims[t, at, 1, j % actions] += 2
+                if e > 0:
+                    prev = int(paths[t, w, e - 1])
+                    assert case["child"][t, prev >> 8, prev & 0xFF] == at
+    assert np.array_equal(h["node_inflight"][:T], claims)
+    duct.launch_backup(d, None, None, virtual_loss=2)
+    torch.cuda.synchronize()
+    h = to_host(d)
+    for k in ("child", "node_w", "node_n", "node_inflight"):
+        assert np.array_equal(h[k], many[k]), k
+
+
 def test_bad_shapes_are_refused():
     case = do.make_case(2, actions=8, depth=3, nodes=32, warps=1, seed=0)
     d = to_device(case)
