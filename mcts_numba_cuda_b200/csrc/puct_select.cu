@@ -40,6 +40,9 @@ enum Reason {
 };
 constexpr int MAX_EVALUATIONS = 2;
 constexpr int NO_EDGE = 0x7FFFFFFF;
+// what root_kernel leaves in the place of a path's length where the traversal goes on: at the child in the place of its result, from
+// the root
+constexpr int FROM_CHILD = -1, FROM_ROOT = -2;
 
 __device__ __forceinline__ int pack(int kind, int node, int slot, int reason) {
     return (reason << REASON_SHIFT) | (kind << KIND_SHIFT) | (slot << SLOT_SHIFT) | node;
@@ -98,6 +101,45 @@ struct EdgeRegs {
     }
 };
 
+// Scores of the expanded edges (LOWEST_INF: none, as for NaN and -inf); returns the best
+template <int EPL>
+__device__ __forceinline__ float score_edges(const EdgeRegs<EPL> &r, float (&score)[EPL], float cpuct, float sqrt_parent, int n_exp, int lane) {
+    float my_best = LOWEST_INF;
+    bool plain = true;
+#pragma unroll
+    for (int k = 0; k < EPL; k++) {
+        const bool visited = r.n[k] > 0;
+        const float up = cpuct * r.prior[k] * sqrt_parent;
+        const int tries = r.n[k] + r.inflight[k] + 1;
+        const float mean = Count(visited ? r.n[k] : 1).divides(r.w[k]);
+        const float v = (visited ? mean : 0.0f) + Count(tries).divides(up);
+        plain = plain && (unsigned)((tries - 1) | r.n[k]) < (1u << 22) && Count::plain(r.w[k], up);
+        score[k] = v;
+    }
+    if (!plain) {   // counts of millions, or values no network gives
+#pragma unroll
+        for (int k = 0; k < EPL; k++) {
+            const float q = r.n[k] > 0 ? r.w[k] / (float)r.n[k] : 0.0f;
+            score[k] = q + cpuct * r.prior[k] * sqrt_parent / (float)(r.n[k] + r.inflight[k] + 1);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < EPL; k++) {
+        score[k] = lane + 32 * k < n_exp && score[k] >= LOWEST ? score[k] : LOWEST_INF;
+        my_best = fmaxf(my_best, score[k]);
+    }
+    return max_of_warp(my_best);
+}
+
+template <int EPL>
+__device__ __forceinline__ int parent_count(const EdgeRegs<EPL> &r, int n_exp, int lane) {
+    int partial = 0;
+#pragma unroll
+    for (int k = 0; k < EPL; k++)
+        if (lane + 32 * k < n_exp) partial += r.n[k] + r.inflight[k];
+    return max(__reduce_add_sync(FULL, partial), 1);
+}
+
 // EPL: edges per lane, ceil(edges / 32) rounded up to 1, 2, 4 or 8 (registers follow it).
 //
 // Traversal i = tree * warps + w is block i, a single warp.  The reference puts the `warps` traversals of a tree into one block
@@ -106,17 +148,28 @@ struct EdgeRegs {
 // down.  Small blocks give the slots back at once; the traversals of a tree still start together (their blocks are
 // neighbours in the grid).  As many blocks as an SM can hold (32) with up to 64 edges.
 // WIDENING: c_pw is not zero.
-template <int EPL, bool WIDENING>
+//
+// RESUMED: root_kernel has been here; see there.
+template <int EPL, bool WIDENING, bool RESUMED>
 __global__ void __launch_bounds__(32, EPL <= 2 ? 32 : (EPL == 4 ? 24 : 16))
 select_kernel(float cpuct, float c_pw, float alpha_pw, int soft_winner, const int *__restrict__ edge_child_id,
               const float *__restrict__ edge_prior, const float *__restrict__ edge_W, const int *__restrict__ edge_N,
               int *edge_inflight, int *node_expand_inflight, const int *__restrict__ node_expanded,
               const int *__restrict__ tree_nodes, int *out_selected_node, int *out_path_eids, int *out_path_len, int nodes,
-              int edges, int warps, int path_depth, int vl) {
+              int edges, int warps, int path_depth, int vl, int trees) {
     const int lane = threadIdx.x;
-    const int traversal = blockIdx.x;
-    const int tree = traversal / warps;
-    const int wid = traversal - tree * warps;
+    int tree, wid, traversal;
+    if (RESUMED) {   // the traversals that go on are the first of their trees, but for ties: they start first, the others leave at once
+        wid = blockIdx.x / trees;
+        tree = blockIdx.x - wid * trees;
+        traversal = tree * warps + wid;
+    } else {
+        traversal = blockIdx.x;
+        tree = traversal / warps;
+        wid = traversal - tree * warps;
+    }
+    const int state = RESUMED ? out_path_len[traversal] : FROM_ROOT;
+    if (RESUMED && state >= 0) return;
     int *path = out_path_eids + (long long)traversal * path_depth;
     const long long tree_nodes_base = (long long)tree * nodes;
     const long long tree_edges_base = tree_nodes_base * edges;
@@ -134,9 +187,16 @@ select_kernel(float cpuct, float c_pw, float alpha_pw, int soft_winner, const in
     r.init(tree_edges_base, edge_child_id, edge_prior, edge_W, edge_N, edge_inflight);
     int *inflight_of_tree = edge_inflight + tree_edges_base;
     int node = 0, depth = 0;
-    int info = expanded[0];
-    r.request(0, lane, edges);
     bool outside = false;      // the child that was picked does not exist
+    if (RESUMED && state == FROM_CHILD) {
+        node = out_selected_node[traversal];
+        depth = 1;
+        outside = (unsigned)node >= (unsigned)node_cnt;
+    }
+    const int start = outside ? 0 : node;
+    int info = expanded[start];
+    r.request(start, lane, edges);
+    if (outside) info = OUTSIDE;
     float sqrt_parent = 0.f;
     int attempt = 0;           // evaluations of this level that ended with a lost claim
     // the claim made on the level above, until its answer is needed
@@ -151,31 +211,7 @@ select_kernel(float cpuct, float c_pw, float alpha_pw, int soft_winner, const in
         // right)
         const int rot = wid - n_exp * (int)(((float)wid + 0.5f) * reciprocal((float)n_exp));
         float score[EPL];
-        float my_best = LOWEST_INF;
-        bool plain = true;
-#pragma unroll
-        for (int k = 0; k < EPL; k++) {
-            const bool visited = r.n[k] > 0;
-            const float up = cpuct * r.prior[k] * sqrt_parent;
-            const int tries = r.n[k] + r.inflight[k] + 1;
-            const float mean = Count(visited ? r.n[k] : 1).divides(r.w[k]);
-            const float v = (visited ? mean : 0.0f) + Count(tries).divides(up);
-            plain = plain && (unsigned)((tries - 1) | r.n[k]) < (1u << 22) && Count::plain(r.w[k], up);
-            score[k] = v;
-        }
-        if (!plain) {   // counts of millions, or values no network gives
-#pragma unroll
-            for (int k = 0; k < EPL; k++) {
-                const float q = r.n[k] > 0 ? r.w[k] / (float)r.n[k] : 0.0f;
-                score[k] = q + cpuct * r.prior[k] * sqrt_parent / (float)(r.n[k] + r.inflight[k] + 1);
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < EPL; k++) {
-            score[k] = lane + 32 * k < n_exp && score[k] >= LOWEST ? score[k] : LOWEST_INF;
-            my_best = fmaxf(my_best, score[k]);
-        }
-        const float top = max_of_warp(my_best);
+        const float top = score_edges(r, score, cpuct, sqrt_parent, n_exp, lane);
         if (top == LOWEST_INF) return NO_EDGE;
         // the bits are compared: +0 is above -0
         if (EPL <= 2) {
@@ -199,13 +235,6 @@ select_kernel(float cpuct, float c_pw, float alpha_pw, int soft_winner, const in
         }
         const int tie = (int)__reduce_min_sync(FULL, (unsigned)my_tie);
         return tie + rot >= n_exp ? tie + rot - n_exp : tie + rot;
-    };
-    auto parent_count = [&](int n_exp) {
-        int partial = 0;
-#pragma unroll
-        for (int k = 0; k < EPL; k++)
-            if (lane + 32 * k < n_exp) partial += r.n[k] + r.inflight[k];
-        return max(__reduce_add_sync(FULL, partial), 1);
     };
     auto quota_of = [&](int parent_eff) {
         const float quota = (alpha_pw == 0.5f) ? c_pw * root_of_count(parent_eff) : c_pw * powf((float)parent_eff, alpha_pw);
@@ -251,7 +280,7 @@ select_kernel(float cpuct, float c_pw, float alpha_pw, int soft_winner, const in
         // ---- the usual level: two or more edges, no room for another, a score, and the claim of the level above held
         if (attempt == 0) while ((unsigned)(info - 2) < several && depth < path_depth) {
             if (!alone && !claim_held()) break;
-            const int parent_eff = parent_count(info);
+            const int parent_eff = parent_count(r, info, lane);
             sqrt_parent = root_of_count(parent_eff);
             if (WIDENING && quota_of(parent_eff) > info) break;
             const int best = arg_max(info);
@@ -289,7 +318,7 @@ select_kernel(float cpuct, float c_pw, float alpha_pw, int soft_winner, const in
         const bool at_end = outside || info < 0 || info > edges || depth >= path_depth;
         int allowed = 1, best = NO_EDGE;
         if (!at_end && (n_exp != 1 || WIDENING)) {
-            const int parent_eff = parent_count(n_exp);
+            const int parent_eff = parent_count(r, n_exp, lane);
             if (attempt == 0) sqrt_parent = root_of_count(parent_eff);   // another evaluation keeps the parent's count
             if (WIDENING) allowed = quota_of(parent_eff);
             if (n_exp > 1) best = arg_max(n_exp);
@@ -354,6 +383,109 @@ select_kernel(float cpuct, float c_pw, float alpha_pw, int soft_winner, const in
     }
 }
 
+// The root for all traversals of a tree, by one warp.  Traversals that start together see the same counts, so there is one
+// evaluation to make, not one each; those that want the same edge want it at the same time, and the first of them has it.  The others
+// evaluate once more and, under the strict rule, are BUSY if they lose again: with eight traversals a tree six of them, whose warps
+// did nothing but that.  The traversals that hold a claim (and those of a root that is not the usual one: two edges
+// or more, a score) go on in select_kernel<., ., RESUMED>.  4096 trees x 64 edges x 16 levels x 8 traversals: 95 us in one kernel, see
+// roots_first.
+constexpr int ROOT_WARPS = 4;
+template <int EPL>
+__global__ void __launch_bounds__(ROOT_WARPS * 32)
+root_kernel(float cpuct, int soft_winner, const int *__restrict__ edge_child_id, const float *__restrict__ edge_prior,
+            const float *__restrict__ edge_W, const int *__restrict__ edge_N, int *edge_inflight, const int *__restrict__ node_expanded,
+            const int *__restrict__ tree_nodes, int *out_selected_node, int *out_path_eids, int *out_path_len, int trees, int nodes, int edges,
+            int warps, int path_depth, int vl) {
+    const int lane = threadIdx.x & 31, tree = blockIdx.x * ROOT_WARPS + (threadIdx.x >> 5);
+    if (tree >= trees) return;
+    const bool mine = lane < warps;   // lane w: traversal w
+    const long long traversal = (long long)tree * warps + lane;
+    const int node_cnt = tree_nodes[tree];
+    const long long tree_edges = (long long)tree * nodes * edges;
+    int n_exp = 0;
+    EdgeRegs<EPL> r;
+    r.init(tree_edges, edge_child_id, edge_prior, edge_W, edge_N, edge_inflight);
+    if (path_depth >= 1 && nodes > 0 && node_cnt > 0 && node_cnt <= nodes && node_cnt <= NODE_LIMIT && edges > 0 && edges <= EDGE_LIMIT) {
+        n_exp = node_expanded[(long long)tree * nodes];
+        r.request(0, lane, edges);
+    }
+    bool usual = n_exp >= 2 && n_exp <= edges;
+    float sqrt_parent = 0.f;
+    if (usual) sqrt_parent = root_of_count(parent_count(r, n_exp, lane));
+    bool open = mine;          // the traversal has no claim and no result yet
+    for (int evaluation = 1; usual && evaluation <= MAX_EVALUATIONS; evaluation++) {
+        if (evaluation > 1) r.request(0, lane, edges);
+        float score[EPL];
+        const float top = score_edges(r, score, cpuct, sqrt_parent, n_exp, lane);
+        if (top == LOWEST_INF) {
+            if (evaluation == 1) usual = false;
+            else if (open) {
+                out_selected_node[traversal] = pack(INVALID, NODE_MASK, 0, R_INVALID_NO_VALID_EDGE);
+                out_path_len[traversal] = 0;
+                open = false;
+            }
+            break;
+        }
+        // every lane its own traversal's edge: the first of those with the top score from edge wid modulo n_exp on
+        unsigned even[EPL];
+        int ties = 0;
+#pragma unroll
+        for (int k = 0; k < EPL; k++) {
+            even[k] = __ballot_sync(FULL, __float_as_uint(score[k]) == __float_as_uint(top));
+            ties += __popc(even[k]);
+        }
+        const int rot = lane % n_exp;
+        int best = NO_EDGE, first = NO_EDGE;
+#pragma unroll
+        for (int k = EPL - 1; k >= 0; k--) {
+            if (even[k] == 0u) continue;
+            first = 32 * k + __ffs(even[k]) - 1;
+            const unsigned behind = rot >= 32 * k + 32 ? 0u : (rot > 32 * k ? even[k] >> (rot - 32 * k) << (rot - 32 * k) : even[k]);
+            if (behind != 0u) best = 32 * k + __ffs(behind) - 1;
+        }
+        if (best == NO_EDGE) best = first;
+        // its count and its child, out of the lane that holds them
+        int seen = 0, child = 0;
+#pragma unroll
+        for (int k = 0; k < EPL; k++) {
+            const int c = __shfl_sync(FULL, r.inflight[k], best & 31), to = __shfl_sync(FULL, r.child[k], best & 31);
+            if (k == best >> 5) {
+                seen = c;
+                child = to;
+            }
+        }
+        const unsigned same = __match_any_sync(FULL, open ? best : -1);
+        bool held = false;
+        if (open && __ffs(same) - 1 == lane) held = atomicCAS(&r.inflight_of[best], seen, seen + vl) == seen;
+        if (open && !held && evaluation == MAX_EVALUATIONS && soft_winner != 0) {
+            atomicAdd(&r.inflight_of[best], vl);
+            held = true;
+        }
+        if (held) {
+            out_path_eids[traversal * path_depth] = best;   // node 0
+            out_selected_node[traversal] = child;
+            out_path_len[traversal] = FROM_CHILD;
+            open = false;
+        }
+        if (!__any_sync(FULL, open)) break;
+    }
+    if (open) {
+        out_selected_node[traversal] = pack(BUSY, 0, 0, R_BUSY_WINNER_RECALC);
+        out_path_len[traversal] = usual ? 0 : FROM_ROOT;
+    }
+}
+
+// Whether a launch's roots are done by root_kernel first: where more traversals will find no place at a root, all but two of
+// a tree, than a quarter over what the device holds at once of them (32, 24 or 16 warps an SM).  Fewer cost less than the second
+// launch, 5 us.  Microseconds of the select, one kernel / two (trees x edges x levels x traversals a tree):
+//   4096 x 64 x 16 x 8 95 / 68, x 4 74 / 68   2500 x 64 x 12 x 8 58 / 45   1000 x 64 x 12 x 8 33 / 30   2500 x 19 x 12 x 8 45 / 36
+//   4096 x 8 x 16 x 8 76 / 46   3000 x 100 x 8 x 8 82 / 48   1500 x 200 x 6 x 8 76 / 43, x 4 54 / 43;   not taken: 4096 x 64 x 16 x 2
+//   64 / 68   2500 x 64 x 12 x 4 44 / 45   700 x 64 x 12 x 8 29 / 29   500 x 100 x 8 x 8 27 / 27
+static bool roots_first(int trees, int edges, int warps) {
+    const int warps_of_sm = edges <= 64 ? 32 : (edges <= 128 ? 24 : 16);
+    return warps > 2 && edges >= 2 && edges <= EDGE_LIMIT && 4LL * trees * (warps - 2) > 5LL * warps_of_sm * 148;
+}
+
 // Turns the claims of finished traversals into statistics (v3 edge layout; the reference has this step only for its
 // older node-inflight layout, src/puct/puct_gpu_v2.py:847-927): per path edge inflight -= virtual_loss, N += 1,
 // W += value; an EXPAND result also returns its ticket.  With values == NULL only the claims are released
@@ -403,11 +535,29 @@ static int launch_select(float cpuct, float c_pw, float alpha_pw, int soft_winne
                          int *out_path_eids, int *out_path_len, int trees, int nodes, int edges, int warps, int path_depth,
                          cudaStream_t stream) {
     const unsigned grid = (unsigned)((long long)trees * warps);
+    if (c_pw == 0.0f && roots_first(trees, edges, warps)) {
+#define PUCT_LAUNCH(E)                                                                                                     \
+    do {                                                                                                                  \
+        root_kernel<E><<<((unsigned)trees + ROOT_WARPS - 1) / ROOT_WARPS, ROOT_WARPS * 32, 0, stream>>>(cpuct, soft_winner, edge_child_id, edge_prior, edge_W, edge_N, edge_inflight,       \
+                                                    node_expanded, tree_nodes, out_selected_node, out_path_eids,           \
+                                                    out_path_len, trees, nodes, edges, warps, path_depth, virtual_loss);   \
+        select_kernel<E, false, true><<<grid, 32, 0, stream>>>(                                                           \
+            cpuct, c_pw, alpha_pw, soft_winner, edge_child_id, edge_prior, edge_W, edge_N, edge_inflight,                  \
+            node_expand_inflight, node_expanded, tree_nodes, out_selected_node, out_path_eids, out_path_len, nodes, edges, \
+            warps, path_depth, virtual_loss, trees);                                                                   \
+    } while (0)
+        if (edges <= 32) PUCT_LAUNCH(1);
+        else if (edges <= 64) PUCT_LAUNCH(2);
+        else if (edges <= 128) PUCT_LAUNCH(4);
+        else PUCT_LAUNCH(8);
+#undef PUCT_LAUNCH
+        return (int)cudaGetLastError();
+    }
 #define PUCT_LAUNCH_AS(E, W)                                                                                              \
-    select_kernel<E, W><<<grid, 32, 0, stream>>>(cpuct, c_pw, alpha_pw, soft_winner, edge_child_id, edge_prior, edge_W,     \
+    select_kernel<E, W, false><<<grid, 32, 0, stream>>>(cpuct, c_pw, alpha_pw, soft_winner, edge_child_id, edge_prior, edge_W,     \
                                                  edge_N, edge_inflight, node_expand_inflight, node_expanded, tree_nodes,    \
                                                  out_selected_node, out_path_eids, out_path_len, nodes, edges, warps,       \
-                                                 path_depth, virtual_loss)
+                                                 path_depth, virtual_loss, trees)
 #define PUCT_LAUNCH(E)                        \
     do {                                      \
         if (c_pw != 0.0f) PUCT_LAUNCH_AS(E, true); \

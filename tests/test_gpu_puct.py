@@ -169,6 +169,69 @@ def test_stress_invariants_many_warps(trees, warps, edges, depth):
         assert int(h2["edge_inflight"].sum()) == 0 and int(h2["node_expand_inflight"].sum()) == 0
 
 
+@pytest.mark.parametrize("edges,warps,copies,soft", [(5, 8, 90, 0), (32, 3, 540, 0), (33, 8, 90, 1), (64, 32, 18, 0), (100, 8, 70, 0), (129, 5, 90, 1),
+                                                     (256, 8, 45, 0)])
+def test_roots_of_many_traversals(edges, warps, copies, soft):
+    """So many traversals that the roots are done first, a warp per tree: usual roots, ties, and roots that are left to the select
+    (terminal, one edge, no score); a child that does not exist."""
+    import torch
+    T = 11
+    case = po.layered_case(trees=T, edges=edges, depth=3, warps=warps, seed=edges + warps, nodes_per_level=6)
+    terminal, single, nowhere, ties, scoreless = 10, 9, 8, 7, 6
+    case["node_expanded"][terminal, 0] = po.NODE_TERMINAL
+    case["node_expanded"][single, 0] = 1
+    case["edge_child"][nowhere, 0, :] = case["node_count"][nowhere]
+    case["edge_prior"][ties, 0, :] = 0.25
+    case["edge_prior"][scoreless, 0, :] = np.nan
+    for name in ("edge_n", "edge_w"):
+        case[name][ties, 0, :] = 0
+    many = {k: np.tile(v, (copies,) + (1,) * (v.ndim - 1)) if isinstance(v, np.ndarray) else v for k, v in case.items()}
+    many["trees"] = T * copies
+    per_sm = 32 if edges <= 64 else 24 if edges <= 128 else 16
+    assert 4 * T * copies * (warps - 2) > 5 * per_sm * 148
+    d = puct.to_device(many)
+    kw = dict(cpuct=1.5, c_pw=0.0, soft_winner=soft)
+    puct.launch_select(d, **kw)
+    torch.cuda.synchronize()
+    h = puct.to_host(d)
+    ref = copy.deepcopy(case)
+    po.select(ref, **kw)
+    assert (h["edge_inflight"] >= 0).all()
+    for t in range(T * copies):
+        base = t % T
+        got = [po.decode(h["out_selected"][t, w]) for w in range(warps)]
+        kinds = [g[0] for g in got]
+        claims = 0
+        for w in range(warps):
+            n = int(h["out_len"][t, w])
+            assert (n == 0) == (kinds[w] in (po.BUSY, po.INVALID))
+            walk = 0
+            for k in range(n - 1):       # the recorded path is a real path of the tree
+                enc = int(h["out_path"][t, w, k])
+                assert enc >> 8 == walk
+                walk = int(case["edge_child"][base, walk, enc & 0xFF])
+            assert n == 0 or walk == got[w][2]
+            claims += max(n - 1, 0)
+        assert int(h["edge_inflight"][t].sum()) == claims
+        if base < scoreless:
+            if h["out_len"][t, 0] > 0:       # the first traversal goes where it would go alone
+                assert h["out_path"][t, 0, 0] == ref["out_path"][base, 0, 0]
+            at_root = [w for w in range(warps) if kinds[w] == po.BUSY and got[w][2] == 0]
+            assert len(at_root) == (0 if soft else warps - 2)
+        elif base == scoreless:
+            assert kinds == [po.INVALID] * warps
+        elif base == ties and not soft:
+            first = [int(h["out_path"][t, w, 0]) & 0xFF for w in range(min(warps, edges)) if h["out_len"][t, w] > 0]
+            assert first == [w for w in range(min(warps, edges)) if h["out_len"][t, w] > 0]
+        elif base == nowhere:
+            assert set(kinds) <= {po.INVALID, po.BUSY} and kinds.count(po.INVALID) >= 2 and claims == 0
+        elif base == terminal:
+            assert kinds == [po.TERMINAL] * warps
+    puct.launch_release(d)
+    torch.cuda.synchronize()
+    assert int(puct.to_host(d)["edge_inflight"].sum()) == 0
+
+
 @pytest.mark.skipif(not os.path.exists(REF_LIB), reason="reference kernel not built (reference not mounted at build time)")
 def test_first_edge_distribution_matches_reference_kernel():
     """Many warps: results depend on the schedule, so compare what both kernels choose at the root in aggregate."""
