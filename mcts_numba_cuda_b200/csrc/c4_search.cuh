@@ -689,8 +689,15 @@ __device__ __forceinline__ unsigned fours_with(unsigned lo, unsigned hi, unsigne
 __device__ __forceinline__ unsigned top_low(unsigned occupied_lo) { return occupied_lo + BOTTOM_LO + MARK; }
 __device__ __forceinline__ unsigned top_high(unsigned occupied_hi) { return occupied_hi + BOTTOM_HI; }
 
-template <bool STRAIGHT>
+//   AHEAD (STRAIGHT, where the threads that play idle while the walker makes the next step): the draws come out of a ring per stream
+//   that those threads fill meanwhile, see Draws.
+constexpr int AHEAD_DRAWS = 64;     // of a stream: no fewer than a game can use, 42 and the rest of its last block
+constexpr int AHEAD_STRIDE = AHEAD_DRAWS + PLIES_PER_CHECK + 1;   // floats: the first ones again behind the last, and an odd number
+static_assert(AHEAD_DRAWS >= ROWS * COLS + STRAIGHT_PLIES && STRAIGHT_PLIES <= PLIES_PER_CHECK, "a block of draws is read in one piece");
+
+template <bool STRAIGHT, bool AHEAD = false>
 struct Game {
+    static_assert(STRAIGHT || !AHEAD, "draws made ahead: one game per thread");
     static constexpr int PLIES = STRAIGHT ? STRAIGHT_PLIES : PLIES_PER_CHECK;
     static_assert(PLIES % 2 == 0, "the two sides alternate by the parity of the ply within a block; the way back takes a power of two");
     unsigned even_lo = 0, even_hi = 0, odd_lo = 0, odd_hi = 0, top_lo = 0, top_hi = 0;
@@ -698,6 +705,8 @@ struct Game {
     float row = 0.f, count = 0.f;
     int stones = 0;
     int drawn = 0;        // draws of the game, those behind its end too where STRAIGHT
+    unsigned ring = 0;    // AHEAD: shared-memory address of the stream's ring, and the ring's place of the game's first draw
+    int place = 0;
     unsigned fours = 0;   // of the last block (STRAIGHT: bit k for ply k)
 
     __device__ __forceinline__ void start(const GameSlot &gs, unsigned first_top_lo, unsigned first_top_hi, const ulonglong2 &stream) {
@@ -716,6 +725,12 @@ struct Game {
     }
     __device__ __forceinline__ void play_block(unsigned lut_base, const SearchParams &p) {
         fours = 0u;
+        float ahead[PLIES];
+        if (AHEAD) {
+            const unsigned at = ring + (unsigned)((place + drawn) & (AHEAD_DRAWS - 1)) * 4u;
+#pragma unroll
+            for (int k = 0; k < PLIES; k++) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(ahead[k]) : "r"(at + 4u * k));
+        }
         if (STRAIGHT) drawn += PLIES;
         // (a warp that is alone on its scheduler has no pipe to spare and is better off with the shifts)
         const unsigned two = STRAIGHT ? 2u : p.times2, four = STRAIGHT ? 4u : p.times4, two23 = STRAIGHT ? 1u << 23 : p.times2p23;
@@ -724,7 +739,9 @@ struct Game {
             // ---- one ply (src/mctsnc.py:2059-2064, :2069)
             // float32 u * int16 count -> float32 (:2061); here (u * 2^64) * (count * 2^-64): the same product
             float f;
-            if (STRAIGHT || k == 0) {
+            if (AHEAD) {
+                f = ahead[k];
+            } else if (STRAIGHT || k == 0) {
                 f = rng_uniform_times_2p64(s0, s1);
                 if (!STRAIGHT) drawn++;
             } else {
@@ -760,9 +777,53 @@ struct Game {
         int n = drawn;
         if (fours == 0u) n = __popc(even_lo | odd_lo) + __popc(even_hi | odd_hi) - stones;   // the board is full
         else if (STRAIGHT) n = drawn - PLIES + __ffs(fours);
-        if (STRAIGHT || fours == 0u)
+        if (!AHEAD && (STRAIGHT || fours == 0u))
             for (int k = drawn - n; k > 0; k--) rng_back(s0, s1);
         return n;
+    }
+};
+
+// The draws of a block's streams made ahead: of every stream the next AHEAD_DRAWS, scaled by 2^64, in a ring that starts at `place`.
+// The stream's state in the block's array is the one behind them; `used`: draws of the step's game, made up by refill while the
+// walker makes the next step and the threads that play would wait for it.  A ply has 14 of 58 instructions less then, and
+// nothing is taken back when a game is closed; what the threads lose is a part of the walker's issue slots.  One search of 1000
+// steps, without / with: 1 x 32 ocp 4.66 / 4.45 ms, 8 x 256 ocp 5.77 / 5.64, 4 x 32 acp 5.12 / 4.79; on clusters 4 x 64 acp 5.49 / 5.33, 4 x 128
+// 5.62 / 5.64, 4 x 256 6.07 / 5.99, two of those 6.68 / 6.21.  With two to four warps that play the walker loses more than they
+// gain: 4 x 128 ocp 4.69 / 4.96, 4 x 64 ocp 4.72 / 4.82.
+struct Draws {
+    float *ring;       // [streams][AHEAD_STRIDE]
+    int *place, *used; // [streams]
+    static __host__ __device__ size_t bytes(int streams) { return (size_t)streams * (AHEAD_STRIDE * sizeof(float) + 2 * sizeof(int)); }
+    __device__ __forceinline__ Draws(void *memory, int streams) {
+        ring = reinterpret_cast<float *>(memory);
+        place = reinterpret_cast<int *>(ring + (size_t)streams * AHEAD_STRIDE);
+        used = place + streams;
+    }
+    // `count` more of stream i, over those that have been used
+    __device__ __forceinline__ void make(ulonglong2 *s_rng, int i, int count) {
+        ulonglong2 state = s_rng[i];
+        float *mine = ring + i * AHEAD_STRIDE;
+        int at = place[i];
+        for (; count > 0; count--) {
+            const float f = rng_uniform_times_2p64(state.x, state.y);
+            mine[at] = f;
+            if (at < PLIES_PER_CHECK) mine[AHEAD_DRAWS + at] = f;
+            at = (at + 1) & (AHEAD_DRAWS - 1);
+        }
+        s_rng[i] = state;
+        place[i] = at;
+    }
+    __device__ __forceinline__ void refill(ulonglong2 *s_rng, int i) {
+        const int n = used[i];
+        if (n == 0) return;
+        used[i] = 0;
+        make(s_rng, i, n);
+    }
+    // where the stream stands: before the draws of the ring
+    __device__ __forceinline__ ulonglong2 state_of(const ulonglong2 *s_rng, int i) const {
+        ulonglong2 state = s_rng[i];
+        for (int k = 0; k < AHEAD_DRAWS; k++) rng_back(state.x, state.y);
+        return state;
     }
 };
 
@@ -778,8 +839,9 @@ struct Game {
 // every barrier.
 //
 // STRAIGHT: how a game is played, see the playouts.
-template <bool OCP, int CL, bool STRAIGHT>
-__device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulonglong2 *s_rng, int4 *cache, const int g,
+// AHEAD: draws made ahead (by all warps but the walker's, of which there is at least one), in `ahead`.
+template <bool OCP, int CL, bool STRAIGHT, bool AHEAD>
+__device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulonglong2 *s_rng, int4 *cache, void *ahead, const int g,
                                           const int n_steps, const bool first) {
     namespace cg = cooperative_groups;
     const int cache_n = CL > 1 ? p.cache_nodes : 0;
@@ -806,6 +868,12 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
     // stream (action, t) of the tree sits at local index action * P_local + (t - rank * P_local)
     for (int i = tid; i < (n_streams >> LOG_CL); i += nt)
         s_rng[i] = g_rng[((i >> log2_local) << p.log2_playouts) + rank * P_local + (i & (P_local - 1))];
+    Draws draws(ahead, n_streams >> LOG_CL);
+    if (AHEAD)
+        for (int i = tid; i < (n_streams >> LOG_CL); i += nt) {
+            draws.place[i] = draws.used[i] = 0;
+            draws.make(s_rng, i, AHEAD_DRAWS);
+        }
     if (CL > 1 && tid < 2 * A) s.tally[tid >> 1][tid & 1] = 0;
     if (tid == 0 && rank == 0) {
         load_tree(p, s, g, first, cache, cache_n);
@@ -872,6 +940,13 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
             }
             break;
         }
+        // the others make up the draws that the games have used (five warps: not the one that shares the walker's scheduler)
+        if (AHEAD && CL == 16 && rank == 0) {
+            if (warp & 3)
+                for (int i = tid - 32; i < (n_streams >> LOG_CL); i += 3 * 32) draws.refill(s_rng, i);
+        } else if (AHEAD && !walker) {
+            for (int i = tid - (nt - first_free_item); i < (n_streams >> LOG_CL); i += first_free_item) draws.refill(s_rng, i);
+        }
         if (CL > 1) cg::this_cluster().sync();
         else __syncthreads();
         if (s.mode == MODE_DONE) break;
@@ -889,7 +964,7 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
             // the side to move in the played-out positions: the other side than at the selected node, unless the
             // selected node itself is played out
             const int first_mover = (s.mode == MODE_TREE_FULL) ? meta_turn(s.sel_meta) : -meta_turn(s.sel_meta);
-            Game<STRAIGHT> game;
+            Game<STRAIGHT, AHEAD> game;
             int rng_idx = 0, j = 0;
             int item = tid - (nt - first_free_item);
             if (walker) {
@@ -902,7 +977,11 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
                 const GameSlot gs = s.slot[j];
                 rng_idx = (gs.rng_base >> LOG_CL) + (item & (P_local - 1));
                 const unsigned long long occupied = gs.cur | gs.other;
-                game.start(gs, top_low((unsigned)occupied), top_high((unsigned)(occupied >> 32)), s_rng[rng_idx]);
+                game.start(gs, top_low((unsigned)occupied), top_high((unsigned)(occupied >> 32)), AHEAD ? make_ulonglong2(0, 0) : s_rng[rng_idx]);
+                if (AHEAD) {
+                    game.ring = (unsigned)__cvta_generic_to_shared(draws.ring + rng_idx * AHEAD_STRIDE);
+                    game.place = draws.place[rng_idx];
+                }
             };
             auto close_game = [&]() {
                 int n = game.finish();
@@ -911,7 +990,7 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
                 if (game.marked()) {
                     // u == 1.0f somewhere in this game: replay it through the byte-level emulation of the reference
                     const GameSlot gs = s.slot[j];
-                    const ulonglong2 rs = s_rng[rng_idx];
+                    const ulonglong2 rs = AHEAD ? draws.state_of(s_rng, rng_idx) : s_rng[rng_idx];
                     const EmuResult er = playout_emulated(first_mover > 0 ? gs.other : gs.cur, first_mover > 0 ? gs.cur : gs.other,
                                                           first_mover, rs.x, rs.y);
                     game.s0 = er.s0;
@@ -921,7 +1000,8 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
                     my_ub += er.ub;
                     my_err |= er.err;
                 }
-                s_rng[rng_idx] = make_ulonglong2(game.s0, game.s1);
+                if (AHEAD) draws.used[rng_idx] = n;   // one draw a ply
+                else s_rng[rng_idx] = make_ulonglong2(game.s0, game.s1);
                 my_plies += n;
                 if (winner != 0) atomicAdd(&s.tally[j][winner > 0 ? 1 : 0], 1);
                 item = atomicAdd(&s.next_item, 1);
@@ -984,7 +1064,7 @@ __device__ __forceinline__ void run_slice(const SearchParams &p, Shared &s, ulon
     if (CL > 1) cg::this_cluster().sync();   // also: no block leaves while another may still write to its shared memory
     else __syncthreads();
     for (int i = tid; i < (n_streams >> LOG_CL); i += nt)
-        g_rng[((i >> log2_local) << p.log2_playouts) + rank * P_local + (i & (P_local - 1))] = s_rng[i];
+        g_rng[((i >> log2_local) << p.log2_playouts) + rank * P_local + (i & (P_local - 1))] = AHEAD ? draws.state_of(s_rng, i) : s_rng[i];
     if (rank != 0) return;
     if (tid == 0) {
         store_tree(p, s, g, first);
@@ -1052,7 +1132,7 @@ __device__ __forceinline__ void build_move_lut(MoveEntry *move_lut) {
 #ifndef MCTSNC_C4_MAXNREG
 #define MCTSNC_C4_MAXNREG 64
 #endif
-template <bool OCP, bool STRAIGHT>
+template <bool OCP, bool STRAIGHT, bool AHEAD = false>
 __global__ void __maxnreg__(MCTSNC_C4_MAXNREG) search_kernel(const SearchParams p) {
     __shared__ Shared s;
     extern __shared__ ulonglong2 s_rng[];
@@ -1086,7 +1166,7 @@ __global__ void __maxnreg__(MCTSNC_C4_MAXNREG) search_kernel(const SearchParams 
         const int n_steps = (queued && rem > p.chunk) ? p.chunk : rem;
         long long t_start = 0;
         if (queued && tid == 0) t_start = global_timer_ns();
-        run_slice<OCP, 1, STRAIGHT>(p, s, s_rng, nullptr, g, n_steps, p.first != 0 && rem == p.steps);
+        run_slice<OCP, 1, STRAIGHT, AHEAD>(p, s, s_rng, nullptr, s_rng + (OCP ? 1 : A) * p.n_playouts, g, n_steps, p.first != 0 && rem == p.steps);
         if (!queued) break;
         __syncthreads();  // every thread's writes of the slice precede the fence of thread 0
         if (tid == 0) {
@@ -1098,17 +1178,18 @@ __global__ void __maxnreg__(MCTSNC_C4_MAXNREG) search_kernel(const SearchParams 
 
 // A cluster of CL blocks per tree: launches with few trees (one search), where a step of a tree is bound by what one SM can play.
 // Launched with the cluster dimension as a launch attribute; cluster c grows tree c for the whole launch.  THREADS: of a block.
-template <bool OCP, int CL>
+template <bool OCP, int CL, bool AHEAD>
 __device__ __forceinline__ void run_cluster(const SearchParams &p) {
     __shared__ Shared s;
     extern __shared__ ulonglong2 s_rng[];
     build_move_lut(s.move_lut);
     const int n_local = ((OCP ? 1 : A) * p.n_playouts) / CL;   // streams this block keeps; the record cache follows
-    run_slice<OCP, CL, true>(p, s, s_rng, reinterpret_cast<int4 *>(s_rng + n_local), (int)(blockIdx.x / CL), p.steps, p.first != 0);
+    int4 *cache = reinterpret_cast<int4 *>(s_rng + n_local);
+    run_slice<OCP, CL, true, AHEAD>(p, s, s_rng, cache, cache + p.cache_nodes, (int)(blockIdx.x / CL), p.steps, p.first != 0);
 }
 
-template <bool OCP, int CL, int THREADS>
-__global__ void __launch_bounds__(THREADS, 2) search_cluster_kernel(const SearchParams p) { run_cluster<OCP, CL>(p); }
+template <bool OCP, int CL, int THREADS, bool AHEAD>
+__global__ void __launch_bounds__(THREADS, 2) search_cluster_kernel(const SearchParams p) { run_cluster<OCP, CL, AHEAD>(p); }
 
 // Clusters of 8 blocks of 256 threads, or -- from as many games a step as those blocks have threads beside the walking warp (1792) -- of
 // 16 blocks of 128 and a warp for the walk: a scheduler has one warp of games then instead of two.  4 trees, ACP 64 /
@@ -1122,7 +1203,7 @@ constexpr int WIDE_CLUSTER_BLOCKS = 16, WIDE_CLUSTER_THREADS = 160, WIDE_CLUSTER
 // 11.14 with a block per tree.  Where both fit the cap costs: 1 / 8 searches of 4 x 64 acp 3.16 / 3.57 ms against 2.91 / 3.24.
 template <bool OCP>
 __global__ void __launch_bounds__(CLUSTER_THREADS, 4) search_packed_cluster_kernel(const SearchParams p) {
-    run_cluster<OCP, CLUSTER_BLOCKS>(p);
+    run_cluster<OCP, CLUSTER_BLOCKS, false>(p);
 }
 
 }  // namespace c4

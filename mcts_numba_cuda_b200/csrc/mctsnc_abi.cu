@@ -74,7 +74,7 @@ struct mctsnc_handle {
     int tpb_roa = 0;
     int sm_count = 0;
     bool cluster_ok = false;      // thread-block clusters can be launched (and MCTSNC_B200_NO_CLUSTER is not set)
-    int cluster_fit[3][2] = {};   // clusters that fit on the device at once, [ClusterForm][small record cache] (0: not asked yet, -1: unknown)
+    int cluster_fit[4][2] = {};   // clusters that fit on the device at once, [ClusterForm][small record cache] (0: not asked yet, -1: unknown)
     int threads = 0;
     int blocks_per_sm = 0;
     long long bytes = 0;
@@ -571,7 +571,7 @@ int choose_threads(mctsnc_handle *h, long long trees) {
 struct PoolShape {
     int trees, walkers, threads;
 };
-constexpr int POOL_SMEM_LIMIT = 226 * 1024;
+constexpr int POOL_SMEM_LIMIT = 226 * 1024, AHEAD_SMEM_LIMIT = 200 * 1024;
 
 const void *pool_kernel_ptr(bool ocp) { return ocp ? (const void *)c4::pool_kernel<true> : (const void *)c4::pool_kernel<false>; }
 
@@ -815,14 +815,16 @@ int launch_search_gomoku(mctsnc_handle *h, int batch, int steps, int first, cuda
     return (int)cudaGetLastError();
 }
 
-// the forms a cluster per tree comes in, in the order they are tried
-enum ClusterForm { WIDE, PLAIN, PACKED };
+// the forms a cluster per tree comes in, in the order they are tried (WIDE and AHEAD: draws made ahead, a block on an SM)
+enum ClusterForm { WIDE, AHEAD, PLAIN, PACKED, CLUSTER_FORMS };
 
 const void *cluster_kernel_ptr(bool ocp, int form) {
-    if (form == WIDE) return (const void *)c4::search_cluster_kernel<false, c4::WIDE_CLUSTER_BLOCKS, c4::WIDE_CLUSTER_THREADS>;   // acp only
+    if (form == WIDE) return (const void *)c4::search_cluster_kernel<false, c4::WIDE_CLUSTER_BLOCKS, c4::WIDE_CLUSTER_THREADS, true>;   // acp only
     if (form == PACKED) return ocp ? (const void *)c4::search_packed_cluster_kernel<true> : (const void *)c4::search_packed_cluster_kernel<false>;
-    return ocp ? (const void *)c4::search_cluster_kernel<true, c4::CLUSTER_BLOCKS, c4::CLUSTER_THREADS>
-               : (const void *)c4::search_cluster_kernel<false, c4::CLUSTER_BLOCKS, c4::CLUSTER_THREADS>;
+    if (form == AHEAD) return ocp ? (const void *)c4::search_cluster_kernel<true, c4::CLUSTER_BLOCKS, c4::CLUSTER_THREADS, true>
+                                  : (const void *)c4::search_cluster_kernel<false, c4::CLUSTER_BLOCKS, c4::CLUSTER_THREADS, true>;
+    return ocp ? (const void *)c4::search_cluster_kernel<true, c4::CLUSTER_BLOCKS, c4::CLUSTER_THREADS, false>
+               : (const void *)c4::search_cluster_kernel<false, c4::CLUSTER_BLOCKS, c4::CLUSTER_THREADS, false>;
 }
 
 int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_t stream) {
@@ -881,8 +883,8 @@ int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_
         const bool ocp = is_ocp(h->cfg);
         // the wide cluster first where a step has games for it (an ocp step never has: 512 at most); then the first form that fits
         // on the device
-        for (int form = !ocp && h->A * h->cfg.n_playouts >= c4::WIDE_CLUSTER_MIN_GAMES ? WIDE : PLAIN; form <= PACKED; form++) {
-            const bool wide = form == WIDE;
+        for (int form = !ocp && h->A * h->cfg.n_playouts >= c4::WIDE_CLUSTER_MIN_GAMES ? WIDE : AHEAD; form <= PACKED; form++) {
+            const bool wide = form == WIDE, ahead = form == WIDE || form == AHEAD;
             const int blocks = wide ? c4::WIDE_CLUSTER_BLOCKS : c4::CLUSTER_BLOCKS;
             const void *kernel = cluster_kernel_ptr(ocp, form);
             if (wide && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
@@ -904,12 +906,13 @@ int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_
             // The first records of a tree stay in the first block's shared memory: many if every block can have an SM to itself,
             // else few.  All clusters of the launch have to be on the device at once (clusters do not spread over GPCs, so fewer
             // fit than blocks / 8): a tree whose cluster waits for another to finish would take two searches' time.  A wide cluster
-            // is for blocks that have an SM each, a packed one for blocks that share it.
+            // and one with draws made ahead are for blocks that have an SM each, a packed one for blocks that share it.
             bool fits = false;
             const bool own_sm = trees * blocks <= h->sm_count;
-            for (int small = own_sm && form != PACKED ? 0 : 1; small < (wide ? 1 : 2) && !fits; small++) {
+            for (int small = own_sm && form != PACKED ? 0 : 1; small < (ahead ? 1 : 2) && !fits; small++) {
                 p.cache_nodes = small ? 2048 : MCTSNC_C4_CACHE_NODES;
-                lc.dynamicSmemBytes = h->dyn_smem / blocks + sizeof(int4) * (size_t)p.cache_nodes;
+                lc.dynamicSmemBytes = h->dyn_smem / blocks + sizeof(int4) * (size_t)p.cache_nodes +
+                                      (ahead ? c4::Draws::bytes((int)(h->dyn_smem / sizeof(ulonglong2)) / blocks) : 0);
                 int &fit = h->cluster_fit[form][small];
                 if (fit == 0) {
                     int n = 0;
@@ -954,7 +957,17 @@ int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_
     if (h->cfg.threads_per_tree == 0 && trees <= h->sm_count && threads + 32 <= 1024) threads += 32;
     int per_sm = 0;
     const void *kernel = search_kernel_ptr(h->cfg, play_straight(h->cfg, threads));
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, h->dyn_smem) != cudaSuccess || per_sm < 1)
+    size_t smem = h->dyn_smem;
+    // The threads that play make their draws while that warp walks (see Draws), where shared memory has room for them; two to four
+    // warps do not.
+    const size_t with_draws = smem + c4::Draws::bytes((int)(smem / sizeof(ulonglong2)));
+    const int playing_warps = h->threads / 32;
+    if (threads > h->threads && play_straight(h->cfg, h->threads) && (playing_warps == 1 || playing_warps > 4) && with_draws <= (size_t)AHEAD_SMEM_LIMIT) {
+        kernel = is_ocp(h->cfg) ? (const void *)c4::search_kernel<true, true, true> : (const void *)c4::search_kernel<false, true, true>;
+        CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AHEAD_SMEM_LIMIT));
+        smem = with_draws;
+    }
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess || per_sm < 1)
         return MCTSNC_E_BAD_ARGUMENT;
     h->blocks_per_sm = per_sm;
     // More trees than blocks fit on the device at once: a persistent grid takes slices of SLICE_STEPS steps from the
@@ -969,7 +982,7 @@ int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_
         p.places = (int)resident;
     }
     void *args[] = {&p};
-    CUDA_TRY(cudaLaunchKernel(kernel, dim3(grid), dim3((unsigned)threads), args, h->dyn_smem, stream));
+    CUDA_TRY(cudaLaunchKernel(kernel, dim3(grid), dim3((unsigned)threads), args, smem, stream));
     if (p.queue) check_queue_kernel<<<(unsigned)((trees + 255) / 256), 256, 0, stream>>>(h->remaining, h->state, (int)trees);
     return (int)cudaGetLastError();
 }

@@ -46,3 +46,22 @@ def test_late_positions_match_oracle_whatever_thread_plays_a_game(variant, n_pla
         compare_trees(ai, orc)
         assert int(best) == orc.best_action
         assert (ai._res["playouts"], ai._res["plies"]) == (orc.playouts, orc.plies)
+
+
+@pytest.mark.parametrize("variant,n_trees,n_playouts,empty,steps", [
+    ("ocp_thrifty", 1, 32, 20, 150), ("ocp_prodigal", 2, 256, 3, 60), ("ocp_prodigal", 1, 512, 30, 60), ("acp_prodigal", 2, 32, 12, 60),
+    ("acp_thrifty", 1, 64, 42, 60), ("acp_prodigal", 3, 128, 9, 60), ("acp_prodigal", 9, 256, 16, 40), ("acp_thrifty", 1, 512, 42, 40)])
+def test_draws_made_ahead_match_oracle(variant, n_trees, n_playouts, empty, steps):
+    """A block or a cluster whose SMs are its own: the threads that play make the draws between the steps.  The streams have to stand
+    where the games left them: the next search starts from there."""
+    board, fills, turn = late_root(empty, seed=empty) if empty < 42 else (np.zeros((6, 7), np.int8), np.zeros(7, np.int8), 1)
+    ai = MCTSNC((6, 7), 7, 7, search_time_limit=np.inf, search_steps_limit=steps, n_trees=n_trees, n_playouts=n_playouts, variant=variant,
+                seed=11, verbose_info=False)
+    ai.init_device_side_arrays()
+    orc = OracleMCTSNC((6, 7), 7, 7, n_trees=n_trees, n_playouts=n_playouts, variant=variant, seed=11, node_capacity=steps * 7 + 8)
+    for _ in range(3):
+        best = ai.run(board, fills, turn)
+        orc.run(board, fills, turn, steps)
+        compare_trees(ai, orc)
+        assert int(best) == orc.best_action
+        assert (ai._res["playouts"], ai._res["plies"]) == (orc.playouts, orc.plies)
