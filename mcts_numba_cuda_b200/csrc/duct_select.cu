@@ -64,11 +64,12 @@ select_kernel(float cpuct, int virtual_loss, int *child_all, const float *__rest
               int path_depth) {
     constexpr int GROUP = 2 * LANES, PER_WARP = 32 / GROUP;
     constexpr int SLOTS = (LANES * LANES + GROUP - 1) / GROUP;   // child ids a lane may hold
+    const unsigned block = block_after_the_kernel_before();
     const int lane = threadIdx.x & 31;
     const int sub = lane & (GROUP - 1), base = lane & ~(GROUP - 1);   // lane within the traversal, its first lane
     const int player = sub / LANES, action = sub & (LANES - 1);
     // the traversals of a warp belong to neighbouring trees (those of one tree would lose each other's claims in step)
-    const int unit = (int)blockIdx.x * WARPS_PER_BLOCK + (int)(threadIdx.x >> 5);
+    const int unit = (int)block * WARPS_PER_BLOCK + (int)(threadIdx.x >> 5);
     const int first_tree = unit / warps * PER_WARP, wid = unit % warps;
     const bool exists = first_tree + lane / GROUP < trees;
     const int tree = exists ? first_tree + lane / GROUP : 0;
@@ -285,11 +286,12 @@ group_select_kernel(float cpuct, int virtual_loss, int *child_all, const float *
                     const int *__restrict__ node_n, int *node_inflight_all, const int *__restrict__ node_terminal,
                     const int *__restrict__ tree_nodes, int *out_selected, int *out_path, int *out_len, int trees, int nodes, int A, int warps,
                     int path_depth) {
+    const unsigned block = block_after_the_kernel_before();
     const int lane = threadIdx.x & 31;
     const int sub = lane & (GROUP_LANES - 1), base = lane & ~(GROUP_LANES - 1);   // lane within the traversal, its first lane
     const int trees_per_warp = GROUPS / warps;
     const int mine = (lane / GROUP_LANES) / warps, wid = (lane / GROUP_LANES) - mine * warps;   // tree of the warp, traversal of the tree
-    const int unit = (int)blockIdx.x * GROUP_WARPS + (int)(threadIdx.x >> 5);
+    const int unit = (int)block * GROUP_WARPS + (int)(threadIdx.x >> 5);
     const bool exists = mine < trees_per_warp && unit * trees_per_warp + mine < trees;
     const int tree = exists ? unit * trees_per_warp + mine : 0;
     const int out = tree * warps + wid;
@@ -490,7 +492,7 @@ static unsigned select_blocks(int trees, int trees_per_warp, int warps) {
 __global__ void backup_kernel(int virtual_loss, int *child, float *node_w, int *node_n, int *node_inflight, const int *out_selected,
                               const int *out_path, const int *out_len, const float *values, const int *new_child, int nodes, int A,
                               int traversals, int warps, int path_depth, int log2_lanes) {
-    const BackupLane at_work(traversals, log2_lanes);
+    const BackupLane at_work(block_after_the_kernel_before(), traversals, log2_lanes);
     const int out = at_work.traversal;
     if (out < 0) return;
     const int len = out_len[out];
@@ -530,7 +532,7 @@ extern "C" int duct_select_launch(float cpuct, int virtual_loss, int *child, con
         warps > 32 || path_depth <= 0 || virtual_loss < 0)
         return (int)cudaErrorInvalidValue;
 #define DUCT_LAUNCH(L)                                                                                                        \
-    duct::select_kernel<L><<<duct::select_blocks(trees, 16 / L, warps), duct::WARPS_PER_BLOCK * 32, 0, (cudaStream_t)stream>>>( \
+    select_math::launch_behind(duct::select_kernel<L>, duct::select_blocks(trees, 16 / L, warps), duct::WARPS_PER_BLOCK * 32, (cudaStream_t)stream,  \
         cpuct, virtual_loss, child, node_prior, node_w, node_n, node_inflight, node_terminal, tree_nodes, out_selected,       \
         out_path, out_len, trees, nodes, actions, warps, path_depth)
     if (duct::traversals_in_step(trees, actions, warps)) {
@@ -539,7 +541,7 @@ extern "C" int duct_select_launch(float cpuct, int virtual_loss, int *child, con
         const unsigned blocks = (unsigned)((units + duct::GROUP_WARPS - 1) / duct::GROUP_WARPS);
         const bool vectors = duct::rows_take_vectors(actions, node_prior, node_w, node_n, node_inflight);
 #define DUCT_GROUP_LAUNCH(APL, V)                                                                                             \
-    duct::group_select_kernel<APL, V><<<blocks, duct::GROUP_WARPS * 32, 0, (cudaStream_t)stream>>>(                          \
+    select_math::launch_behind(duct::group_select_kernel<APL, V>, blocks, duct::GROUP_WARPS * 32, (cudaStream_t)stream,                           \
         cpuct, virtual_loss, child, node_prior, node_w, node_n, node_inflight, node_terminal, tree_nodes, out_selected,       \
         out_path, out_len, trees, nodes, actions, warps, path_depth)
         if (actions <= 4) DUCT_GROUP_LAUNCH(1, false);
@@ -565,7 +567,7 @@ extern "C" int duct_backup_launch(int virtual_loss, int *child, float *node_w, i
         return (int)cudaErrorInvalidValue;
     if ((long long)trees * warps > 0x7FFFFFFF) return (int)cudaErrorInvalidValue;
     const select_math::BackupGrid g(trees * warps, path_depth);
-    duct::backup_kernel<<<g.blocks, g.THREADS, 0, (cudaStream_t)stream>>>(virtual_loss, child, node_w, node_n, node_inflight, out_selected,
+    select_math::launch_behind(duct::backup_kernel, g.blocks, g.THREADS, (cudaStream_t)stream, virtual_loss, child, node_w, node_n, node_inflight, out_selected,
                                                                           out_path, out_len, values, new_child, nodes, actions,
                                                                           trees * warps, warps, path_depth, g.log2_lanes);
     return (int)cudaGetLastError();

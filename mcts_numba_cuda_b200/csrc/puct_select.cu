@@ -157,14 +157,15 @@ select_kernel(float cpuct, float c_pw, float alpha_pw, int soft_winner, const in
               int *edge_inflight, int *node_expand_inflight, const int *__restrict__ node_expanded,
               const int *__restrict__ tree_nodes, int *out_selected_node, int *out_path_eids, int *out_path_len, int nodes,
               int edges, int warps, int path_depth, int vl, int trees) {
+    const unsigned block = block_after_the_kernel_before();
     const int lane = threadIdx.x;
     int tree, wid, traversal;
     if (RESUMED) {   // the traversals that go on are the first of their trees, but for ties: they start first, the others leave at once
-        wid = blockIdx.x / trees;
-        tree = blockIdx.x - wid * trees;
+        wid = block / trees;
+        tree = block - wid * trees;
         traversal = tree * warps + wid;
     } else {
-        traversal = blockIdx.x;
+        traversal = block;
         tree = traversal / warps;
         wid = traversal - tree * warps;
     }
@@ -396,7 +397,8 @@ root_kernel(float cpuct, int soft_winner, const int *__restrict__ edge_child_id,
             const float *__restrict__ edge_W, const int *__restrict__ edge_N, int *edge_inflight, const int *__restrict__ node_expanded,
             const int *__restrict__ tree_nodes, int *out_selected_node, int *out_path_eids, int *out_path_len, int trees, int nodes, int edges,
             int warps, int path_depth, int vl) {
-    const int lane = threadIdx.x & 31, tree = blockIdx.x * ROOT_WARPS + (threadIdx.x >> 5);
+    const unsigned block = block_after_the_kernel_before();
+    const int lane = threadIdx.x & 31, tree = block * ROOT_WARPS + (threadIdx.x >> 5);
     if (tree >= trees) return;
     const bool mine = lane < warps;   // lane w: traversal w
     const long long traversal = (long long)tree * warps + lane;
@@ -495,7 +497,7 @@ __global__ void backup_kernel(int virtual_loss, float *edge_W, int *edge_N, int 
                               const int *__restrict__ out_path_eids, const int *__restrict__ out_path_len,
                               const float *__restrict__ path_edge_values, int traversals, int nodes, int edges, int warps,
                               int path_depth, int log2_lanes) {
-    const BackupLane at_work(traversals, log2_lanes);
+    const BackupLane at_work(block_after_the_kernel_before(), traversals, log2_lanes);
     const int out_ix = at_work.traversal;
     if (out_ix < 0) return;
     const int tree = out_ix / warps;
@@ -538,10 +540,10 @@ static int launch_select(float cpuct, float c_pw, float alpha_pw, int soft_winne
     if (c_pw == 0.0f && roots_first(trees, edges, warps)) {
 #define PUCT_LAUNCH(E)                                                                                                     \
     do {                                                                                                                  \
-        root_kernel<E><<<((unsigned)trees + ROOT_WARPS - 1) / ROOT_WARPS, ROOT_WARPS * 32, 0, stream>>>(cpuct, soft_winner, edge_child_id, edge_prior, edge_W, edge_N, edge_inflight,       \
+        select_math::launch_behind(root_kernel<E>, ((unsigned)trees + ROOT_WARPS - 1) / ROOT_WARPS, ROOT_WARPS * 32, stream, cpuct, soft_winner, edge_child_id, edge_prior, edge_W, edge_N, edge_inflight,       \
                                                     node_expanded, tree_nodes, out_selected_node, out_path_eids,           \
                                                     out_path_len, trees, nodes, edges, warps, path_depth, virtual_loss);   \
-        select_kernel<E, false, true><<<grid, 32, 0, stream>>>(                                                           \
+        select_math::launch_behind(select_kernel<E, false, true>, grid, 32, stream,                                                            \
             cpuct, c_pw, alpha_pw, soft_winner, edge_child_id, edge_prior, edge_W, edge_N, edge_inflight,                  \
             node_expand_inflight, node_expanded, tree_nodes, out_selected_node, out_path_eids, out_path_len, nodes, edges, \
             warps, path_depth, virtual_loss, trees);                                                                   \
@@ -554,7 +556,7 @@ static int launch_select(float cpuct, float c_pw, float alpha_pw, int soft_winne
         return (int)cudaGetLastError();
     }
 #define PUCT_LAUNCH_AS(E, W)                                                                                              \
-    select_kernel<E, W, false><<<grid, 32, 0, stream>>>(cpuct, c_pw, alpha_pw, soft_winner, edge_child_id, edge_prior, edge_W,     \
+    select_math::launch_behind(select_kernel<E, W, false>, grid, 32, stream, cpuct, c_pw, alpha_pw, soft_winner, edge_child_id, edge_prior, edge_W,     \
                                                  edge_N, edge_inflight, node_expand_inflight, node_expanded, tree_nodes,    \
                                                  out_selected_node, out_path_eids, out_path_len, nodes, edges, warps,       \
                                                  path_depth, virtual_loss, trees)
@@ -609,7 +611,7 @@ extern "C" int puct_backup_launch(int virtual_loss, float *edge_W, int *edge_N, 
     if (trees <= 0 || warps <= 0 || warps > 32) return (int)cudaErrorInvalidValue;
     if ((long long)trees * warps > 0x7FFFFFFF) return (int)cudaErrorInvalidValue;
     const select_math::BackupGrid g(trees * warps, path_depth);
-    puct::backup_kernel<<<g.blocks, g.THREADS, 0, (cudaStream_t)stream>>>(virtual_loss, edge_W, edge_N, edge_inflight, node_expand_inflight,
+    select_math::launch_behind(puct::backup_kernel, g.blocks, g.THREADS, (cudaStream_t)stream, virtual_loss, edge_W, edge_N, edge_inflight, node_expand_inflight,
                                                                           tree_nodes, out_selected_node, out_path_eids, out_path_len,
                                                                           path_edge_values, trees * warps, nodes, edges, warps,
                                                                           path_depth, g.log2_lanes);

@@ -187,8 +187,9 @@ select_kernel(float cpuct, float c_pw, float alpha_pw, const int *__restrict__ e
               const float *__restrict__ edge_W, const int *__restrict__ edge_N, int *node_inflight_all, int *node_expand_inflight,
               const int *__restrict__ node_expanded, const int *__restrict__ tree_nodes, int *out_selected_node, int *out_path_eids,
               int *out_path_len, int nodes, int edges, int warps, int path_depth) {
+    const unsigned block = block_after_the_kernel_before();
     const int lane = threadIdx.x;
-    const int traversal = blockIdx.x;
+    const int traversal = block;
     const int tree = traversal / warps;
     const int wid = traversal - tree * warps;
     int *path = out_path_eids + (long long)traversal * path_depth;
@@ -397,7 +398,7 @@ __global__ void backup_kernel(int virtual_loss, const int *__restrict__ edge_chi
                               const int *__restrict__ out_selected_node, const int *__restrict__ out_path_eids,
                               const int *__restrict__ out_path_len, const float *__restrict__ path_edge_values, int traversals, int nodes,
                               int edges, int warps, int path_depth, int log2_lanes) {
-    const BackupLane at_work(traversals, log2_lanes);
+    const BackupLane at_work(block_after_the_kernel_before(), traversals, log2_lanes);
     const int traversal = at_work.traversal;
     if (traversal < 0) return;
     const int tree = traversal / warps;
@@ -444,7 +445,7 @@ extern "C" int puct_v2_select_launch(int variant, float cpuct, float c_pw, float
     const unsigned grid = (unsigned)((long long)trees * warps);
     const cudaStream_t s = (cudaStream_t)stream;
 #define PUCT_V2_LAUNCH(P, E, W)                                                                                              \
-    puct_v2::select_kernel<P, E, W><<<grid, 32, 0, s>>>(cpuct, c_pw, alpha_pw, edge_child_id, edge_prior, edge_W, edge_N,    \
+    select_math::launch_behind(puct_v2::select_kernel<P, E, W>, grid, 32, s, cpuct, c_pw, alpha_pw, edge_child_id, edge_prior, edge_W, edge_N,    \
                                                         node_inflight, node_expand_inflight, node_expanded, tree_nodes,      \
                                                         out_selected_node, out_path_eids, out_path_len, nodes, edges, warps, \
                                                         path_depth)
@@ -471,7 +472,7 @@ extern "C" int puct_v2_backup_launch(int virtual_loss, const int *edge_child_id,
     if (trees <= 0 || warps <= 0 || warps > 32) return (int)cudaErrorInvalidValue;
     if ((long long)trees * warps > 0x7FFFFFFF) return (int)cudaErrorInvalidValue;
     const select_math::BackupGrid g(trees * warps, path_depth);
-    puct_v2::backup_kernel<<<g.blocks, g.THREADS, 0, (cudaStream_t)stream>>>(virtual_loss, edge_child_id, edge_W, edge_N, node_inflight,
+    select_math::launch_behind(puct_v2::backup_kernel, g.blocks, g.THREADS, (cudaStream_t)stream, virtual_loss, edge_child_id, edge_W, edge_N, node_inflight,
                                                                              node_expand_inflight, tree_nodes, out_selected_node,
                                                                              out_path_eids, out_path_len, path_edge_values,
                                                                              trees * warps, nodes, edges, warps, path_depth,
