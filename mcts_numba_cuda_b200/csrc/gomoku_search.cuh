@@ -879,6 +879,7 @@ static_assert((THREAD_WORDS * DYN_THREADS) % 4 == 0 && SHEET_WORDS % 4 == 0 && T
 template <bool OCP, bool ONE_TREE>
 __global__ void __launch_bounds__(DYN_THREADS) playout_dynamic_kernel(const __grid_constant__ Params p, int total_trees) {
     constexpr int REFILL_MIN = ONE_TREE ? 8 : 12;
+    if (ONE_TREE) asm volatile("griddepcontrol.wait;" ::: "memory");   // the step before: its blocks may still be here
     extern __shared__ __align__(16) unsigned s_mem[];
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
@@ -979,6 +980,7 @@ __global__ void __launch_bounds__(DYN_THREADS) playout_dynamic_kernel(const __gr
         // what this warp's lanes have written comes before its arrival, and the step after all arrivals
         __threadfence();
         __syncwarp();
+        asm volatile("griddepcontrol.launch_dependents;");   // the next step's blocks may come, once all of this one are here
         int arrived = 0;
         if (lane == 0) arrived = atomicAdd(&p.work[p.tree_base].done, 1);
         arrived = __shfl_sync(0xFFFFFFFFu, arrived, 0);
