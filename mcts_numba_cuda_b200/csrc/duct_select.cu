@@ -226,8 +226,8 @@ select_kernel(float cpuct, int virtual_loss, int *child_all, const float *__rest
 // The claims of earlier turns are seen: __syncwarp orders them before the next loads, and no other warp is in the tree.
 // The child of the joint action is loaded when it is known: a node's whole row of children, loaded ahead as in
 // select_kernel, is as much as all its statistics, and with every traversal on the device at once memory's throughput counts.
-// What bounds it: instructions (the logic pipe two thirds busy) and two round trips to memory a level; 4096 trees x 8 actions x 8
-// traversals x 16 levels 159 us with select_kernel, 95 so (111 with all choices of a level in one turn, which takes the whole
+// What bounds it: a chain of two round trips to memory and some 400 instructions a turn (1500 trees: 31 % of the issue slots, half of a
+// warp's time waiting for memory); 4096 trees x 8 actions x 8 traversals x 16 levels 159 us with select_kernel, 95 so (111 with all choices of a level in one turn, which takes the whole
 // warp along).
 // VECTORS: rows of 4 * APL actions on addresses that take a lane's actions in one load.
 constexpr int GROUP_LANES = 4, GROUPS = 8, GROUP_WARPS = 4;

@@ -884,7 +884,7 @@ int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_
     p.times2p23 = 1u << 23;
     // Few trees (one search, a few searches): a cluster of blocks per tree, so that the games of a step are played on
     // several SMs at once.  Measured, 4 x 256 acp_prodigal, 2000 steps, 1 / 4 / 8 searches in one launch: 13.7 / 14.4 / 20.6 ms with
-    // clusters against 42.2 with a block of 1024 threads per tree; 500 steps, 9 / 12 / 16 searches: 5.0 / 5.6 / 7.0 against 11.1 --
+    // clusters against 42.2 with a block of 1024 threads per tree (12.6 for one with draws made ahead); 500 steps, 9 / 12 / 16 searches: 5.0 / 5.6 / 7.0 against 11.1 --
     // up to four cluster blocks per SM pay, and more do not fit.
     // Only where a step has more than 256 games (ACP with 64 playouts or more, OCP with 512).  One search of 2000 steps, 4
     // trees, with a block / with clusters: ACP 8 / 16 / 32 / 64 / 128 / 256 / 512 playouts 9.1 / 9.3 / 11.7 / 16.6 / 25.4 / 42.2 / 64.5 ms
