@@ -597,7 +597,8 @@ bool choose_pool(const mctsnc_handle *h, long long trees, int steps, PoolShape *
     const bool large = games >= 896;
     if (h->cfg.threads_per_tree > 0 || steps <= SLICE_STEPS || games <= 32 || trees <= (large ? h->sm_count + h->sm_count / 6 : h->sm_count)) return false;
     const long long need = (trees + h->sm_count - 1) / h->sm_count;
-    const long long most = (long long)ceilf(150.f / sqrtf((float)games));   // 4 trees of 1792 games, 10 of 256, 14 of 128
+    // 5 trees of 1792 games (256 roots of 4 x 256, 2000 steps: 86.3 ms with 4, 84.5 with 5, 96.5 with 6), 10 of 256, 14 of 128
+    const long long most = (long long)ceilf((large ? 180.f : 150.f) / sqrtf((float)games));
     long long k = need;
     if (large) k = (long long)(0.72f * (float)trees / (float)h->sm_count + 0.6f);
     else if (need > 3 && games > 128 && need * games > 2048) k = need * 18 / 25 < 3 ? 3 : need * 18 / 25;

@@ -61,3 +61,22 @@ def test_pooled_trees_that_fill_up_equal_a_block_per_tree(variant):
     for b in (0, roots - 1):
         for name in ("trees_ns", "trees_ns_wins", "trees_playout_outcomes", "trees_actions_expanded"):
             assert np.array_equal(*(ai.export(name, b) for ai in handles)), name
+
+
+def test_a_search_over_several_launches_equals_one():
+    """A search of many trees under a time limit: its launches go on from what the one before has left."""
+    kw = dict(n_trees=200, n_playouts=16, variant="acp_prodigal", seed=4, verbose_info=False)
+    board, fills = np.zeros((6, 7), np.int8), np.zeros(7, np.int8)
+    timed = MCTSNC((6, 7), 7, 7, search_time_limit=0.03, search_steps_limit=np.inf, **kw)
+    timed.init_device_side_arrays()
+    best = timed.run(board, fills, 1)
+    assert timed.steps > 70 and timed.launch_geometry()["blocks_per_sm"] == 2        # launches of 2 ms, trees of a block
+    whole = MCTSNC((6, 7), 7, 7, search_time_limit=np.inf, search_steps_limit=float(timed.steps), **kw)
+    whole.init_device_side_arrays()
+    assert best == whole.run(board, fills, 1)
+    for name in ("playouts", "plies", "total_nodes", "depth_sum"):
+        assert timed._res[name] == whole._res[name], name
+    sizes = timed.export("trees_sizes")
+    assert np.array_equal(sizes, whole.export("trees_sizes"))
+    for name in ("trees_ns", "trees_ns_wins"):
+        assert np.array_equal(timed.export(name, max_nodes=int(sizes.max())), whole.export(name, max_nodes=int(sizes.max()))), name
