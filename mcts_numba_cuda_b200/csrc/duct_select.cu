@@ -64,6 +64,7 @@ select_kernel(float cpuct, int virtual_loss, int *child_all, const float *__rest
               int path_depth) {
     constexpr int GROUP = 2 * LANES, PER_WARP = 32 / GROUP;
     constexpr int SLOTS = (LANES * LANES + GROUP - 1) / GROUP;   // child ids a lane may hold
+    let_the_next_kernel_come();
     const unsigned block = block_after_the_kernel_before();
     const int lane = threadIdx.x & 31;
     const int sub = lane & (GROUP - 1), base = lane & ~(GROUP - 1);   // lane within the traversal, its first lane
@@ -286,6 +287,7 @@ group_select_kernel(float cpuct, int virtual_loss, int *child_all, const float *
                     const int *__restrict__ node_n, int *node_inflight_all, const int *__restrict__ node_terminal,
                     const int *__restrict__ tree_nodes, int *out_selected, int *out_path, int *out_len, int trees, int nodes, int A, int warps,
                     int path_depth) {
+    let_the_next_kernel_come();
     const unsigned block = block_after_the_kernel_before();
     const int lane = threadIdx.x & 31;
     const int sub = lane & (GROUP_LANES - 1), base = lane & ~(GROUP_LANES - 1);   // lane within the traversal, its first lane

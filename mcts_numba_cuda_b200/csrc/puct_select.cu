@@ -157,6 +157,7 @@ select_kernel(float cpuct, float c_pw, float alpha_pw, int soft_winner, const in
               int *edge_inflight, int *node_expand_inflight, const int *__restrict__ node_expanded,
               const int *__restrict__ tree_nodes, int *out_selected_node, int *out_path_eids, int *out_path_len, int nodes,
               int edges, int warps, int path_depth, int vl, int trees) {
+    let_the_next_kernel_come();
     const unsigned block = block_after_the_kernel_before();
     const int lane = threadIdx.x;
     int tree, wid, traversal;
@@ -397,6 +398,7 @@ root_kernel(float cpuct, int soft_winner, const int *__restrict__ edge_child_id,
             const float *__restrict__ edge_W, const int *__restrict__ edge_N, int *edge_inflight, const int *__restrict__ node_expanded,
             const int *__restrict__ tree_nodes, int *out_selected_node, int *out_path_eids, int *out_path_len, int trees, int nodes, int edges,
             int warps, int path_depth, int vl) {
+    let_the_next_kernel_come();
     const unsigned block = block_after_the_kernel_before();
     const int lane = threadIdx.x & 31, tree = block * ROOT_WARPS + (threadIdx.x >> 5);
     if (tree >= trees) return;

@@ -187,6 +187,7 @@ select_kernel(float cpuct, float c_pw, float alpha_pw, const int *__restrict__ e
               const float *__restrict__ edge_W, const int *__restrict__ edge_N, int *node_inflight_all, int *node_expand_inflight,
               const int *__restrict__ node_expanded, const int *__restrict__ tree_nodes, int *out_selected_node, int *out_path_eids,
               int *out_path_len, int nodes, int edges, int warps, int path_depth) {
+    let_the_next_kernel_come();
     const unsigned block = block_after_the_kernel_before();
     const int lane = threadIdx.x;
     const int traversal = block;
