@@ -33,8 +33,10 @@ constexpr int POOL_ADDRESS_BITS = 18;
 constexpr unsigned POOL_FREE = (1u << POOL_ADDRESS_BITS) - 1u;
 constexpr unsigned POOL_MEMORY = 227 * 1024;        // of an SM; an address below it is a slot
 __device__ __forceinline__ unsigned pool_cell(unsigned entry, unsigned address) { return (entry << POOL_ADDRESS_BITS) | address; }
-// Looks of an idle warp for work before the launch is given up (a second or more; it waits for a walker, which waits for no
-// other block)
+// Looks of an idle warp for work before it takes its wait for endless; the pauses between them are nominally 0.08 s (walkers) and 0.4 s
+// (players).  A walker waits for games that are played or handed out, some hundred microseconds at most, and gives the launch up.  A player
+// may wait as long as the walkers have nothing to play: steps that select a terminal node play no game, and a tree with a won root
+// has stretches of millions of them.  It gives up when no tree of the block has gone on since its last such wait.
 constexpr int POOL_IDLE_LIMIT = 1 << 22;
 
 enum PoolPhase { POOL_EMPTY, POOL_READY, POOL_PENDING, POOL_PLAYING };
@@ -64,7 +66,9 @@ struct Pool {
     unsigned next_ticket, next_entry;
     int walkers_left;
     int given_up;
+    unsigned seen[32];   // by a warp that plays, see pool_moves
 };
+static_assert(sizeof(Pool) % 16 == 0, "the trees follow");
 
 __host__ __device__ __forceinline__ size_t pool_bytes(int trees, int streams) {
     return sizeof(Pool) + (size_t)trees * (sizeof(PoolTree) + A * sizeof(PoolSlot) + sizeof(ulonglong2) * (size_t)streams);
@@ -81,6 +85,19 @@ __device__ __forceinline__ void store_release(unsigned *p, unsigned v) {
 }
 __device__ __forceinline__ void add_release(unsigned *p, unsigned v) {
     asm volatile("red.release.cta.shared.add.u32 [%0], %1;" ::"r"(shared_address(p)), "r"(v) : "memory");
+}
+
+// Whether a tree of the block has made a step since this warp asked last, and the launch has not been given up: a slice's start and the
+// steps made of it, which only grow, summed over the trees.  Neither in the players' loop nor with a vote, which make that loop slower
+// (256 roots of 4 x 256 acp 2 %, 200 of 4 x 64 5 %); with a count kept by the walkers an ocp batch is 1 to 6 % slower.
+__device__ __noinline__ bool pool_moves(Pool &pool, const PoolTree *trees, int n) {
+    long long now = 0;
+    for (int k = 0; k < n; k++) now += *(volatile const long long *)&trees[k].t_start + *(volatile const int *)&trees[k].step;
+    volatile unsigned &seen = pool.seen[threadIdx.x >> 5];
+    const bool moves = (unsigned)now != seen;
+    __syncwarp();
+    seen = (unsigned)now;
+    return moves && !*(volatile int *)&pool.given_up;
 }
 
 template <bool OCP>
@@ -331,8 +348,11 @@ __device__ __forceinline__ void pool_play(const SearchParams &p, Pool &pool, Poo
             if (*(volatile int *)&pool.walkers_left == 0) break;
             __nanosleep(100);
             if (++idle > POOL_IDLE_LIMIT || *(volatile int *)&pool.given_up) {
-                *(volatile int *)&pool.given_up = 1;
-                break;
+                idle = 0;
+                if (!pool_moves(pool, trees, p.pool_trees)) {
+                    *(volatile int *)&pool.given_up = 1;
+                    break;
+                }
             }
         } else {
             idle = 0;
@@ -354,6 +374,7 @@ __global__ void __launch_bounds__(1024, 1) pool_kernel(const SearchParams p) {
         pool.next_entry = 0u;
         pool.walkers_left = p.pool_walkers;
         pool.given_up = 0;
+        for (int i = 0; i < 32; i++) pool.seen[i] = 0u;
     }
     __syncthreads();
     const int warp = threadIdx.x >> 5;

@@ -80,3 +80,29 @@ def test_a_search_over_several_launches_equals_one():
     assert np.array_equal(sizes, whole.export("trees_sizes"))
     for name in ("trees_ns", "trees_ns_wins"):
         assert np.array_equal(timed.export(name, max_nodes=int(sizes.max())), whole.export(name, max_nodes=int(sizes.max()))), name
+
+
+@pytest.mark.parametrize("empty,seed", [(11, 84), (13, 37)])
+def test_pooled_trees_outlast_a_million_steps_without_a_game(empty, seed):
+    """The mover wins at once: from some step before 2000 to one after 1500000 every step selects the won child, and no game is played;
+    then there are games again.  The players of a block wait that long, for seconds."""
+    steps, roots = 1_700_000, 200
+    board, fills, turn = late_root(empty, seed)
+    orc = OracleMCTSNC((6, 7), 7, 7, n_trees=1, n_playouts=64, variant="ocp_prodigal", seed=3, node_capacity=20000)
+    orc.run(board, fills, turn, 2000)
+    early = orc.plies
+    orc = OracleMCTSNC((6, 7), 7, 7, n_trees=1, n_playouts=64, variant="ocp_prodigal", seed=3, node_capacity=20000)
+    orc.run(board, fills, turn, 1_500_000)
+    assert orc.plies == early
+    orc = OracleMCTSNC((6, 7), 7, 7, n_trees=1, n_playouts=64, variant="ocp_prodigal", seed=3, node_capacity=20000)
+    orc.run(board, fills, turn, steps)
+    assert orc.plies > early
+    ai = MCTSNC((6, 7), 7, 7, search_time_limit=np.inf, search_steps_limit=steps, n_trees=1, n_playouts=64, variant="ocp_prodigal", seed=3,
+                verbose_info=False, max_batch=roots, device_memory=2e6 / 2 ** 30)      # far more nodes than the tree comes to
+    ai.init_device_side_arrays()
+    out = ai.run_batch(np.stack([board] * roots), np.stack([fills] * roots), np.full(roots, turn), steps=steps)
+    assert ai.launch_geometry()["blocks_per_sm"] == 2      # trees of a block
+    assert (out["status"] == 0).all()
+    assert (out["playouts"] == orc.playouts).all() and (out["plies"] == orc.plies).all()
+    for b in (0, roots - 1):
+        compare_trees(ai, orc, search=b)
