@@ -58,9 +58,9 @@ constexpr int WARPS_PER_BLOCK = 8;
 // LANES lanes per player, action = lane within them; 2 * LANES lanes per traversal, the traversals of a warp side by side
 template <int LANES>
 __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32)
-select_kernel(float cpuct, int virtual_loss, int *child_all, const float *__restrict__ node_prior, const float *__restrict__ node_w,
-              const int *__restrict__ node_n, int *node_inflight_all, const int *__restrict__ node_terminal,
-              const int *__restrict__ tree_nodes, int *out_selected, int *out_path, int *out_len, int trees, int nodes, int A, int warps,
+select_kernel(float cpuct, int virtual_loss, int *child_all, const float *node_prior, const float *node_w,
+              const int *node_n, int *node_inflight_all, const int *node_terminal,
+              const int *tree_nodes, int *out_selected, int *out_path, int *out_len, int trees, int nodes, int A, int warps,
               int path_depth) {
     constexpr int GROUP = 2 * LANES, PER_WARP = 32 / GROUP;
     constexpr int SLOTS = (LANES * LANES + GROUP - 1) / GROUP;   // child ids a lane may hold
@@ -239,18 +239,18 @@ __device__ __forceinline__ void load_row(T (&v)[APL], const T *p, int actions, b
     unsigned raw[APL];
     const unsigned *q = reinterpret_cast<const unsigned *>(p);
     if (VECTORS && APL == 2) {
-        const uint2 x = fresh ? __ldcv(reinterpret_cast<const uint2 *>(q)) : __ldg(reinterpret_cast<const uint2 *>(q));
+        const uint2 x = fresh ? __ldcv(reinterpret_cast<const uint2 *>(q)) : *reinterpret_cast<const uint2 *>(q);
         raw[0] = x.x;
         raw[APL > 1 ? 1 : 0] = x.y;
     } else if (VECTORS && APL == 4) {
-        const uint4 x = fresh ? __ldcv(reinterpret_cast<const uint4 *>(q)) : __ldg(reinterpret_cast<const uint4 *>(q));
+        const uint4 x = fresh ? __ldcv(reinterpret_cast<const uint4 *>(q)) : *reinterpret_cast<const uint4 *>(q);
         raw[0] = x.x;
         raw[APL > 1 ? 1 : 0] = x.y;
         raw[APL > 2 ? 2 : 0] = x.z;
         raw[APL > 3 ? 3 : 0] = x.w;
     } else {
 #pragma unroll
-        for (int k = 0; k < APL; k++) raw[k] = k < actions ? (fresh ? __ldcv(q + k) : __ldg(q + k)) : 0u;
+        for (int k = 0; k < APL; k++) raw[k] = k < actions ? (fresh ? __ldcv(q + k) : q[k]) : 0u;
     }
 #pragma unroll
     for (int k = 0; k < APL; k++) v[k] = *reinterpret_cast<T *>(&raw[k]);
@@ -283,9 +283,9 @@ __device__ __forceinline__ void scores(float (&value)[2][APL], float cpuct, cons
 
 template <int APL, bool VECTORS>
 __global__ void __launch_bounds__(GROUP_WARPS * 32, 7)
-group_select_kernel(float cpuct, int virtual_loss, int *child_all, const float *__restrict__ node_prior, const float *__restrict__ node_w,
-                    const int *__restrict__ node_n, int *node_inflight_all, const int *__restrict__ node_terminal,
-                    const int *__restrict__ tree_nodes, int *out_selected, int *out_path, int *out_len, int trees, int nodes, int A, int warps,
+group_select_kernel(float cpuct, int virtual_loss, int *child_all, const float *node_prior, const float *node_w,
+                    const int *node_n, int *node_inflight_all, const int *node_terminal,
+                    const int *tree_nodes, int *out_selected, int *out_path, int *out_len, int trees, int nodes, int A, int warps,
                     int path_depth) {
     let_the_next_kernel_come();
     const unsigned block = block_after_the_kernel_before();

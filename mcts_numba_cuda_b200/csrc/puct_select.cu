@@ -152,10 +152,10 @@ __device__ __forceinline__ int parent_count(const EdgeRegs<EPL> &r, int n_exp, i
 // RESUMED: root_kernel has been here; see there.
 template <int EPL, bool WIDENING, bool RESUMED>
 __global__ void __launch_bounds__(32, EPL <= 2 ? 32 : (EPL == 4 ? 24 : 16))
-select_kernel(float cpuct, float c_pw, float alpha_pw, int soft_winner, const int *__restrict__ edge_child_id,
-              const float *__restrict__ edge_prior, const float *__restrict__ edge_W, const int *__restrict__ edge_N,
-              int *edge_inflight, int *node_expand_inflight, const int *__restrict__ node_expanded,
-              const int *__restrict__ tree_nodes, int *out_selected_node, int *out_path_eids, int *out_path_len, int nodes,
+select_kernel(float cpuct, float c_pw, float alpha_pw, int soft_winner, const int *edge_child_id,
+              const float *edge_prior, const float *edge_W, const int *edge_N,
+              int *edge_inflight, int *node_expand_inflight, const int *node_expanded,
+              const int *tree_nodes, int *out_selected_node, int *out_path_eids, int *out_path_len, int nodes,
               int edges, int warps, int path_depth, int vl, int trees) {
     let_the_next_kernel_come();
     const unsigned block = block_after_the_kernel_before();
@@ -394,9 +394,9 @@ select_kernel(float cpuct, float c_pw, float alpha_pw, int soft_winner, const in
 constexpr int ROOT_WARPS = 4;
 template <int EPL>
 __global__ void __launch_bounds__(ROOT_WARPS * 32)
-root_kernel(float cpuct, int soft_winner, const int *__restrict__ edge_child_id, const float *__restrict__ edge_prior,
-            const float *__restrict__ edge_W, const int *__restrict__ edge_N, int *edge_inflight, const int *__restrict__ node_expanded,
-            const int *__restrict__ tree_nodes, int *out_selected_node, int *out_path_eids, int *out_path_len, int trees, int nodes, int edges,
+root_kernel(float cpuct, int soft_winner, const int *edge_child_id, const float *edge_prior,
+            const float *edge_W, const int *edge_N, int *edge_inflight, const int *node_expanded,
+            const int *tree_nodes, int *out_selected_node, int *out_path_eids, int *out_path_len, int trees, int nodes, int edges,
             int warps, int path_depth, int vl) {
     let_the_next_kernel_come();
     const unsigned block = block_after_the_kernel_before();
@@ -495,9 +495,9 @@ static bool roots_first(int trees, int edges, int warps) {
 // W += value; an EXPAND result also returns its ticket.  With values == NULL only the claims are released
 // (src/puct/test_puct_gpu_v3.py:274-332).
 __global__ void backup_kernel(int virtual_loss, float *edge_W, int *edge_N, int *edge_inflight, int *node_expand_inflight,
-                              const int *__restrict__ tree_nodes, const int *__restrict__ out_selected_node,
-                              const int *__restrict__ out_path_eids, const int *__restrict__ out_path_len,
-                              const float *__restrict__ path_edge_values, int traversals, int nodes, int edges, int warps,
+                              const int *tree_nodes, const int *out_selected_node,
+                              const int *out_path_eids, const int *out_path_len,
+                              const float *path_edge_values, int traversals, int nodes, int edges, int warps,
                               int path_depth, int log2_lanes) {
     const BackupLane at_work(block_after_the_kernel_before(), traversals, log2_lanes);
     const int out_ix = at_work.traversal;

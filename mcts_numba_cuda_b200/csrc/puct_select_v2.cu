@@ -183,9 +183,9 @@ __device__ __forceinline__ int expansion_ticket(int *tickets, int n_exp, int all
 // tree learns from its own visits what it would read before them).
 template <bool PRECLAIM, int EPL, bool WIDENING>
 __global__ void __launch_bounds__(32, EPL <= 2 ? 32 : (EPL == 4 ? 24 : 16))
-select_kernel(float cpuct, float c_pw, float alpha_pw, const int *__restrict__ edge_child_id, const float *__restrict__ edge_prior,
-              const float *__restrict__ edge_W, const int *__restrict__ edge_N, int *node_inflight_all, int *node_expand_inflight,
-              const int *__restrict__ node_expanded, const int *__restrict__ tree_nodes, int *out_selected_node, int *out_path_eids,
+select_kernel(float cpuct, float c_pw, float alpha_pw, const int *edge_child_id, const float *edge_prior,
+              const float *edge_W, const int *edge_N, int *node_inflight_all, int *node_expand_inflight,
+              const int *node_expanded, const int *tree_nodes, int *out_selected_node, int *out_path_eids,
               int *out_path_len, int nodes, int edges, int warps, int path_depth) {
     let_the_next_kernel_come();
     const unsigned block = block_after_the_kernel_before();
@@ -394,10 +394,10 @@ select_kernel(float cpuct, float c_pw, float alpha_pw, const int *__restrict__ e
 
 // _backup_kernel_native (:847-927): per path edge the child's visit is given back, the edge gets N += 1 and W += value;
 // an EXPAND result returns its ticket.  With values == NULL only the visits and the ticket are released.
-__global__ void backup_kernel(int virtual_loss, const int *__restrict__ edge_child_id, float *edge_W, int *edge_N,
-                              int *node_inflight, int *node_expand_inflight, const int *__restrict__ tree_nodes,
-                              const int *__restrict__ out_selected_node, const int *__restrict__ out_path_eids,
-                              const int *__restrict__ out_path_len, const float *__restrict__ path_edge_values, int traversals, int nodes,
+__global__ void backup_kernel(int virtual_loss, const int *edge_child_id, float *edge_W, int *edge_N,
+                              int *node_inflight, int *node_expand_inflight, const int *tree_nodes,
+                              const int *out_selected_node, const int *out_path_eids,
+                              const int *out_path_len, const float *path_edge_values, int traversals, int nodes,
                               int edges, int warps, int path_depth, int log2_lanes) {
     const BackupLane at_work(block_after_the_kernel_before(), traversals, log2_lanes);
     const int traversal = at_work.traversal;

@@ -213,3 +213,18 @@ def test_the_extension_is_named_for_its_interpreter():
     """Another interpreter on the same checkout finds it stale and builds its own."""
     assert build.WAVE_PATH == os.path.join(build.HERE, "_wave" + sysconfig.get_config_var("EXT_SUFFIX"))
     assert os.path.samefile(importlib.import_module("mcts_numba_cuda_b200._wave").__file__, build.WAVE_PATH)
+
+
+def test_kernels_launched_behind_others_have_no_read_only_pointers():
+    """Their blocks may be on the device while the kernel before still writes what they will read after their wait; the read-only
+    data path is only for what nobody writes while the kernel lives."""
+    csrc = os.path.join(ROOT, "mcts_numba_cuda_b200", "csrc")
+    behind = 0
+    for name in sorted(os.listdir(csrc)):
+        with open(os.path.join(csrc, name)) as f:
+            text = re.sub(r"//[^\n]*", "", f.read())
+        if "griddepcontrol.wait" not in text and "block_after_the_kernel_before" not in text:
+            continue
+        behind += 1
+        assert not re.search(r"__restrict__|__ldg\s*\(|ld\.global\.nc", text), name
+    assert behind >= 5
