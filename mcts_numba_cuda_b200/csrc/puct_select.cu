@@ -418,7 +418,10 @@ root_kernel(float cpuct, int soft_winner, const int *edge_child_id, const float 
     if (usual) sqrt_parent = root_of_count(parent_count(r, n_exp, lane));
     bool open = mine;          // the traversal has no claim and no result yet
     for (int evaluation = 1; usual && evaluation <= MAX_EVALUATIONS; evaluation++) {
-        if (evaluation > 1) r.request(0, lane, edges);
+        if (evaluation > 1) {
+            __syncwarp();   // the claims just made, each by a lane of its own, are seen
+            r.request(0, lane, edges);
+        }
         float score[EPL];
         const float top = score_edges(r, score, cpuct, sqrt_parent, n_exp, lane);
         if (top == LOWEST_INF) {

@@ -232,6 +232,27 @@ def test_roots_of_many_traversals(edges, warps, copies, soft):
     assert int(puct.to_host(d)["edge_inflight"].sum()) == 0
 
 
+@pytest.mark.parametrize("edges,warps,copies", [(8, 8, 90), (64, 8, 90), (100, 8, 70), (200, 8, 45)])
+def test_the_second_choice_at_a_root_sees_the_first_claim(edges, warps, copies):
+    """Roots done first: the loser that is next in line chooses again with the winner's claim in the counts, each a lane of one warp."""
+    T, vl, cpuct = 11, 3, 1.5
+    case = po.layered_case(trees=T, edges=edges, depth=3, warps=warps, seed=edges, nodes_per_level=6)
+    many = {k: np.tile(v, (copies,) + (1,) * (v.ndim - 1)) if isinstance(v, np.ndarray) else v for k, v in case.items()}
+    many["trees"] = T * copies
+    h = run_ours(many, cpuct=cpuct, c_pw=0.0, virtual_loss=vl)[1]
+    for base in range(T):
+        n_exp = int(case["node_expanded"][base, 0])
+        sqrt_parent = np.sqrt(np.float32(case["edge_n"][base, 0, :n_exp].sum()), dtype=np.float32)
+        inflight = np.zeros(n_exp, int)
+        for wid in (0, 1):
+            scores = [po._score(cpuct, case["edge_prior"][base, 0, e], case["edge_w"][base, 0, e], int(case["edge_n"][base, 0, e]),
+                                int(inflight[e]), sqrt_parent) for e in range(n_exp)]
+            best = int(np.argmax(scores))
+            assert sorted(scores)[-1] > sorted(scores)[-2]
+            assert (h["out_path"][base::T, wid, 0] == best).all()
+            inflight[best] += vl
+
+
 @pytest.mark.skipif(not os.path.exists(REF_LIB), reason="reference kernel not built (reference not mounted at build time)")
 def test_first_edge_distribution_matches_reference_kernel():
     """Many warps: results depend on the schedule, so compare what both kernels choose at the root in aggregate."""
