@@ -65,6 +65,9 @@ struct DevResult {
     float stage_ms[4];   // mean over the search's trees of TreeState::stage_ms
 };
 
+// the forms a cluster per tree comes in, in the order they are tried (WIDE and AHEAD: draws made ahead, a block on an SM)
+enum ClusterForm { WIDE, AHEAD, PLAIN, PACKED, CLUSTER_FORMS };
+
 }  // namespace
 
 struct mctsnc_handle {
@@ -74,7 +77,7 @@ struct mctsnc_handle {
     int tpb_roa = 0;
     int sm_count = 0;
     bool cluster_ok = false;      // thread-block clusters can be launched (and MCTSNC_B200_NO_CLUSTER is not set)
-    int cluster_fit[4][2] = {};   // clusters that fit on the device at once, [ClusterForm][small record cache] (0: not asked yet, -1: unknown)
+    int cluster_fit[CLUSTER_FORMS][2] = {};   // clusters that fit on the device at once, [ClusterForm][small record cache] (0: not asked yet, -1: unknown)
     int threads = 0;
     int blocks_per_sm = 0;
     long long bytes = 0;
@@ -828,9 +831,6 @@ int launch_search_gomoku(mctsnc_handle *h, int batch, int steps, int first, cuda
     }
     return (int)cudaGetLastError();
 }
-
-// the forms a cluster per tree comes in, in the order they are tried (WIDE and AHEAD: draws made ahead, a block on an SM)
-enum ClusterForm { WIDE, AHEAD, PLAIN, PACKED, CLUSTER_FORMS };
 
 const void *cluster_kernel_ptr(bool ocp, int form) {
     if (form == WIDE) return (const void *)c4::search_cluster_kernel<false, c4::WIDE_CLUSTER_BLOCKS, c4::WIDE_CLUSTER_THREADS, true>;   // acp only

@@ -435,12 +435,8 @@ root_kernel(float cpuct, int soft_winner, const int *edge_child_id, const float 
         }
         // every lane its own traversal's edge: the first of those with the top score from edge wid modulo n_exp on
         unsigned even[EPL];
-        int ties = 0;
 #pragma unroll
-        for (int k = 0; k < EPL; k++) {
-            even[k] = __ballot_sync(FULL, __float_as_uint(score[k]) == __float_as_uint(top));
-            ties += __popc(even[k]);
-        }
+        for (int k = 0; k < EPL; k++) even[k] = __ballot_sync(FULL, __float_as_uint(score[k]) == __float_as_uint(top));
         const int rot = lane % n_exp;
         int best = NO_EDGE, first = NO_EDGE;
 #pragma unroll
