@@ -474,7 +474,7 @@ group_select_kernel(float cpuct, int virtual_loss, int *child_all, const float *
 //   12: 1000 x 4 27 / 30
 static bool traversals_in_step(int trees, int actions, int warps) {
     const int per_warp = actions <= 4 ? 4 : (actions <= 8 ? 2 : 1);
-    return warps >= 2 && warps <= GROUPS && ((long long)trees + per_warp - 1) / per_warp * warps > 32 * 148;
+    return warps >= 2 && warps <= GROUPS && ((long long)trees + per_warp - 1) / per_warp * warps > 32 * sm_count();
 }
 
 // whether every row of A words starts where a load of A / 4 words may

@@ -486,7 +486,7 @@ root_kernel(float cpuct, int soft_winner, const int *edge_child_id, const float 
 //   64 / 68   2500 x 64 x 12 x 4 44 / 45   700 x 64 x 12 x 8 29 / 29   500 x 100 x 8 x 8 27 / 27
 static bool roots_first(int trees, int edges, int warps) {
     const int warps_of_sm = edges <= 64 ? 32 : (edges <= 128 ? 24 : 16);
-    return warps > 2 && edges >= 2 && edges <= EDGE_LIMIT && 4LL * trees * (warps - 2) > 5LL * warps_of_sm * 148;
+    return warps > 2 && edges >= 2 && edges <= EDGE_LIMIT && 4LL * trees * (warps - 2) > 5LL * warps_of_sm * sm_count();
 }
 
 // Turns the claims of finished traversals into statistics (v3 edge layout; the reference has this step only for its
