@@ -408,6 +408,7 @@ def run_puct(args):
     # (the others lost their claims and read a node or two)
     bytes_per_level = 16 * E + 16
     achieved = levels * bytes_per_level / (ms * 1e-3) / 1e9
+    kernel = _abi.lib().puct_select_kernel_name(0.0, T, E, Wp).decode()
     prof = profiler_readings("puct", f"{E},{D},{Wp}")
     line = {"metric": "PUCT selections/sec (select kernel only, CUDA events)", "value": sel / (ms * 1e-3), "unit": "selections/s",
             "n_gpus": 1, "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True,
@@ -421,8 +422,8 @@ def run_puct(args):
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": pk["hbm_gbs"], "unit": "GB/s",
                          "frac": achieved / pk["hbm_gbs"], "traffic": None if prof is None else T * prof["dram_bytes_per_tree"],
                          "traffic_unit": "bytes per launch, scaled by trees from an ncu capture of a smaller case", "peak_source": pk["source"],
-                         "kernel": "puct::select_kernel", "bytes_per_level": bytes_per_level, "levels": levels},
-            "gpu_launches": 2 * (args.steps + args.warmup) * 2, "clocks": clocks}
+                         "kernel": kernel, "bytes_per_level": bytes_per_level, "levels": levels},
+            "gpu_launches": 2 * (args.steps + args.warmup) * (1 + len(kernel.split("+"))), "clocks": clocks}
     return line
 
 
@@ -517,7 +518,7 @@ def run_duct(args):
                          "frac": achieved / pk["hbm_gbs"],
                          "traffic": None if prof is None else T * prof["dram_bytes_per_tree"],
                          "traffic_unit": "bytes per launch, scaled by trees from an ncu capture of a smaller case",
-                         "peak_source": pk["source"], "kernel": "duct::select_kernel", "bytes_per_selection": bytes_per_sel},
+                         "peak_source": pk["source"], "kernel": _abi.lib().duct_select_kernel_name(T, A, Wp).decode(), "bytes_per_selection": bytes_per_sel},
             "cpu_baseline": cpu, "gpu_launches": 2 * (args.steps + args.warmup), "clocks": clocks}
     return line
 
@@ -741,11 +742,6 @@ def main():
     inst_achieved = plies_per_launch * G["inst_per_ply"] / (kernel_ms * 1e-3)
     workload_key = f"{args.variant},{args.trees},{args.playouts},{args.search_steps},{B}"
     prof = profiler_readings(args.game, workload_key)
-    pooled = B * args.trees > sm_count and args.playouts * (A if "acp" in args.variant else 1) > 32 and args.search_steps > 32
-    if args.game == "c4":
-        kernel_name = "c4::pool_kernel" if pooled else "c4::search_kernel"
-    else:
-        kernel_name = "gomoku::search_block_kernel" if geo["threads_per_tree"] != 224 else "gomoku::playout_dynamic_kernel (+ tree_step_kernel)"
     line = {
         "metric": "playouts/sec", "value": value, "unit": "playouts/s", "n_gpus": n_gpus, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": dev_ms / args.steps, "higher_is_better": True, "scaling": "weak",
@@ -756,7 +752,7 @@ def main():
         "roofline": {"bound": "issue", "achieved": inst_achieved / 1e12, "peak": peak_inst / 1e12, "unit": "T thread-inst/s",
                      "frac": inst_achieved / peak_inst, "peak_source": f"{sm_count} SMs x 4 schedulers x 32 lanes x {pk['sm_max_mhz']:.0f} MHz ({pk['source']} clock)",
                      "traffic": None if prof is None else prof.get("dram_bytes_per_launch"),
-                     "traffic_unit": "DRAM bytes per launch (ncu)", "kernel": kernel_name, "kernel_ms": kernel_ms,
+                     "traffic_unit": "DRAM bytes per launch (ncu)", "kernel": geo["kernel"], "kernel_ms": kernel_ms,
                      "work_unit": "playout ply", "inst_per_ply_yardstick": G["inst_per_ply"],
                      "plies_per_playout": plies_per_launch / max(playouts_per_launch, 1), "plies_per_launch": plies_per_launch,
                      "profiler": None if prof is None else {k: prof.get(k) for k in ("case", "alu_pipe_pct", "issue_active_pct",

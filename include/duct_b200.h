@@ -43,6 +43,9 @@ int duct_select_launch(float cpuct, int virtual_loss, int *child, const float *n
                        int *out_selected, int *out_path, int *out_len, int trees, int nodes, int actions, int warps,
                        int path_depth, void *stream);
 
+/* Name of the kernel that duct_select_launch runs for these sizes; the library keeps the text. */
+const char *duct_select_kernel_name(int trees, int actions, int warps);
+
 int duct_backup_launch(int virtual_loss, int *child, float *node_w, int *node_n, int *node_inflight, const int *out_selected,
                        const int *out_path, const int *out_len, const float *values, const int *new_child, int trees, int nodes,
                        int actions, int warps, int path_depth, void *stream);

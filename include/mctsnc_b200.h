@@ -184,6 +184,9 @@ int mctsnc_export_rng(mctsnc_handle *h, int32_t search, int32_t which, uint64_t 
 int mctsnc_query(mctsnc_handle *h, int32_t *threads_per_tree, int32_t *blocks_per_sm, int32_t *sm_count,
                  int64_t *bytes_allocated);
 
+/* Name of the kernel that grew the trees of the last search launch, "" before the first; the library keeps the text. */
+const char *mctsnc_search_kernel(mctsnc_handle *h);
+
 /* Diagnostic, no counterpart in the reference: record every slice of the following batched Connect-4 launches that run
    through the work queue (more trees than blocks fit on the device): 4 int64 per slice -- tree, start and end of the
    slice in nanoseconds of the device's global timer, (SM id << 32) | steps run.  max_records = 0 switches it off.

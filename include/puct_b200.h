@@ -24,6 +24,9 @@ int puct_select_winner_recalc_launch(float cpuct, float c_pw, float alpha_pw, in
                                      int *out_selected_node, int *out_path_eids, int *out_path_len, int trees, int nodes,
                                      int edges, int warps, int path_depth, void *stream);
 
+/* Name of the kernel, or of the two, that the select launches above run for these sizes; the library keeps the text. */
+const char *puct_select_kernel_name(float c_pw, int trees, int edges, int warps);
+
 /* Replaces puct_cpp_cuda_error_string, src/puct/puct_gpu_v3_cpp.cu:483-485. */
 const char *puct_cpp_cuda_error_string(int code);
 

@@ -23,15 +23,15 @@ E_BAD_ARGUMENT, E_UNSUPPORTED, E_NO_MEMORY, E_BAD_ROOT, E_CAPACITY, E_NO_DEVICE 
 EXPORTED = ["mctsnc_create", "mctsnc_destroy", "mctsnc_reset_rng", "mctsnc_run", "mctsnc_run_batch",
             "mctsnc_search_batch_device", "mctsnc_finish_batch_device", "mctsnc_launch_batch_device",
             "mctsnc_reduce_trees_device", "mctsnc_export", "mctsnc_export_rng",
-            "mctsnc_query", "mctsnc_search_c4_static", "mctsnc_trace_slices", "mctsnc_read_slices",
+            "mctsnc_query", "mctsnc_search_kernel", "mctsnc_search_c4_static", "mctsnc_trace_slices", "mctsnc_read_slices",
             "mctsnc_exchange_create", "mctsnc_exchange_connect", "mctsnc_exchange_allreduce", "mctsnc_exchange_status",
             "mctsnc_exchange_destroy", "mctsnc_error_string"]
 EXCHANGE_HANDLE_BYTES, EXCHANGE_TIMEOUT = 64, 1
 # the PUCT entry points keep the names of the reference's native library (include/puct_b200.h)
 EXPORTED_PUCT = ["puct_select_winner_recalc_launch", "puct_select_virtual_loss_launch", "puct_backup_launch",
-                 "puct_cpp_cuda_error_string", "puct_v2_select_launch", "puct_v2_backup_launch"]
+                 "puct_cpp_cuda_error_string", "puct_select_kernel_name", "puct_v2_select_launch", "puct_v2_backup_launch"]
 # decoupled-UCT select for simultaneous moves: no counterpart in the reference (include/duct_b200.h)
-EXPORTED_DUCT = ["duct_select_launch", "duct_backup_launch"]
+EXPORTED_DUCT = ["duct_select_launch", "duct_select_kernel_name", "duct_backup_launch"]
 
 
 class Config(ctypes.Structure):
@@ -108,6 +108,11 @@ def lib():
         L.mctsnc_error_string.restype = ctypes.c_char_p
         for name in EXPORTED[:-1]:
             getattr(L, name).restype = ctypes.c_int
+        L.mctsnc_search_kernel.argtypes = [vp]
+        L.puct_select_kernel_name.argtypes = [ctypes.c_float, ctypes.c_int, ctypes.c_int, ctypes.c_int]
+        L.duct_select_kernel_name.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_int]
+        for name in ("mctsnc_search_kernel", "puct_select_kernel_name", "duct_select_kernel_name"):
+            getattr(L, name).restype = ctypes.c_char_p
         assert ctypes.sizeof(Result) == RESULT_DTYPE.itemsize
         _lib = L
     return _lib

@@ -561,6 +561,10 @@ extern "C" int duct_select_launch(float cpuct, int virtual_loss, int *child, con
     return (int)cudaGetLastError();
 }
 
+extern "C" const char *duct_select_kernel_name(int trees, int actions, int warps) {
+    return duct::traversals_in_step(trees, actions, warps) ? "duct::group_select_kernel" : "duct::select_kernel";
+}
+
 extern "C" int duct_backup_launch(int virtual_loss, int *child, float *node_w, int *node_n, int *node_inflight,
                                   const int *out_selected, const int *out_path, const int *out_len, const float *values,
                                   const int *new_child, int trees, int nodes, int actions, int warps, int path_depth, void *stream) {

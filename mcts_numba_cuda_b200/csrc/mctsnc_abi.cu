@@ -80,6 +80,7 @@ struct mctsnc_handle {
     int cluster_fit[CLUSTER_FORMS][2] = {};   // clusters that fit on the device at once, [ClusterForm][small record cache] (0: not asked yet, -1: unknown)
     int threads = 0;
     int blocks_per_sm = 0;
+    const char *kernel = "";     // of the last search launch
     long long bytes = 0;
     long long n_trees_total = 0;  // max_batch * n_trees
     long long rng_per_search = 0; // playout streams per search of this handle
@@ -758,6 +759,7 @@ int launch_search_gomoku(mctsnc_handle *h, int batch, int steps, int first, cuda
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kernel, threads, smem) == cudaSuccess &&
             trees <= (long long)fit * h->sm_count) {
             h->threads = threads;
+            h->kernel = "gomoku::search_block_kernel";
             h->blocks_per_sm = fit;
             return (int)cudaLaunchKernel(kernel, dim3((unsigned)trees), dim3((unsigned)threads), args, smem, stream);
         }
@@ -776,6 +778,7 @@ int launch_search_gomoku(mctsnc_handle *h, int batch, int steps, int first, cuda
         per_sm = 1;
     const long long resident = (long long)per_sm * h->sm_count;
     h->threads = gomoku::DYN_THREADS;
+    h->kernel = "gomoku::playout_dynamic_kernel";
     h->blocks_per_sm = per_sm;
     CUDA_TRY(cudaEventRecord(h->g_fork, stream));
     for (int g = 0; g < groups; g++) CUDA_TRY(cudaStreamWaitEvent(h->g_stream[g], h->g_fork, 0));
@@ -839,6 +842,12 @@ const void *cluster_kernel_ptr(bool ocp, int form) {
                                   : (const void *)c4::search_cluster_kernel<false, c4::CLUSTER_BLOCKS, c4::CLUSTER_THREADS, true>;
     return ocp ? (const void *)c4::search_cluster_kernel<true, c4::CLUSTER_BLOCKS, c4::CLUSTER_THREADS, false>
                : (const void *)c4::search_cluster_kernel<false, c4::CLUSTER_BLOCKS, c4::CLUSTER_THREADS, false>;
+}
+
+const char *cluster_kernel_name(int form) {
+    if (form == WIDE) return "c4::search_cluster_kernel, 16 blocks, draws ahead";
+    if (form == AHEAD) return "c4::search_cluster_kernel, 8 blocks, draws ahead";
+    return form == PACKED ? "c4::search_packed_cluster_kernel" : "c4::search_cluster_kernel, 8 blocks";
 }
 
 int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_t stream) {
@@ -940,6 +949,7 @@ int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_
             h->threads = wide ? (c4::WIDE_CLUSTER_THREADS - 32) * blocks : c4::CLUSTER_THREADS * blocks;
             h->blocks_per_sm = 1;
             void *args[] = {&p};
+            h->kernel = cluster_kernel_name(form);
             if (cudaLaunchKernelExC(&lc, kernel, args) == cudaSuccess) return 0;
             cudaGetLastError();      // the launch was refused (nothing ran): one block per tree from now on
             h->cluster_ok = false;
@@ -957,6 +967,7 @@ int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_
         p.places = pool.trees * (int)grid;
         if (trees > p.places) use_queue(h, p, trees, steps, stream);
         h->threads = pool.threads / pool.trees;
+        h->kernel = "c4::pool_kernel";
         h->blocks_per_sm = pool.trees;
         void *args[] = {&p};
         CUDA_TRY(cudaLaunchKernel(kernel, dim3(grid), dim3((unsigned)pool.threads), args,
@@ -966,6 +977,7 @@ int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_
     }
     int threads = h->cfg.threads_per_tree > 0 ? h->cfg.threads_per_tree : choose_threads(h, trees);
     h->threads = threads;
+    h->kernel = "c4::search_kernel";
     // A tree that has an SM to itself gets a warp more, for the walker: it works out the counts and logarithms of the backup
     // while the others play (one warp for 32 games and the walker: 5.9 us a step, two: 4.4).
     if (h->cfg.threads_per_tree == 0 && trees <= h->sm_count && threads + 32 <= 1024) threads += 32;
@@ -980,6 +992,7 @@ int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_
         kernel = is_ocp(h->cfg) ? (const void *)c4::search_kernel<true, true, true> : (const void *)c4::search_kernel<false, true, true>;
         CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AHEAD_SMEM_LIMIT));
         smem = with_draws;
+        h->kernel = "c4::search_kernel, draws ahead";
     }
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess || per_sm < 1)
         return MCTSNC_E_BAD_ARGUMENT;
@@ -1595,6 +1608,8 @@ extern "C" int mctsnc_query(mctsnc_handle *h, int32_t *threads_per_tree, int32_t
     if (bytes_allocated) *bytes_allocated = h->bytes;
     return 0;
 }
+
+extern "C" const char *mctsnc_search_kernel(mctsnc_handle *h) { return h ? h->kernel : ""; }
 
 extern "C" int mctsnc_trace_slices(mctsnc_handle *h, int32_t max_records) {
     if (!h || max_records < 0) return MCTSNC_E_BAD_ARGUMENT;

@@ -619,5 +619,9 @@ extern "C" int puct_backup_launch(int virtual_loss, float *edge_W, int *edge_N, 
     return (int)cudaGetLastError();
 }
 
+extern "C" const char *puct_select_kernel_name(float c_pw, int trees, int edges, int warps) {
+    return c_pw == 0.0f && puct::roots_first(trees, edges, warps) ? "puct::root_kernel + puct::select_kernel" : "puct::select_kernel";
+}
+
 // Same meaning as puct_cpp_cuda_error_string of src/puct/puct_gpu_v3_cpp.cu:483-485.
 extern "C" const char *puct_cpp_cuda_error_string(int code) { return cudaGetErrorString(static_cast<cudaError_t>(code)); }

@@ -423,7 +423,7 @@ class MCTSNC:
 
     def launch_geometry(self):
         """Geometry of the last search launch: threads per tree, resident blocks per SM (where a block grows several trees: the trees of
-        an SM), SMs of the device and the bytes of device memory the handle holds.  A Connect-4 batch with more trees than ``blocks_per_sm * sm_count`` and more
+        an SM), SMs of the device, the bytes of device memory the handle holds and the name of the kernel that grew the trees.  A Connect-4 batch with more trees than ``blocks_per_sm * sm_count`` and more
         than ``SLICE_STEPS`` steps runs as a persistent grid fed by the work queue."""
         if self._handle is None:
             raise RuntimeError("[MCTSNC: init_device_side_arrays() has to be called first]")
@@ -432,7 +432,7 @@ class MCTSNC:
         _abi.check(_abi.lib().mctsnc_query(self._handle, ctypes.byref(thr), ctypes.byref(per_sm), ctypes.byref(sms),
                                            ctypes.byref(nbytes)))
         return {"threads_per_tree": thr.value, "blocks_per_sm": per_sm.value, "sm_count": sms.value,
-                "device_bytes": nbytes.value}
+                "device_bytes": nbytes.value, "kernel": _abi.lib().mctsnc_search_kernel(self._handle).decode()}
 
     def trace_slices(self, max_records):
         """Diagnostic: record every slice of the following batched launches that go through the work queue

@@ -228,3 +228,13 @@ def test_kernels_launched_behind_others_have_no_read_only_pointers():
         behind += 1
         assert not re.search(r"__restrict__|__ldg\s*\(|ld\.global\.nc", text), name
     assert behind >= 5
+
+
+def test_wave_kernels_are_named_by_the_rules_that_choose_them():
+    L = _abi.lib()
+    assert L.puct_select_kernel_name(0.0, 4096, 64, 8) == b"puct::root_kernel + puct::select_kernel"
+    for c_pw, trees, edges, warps in ((1.0, 4096, 64, 8), (0.0, 4096, 64, 2), (0.0, 100, 19, 8), (0.0, 4096, 300, 8)):
+        assert L.puct_select_kernel_name(c_pw, trees, edges, warps) == b"puct::select_kernel"
+    assert L.duct_select_kernel_name(4096, 8, 8) == b"duct::group_select_kernel"
+    for trees, actions, warps in ((4096, 8, 1), (4096, 8, 9), (100, 8, 8)):
+        assert L.duct_select_kernel_name(trees, actions, warps) == b"duct::select_kernel"
