@@ -65,8 +65,10 @@ struct DevResult {
     float stage_ms[4];   // mean over the search's trees of TreeState::stage_ms
 };
 
-// the forms a cluster per tree comes in, in the order they are tried (WIDE and AHEAD: draws made ahead, a block on an SM)
-enum ClusterForm { WIDE, AHEAD, PLAIN, PACKED, CLUSTER_FORMS };
+// the forms a cluster per tree comes in, in the order they are tried (WIDE_AHEAD and AHEAD: draws made ahead, a block on an SM)
+enum ClusterForm { WIDE_AHEAD, WIDE, AHEAD, PLAIN, PACKED, CLUSTER_FORMS };
+bool is_wide(int form) { return form == WIDE_AHEAD || form == WIDE; }
+bool is_ahead(int form) { return form == WIDE_AHEAD || form == AHEAD; }
 
 }  // namespace
 
@@ -836,7 +838,9 @@ int launch_search_gomoku(mctsnc_handle *h, int batch, int steps, int first, cuda
 }
 
 const void *cluster_kernel_ptr(bool ocp, int form) {
-    if (form == WIDE) return (const void *)c4::search_cluster_kernel<false, c4::WIDE_CLUSTER_BLOCKS, c4::WIDE_CLUSTER_THREADS, true>;   // acp only
+    // acp only
+    if (form == WIDE_AHEAD) return (const void *)c4::search_cluster_kernel<false, c4::WIDE_CLUSTER_BLOCKS, c4::WIDE_CLUSTER_THREADS, true>;
+    if (form == WIDE) return (const void *)c4::search_cluster_kernel<false, c4::WIDE_CLUSTER_BLOCKS, c4::WIDE_CLUSTER_THREADS, false>;
     if (form == PACKED) return ocp ? (const void *)c4::search_packed_cluster_kernel<true> : (const void *)c4::search_packed_cluster_kernel<false>;
     if (form == AHEAD) return ocp ? (const void *)c4::search_cluster_kernel<true, c4::CLUSTER_BLOCKS, c4::CLUSTER_THREADS, true>
                                   : (const void *)c4::search_cluster_kernel<false, c4::CLUSTER_BLOCKS, c4::CLUSTER_THREADS, true>;
@@ -844,8 +848,26 @@ const void *cluster_kernel_ptr(bool ocp, int form) {
                : (const void *)c4::search_cluster_kernel<false, c4::CLUSTER_BLOCKS, c4::CLUSTER_THREADS, false>;
 }
 
+// Draws made ahead (c4::Draws) cost a launch 64 draws of every stream at its begin and the way back at its end, 3 us where a
+// thread has one stream and 7 where it has two, and save a part of a step.  Launches of fewer steps than this play without: us with /
+// without, 8 and 16 steps, 1 x 32 ocp 47.7 / 46.9 and 80.9 / 82.0, 8 x 256 ocp 67.5 / 65.4 and 110.5 / 110.5, 4 x 32 acp 61.3 / 61.3 and 101.3 /
+// 104.5; clusters 4 x 64 acp 54.0 / 53.2 and 97.2 / 98.4, 4 x 512 ocp 56.0 / 55.2 and 100.2 / 102.3, 4 x 256 acp 57.4 / 56.1 and 101.2 / 101.4.
+constexpr int AHEAD_MIN_STEPS = 16;
+
+// And of clusters, by the streams of a block; us with / without, 32, 64, 200 and 1000 steps:
+//   8 blocks, 64 streams (512 ocp) 189 / 195, 365 / 378, 1110 / 1159, 5697 / 5847; 56 (64 acp) 184 / 187, 354 / 363, 1078 / 1116, 5418 / 5608;
+//   112 (128 acp), four warps that play beside the walker's: never, 193 / 188, 373 / 367, 1139 / 1129, 5739 / 5697; 224 (256 acp, 12
+//   trees) 214 / 222, 414 / 430, 1274 / 1329, 6372 / 6564; 448 (512 acp), two a thread: no gain, 633 / 633, 1961 / 1962, 9415 / 9419 from 64 steps;
+//   16 blocks, 112 streams (256 acp) 186 / 190, 358 / 372, 1094 / 1144, 5726 / 5824; 224 (512 acp) 275 / 270, 528 / 528, 1570 / 1618,
+//   7539 / 7934.
+bool cluster_draws_pay(int steps, int streams, bool wide) {
+    if (wide) return steps >= (streams > c4::WIDE_CLUSTER_THREADS ? 4 * AHEAD_MIN_STEPS : AHEAD_MIN_STEPS);
+    return steps >= AHEAD_MIN_STEPS && (streams <= 64 || (streams > 128 && streams <= c4::CLUSTER_THREADS));
+}
+
 const char *cluster_kernel_name(int form) {
-    if (form == WIDE) return "c4::search_cluster_kernel, 16 blocks, draws ahead";
+    if (form == WIDE_AHEAD) return "c4::search_cluster_kernel, 16 blocks, draws ahead";
+    if (form == WIDE) return "c4::search_cluster_kernel, 16 blocks";
     if (form == AHEAD) return "c4::search_cluster_kernel, 8 blocks, draws ahead";
     return form == PACKED ? "c4::search_packed_cluster_kernel" : "c4::search_cluster_kernel, 8 blocks";
 }
@@ -906,9 +928,14 @@ int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_
         const bool ocp = is_ocp(h->cfg);
         // the wide cluster first where a step has games for it (an ocp step never has: 512 at most); then the first form that fits
         // on the device
-        for (int form = !ocp && h->A * h->cfg.n_playouts >= c4::WIDE_CLUSTER_MIN_GAMES ? WIDE : AHEAD; form <= PACKED; form++) {
-            const bool wide = form == WIDE, ahead = form == WIDE || form == AHEAD;
+        for (int form = !ocp && h->A * h->cfg.n_playouts >= c4::WIDE_CLUSTER_MIN_GAMES ? WIDE_AHEAD : AHEAD; form <= PACKED; form++) {
+            const bool wide = is_wide(form), ahead = is_ahead(form);
             const int blocks = wide ? c4::WIDE_CLUSTER_BLOCKS : c4::CLUSTER_BLOCKS;
+            const int streams = (int)(h->dyn_smem / sizeof(ulonglong2)) / blocks;   // of a block
+            if (ahead && !cluster_draws_pay(steps, streams, wide)) continue;
+            // 16 blocks without draws made ahead come before 8 with them only where those do not pay either (8 trees of 512: 64, 200 and
+            // 1000 steps 590, 1879, 9093 us against 632, 1960, 9415; of 256, 9 trees, with 16 / with 8: 410 / 410, 1249 / 1271, 6368 / 6342)
+            if (form == WIDE && cluster_draws_pay(steps, (int)(h->dyn_smem / sizeof(ulonglong2)) / c4::CLUSTER_BLOCKS, false)) continue;
             const void *kernel = cluster_kernel_ptr(ocp, form);
             if (wide && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
                 cudaGetLastError();
@@ -932,10 +959,10 @@ int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_
             // and one with draws made ahead are for blocks that have an SM each, a packed one for blocks that share it.
             bool fits = false;
             const bool own_sm = trees * blocks <= h->sm_count;
-            for (int small = own_sm && form != PACKED ? 0 : 1; small < (ahead ? 1 : 2) && !fits; small++) {
+            for (int small = own_sm && form != PACKED ? 0 : 1; small < (wide || ahead ? 1 : 2) && !fits; small++) {
                 p.cache_nodes = small ? 2048 : MCTSNC_C4_CACHE_NODES;
                 lc.dynamicSmemBytes = h->dyn_smem / blocks + sizeof(int4) * (size_t)p.cache_nodes +
-                                      (ahead ? c4::Draws::bytes((int)(h->dyn_smem / sizeof(ulonglong2)) / blocks) : 0);
+                                      (ahead ? c4::Draws::bytes(streams) : 0);
                 int &fit = h->cluster_fit[form][small];
                 if (fit == 0) {
                     int n = 0;
@@ -988,7 +1015,8 @@ int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_
     // warps do not.
     const size_t with_draws = smem + c4::Draws::bytes((int)(smem / sizeof(ulonglong2)));
     const int playing_warps = h->threads / 32;
-    if (threads > h->threads && play_straight(h->cfg, h->threads) && (playing_warps == 1 || playing_warps > 4) && with_draws <= (size_t)AHEAD_SMEM_LIMIT) {
+    if (steps >= AHEAD_MIN_STEPS && threads > h->threads && play_straight(h->cfg, h->threads) && (playing_warps == 1 || playing_warps > 4) &&
+        with_draws <= (size_t)AHEAD_SMEM_LIMIT) {
         kernel = is_ocp(h->cfg) ? (const void *)c4::search_kernel<true, true, true> : (const void *)c4::search_kernel<false, true, true>;
         CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AHEAD_SMEM_LIMIT));
         smem = with_draws;

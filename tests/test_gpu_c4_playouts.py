@@ -65,3 +65,25 @@ def test_draws_made_ahead_match_oracle(variant, n_trees, n_playouts, empty, step
         compare_trees(ai, orc)
         assert int(best) == orc.best_action
         assert (ai._res["playouts"], ai._res["plies"]) == (orc.playouts, orc.plies)
+
+
+@pytest.mark.parametrize("variant,n_trees,n_playouts,steps,kernel", [
+    ("ocp_thrifty", 1, 32, 15, "search_kernel"), ("ocp_thrifty", 1, 32, 16, "search_kernel, draws ahead"),
+    ("acp_prodigal", 4, 64, 15, "search_cluster_kernel, 8 blocks"), ("acp_prodigal", 4, 64, 16, "search_cluster_kernel, 8 blocks, draws ahead"),
+    ("acp_thrifty", 2, 128, 40, "search_cluster_kernel, 8 blocks"), ("acp_prodigal", 12, 256, 16, "search_cluster_kernel, 8 blocks, draws ahead"),
+    ("acp_prodigal", 2, 256, 15, "search_cluster_kernel, 16 blocks"), ("acp_thrifty", 2, 256, 16, "search_cluster_kernel, 16 blocks, draws ahead"),
+    ("acp_prodigal", 1, 512, 63, "search_cluster_kernel, 16 blocks"), ("acp_prodigal", 1, 512, 64, "search_cluster_kernel, 16 blocks, draws ahead")])
+def test_draws_are_made_ahead_only_where_they_pay(variant, n_trees, n_playouts, steps, kernel):
+    """A launch of a few steps does not get back what the draws cost at its begin and end.  A long search, a short one and a long one on the
+    streams that the one before has left."""
+    board, fills, turn = late_root(30, seed=4)
+    ai = MCTSNC((6, 7), 7, 7, search_time_limit=np.inf, search_steps_limit=steps, n_trees=n_trees, n_playouts=n_playouts, variant=variant,
+                seed=6, verbose_info=False)
+    ai.init_device_side_arrays()
+    orc = OracleMCTSNC((6, 7), 7, 7, n_trees=n_trees, n_playouts=n_playouts, variant=variant, seed=6, node_capacity=steps * 7 + 8)
+    for count in (steps, 5, steps):
+        best = ai.run(board, fills, turn, forced_search_steps_limit=count)
+        assert ai.launch_geometry()["kernel"] == "c4::" + (kernel if count == steps else kernel.replace(", draws ahead", ""))
+        orc.run(board, fills, turn, count)
+        compare_trees(ai, orc)
+        assert int(best) == orc.best_action and ai._res["plies"] == orc.plies
