@@ -603,8 +603,15 @@ bool choose_pool(const mctsnc_handle *h, long long trees, int steps, PoolShape *
     const bool large = games >= 896;
     if (h->cfg.threads_per_tree > 0 || steps <= SLICE_STEPS || games <= 32 || trees <= (large ? h->sm_count + h->sm_count / 6 : h->sm_count)) return false;
     const long long need = (trees + h->sm_count - 1) / h->sm_count;
-    // 5 trees of 1792 games (256 roots of 4 x 256, 2000 steps: 86.3 ms with 4, 84.5 with 5, 96.5 with 6), 10 of 256, 14 of 128
-    const long long most = (long long)ceilf((large ? 180.f : 150.f) / sqrtf((float)games));
+    // 4 trees of 1792 games, 10 of 256, 14 of 128.  One more of 896 games and more pays where the trees are many for the places, and the more
+    // so the longer they take turns with them: ms with 4 / 5 trees of 1792 games, 200, 500, 1000 and 2000 steps, 908 trees (1.23 a place of
+    // the 5) 9.03 / 10.07, 20.8 / 24.7, 39.6 / 45.0, 75.4 / 83.7; 980 (1.32) 9.72 / 10.15, 22.6 / 23.3, 43.2 / 44.0, 82.5 / 82.6; 1024 (1.38) 10.12 /
+    // 10.38, 23.7 / 23.8, 45.2 / 44.8, 86.4 / 84.7; 1220 (1.65) 11.50 / 11.56, 27.1 / 26.9, 51.7 / 50.5, 99.1 / 95.3; with 6 / 7 of 896 games 1352
+    // (1.30) 6.87 / 7.05, 16.1 / 16.5, 31.1 / 31.6, 60.5 / 60.8; 1420 (1.37) 7.25 / 7.36, 17.1 / 17.0, 33.0 / 32.2, 64.3 / 61.8; 1536 (1.48) 7.75 /
+    // 7.74, 18.4 / 18.1, 35.4 / 34.7, 69.1 / 66.8; 40 and 100 steps of 2048 trees of 896 games 2.40 / 2.57 and 5.28 / 5.30, of 1536 of 1792 3.50 / 3.73
+    // and 7.59 / 7.71.
+    long long most = (long long)ceilf(150.f / sqrtf((float)games));
+    if (large && steps >= 200 && (double)trees >= (1.31 + 45. / steps) * (double)((most + 1) * h->sm_count)) most++;
     long long k = need;
     if (large) k = (long long)(0.72f * (float)trees / (float)h->sm_count + 0.6f);
     else if (need > 3 && games > 128 && need * games > 2048) k = need * 18 / 25 < 3 ? 3 : need * 18 / 25;

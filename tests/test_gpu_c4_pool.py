@@ -106,3 +106,16 @@ def test_pooled_trees_outlast_a_million_steps_without_a_game(empty, seed):
     assert (out["playouts"] == orc.playouts).all() and (out["plies"] == orc.plies).all()
     for b in (0, roots - 1):
         compare_trees(ai, orc, search=b)
+
+
+@pytest.mark.parametrize("n_playouts,roots,steps,at_once", [(256, 227, 2000, 4), (256, 256, 600, 4), (256, 256, 700, 5), (256, 384, 100, 4),
+                                                            (256, 384, 300, 5), (128, 338, 1000, 6), (128, 384, 500, 7), (128, 384, 200, 6), (512, 256, 500, 3)])
+def test_a_tree_more_on_an_sm_only_where_many_wait_for_long(n_playouts, roots, steps, at_once):
+    boards, fills, turns = c4_random_roots(roots, 20, seed=3)
+    ai = MCTSNC((6, 7), 7, 7, search_time_limit=np.inf, search_steps_limit=steps, n_trees=4, n_playouts=n_playouts, variant="acp_prodigal", seed=5,
+                verbose_info=False, max_batch=roots)
+    ai.init_device_side_arrays()
+    out = ai.run_batch(boards, fills, turns, steps=steps)
+    assert ai.launch_geometry()["blocks_per_sm"] == at_once
+    assert (out["status"] & _abi.STATUS_INTERNAL == 0).all() and (out["steps"] == steps).all()
+    assert (out["root_ns"][:, :7].sum(axis=1) > 0).all()
