@@ -619,6 +619,11 @@ bool choose_pool(const mctsnc_handle *h, long long trees, int steps, PoolShape *
     if (k < 1) k = 1;
     if (k > c4::POOL_MAX_TREES) k = c4::POOL_MAX_TREES;
     while (k > 1 && c4::pool_bytes((int)k, (int)(h->rng_per_search / h->cfg.n_trees)) > (size_t)POOL_SMEM_LIMIT) k--;
+    // Trees that take turns with one place an SM, and not enough steps to make up for the first turns: us with a block per tree / with the
+    // pool, 896 games, 33, 48, 64 and 100 steps, 210 trees 698 / 804, 1002 / 1011, 1319 / 1232, 2041 / 1790; 250 728 / 890, 1027 / 1107, 1366 / 1332, 2081 /
+    // 1874; 286 727 / 960, 1040 / 1189, 1364 / 1420, 2083 / 2008; 1792 games, 33, 40 and 48 steps, 210 trees 1109 / 1101, 1346 / 1246, 1588 / 1404; 250
+    // 1157 / 1248, 1387 / 1383, 1651 / 1539; 286 1151 / 1340, 1385 / 1484, 1643 / 1647; 3584 games, 250 trees 1993 / 2022, 2392 / 2235, 2837 / 2497.
+    if (k == 1 && steps < (games < 1792 ? 60 : 40) && 20 * trees > 29 * h->sm_count) return false;
     shape->trees = (int)k;
     shape->walkers = (int)(k + 1) / 2;
     if (games <= 512 && shape->walkers < 5) shape->walkers = k < 5 ? (int)k : 5;

@@ -119,3 +119,20 @@ def test_a_tree_more_on_an_sm_only_where_many_wait_for_long(n_playouts, roots, s
     assert ai.launch_geometry()["blocks_per_sm"] == at_once
     assert (out["status"] & _abi.STATUS_INTERNAL == 0).all() and (out["steps"] == steps).all()
     assert (out["root_ns"][:, :7].sum(axis=1) > 0).all()
+
+
+@pytest.mark.parametrize("n_playouts,roots,steps,kernel", [(128, 250, 36, "c4::search_kernel"), (128, 250, 60, "c4::pool_kernel"),
+                                                           (128, 210, 33, "c4::pool_kernel"), (128, 290, 33, "c4::pool_kernel"),
+                                                           (256, 250, 39, "c4::search_kernel"), (256, 250, 40, "c4::pool_kernel")])
+def test_few_steps_of_trees_in_turns_have_a_block_per_tree(n_playouts, roots, steps, kernel):
+    boards, fills, turns = c4_random_roots(roots, 20, seed=4)
+    ai = MCTSNC((6, 7), 7, 7, search_time_limit=np.inf, search_steps_limit=steps, n_trees=1, n_playouts=n_playouts, variant="acp_prodigal", seed=5,
+                verbose_info=False, max_batch=roots)
+    ai.init_device_side_arrays()
+    out = ai.run_batch(boards, fills, turns, steps=steps)
+    assert ai.launch_geometry()["kernel"] == kernel and (out["status"] & _abi.STATUS_INTERNAL == 0).all()
+    for b in (0, roots - 1):
+        orc = OracleMCTSNC((6, 7), 7, 7, n_trees=1, n_playouts=n_playouts, variant="acp_prodigal", seed=5, node_capacity=steps * 7 + 8)
+        orc.run(boards[b], fills[b], int(turns[b]), steps)
+        assert (out["playouts"][b], out["plies"][b], out["best_action"][b]) == (orc.playouts, orc.plies, orc.best_action)
+        compare_trees(ai, orc, search=b)
