@@ -136,3 +136,20 @@ def test_few_steps_of_trees_in_turns_have_a_block_per_tree(n_playouts, roots, st
         orc.run(boards[b], fills[b], int(turns[b]), steps)
         assert (out["playouts"][b], out["plies"][b], out["best_action"][b]) == (orc.playouts, orc.plies, orc.best_action)
         compare_trees(ai, orc, search=b)
+
+
+def test_draws_of_one_in_pooled_trees_are_replayed_like_the_oracle():
+    """Games that meet a uniform draw of exactly 1.0f, with either side to move first, found in a block of several trees."""
+    roots, steps, kw = 100, 40, dict(n_trees=4, n_playouts=256, variant="acp_prodigal", seed=7)
+    boards, fills, turns = c4_random_roots(roots, 20, seed=1)
+    ai = MCTSNC((6, 7), 7, 7, search_time_limit=np.inf, search_steps_limit=steps, verbose_info=False, max_batch=roots, **kw)
+    ai.init_device_side_arrays()
+    out = ai.run_batch(boards, fills, turns, steps=steps)
+    assert ai.launch_geometry()["kernel"] == "c4::pool_kernel" and ai.launch_geometry()["blocks_per_sm"] == 2
+    for b, ub in ((0, 1), (20, 1), (40, 1), (10, 0)):       # the first mover of the game is -1, +1, -1
+        orc = OracleMCTSNC((6, 7), 7, 7, node_capacity=steps * 7 + 8, **kw)
+        orc.run(boards[b], fills[b], int(turns[b]), steps)
+        assert orc.ub_draws == ub == out["ub_draws"][b]
+        assert bool(out["status"][b] & _abi.STATUS_UB_DRAW) == bool(ub) and out["status"][b] & _abi.STATUS_INTERNAL == 0
+        assert (out["playouts"][b], out["plies"][b], out["best_action"][b]) == (orc.playouts, orc.plies, orc.best_action)
+        compare_trees(ai, orc, search=b)
