@@ -95,7 +95,8 @@ typedef struct mctsnc_result {
     int32_t max_size;
     int32_t reserved;
     /* time spent in the four stages of the steps (select, expand, playouts, backup), milliseconds, mean over this
-       handle's trees of the time their blocks spent there (SM cycle counter at the nominal clock); the reference's
+       handle's trees of the time their blocks spent there (SM cycle counter at the nominal clock; the playouts of a tree whose
+       block grows others too hold its waits for them); the reference's
        time_select / time_expand / time_playout / time_backup (src/mctsnc.py:606-686) are host clocks around launches */
     float stage_ms[4];
     float reduce_ms[2];          /* CUDA-event time of the two final reductions (mctsnc_run only; 0 for batch calls) */

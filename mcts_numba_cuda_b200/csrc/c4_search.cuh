@@ -787,9 +787,9 @@ struct Game {
 // The stream's state in the block's array is the one behind them; `used`: draws of the step's game, made up by refill while the
 // walker makes the next step and the threads that play would wait for it.  A ply has 14 of 58 instructions less then, and
 // nothing is taken back when a game is closed; what the threads lose is a part of the walker's issue slots.  One search of 1000
-// steps, without / with: 1 x 32 ocp 4.66 / 4.45 ms, 8 x 256 ocp 5.77 / 5.64, 4 x 32 acp 5.12 / 4.79; on clusters 4 x 64 acp 5.49 / 5.33, 4 x 128
-// 5.62 / 5.64, 4 x 256 6.07 / 5.99, two of those 6.68 / 6.21.  With two to four warps that play the walker loses more than they
-// gain: 4 x 128 ocp 4.69 / 4.96, 4 x 64 ocp 4.72 / 4.82.
+// steps, without / with: 1 x 32 ocp 4.75 / 4.57 ms, 8 x 256 ocp 5.61 / 5.57, 4 x 32 acp 5.31 / 4.92; on clusters 4 x 64 acp 5.59 / 5.41, 4 x 256
+// 5.81 / 5.72, 4 x 512 7.93 / 7.51.  With two to four warps that play the walker loses more than they gain: 4 x 128 ocp 4.69 / 4.96, 4 x 64
+// ocp 4.72 / 4.82, on clusters 4 x 128 acp 5.67 / 5.70.
 struct Draws {
     float *ring;       // [streams][AHEAD_STRIDE]
     int *place, *used; // [streams]
@@ -1158,8 +1158,8 @@ __global__ void __maxnreg__(MCTSNC_C4_MAXNREG) search_kernel(const SearchParams 
             if (tid == 0) {
                 // Where a quarter more trees than blocks share the queue, the next tree is taken before the last one is put back, so that
                 // trees go round the SMs: a tree with slow neighbours on its SM falls behind, has the most time left, and would be what
-                // its own block takes next (256 x 4 x 256 acp, 300 steps, 20.7 instead of 22.4 ms; 256 x 8 x 256 ocp, 500 steps,
-                // 16.9 instead of 18.2).  Where hardly any tree waits that order exchanges the trees with the most time left for those
+                // its own block takes next (with a block per tree for all of them: 256 x 4 x 256 acp, 300 steps, 20.7 instead of 22.4 ms;
+                // 256 x 8 x 256 ocp, 500 steps, 16.9 instead of 18.2).  Where hardly any tree waits that order exchanges the trees with the most time left for those
                 // with the least at every slice (600 x 4 x 128 ocp, 1000 steps, 2400 trees on 2368 blocks: 32.8 instead of 24.7 ms).
                 int next = -1;
                 const int held = s.held;

@@ -66,7 +66,8 @@ struct TreeState {
     unsigned long long ub_draws;
     float us_per_step;   // work queue: smoothed time per step of the tree's slices in the current launch (microseconds)
     // time this tree's block spent in the four stages of its steps since the search began, in milliseconds at the nominal
-    // SM clock (cycle counter of the SM the block ran on): select, expand, playouts, backup.  The reference times the same
+    // SM clock (cycle counter of the SM the block ran on): select, expand, playouts (where the block grows other trees too, with the waits
+    // for them), backup.  The reference times the same
     // stages with host clocks around its launches (src/mctsnc.py:606-686).
     float stage_ms[4];
     int max_depth;       // deepest node, and

@@ -222,8 +222,9 @@ select_kernel(float cpuct, int virtual_loss, int *child_all, const float *node_p
 // Who meets whom is known in registers: of the traversals of a tree that want the same action in the same turn the first has
 // it, and their counts are from the same moment, so the others are those whose compare-and-swap would fail.  A claim
 // is therefore an addition that nobody waits for.  A third choice, which needs no answer, follows the second at once, as it does in
-// select_kernel while the winners still wait for theirs; with that the same paths come out (4096 trees x 8 actions x 8
-// traversals: 0.1 % of the counts differ between two runs of select_kernel, and as many between it and this kernel).
+// select_kernel while the winners still wait for theirs; with that nearly the same paths come out (counts that differ after a wave and
+// its backup, between two runs of select_kernel / between it and this kernel: 4096 trees x 8 actions x 8 traversals 0.09 / 0.12 %, two
+// waves one after the other 0.75 / 0.78 %; 2500 x 8 x 4 0.012 / 0.015 %; 4096 x 7 x 8 0.22 / 0.33 %).
 // The claims of earlier turns are seen: __syncwarp orders them before the next loads, and no other warp is in the tree.
 // The child of the joint action is loaded when it is known: a node's whole row of children, loaded ahead as in
 // select_kernel, is as much as all its statistics, and with every traversal on the device at once memory's throughput counts.

@@ -541,8 +541,9 @@ const void *search_kernel_ptr(const mctsnc_config &c, bool straight) {
     return is_ocp(c) ? (const void *)c4::search_kernel<true, false> : (const void *)c4::search_kernel<false, false>;
 }
 
-// Threads that play the games of one tree in a block of its own (choose_pool has looked at the launch before), from the games a step plays (n_playouts, times the children of a node for
-// the ACP variants) and from how many trees there are for the device.
+// Threads that play the games of one tree in a block of its own, from the games a step plays (n_playouts, times the children of a node
+// for the ACP variants) and from how many trees there are for the device.  Launches of more trees than SMs come here only where
+// choose_pool leaves them: up to 32 games or 32 steps, and what it says of few steps; the figures below for such trees are of longer launches.
 //   Many trees (at least two per SM): a quarter of the games, between 32 and 320; half of them when a step has at most 256
 //   games.  Measured on 256 roots, G playouts/s: ACP 4 x 256 (1792 games a step), 500 steps, 18.2 / 20.3 / 20.2 / 18.7 / 19.0 / 19.0 at 256 /
 //   288 / 320 / 352 / 384 / 512 threads (a thread of a smaller block plays more games per step, so less of a step is spent
@@ -597,7 +598,7 @@ const void *pool_kernel_ptr(bool ocp) { return ocp ? (const void *)c4::pool_kern
 // of fewer trees fill the lanes, fewer, so that the work queue can even out the SMs.
 // Walkers: one for two trees, more where the games are few and the walk is most of a step.  Players: enough lanes, but a lane
 // of a smaller block plays its ply sooner.
-// Launches of up to SLICE_STEPS steps keep the block per tree.
+// Launches of up to SLICE_STEPS steps keep the block per tree.  (The table is of six trees of 896 games and four of 1792 at most.)
 bool choose_pool(const mctsnc_handle *h, long long trees, int steps, PoolShape *shape) {
     const int games = h->cfg.n_playouts * (is_ocp(h->cfg) ? 1 : h->A);
     const bool large = games >= 896;
@@ -927,9 +928,9 @@ int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_
     p.times4 = 4u;
     p.times2p23 = 1u << 23;
     // Few trees (one search, a few searches): a cluster of blocks per tree, so that the games of a step are played on
-    // several SMs at once.  Measured, 4 x 256 acp_prodigal, 2000 steps, 1 / 4 / 8 searches in one launch: 13.7 / 14.4 / 20.6 ms with
-    // clusters against 42.2 with a block of 1024 threads per tree (12.6 for one with draws made ahead); 500 steps, 9 / 12 / 16 searches: 5.0 / 5.6 / 7.0 against 11.1 --
-    // up to four cluster blocks per SM pay, and more do not fit.
+    // several SMs at once.  Measured without draws made ahead, 4 x 256 acp_prodigal, 2000 steps, 1 / 4 / 8 searches in one launch: 13.7 /
+    // 14.4 / 20.6 ms with clusters (one, with them, 12.6) against 42.2 with a block of 1024 threads per tree; 500 steps, 9 / 12 / 16 searches:
+    // 5.0 / 5.6 / 7.0 against 11.1 -- up to four cluster blocks per SM pay, and more do not fit.
     // Only where a step has more than 256 games (ACP with 64 playouts or more, OCP with 512).  One search of 2000 steps, 4
     // trees, with a block / with clusters: ACP 8 / 16 / 32 / 64 / 128 / 256 / 512 playouts 9.1 / 9.3 / 11.7 / 16.6 / 25.4 / 42.2 / 64.5 ms
     // against 11.2 / 11.4 / 11.8 / 12.0 / 12.5 / 13.7 / 18.2; OCP 128 / 256 / 512 playouts 10.1 / 12.3 / 17.6 against 12.2 / 12.4 / 12.7: with few
@@ -1038,9 +1039,9 @@ int launch_search(mctsnc_handle *h, int batch, int steps, int first, cudaStream_
         return MCTSNC_E_BAD_ARGUMENT;
     h->blocks_per_sm = per_sm;
     // More trees than blocks fit on the device at once: a persistent grid takes slices of SLICE_STEPS steps from the
-    // work queue, so that trees with long games do not keep a few SMs busy after the others have run out of work
-    // (1024 trees of 2000 steps, 4 x 256 acp_prodigal: 156 ms with one block per tree, 115 with the queue; 3200 trees of 4 x 128
-    // ocp_prodigal, 1000 steps: 37.3 and 29.0).  Otherwise block b grows tree b for the whole launch.
+    // work queue, so that trees with long games do not keep a few SMs busy after the others have run out of work (a block per tree in
+    // both, as with an explicit threads_per_tree: 1024 trees of 2000 steps, 4 x 256 acp_prodigal, 156 ms without the queue, 115 with it; 3200
+    // trees of 4 x 128 ocp_prodigal, 1000 steps, 37.3 and 29.0).  Otherwise block b grows tree b for the whole launch.
     const long long resident = (long long)per_sm * h->sm_count;
     unsigned grid = (unsigned)trees;
     if (trees > resident && steps > SLICE_STEPS) {

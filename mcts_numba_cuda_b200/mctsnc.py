@@ -329,8 +329,8 @@ class MCTSNC:
         self.device_time = r["device_ms"] * 1e-3
         # The loop runs on the device in one piece: its CUDA-event time is the loop time.  The per-stage times of the
         # reference (host clocks around each launch, src/mctsnc.py:606-686) are here the time a tree's thread block spent in
-        # each stage, counted on the device (mean over the trees, which run side by side); the two reductions are timed
-        # with CUDA events.
+        # each stage, counted on the device (mean over the trees, which run side by side); where a block grows several trees, the
+        # playouts hold the waits for free threads and for the warp that walks too.  The two reductions are timed with CUDA events.
         self.time_loop = self.device_time
         self.time_select, self.time_expand, self.time_playout, self.time_backup = (1e-3 * x for x in stage_ms)
         self.time_reduce_over_trees, self.time_reduce_over_actions = (1e-3 * x for x in reduce_ms)
