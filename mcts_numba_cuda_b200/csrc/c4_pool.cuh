@@ -5,8 +5,8 @@
 // in shared memory: a lane whose game is over takes the next one, whichever tree it belongs to.
 //
 // Measured with the same plies in both: 256 roots of 4 x 256 acp, 400 steps, 22.7 ms with a block per tree, 19.1 with the pool; of 8 x 128
-// ocp 8.65 and 6.2; a step's lanes 27 to 28 of 32 in play instead of 21.  What bounds it: issue slots (87 % busy) and the logic pipe
-// (83 %) where games are many; where they are few (ocp: 15 to 22 lanes) the chain of a step, walk and longest game.
+// ocp 8.65 and 6.2; a step's lanes 27 of 32 in play instead of 21.  What bounds it: issue slots (87 % busy) and the logic pipe
+// (83 %) where games are many; where they are few (ocp: 22 to 23 lanes) the chain of a step, walk and longest game.
 //
 // The first `walkers` warps select, expand and back up, each for the trees w, w + walkers, ... of the block; the others play.
 // Every game slot that a step needs played out becomes an entry of the queue, P games with one ticket each: ticket t is
